@@ -3,6 +3,7 @@
 // the reference's C operator interface (k3_rocm_ops.h); the kernels are new.
 #include "k3_common.cuh"
 #include "k3_moe_ops.h"
+#include "k3_route_block.cuh"
 
 #include <math.h>
 
@@ -204,89 +205,45 @@ rms_norm_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ in,
 }
 
 // ------------------------------------------------------------ router top-k
-// One warp per score row.  Lane l owns experts l, l+32, ...; top_k rounds of a
-// warp arg-max under the order (score+bias descending, expert id ascending),
-// which is the order the reference's insertion oracle and bitonic kernel
-// produce (k3_rocm_ops.cu:1398-1449).  Weights: raw score / (1e-20 + sum of the
-// selected raw scores in rank order) * scale.
-constexpr int kMaxPerLane = 32;  // 1024 experts / 32 lanes
-
-__global__ void __launch_bounds__(128)
+// One block per score row (k3_route_block.cuh): order score + bias descending, expert id
+// ascending on ties, which is the order the reference's insertion oracle and bitonic kernel
+// produce (k3_rocm_ops.cu:1398-1449).  Weights: raw score / (1e-20 + sum of the selected
+// raw scores in rank order) * scale.  Bound by latency, not bytes: one warp per row with
+// top_k rounds of arg-max over 28 scores per lane took 25 us for one row of 896 and 129 us
+// for 8192 rows; eight warps that find a threshold first and rank the few dozen scores
+// above it take under 7 us and 47 us.
+__global__ void __launch_bounds__(kThreads)
 router_topk_kernel(uint32_t *__restrict__ ids_out, float *__restrict__ weights_out,
                    const float *__restrict__ logits, const float *__restrict__ bias,
                    uint32_t vectors, uint32_t experts, uint32_t top_k, float scale) {
-    const uint32_t lane = threadIdx.x % kWarp;
-    const uint32_t warps_per_block = blockDim.x / kWarp;
-    const uint32_t per_lane = (experts + kWarp - 1) / kWarp;
-    for (uint32_t v = blockIdx.x * warps_per_block + threadIdx.x / kWarp; v < vectors;
-         v += gridDim.x * warps_per_block) {
+    __shared__ RouteScratch rs;
+    __shared__ uint32_t ids_s[32];
+    __shared__ float weights_s[32];
+    float b[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; j++) {
+        const uint32_t e = threadIdx.x + j * kThreads;
+        b[j] = e < experts ? bias[e] : 0.f;
+    }
+    for (uint32_t v = blockIdx.x; v < vectors; v += gridDim.x) {
         const float *row = logits + (uint64_t)v * experts;
-        float choice[kMaxPerLane];
-        float score[kMaxPerLane];
+        float l[4];
 #pragma unroll
-        for (int i = 0; i < kMaxPerLane; i++) {
-            const uint32_t e = lane + (uint32_t)i * kWarp;
-            if ((uint32_t)i < per_lane && e < experts) {
-                const float s = sigmoid_exact(row[e]);
-                score[i] = s;
-                choice[i] = s + bias[e];
-            } else {
-                score[i] = 0.f;
-                choice[i] = -INFINITY;
-            }
+        for (uint32_t j = 0; j < 4u; j++) {
+            const uint32_t e = threadIdx.x + j * kThreads;
+            l[j] = e < experts ? row[e] : 0.f;
         }
-        uint32_t taken = 0u;  // bit i: local candidate i already selected
-        float my_weight = 0.f;
-        uint32_t my_id = 0u;
-        float denominator = 1e-20f;
-        for (uint32_t rank = 0; rank < top_k; rank++) {
-            // local best: largest choice, smallest index on ties (ascending scan, strict >)
-            float best = -INFINITY;
-            int best_i = -1;
 #pragma unroll
-            for (int i = 0; i < kMaxPerLane; i++) {
-                const bool usable = ((taken >> i) & 1u) == 0u && (uint32_t)i < per_lane &&
-                                    lane + (uint32_t)i * kWarp < experts;
-                if (usable && (best_i < 0 || choice[i] > best)) {
-                    best = choice[i];
-                    best_i = i;
-                }
-            }
-            uint32_t best_id = best_i < 0 ? 0xffffffffu : lane + (uint32_t)best_i * kWarp;
-            float win = best;
-            uint32_t win_id = best_id;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float oc = __shfl_xor_sync(0xffffffffu, win, o);
-                const uint32_t oid = __shfl_xor_sync(0xffffffffu, win_id, o);
-                const bool take = (oid != 0xffffffffu) &&
-                                  (win_id == 0xffffffffu || oc > win || (oc == win && oid < win_id));
-                if (take) {
-                    win = oc;
-                    win_id = oid;
-                }
-            }
-            // owner marks the winner and publishes its raw score
-            float raw = 0.f;
-            if (win_id != 0xffffffffu && (win_id % kWarp) == lane) {
-                const int i = (int)(win_id / kWarp);
-                taken |= 1u << i;
-#pragma unroll
-                for (int j = 0; j < kMaxPerLane; j++) {
-                    if (j == i) raw = score[j];
-                }
-            }
-            raw = __shfl_sync(0xffffffffu, raw, win_id == 0xffffffffu ? 0 : (int)(win_id % kWarp));
-            denominator += raw;
-            if (lane == rank) {
-                my_weight = raw;
-                my_id = win_id;
-            }
+        for (uint32_t j = 0; j < 4u; j++) {
+            const uint32_t e = threadIdx.x + j * kThreads;
+            const float s = sigmoid_exact(l[j]);
+            rs.score[e] = s;
+            rs.choice[e] = s + b[j];
         }
-        if (lane < top_k) {
-            ids_out[(uint64_t)v * top_k + lane] = my_id;
-            weights_out[(uint64_t)v * top_k + lane] =
-                __fmul_rn(__fdiv_rn(my_weight, denominator), scale);
+        route_select_block(rs, ids_s, weights_s, experts, top_k, scale);
+        if (threadIdx.x < top_k) {
+            ids_out[(uint64_t)v * top_k + threadIdx.x] = ids_s[threadIdx.x];
+            weights_out[(uint64_t)v * top_k + threadIdx.x] = weights_s[threadIdx.x];
         }
     }
 }
@@ -434,7 +391,7 @@ extern "C" bool k3_rocm_router_topk_f32_batch(void *expert_ids, void *expert_wei
         expert_count > 1024u || top_k > 32u || scaling_factor <= 0.0f) {
         return false;
     }
-    router_topk_kernel<<<grid_for(vector_count, 4), 128, 0, (cudaStream_t)stream>>>(
+    router_topk_kernel<<<grid_for(vector_count, 1), kThreads, 0, (cudaStream_t)stream>>>(
         (uint32_t *)expert_ids, (float *)expert_weights, (const float *)logits,
         (const float *)correction_bias, vector_count, expert_count, top_k, scaling_factor);
     return launch_ok();

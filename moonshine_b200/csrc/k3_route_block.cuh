@@ -1,5 +1,4 @@
-// Top-k routing of one token by a whole thread block from the per-expert scores the
-// router rows left in memory: choice = sigmoid(logit) + bias decides (larger first,
+// Top-k routing of one token by a whole thread block from its per-expert scores: choice = sigmoid(logit) + bias decides (larger first,
 // lower expert id on ties, k3_rocm_ops.cu:1385-1450 / tests/test_k3_moe_smoke.cu:215-253),
 // weight = score / (1e-20 + sum of the selected scores in rank order) * scale.
 //
@@ -48,30 +47,12 @@ K3_DEVINL void route_round(uint32_t (&key)[4], uint32_t warp, uint32_t lane, uin
     }
 }
 
-// All threads of a block of at least 256 threads call this (it contains block barriers).
-// route_words: f32 [2][1024] = scores, choices.  Results: ids_s / weights_s [top_k] in
-// shared memory, valid after the call for every thread.
-K3_DEVINL void route_topk_block(RouteScratch &rs, uint32_t *ids_s, float *weights_s, const float *route_words,
-                                uint32_t experts, uint32_t top_k, float route_scale) {
+// All threads of a block of at least 256 threads call this (it contains block barriers) after
+// filling rs.score / rs.choice for every expert; no barrier is needed in between.  Results:
+// ids_s / weights_s [top_k] in shared memory, valid after the call for every thread.
+K3_DEVINL void route_select_block(RouteScratch &rs, uint32_t *ids_s, float *weights_s, uint32_t experts,
+                                  uint32_t top_k, float route_scale) {
     const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-    {
-        // all of a thread's loads in flight at once (blockDim >= 256: at most four experts each)
-        float sc[4], ch[4];
-#pragma unroll
-        for (uint32_t j = 0; j < 4u; j++) {
-            const uint32_t e = threadIdx.x + j * blockDim.x;
-            sc[j] = e < experts ? __ldcg(route_words + e) : 0.f;
-            ch[j] = e < experts ? __ldcg(route_words + 1024u + e) : 0.f;
-        }
-#pragma unroll
-        for (uint32_t j = 0; j < 4u; j++) {
-            const uint32_t e = threadIdx.x + j * blockDim.x;
-            if (e < 1024u) {
-                rs.score[e] = sc[j];
-                rs.choice[e] = ch[j];
-            }
-        }
-    }
     if (threadIdx.x == 0) rs.passed = 0u;
     if (threadIdx.x < 32u) {
         ids_s[threadIdx.x] = 0xffffffffu;
@@ -159,6 +140,28 @@ K3_DEVINL void route_topk_block(RouteScratch &rs, uint32_t *ids_s, float *weight
         if (lane < top_k) weights_s[lane] = w;
     }
     __syncthreads();
+}
+
+// The same from scores another kernel left in memory: route_words f32 [2][1024] = scores, choices.
+K3_DEVINL void route_topk_block(RouteScratch &rs, uint32_t *ids_s, float *weights_s, const float *route_words,
+                                uint32_t experts, uint32_t top_k, float route_scale) {
+    // all of a thread's loads in flight at once (blockDim >= 256: at most four experts each)
+    float sc[4], ch[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; j++) {
+        const uint32_t e = threadIdx.x + j * blockDim.x;
+        sc[j] = e < experts ? __ldcg(route_words + e) : 0.f;
+        ch[j] = e < experts ? __ldcg(route_words + 1024u + e) : 0.f;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; j++) {
+        const uint32_t e = threadIdx.x + j * blockDim.x;
+        if (e < 1024u) {
+            rs.score[e] = sc[j];
+            rs.choice[e] = ch[j];
+        }
+    }
+    route_select_block(rs, ids_s, weights_s, experts, top_k, route_scale);
 }
 
 }  // namespace k3
