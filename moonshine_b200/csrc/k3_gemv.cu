@@ -10,6 +10,7 @@
 // Batch entry points run the same code per input row, hence batch == repeated
 // single-row calls byte for byte, and the batch_tile argument is validated
 // but does not change any result.
+#include "k3_exact_gemm.cuh"
 #include "k3_gemv.cuh"
 #include "k3_moe_ops.h"
 
@@ -99,79 +100,6 @@ bf16_gemm_kernel(Out *__restrict__ out, const uint16_t *__restrict__ w,
     }
 }
 
-// --------------------------------------------------------------------- Q8
-// One warp per weight row.  Virtual lane = octet mod 256 = 32*i + u for thread
-// u, slot i; 8 sequential fused multiply-adds per octet.
-template <int VT>
-__global__ void __launch_bounds__(256)
-q8_gemm_kernel(uint16_t *__restrict__ out, const int8_t *__restrict__ q,
-               const void *__restrict__ scales, const uint16_t *__restrict__ x,
-               uint32_t vectors, uint32_t rows, uint32_t columns, uint32_t block,
-               int scale_f16) {
-    const uint32_t lane = threadIdx.x % kWarp;
-    const uint32_t warps = (gridDim.x * blockDim.x) / kWarp;
-    const uint32_t octets = columns / 8u;
-    const uint32_t blocks_per_row = columns / block;
-    for (uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp; row < rows;
-         row += warps) {
-        const int8_t *qr = q + (uint64_t)row * columns;
-        const uint64_t sbase = (uint64_t)row * blocks_per_row;
-        for (uint32_t v0 = 0; v0 < vectors; v0 += VT) {
-            float acc[VT][8];
-#pragma unroll
-            for (int v = 0; v < VT; v++)
-#pragma unroll
-                for (int i = 0; i < 8; i++) acc[v][i] = 0.f;
-            for (uint32_t o0 = 0; o0 < octets; o0 += 256u) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const uint32_t octet = o0 + 32u * i + lane;
-                    if (octet >= octets) continue;
-                    const uint2 wq = *reinterpret_cast<const uint2 *>(qr + (uint64_t)octet * 8u);
-                    const uint32_t sidx = (octet * 8u) / block;
-                    const float s = scale_f16
-                                        ? __half2float(reinterpret_cast<const __half *>(scales)[sbase + sidx])
-                                        : reinterpret_cast<const float *>(scales)[sbase + sidx];
-                    float wf[8];
-#pragma unroll
-                    for (int b = 0; b < 4; b++) {
-                        wf[b] = __fmul_rn((float)(int8_t)(wq.x >> (8 * b)), s);
-                        wf[4 + b] = __fmul_rn((float)(int8_t)(wq.y >> (8 * b)), s);
-                    }
-#pragma unroll
-                    for (int v = 0; v < VT; v++) {
-                        if (v0 + v >= vectors) break;
-                        const uint4 xq = *reinterpret_cast<const uint4 *>(
-                            x + (uint64_t)(v0 + v) * columns + (uint64_t)octet * 8u);
-                        float a = acc[v][i];
-                        a = fmaf(wf[0], bf16_lo(xq.x), a);
-                        a = fmaf(wf[1], bf16_hi(xq.x), a);
-                        a = fmaf(wf[2], bf16_lo(xq.y), a);
-                        a = fmaf(wf[3], bf16_hi(xq.y), a);
-                        a = fmaf(wf[4], bf16_lo(xq.z), a);
-                        a = fmaf(wf[5], bf16_hi(xq.z), a);
-                        a = fmaf(wf[6], bf16_lo(xq.w), a);
-                        a = fmaf(wf[7], bf16_hi(xq.w), a);
-                        acc[v][i] = a;
-                    }
-                }
-            }
-#pragma unroll
-            for (int v = 0; v < VT; v++) {
-                if (v0 + v >= vectors) break;
-                // tree: widths 128, 64, 32 are slot-to-slot, 16..1 lane-to-lane
-                float p0 = acc[v][0] + acc[v][4], p1 = acc[v][1] + acc[v][5];
-                float p2 = acc[v][2] + acc[v][6], p3 = acc[v][3] + acc[v][7];
-                p0 += p2; p1 += p3;
-                p0 += p1;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) p0 += __shfl_down_sync(0xffffffffu, p0, o);
-                if (lane == 0) out[(uint64_t)(v0 + v) * rows + row] = float_to_bf16_bits(p0);
-            }
-        }
-    }
-}
-
 // ------------------------------------------------------------------ MXFP4
 // Item = 32 rows.  Two input rows per pass (MMA columns 0-3 and 4-7).
 template <bool kAligned16>
@@ -204,18 +132,44 @@ mxfp4_gemm_kernel(uint16_t *__restrict__ out, const uint8_t *__restrict__ packed
     }
 }
 
+template <typename Out, int kR, int kV, int kSR, int kSV>
+void launch_exact_bf16(void *output, const void *weights, const void *input, uint32_t vectors, uint32_t rows,
+                       uint32_t columns, cudaStream_t stream) {
+    const dim3 grid((rows + kR * kSR - 1u) / (kR * kSR), (vectors + kV * kSV - 1u) / (kV * kSV));
+    exact_bf16_kernel<Out, kR, kV, kSR, kSV><<<grid, 64 * kSR * kSV, 0, stream>>>(
+        (Out *)output, (const uint16_t *)weights, (const uint16_t *)input, vectors, rows, columns);
+}
+
 template <typename Out>
 bool launch_bf16(void *output, const void *weights, const void *input, uint32_t vectors,
                  uint32_t rows, uint32_t columns, cudaStream_t stream) {
-    const uint32_t blocks = (uint32_t)std::min<uint64_t>(((uint64_t)rows + 7) / 8, (uint64_t)sm_count() * 8);
-    if (vectors == 1u) {
-        bf16_gemm_kernel<Out, 1><<<blocks, 256, 0, stream>>>(
-            (Out *)output, (const uint16_t *)weights, (const uint16_t *)input, vectors, rows, columns);
+    if (columns % 4u != 0u || ((((uintptr_t)weights) | ((uintptr_t)input)) & 7u) != 0) {
+        // ragged columns or odd bases: one warp per weight row, element by element where it must
+        const uint32_t blocks = (uint32_t)std::min<uint64_t>(((uint64_t)rows + 7) / 8, (uint64_t)sm_count() * 8);
+        auto kernel = vectors == 1u ? bf16_gemm_kernel<Out, 1> : bf16_gemm_kernel<Out, 4>;
+        kernel<<<blocks, 256, 0, stream>>>((Out *)output, (const uint16_t *)weights, (const uint16_t *)input, vectors,
+                                           rows, columns);
+    } else if (vectors == 1u) {
+        launch_exact_bf16<Out, 1, 1, 4, 1>(output, weights, input, vectors, rows, columns, stream);
+    } else if (vectors == 2u) {
+        launch_exact_bf16<Out, 1, 2, 4, 1>(output, weights, input, vectors, rows, columns, stream);
+    } else if (vectors <= 4u) {
+        launch_exact_bf16<Out, 2, 4, 4, 1>(output, weights, input, vectors, rows, columns, stream);
+    } else if (vectors <= 16u) {
+        launch_exact_bf16<Out, 2, 4, 2, 2>(output, weights, input, vectors, rows, columns, stream);
     } else {
-        bf16_gemm_kernel<Out, 4><<<blocks, 256, 0, stream>>>(
-            (Out *)output, (const uint16_t *)weights, (const uint16_t *)input, vectors, rows, columns);
+        launch_exact_bf16<Out, 4, 4, 4, 2>(output, weights, input, vectors, rows, columns, stream);
     }
     return launch_ok();
+}
+
+template <int kR, int kV>
+void launch_exact_q8(void *output, const void *quantized, const void *scales, const void *input, uint32_t vectors,
+                     uint32_t rows, uint32_t columns, uint32_t block, int scale_type, cudaStream_t stream) {
+    const dim3 grid((rows + kR - 1u) / kR, (vectors + kV - 1u) / kV);
+    exact_q8_kernel<kR, kV><<<grid, 256, 0, stream>>>(
+        (uint16_t *)output, (const int8_t *)quantized, scales, (const uint16_t *)input, vectors, rows, columns, block,
+        scale_type);
 }
 
 }  // namespace
@@ -280,15 +234,15 @@ extern "C" bool k3_moe_q8_gemm_bf16(void *output, const void *quantized, const v
         return false;
     }
     if ((((uintptr_t)quantized) & 7u) != 0 || (((uintptr_t)input) & 15u) != 0) return false;
-    const uint32_t blocks = (uint32_t)std::min<uint64_t>(((uint64_t)rows + 7) / 8, (uint64_t)sm_count() * 8);
+    cudaStream_t st = (cudaStream_t)stream;
     if (vector_count == 1u) {
-        q8_gemm_kernel<1><<<blocks, 256, 0, (cudaStream_t)stream>>>(
-            (uint16_t *)output, (const int8_t *)quantized, scales, (const uint16_t *)input,
-            vector_count, rows, columns, block, scale_type);
+        launch_exact_q8<4, 1>(output, quantized, scales, input, vector_count, rows, columns, block, scale_type, st);
+    } else if (vector_count <= 2u) {
+        launch_exact_q8<4, 2>(output, quantized, scales, input, vector_count, rows, columns, block, scale_type, st);
+    } else if (vector_count <= 4u) {
+        launch_exact_q8<4, 4>(output, quantized, scales, input, vector_count, rows, columns, block, scale_type, st);
     } else {
-        q8_gemm_kernel<4><<<blocks, 256, 0, (cudaStream_t)stream>>>(
-            (uint16_t *)output, (const int8_t *)quantized, scales, (const uint16_t *)input,
-            vector_count, rows, columns, block, scale_type);
+        launch_exact_q8<4, 8>(output, quantized, scales, input, vector_count, rows, columns, block, scale_type, st);
     }
     return launch_ok();
 }
