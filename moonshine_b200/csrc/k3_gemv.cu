@@ -11,7 +11,7 @@
 // single-row calls byte for byte, and the batch_tile argument is validated
 // but does not change any result.
 #include "k3_exact_gemm.cuh"
-#include "k3_gemv.cuh"
+#include "k3_mxfp4_rows.cuh"
 #include "k3_moe_ops.h"
 
 #include <algorithm>
@@ -100,38 +100,6 @@ bf16_gemm_kernel(Out *__restrict__ out, const uint16_t *__restrict__ w,
     }
 }
 
-// ------------------------------------------------------------------ MXFP4
-// Item = 32 rows.  Two input rows per pass (MMA columns 0-3 and 4-7).
-template <bool kAligned16>
-__global__ void __launch_bounds__(kGemvThreads)
-mxfp4_gemm_kernel(uint16_t *__restrict__ out, const uint8_t *__restrict__ packed,
-                  const uint8_t *__restrict__ scales, const uint16_t *__restrict__ x,
-                  uint32_t vectors, uint32_t rows, uint32_t k, uint32_t k_pad) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const GemvSmem sm = carve_gemv_smem(smem_raw, k_pad);
-    __half *xs = sm.xs;
-    float *red = sm.red, *out_s = sm.out_s, *inv_scale = sm.inv_scale, *scratch = sm.scratch;
-    const uint32_t items = (rows + kGemvRowsPerItem - 1) / kGemvRowsPerItem;
-    for (uint32_t v0 = 0; v0 < vectors; v0 += 2u) {
-        const uint32_t nvec = min(2u, vectors - v0);
-        __syncthreads();
-        stage_vectors_f16(xs, inv_scale, x + (uint64_t)v0 * k,
-                          nvec > 1u ? x + (uint64_t)(v0 + 1u) * k : nullptr, k, k_pad, scratch);
-        for (uint32_t item = blockIdx.x; item < items; item += gridDim.x) {
-            const uint32_t row0 = item * kGemvRowsPerItem;
-            mxfp4_item_32rows<kAligned16>(out_s, red, packed, scales, row0, rows, k, xs, k_pad,
-                                          nvec, inv_scale);
-            if (threadIdx.x < 64u) {
-                const uint32_t vec = threadIdx.x >> 5, r = threadIdx.x & 31u;
-                if (vec < nvec && row0 + r < rows) {
-                    out[(uint64_t)(v0 + vec) * rows + row0 + r] =
-                        float_to_bf16_bits(out_s[vec * 32u + r]);
-                }
-            }
-        }
-    }
-}
-
 template <typename Out, int kR, int kV, int kSR, int kSV>
 void launch_exact_bf16(void *output, const void *weights, const void *input, uint32_t vectors, uint32_t rows,
                        uint32_t columns, cudaStream_t stream) {
@@ -160,6 +128,19 @@ bool launch_bf16(void *output, const void *weights, const void *input, uint32_t 
     } else {
         launch_exact_bf16<Out, 4, 4, 4, 2>(output, weights, input, vectors, rows, columns, stream);
     }
+    return launch_ok();
+}
+
+template <int kTiles, int kBlocks, int kTeams>
+bool launch_mxfp4(void *output, const void *packed, const void *scales, const void *input, uint32_t vectors,
+                  uint32_t rows, uint32_t columns, cudaStream_t stream) {
+    constexpr size_t smem = mxfp4_tile_smem<kTiles, kBlocks, kTeams>();
+    auto kernel = mxfp4_tile_kernel<kTiles, kBlocks, kTeams>;
+    if (!set_max_dynamic_smem((const void *)kernel, smem)) return false;
+    const dim3 grid((rows + 16u * kBlocks - 1u) / (16u * kBlocks), (vectors + 8u * kTiles - 1u) / (8u * kTiles));
+    kernel<<<grid, 32 * kBlocks * kTeams, smem, stream>>>((uint16_t *)output, (const uint8_t *)packed,
+                                                          (const uint8_t *)scales, (const uint16_t *)input, vectors,
+                                                          rows, columns);
     return launch_ok();
 }
 
@@ -282,23 +263,36 @@ extern "C" bool k3_rocm_mxfp4_gemm_tiled_bf16(void *output, const void *packed,
     }
     if (batch_tile != 16u && batch_tile != 32u && batch_tile != 64u) return false;
     if ((((uintptr_t)packed) & 7u) != 0) return false;   // the format guarantees 8 bytes
-    const uint32_t k_pad = (columns + 127u) / 128u * 128u;
-    const size_t smem = gemv_smem_bytes(k_pad);
-    const uint32_t items = (rows + kGemvRowsPerItem - 1) / kGemvRowsPerItem;
-    const uint32_t blocks = std::min(items, (uint32_t)sm_count() * 2u);
-    const bool aligned = (((uintptr_t)packed) & 15u) == 0;
-    auto kernel = aligned ? mxfp4_gemm_kernel<true> : mxfp4_gemm_kernel<false>;
-    if (smem > 48 * 1024) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return false;
+    cudaStream_t st = (cudaStream_t)stream;
+    const uint32_t tiles = (vector_count + 7u) / 8u;
+    const bool wide = (((uintptr_t)input) & 15u) == 0;
+    if (tiles == 1u || !wide) {
+        auto kernel = wide ? mxfp4_rows_kernel<true> : mxfp4_rows_kernel<false>;
+        kernel<<<dim3((rows + 15u) / 16u, tiles), 32 * kMxSplits, 0, st>>>(
+            (uint16_t *)output, (const uint8_t *)packed, (const uint8_t *)scales, (const uint16_t *)input, vector_count,
+            rows, columns);
+        return launch_ok();
+    }
+    // Vectors in passes of equal width, at most seven tiles of accumulators: a block's time is
+    // about tiles + 3 (the dequantisation), and what counts is that of the waves it takes.
+    uint32_t best = 7u, best_cost = 0xffffffffu;
+    for (uint32_t width = 2u; width <= 7u; width++) {
+        const uint32_t block_rows = width <= 3u ? 32u : 64u;
+        const uint64_t blocks = (uint64_t)((rows + block_rows - 1u) / block_rows) * ((tiles + width - 1u) / width);
+        const uint64_t cost = (blocks + sm_count() - 1u) / sm_count() * (width + 3u);
+        if (cost < best_cost) {
+            best = width;
+            best_cost = (uint32_t)std::min<uint64_t>(cost, 0xfffffffeu);
         }
     }
-    kernel<<<blocks, kGemvThreads, smem, (cudaStream_t)stream>>>(
-        (uint16_t *)output, (const uint8_t *)packed, (const uint8_t *)scales,
-        (const uint16_t *)input, vector_count, rows, columns, k_pad);
-    return launch_ok();
+    switch (best) {
+        case 2: return launch_mxfp4<2, 2, 8>(output, packed, scales, input, vector_count, rows, columns, st);
+        case 3: return launch_mxfp4<3, 2, 8>(output, packed, scales, input, vector_count, rows, columns, st);
+        case 4: return launch_mxfp4<4, 4, 4>(output, packed, scales, input, vector_count, rows, columns, st);
+        case 5: return launch_mxfp4<5, 4, 4>(output, packed, scales, input, vector_count, rows, columns, st);
+        case 6: return launch_mxfp4<6, 4, 4>(output, packed, scales, input, vector_count, rows, columns, st);
+        default: return launch_mxfp4<7, 4, 4>(output, packed, scales, input, vector_count, rows, columns, st);
+    }
 }
 
 extern "C" bool k3_rocm_mxfp4_gemm_bf16(void *output, const void *packed, const void *scales,
