@@ -1,8 +1,9 @@
 """Build the native library in-tree with nvcc for sm_100a.
 
 ``python -m moonshine_b200.build`` compiles every ``csrc/*.cu`` into
-``moonshine_b200/libk3moe.so``.  Object files are cached under
-``moonshine_b200/_build`` and rebuilt when a source or header is newer.
+``moonshine_b200/libk3moe.so`` and ``csrc/k3_pyops.cpp``, the CPython bindings of
+its entry points, into ``moonshine_b200/_k3ops.so``.  Object files are cached
+under ``moonshine_b200/_build`` and rebuilt when a source or header is newer.
 """
 from __future__ import annotations
 
@@ -10,6 +11,7 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -17,6 +19,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libk3moe.so")
+BINDINGS = os.path.join(HERE, "_k3ops.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -61,7 +64,7 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False) 
         if verbose or res.returncode != 0 or ptxas_info:
             sys.stderr.write(" ".join(cmd) + "\n" + res.stdout + res.stderr)
         if res.returncode != 0:
-            raise RuntimeError("nvcc failed for " + cmd[-3])
+            raise RuntimeError("compilation failed: " + " ".join(cmd))
 
     with ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as pool:
         list(pool.map(run, jobs))
@@ -71,6 +74,11 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False) 
         if res.returncode != 0:
             sys.stderr.write(res.stdout + res.stderr)
             raise RuntimeError("link failed")
+    src = os.path.join(CSRC, "k3_pyops.cpp")
+    if force or not os.path.exists(BINDINGS) or os.path.getmtime(BINDINGS) < max(os.path.getmtime(src), hdr_time):
+        run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall",
+             "-I", os.path.join(ROOT, "include"), "-I", sysconfig.get_paths()["include"], "-o", BINDINGS, src,
+             "-L", HERE, "-l:libk3moe.so", "-Wl,-rpath,$ORIGIN"])
     return LIB
 
 

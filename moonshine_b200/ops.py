@@ -64,8 +64,15 @@ def _make(name, restype, argtypes):
     return call
 
 
-for _name, (_res, _args) in _native.SIGNATURES.items():
-    globals()[_name] = _make(_name, _res, _args)
+_CALLS = {_name: _make(_name, _res, _args) for _name, (_res, _args) in _native.SIGNATURES.items()}
+try:
+    # the same functions with their arguments converted in C (csrc/k3_pyops.cpp): a ctypes call
+    # takes longer than most operators run
+    from . import _k3ops
+    _CALLS.update(_k3ops.bind(_CALLS, torch.Tensor, torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice))
+except (ImportError, AttributeError):        # not built, or a torch without these: the ctypes forms stay
+    pass
+globals().update(_CALLS)
 
 ACT_SITU, ACT_SWIGLU = 0, 1
 Q8_F32, Q8_F16 = 0, 1
