@@ -424,6 +424,7 @@ decode_router_kernel(DecodeArgs a) {
 __global__ void __launch_bounds__(256)
 decode_terms_kernel(const uint16_t *__restrict__ x, uint8_t *x_terms, uint8_t *x_sf, uint32_t *control,
                     uint32_t hidden) {
+    pdl_wait();
     const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
     if (blockIdx.x == 0 && threadIdx.x < 64u) control[threadIdx.x] = 0u;
     const uint32_t blk = blockIdx.x * 8u + warp;
@@ -771,9 +772,10 @@ bool k3_decode_experts_token(const k3_moe_layer_desc *d, const void *x, const vo
     }
     uint8_t *x_terms = nullptr, *x_sf = nullptr;
     k3_decode_mx_vector_scratch(d, scratch, (void **)&x_terms, (void **)&x_sf);
-    decode_terms_kernel<<<(d->hidden / 32u + 7u) / 8u, 256, 0, stream>>>(
-        (const uint16_t *)x, x_terms, x_sf, (uint32_t *)k3_decode_mx_control_words(d, scratch), d->hidden);
-    if (!launch_ok()) return false;
+    if (!launch_chained(decode_terms_kernel, (d->hidden / 32u + 7u) / 8u, 256, 0, stream, (const uint16_t *)x, x_terms,
+                        x_sf, (uint32_t *)k3_decode_mx_control_words(d, scratch), d->hidden)) {
+        return false;
+    }
     return k3_decode_mx_experts(d, const_cast<void *>(ids), nullptr, nullptr, act, rows_out, scratch, nullptr, nullptr,
                                 0u, stream);
 }

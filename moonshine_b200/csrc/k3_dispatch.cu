@@ -27,8 +27,8 @@ __device__ uint32_t g_dispatch_status = 0;
 
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 route_hist_kernel(uint32_t *__restrict__ hist, const uint32_t *__restrict__ ids,
-                  uint32_t routes, uint32_t experts, uint32_t chunks,
-                  uint32_t *__restrict__ error_flag) {
+                  uint32_t routes, uint32_t experts, uint32_t chunks) {
+    pdl_wait();
     extern __shared__ uint32_t smem_hist[];   // [kWarpsPerBlock][experts]
     const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
     const uint32_t chunk = blockIdx.x * kWarpsPerBlock + warp;
@@ -41,10 +41,7 @@ route_hist_kernel(uint32_t *__restrict__ hist, const uint32_t *__restrict__ ids,
         for (uint32_t r = begin + lane; r < end; r += kWarp) {
             const uint32_t e = ids[r];
             if (e < experts) atomicAdd(&h[e], 1u);
-            else {                                     // invalid route id
-                atomicExch(error_flag, 1u);
-                g_dispatch_status = 2u;
-            }
+            else g_dispatch_status = 2u;               // invalid route id
         }
         __syncwarp();
         for (uint32_t e = lane; e < experts; e += kWarp) {
@@ -57,6 +54,7 @@ route_hist_kernel(uint32_t *__restrict__ hist, const uint32_t *__restrict__ ids,
 __global__ void __launch_bounds__(kMaxExperts)
 route_scan_kernel(uint32_t *__restrict__ hist, uint32_t *__restrict__ offsets,
                   uint32_t experts, uint32_t chunks) {
+    pdl_wait();
     __shared__ uint32_t warp_sums[kMaxExperts / 32];
     const uint32_t e = threadIdx.x;
     uint32_t running = 0u;
@@ -99,6 +97,7 @@ route_place_kernel(uint32_t *__restrict__ sorted_route, uint32_t *__restrict__ s
                    uint32_t *__restrict__ inv_perm, const uint32_t *__restrict__ hist,
                    const uint32_t *__restrict__ offsets, const uint32_t *__restrict__ ids,
                    uint32_t routes, uint32_t experts, uint32_t chunks, uint32_t top_k) {
+    pdl_wait();
     extern __shared__ uint32_t smem_cursor[];   // [kWarpsPerBlock][experts]
     const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
     const uint32_t chunk = blockIdx.x * kWarpsPerBlock + warp;
@@ -129,6 +128,19 @@ route_place_kernel(uint32_t *__restrict__ sorted_route, uint32_t *__restrict__ s
         }
         __syncwarp();
     }
+}
+
+bool launch_dispatch(uint32_t *hist, void *offsets, void *sorted_route, void *sorted_token, void *inv_perm,
+                     const void *expert_ids, uint32_t routes, uint32_t experts, uint32_t top_k, cudaStream_t stream) {
+    const uint32_t chunks = (routes + kChunk - 1) / kChunk;
+    const uint32_t blocks = (chunks + kWarpsPerBlock - 1) / kWarpsPerBlock;
+    const size_t smem = (size_t)kWarpsPerBlock * experts * sizeof(uint32_t);
+    return launch_chained(route_hist_kernel, blocks, kWarpsPerBlock * 32, smem, stream, hist,
+                          (const uint32_t *)expert_ids, routes, experts, chunks) &&
+           launch_chained(route_scan_kernel, 1, kMaxExperts, 0, stream, hist, (uint32_t *)offsets, experts, chunks) &&
+           launch_chained(route_place_kernel, blocks, kWarpsPerBlock * 32, smem, stream, (uint32_t *)sorted_route,
+                          (uint32_t *)sorted_token, (uint32_t *)inv_perm, hist, (const uint32_t *)offsets,
+                          (const uint32_t *)expert_ids, routes, experts, chunks, top_k);
 }
 
 }  // namespace
@@ -167,22 +179,9 @@ extern "C" bool k3_moe_dispatch_build(void *offsets, void *sorted_route, void *s
     if (routes64 > 0x7fffffffull) return false;
     if (workspace_bytes < k3_moe_dispatch_workspace_bytes(tokens, top_k, experts)) return false;
     const uint32_t routes = (uint32_t)routes64;
-    const uint32_t chunks = (routes + kChunk - 1) / kChunk;
     cudaStream_t stream = (cudaStream_t)stream_pointer;
-    uint32_t *error_flag = (uint32_t *)workspace;          // first 256 bytes: status words
     uint32_t *hist = (uint32_t *)((char *)workspace + 256);
-    if (cudaMemsetAsync(error_flag, 0, 256, stream) != cudaSuccess) return false;
-    const uint32_t blocks = (chunks + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    const size_t smem = (size_t)kWarpsPerBlock * experts * sizeof(uint32_t);
-    route_hist_kernel<<<blocks, kWarpsPerBlock * 32, smem, stream>>>(
-        hist, (const uint32_t *)expert_ids, routes, experts, chunks, error_flag);
-    if (!launch_ok()) return false;
-    route_scan_kernel<<<1, kMaxExperts, 0, stream>>>(hist, (uint32_t *)offsets, experts, chunks);
-    if (!launch_ok()) return false;
-    route_place_kernel<<<blocks, kWarpsPerBlock * 32, smem, stream>>>(
-        (uint32_t *)sorted_route, (uint32_t *)sorted_token, (uint32_t *)inv_perm, hist,
-        (const uint32_t *)offsets, (const uint32_t *)expert_ids, routes, experts, chunks, top_k);
-    return launch_ok();
+    return launch_dispatch(hist, offsets, sorted_route, sorted_token, inv_perm, expert_ids, routes, experts, top_k, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -204,8 +203,8 @@ extern "C" bool k3_moe_dispatch_build(void *offsets, void *sorted_route, void *s
 //   * All calls on one GPU share the array.  Two calls whose kernels overlap in
 //     time (different streams, or different host threads) corrupt each other's
 //     histograms: serialise them on one stream.  The array keeps the previous
-//     call's contents; the status words are cleared and every histogram entry
-//     a call reads is rewritten by that call first.
+//     call's contents; every histogram entry a call reads is rewritten by that
+//     call first.
 //   * The first call on each GPU looks up the array's device address
 //     (cudaGetSymbolAddress, with that GPU current).  Make that first call
 //     outside any stream capture.
@@ -274,33 +273,10 @@ extern "C" bool k3_moe_dispatch_build_noalloc(void *offsets, void *sorted_route,
     unsigned char *scratch = (unsigned char *)scratch_for_current_device(error, error_size);
     if (!scratch) return false;
     const uint32_t routes = (uint32_t)routes64;
-    const uint32_t chunks = (routes + kChunk - 1) / kChunk;
     cudaStream_t stream = (cudaStream_t)stream_pointer;
-    uint32_t *error_flag = (uint32_t *)scratch;                 // status words, must start at zero
-    uint32_t *hist = (uint32_t *)(scratch + 256);               // rewritten below before it is read
-    if (cudaMemsetAsync(error_flag, 0, 256, stream) != cudaSuccess) {
-        (void)cudaGetLastError();
-        set_error(error, error_size, "cudaMemsetAsync of the status words failed");
-        return false;
-    }
-    const uint32_t blocks = (chunks + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    const size_t smem = (size_t)kWarpsPerBlock * experts * sizeof(uint32_t);
-    route_hist_kernel<<<blocks, kWarpsPerBlock * 32, smem, stream>>>(
-        hist, (const uint32_t *)expert_ids, routes, experts, chunks, error_flag);
-    if (!launch_ok()) {
-        set_error(error, error_size, "histogram kernel launch failed");
-        return false;
-    }
-    route_scan_kernel<<<1, kMaxExperts, 0, stream>>>(hist, (uint32_t *)offsets, experts, chunks);
-    if (!launch_ok()) {
-        set_error(error, error_size, "scan kernel launch failed");
-        return false;
-    }
-    route_place_kernel<<<blocks, kWarpsPerBlock * 32, smem, stream>>>(
-        (uint32_t *)sorted_route, (uint32_t *)sorted_token, (uint32_t *)inv_perm, hist,
-        (const uint32_t *)offsets, (const uint32_t *)expert_ids, routes, experts, chunks, top_k);
-    if (!launch_ok()) {
-        set_error(error, error_size, "placement kernel launch failed");
+    uint32_t *hist = (uint32_t *)(scratch + 256);               // rewritten before it is read
+    if (!launch_dispatch(hist, offsets, sorted_route, sorted_token, inv_perm, expert_ids, routes, experts, top_k, stream)) {
+        set_error(error, error_size, "dispatch kernel launch failed");
         return false;
     }
     return true;

@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(kThreads)
 activation_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ gate,
                   const uint16_t *__restrict__ up, uint64_t count, int kind, float beta,
                   float linear_beta) {
+    pdl_wait();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool aligned = ((((uintptr_t)out) | ((uintptr_t)gate) | ((uintptr_t)up)) & 15u) == 0;
@@ -62,10 +63,25 @@ activation_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ gate,
     }
 }
 
+// The same for a row or a few: two elements per thread, so that a row of 3072 spreads over a
+// dozen blocks instead of queueing eight expf / tanhf chains in each of 384 threads.
+__global__ void __launch_bounds__(128)
+activation_pairs_kernel(uint32_t *__restrict__ out, const uint32_t *__restrict__ gate, const uint32_t *__restrict__ up,
+                        uint32_t pairs, int kind, float beta, float linear_beta) {
+    pdl_wait();
+    const uint32_t i = blockIdx.x * 128u + threadIdx.x;
+    if (i >= pairs) return;
+    const uint32_t g = gate[i], u = up[i];
+    const uint32_t lo = float_to_bf16_bits(activation(bf16_lo(g), bf16_lo(u), kind, beta, linear_beta));
+    const uint32_t hi = float_to_bf16_bits(activation(bf16_hi(g), bf16_hi(u), kind, beta, linear_beta));
+    out[i] = lo | (hi << 16);
+}
+
 // ----------------------------------------------------------------------- add
 __global__ void __launch_bounds__(kThreads)
 add_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ a,
            const uint16_t *__restrict__ b, uint64_t count) {
+    pdl_wait();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const bool aligned = ((((uintptr_t)out) | ((uintptr_t)a) | ((uintptr_t)b)) & 15u) == 0;
@@ -98,6 +114,7 @@ template <bool Scatter>
 __global__ void __launch_bounds__(kThreads)
 copy_rows_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ in,
                  const uint32_t *__restrict__ ids, uint32_t rows, uint32_t row_size) {
+    pdl_wait();
     // one warp per row; 16-byte copies when both sides allow it
     const uint32_t warps_per_block = blockDim.x / kWarp;
     const uint32_t lane = threadIdx.x % kWarp;
@@ -126,6 +143,7 @@ __global__ void __launch_bounds__(kThreads)
 weighted_sum_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ vectors,
                     const float *__restrict__ weights, uint32_t tokens, uint32_t count,
                     uint32_t hidden) {
+    pdl_wait();
     extern __shared__ float w_s[];
     const bool wide = (hidden % 8u == 0) &&
                       ((((uintptr_t)out) | ((uintptr_t)vectors)) & 15u) == 0;
@@ -138,8 +156,9 @@ weighted_sum_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ vec
         const uint16_t *v = vectors + (uint64_t)token * count * hidden;
         uint16_t *o = out + (uint64_t)token * hidden;
         if (wide) {
-            for (uint32_t c = threadIdx.x; c < hidden / 8u; c += blockDim.x) {
+            for (uint32_t c = blockIdx.y * blockDim.x + threadIdx.x; c < hidden / 8u; c += gridDim.y * blockDim.x) {
                 float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
                 for (uint32_t r = 0; r < count; r++) {
                     const uint4 q =
                         reinterpret_cast<const uint4 *>(v + (uint64_t)r * hidden)[c];
@@ -162,7 +181,7 @@ weighted_sum_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ vec
                 reinterpret_cast<uint4 *>(o)[c] = make_uint4(r4[0], r4[1], r4[2], r4[3]);
             }
         } else {
-            for (uint32_t d = threadIdx.x; d < hidden; d += blockDim.x) {
+            for (uint32_t d = blockIdx.y * blockDim.x + threadIdx.x; d < hidden; d += gridDim.y * blockDim.x) {
                 float acc = 0.f;
                 for (uint32_t r = 0; r < count; r++) {
                     acc = fmaf(w_s[r], bf16_bits_to_float(v[(uint64_t)r * hidden + d]), acc);
@@ -176,30 +195,70 @@ weighted_sum_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ vec
 // ------------------------------------------------------------------ RMSNorm
 // Sum of squares in the reference's order: 256 strided lanes, one fused
 // multiply-add per element, binary tree (k3_rocm_ops.cu:837-867).
+//
+// A row of up to kNormHeld * 256 columns is read once, all loads in flight, and kept in
+// registers for the second pass; the tree runs over shared memory once (widths 128, 64, 32)
+// and then in every warp by shuffles.  One row of 7168: 6.8 us with a load, a wait and eight
+// barriers per step, 3.1 us in a chain now (bound by two memory round trips).
+constexpr uint32_t kNormHeld = 32;
+
 __global__ void __launch_bounds__(kThreads)
 rms_norm_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ in,
                 const uint16_t *__restrict__ weight, uint32_t vectors, uint32_t hidden,
                 float epsilon) {
-    __shared__ float red[kThreads];
-    for (uint32_t v = blockIdx.x; v < vectors; v += gridDim.x) {
+    pdl_wait();
+    __shared__ float red[2][kThreads];
+    const uint32_t lane = threadIdx.x % kWarp;
+    const bool held = hidden <= kNormHeld * kThreads;
+    uint32_t turn = 0u;
+    for (uint32_t v = blockIdx.x; v < vectors; v += gridDim.x, turn ^= 1u) {
         const uint16_t *x = in + (uint64_t)v * hidden;
+        uint16_t xs[kNormHeld], ws[kNormHeld];
         float sum = 0.f;
-        for (uint32_t d = threadIdx.x; d < hidden; d += kThreads) {
-            const float value = bf16_bits_to_float(x[d]);
-            sum = fmaf(value, value, sum);
+        if (held) {
+#pragma unroll
+            for (uint32_t j = 0; j < kNormHeld; j++) {
+                const uint32_t d = threadIdx.x + j * kThreads;
+                xs[j] = d < hidden ? x[d] : 0u;
+                ws[j] = d < hidden ? weight[d] : 0u;
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < kNormHeld; j++) {
+                const float value = bf16_bits_to_float(xs[j]);
+                sum = fmaf(value, value, sum);             // + 0 past the end changes nothing
+            }
+        } else {
+            for (uint32_t d = threadIdx.x; d < hidden; d += kThreads) {
+                const float value = bf16_bits_to_float(x[d]);
+                sum = fmaf(value, value, sum);
+            }
         }
-        red[threadIdx.x] = sum;
+        float *r = red[turn];                              // the other half may still be read
+        r[threadIdx.x] = sum;
         __syncthreads();
-        for (uint32_t width = kThreads / 2; width > 0; width >>= 1) {
-            if (threadIdx.x < width) red[threadIdx.x] += red[threadIdx.x + width];
-            __syncthreads();
-        }
-        const float reciprocal_std = 1.0f / sqrtf(red[0] / (float)hidden + epsilon);
-        __syncthreads();
-        for (uint32_t d = threadIdx.x; d < hidden; d += kThreads) {
-            const float value = __fmul_rn(__fmul_rn(bf16_bits_to_float(x[d]), reciprocal_std),
-                                          bf16_bits_to_float(weight[d]));
-            out[(uint64_t)v * hidden + d] = float_to_bf16_bits(value);
+        float t0 = r[lane] + r[lane + 128u], t1 = r[lane + 32u] + r[lane + 160u];
+        const float t2 = r[lane + 64u] + r[lane + 192u], t3 = r[lane + 96u] + r[lane + 224u];
+        t0 += t2;
+        t1 += t3;
+        t0 += t1;
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) t0 += __shfl_xor_sync(0xffffffffu, t0, w);
+        const float reciprocal_std = 1.0f / sqrtf(t0 / (float)hidden + epsilon);
+        if (held) {
+#pragma unroll
+            for (uint32_t j = 0; j < kNormHeld; j++) {
+                const uint32_t d = threadIdx.x + j * kThreads;
+                if (d < hidden) {
+                    out[(uint64_t)v * hidden + d] = float_to_bf16_bits(__fmul_rn(
+                        __fmul_rn(bf16_bits_to_float(xs[j]), reciprocal_std), bf16_bits_to_float(ws[j])));
+                }
+            }
+        } else {
+            for (uint32_t d = threadIdx.x; d < hidden; d += kThreads) {
+                const float value = __fmul_rn(__fmul_rn(bf16_bits_to_float(x[d]), reciprocal_std),
+                                              bf16_bits_to_float(weight[d]));
+                out[(uint64_t)v * hidden + d] = float_to_bf16_bits(value);
+            }
         }
     }
 }
@@ -216,6 +275,7 @@ __global__ void __launch_bounds__(kThreads)
 router_topk_kernel(uint32_t *__restrict__ ids_out, float *__restrict__ weights_out,
                    const float *__restrict__ logits, const float *__restrict__ bias,
                    uint32_t vectors, uint32_t experts, uint32_t top_k, float scale) {
+    pdl_wait();
     __shared__ RouteScratch rs;
     __shared__ uint32_t ids_s[32];
     __shared__ float weights_s[32];
@@ -252,6 +312,7 @@ router_topk_kernel(uint32_t *__restrict__ ids_out, float *__restrict__ weights_o
 __global__ void q8_quantize_kernel(int8_t *__restrict__ q, void *__restrict__ scales,
                                    const uint16_t *__restrict__ w, uint64_t blocks,
                                    uint32_t block, int scale_f16) {
+    pdl_wait();
     // one warp per block of `block` elements
     const uint32_t lane = threadIdx.x % kWarp;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
@@ -282,6 +343,7 @@ __global__ void q8_quantize_kernel(int8_t *__restrict__ q, void *__restrict__ sc
 __global__ void q8_dequantize_kernel(uint16_t *__restrict__ w, const int8_t *__restrict__ q,
                                      const void *__restrict__ scales, uint64_t count,
                                      uint32_t block, int scale_f16) {
+    pdl_wait();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
         const uint64_t b = i / block;
@@ -300,11 +362,17 @@ extern "C" bool k3_moe_activation_bf16(void *output, const void *gate, const voi
     if (!output || !gate || !up || element_count == 0) return false;
     if (activation != kActSitu && activation != kActSwiglu) return false;
     if (activation == kActSitu && (beta <= 0.0f || linear_beta <= 0.0f)) return false;
-    activation_kernel<<<grid_for((element_count + 7) / 8, kThreads), kThreads, 0,
-                        (cudaStream_t)stream>>>((uint16_t *)output, (const uint16_t *)gate,
-                                                (const uint16_t *)up, element_count, activation,
-                                                beta, linear_beta);
-    return launch_ok();
+    // below one pair per thread slot of the GPU the chains' latency is all there is
+    const uint64_t pairs = element_count / 2u;
+    if (element_count % 2u == 0 && pairs <= (uint64_t)sm_count() * 1024u &&
+        ((((uintptr_t)output) | ((uintptr_t)gate) | ((uintptr_t)up)) & 3u) == 0) {
+        return launch_chained(activation_pairs_kernel, (uint32_t)((pairs + 127u) / 128u), 128, 0, (cudaStream_t)stream,
+                              (uint32_t *)output, (const uint32_t *)gate, (const uint32_t *)up, (uint32_t)pairs,
+                              activation, beta, linear_beta);
+    }
+    return launch_chained(activation_kernel, grid_for((element_count + 7) / 8, kThreads), kThreads, 0,
+                          (cudaStream_t)stream, (uint16_t *)output, (const uint16_t *)gate, (const uint16_t *)up,
+                          element_count, activation, beta, linear_beta);
 }
 
 extern "C" bool k3_rocm_situ_bf16(void *output, const void *gate, const void *up,
@@ -318,31 +386,25 @@ extern "C" bool k3_rocm_situ_bf16(void *output, const void *gate, const void *up
 extern "C" bool k3_rocm_add_bf16(void *output, const void *left, const void *right,
                                  uint64_t element_count, void *stream) {
     if (!output || !left || !right || element_count == 0) return false;
-    add_kernel<<<grid_for((element_count + 7) / 8, kThreads), kThreads, 0,
-                 (cudaStream_t)stream>>>((uint16_t *)output, (const uint16_t *)left,
-                                         (const uint16_t *)right, element_count);
-    return launch_ok();
+    return launch_chained(add_kernel, grid_for((element_count + 7) / 8, kThreads), kThreads, 0,
+                          (cudaStream_t)stream, (uint16_t *)output, (const uint16_t *)left, (const uint16_t *)right,
+                          element_count);
 }
 
 extern "C" bool k3_rocm_gather_rows_bf16(void *output, const void *input, const void *row_ids,
                                          uint32_t row_count, uint32_t row_size, void *stream) {
     if (!output || !input || !row_ids || row_count == 0u || row_size == 0u) return false;
-    copy_rows_kernel<false><<<grid_for(row_count, kThreads / kWarp), kThreads, 0,
-                              (cudaStream_t)stream>>>((uint16_t *)output,
-                                                      (const uint16_t *)input,
-                                                      (const uint32_t *)row_ids, row_count,
-                                                      row_size);
-    return launch_ok();
+    return launch_chained(copy_rows_kernel<false>, grid_for(row_count, kThreads / kWarp), kThreads, 0,
+                          (cudaStream_t)stream, (uint16_t *)output, (const uint16_t *)input,
+                          (const uint32_t *)row_ids, row_count, row_size);
 }
 
 extern "C" bool k3_rocm_scatter_rows_bf16(void *output, const void *input, const void *row_ids,
                                           uint32_t row_count, uint32_t row_size, void *stream) {
     if (!output || !input || !row_ids || row_count == 0u || row_size == 0u) return false;
-    copy_rows_kernel<true><<<grid_for(row_count, kThreads / kWarp), kThreads, 0,
-                             (cudaStream_t)stream>>>((uint16_t *)output, (const uint16_t *)input,
-                                                     (const uint32_t *)row_ids, row_count,
-                                                     row_size);
-    return launch_ok();
+    return launch_chained(copy_rows_kernel<true>, grid_for(row_count, kThreads / kWarp), kThreads, 0,
+                          (cudaStream_t)stream, (uint16_t *)output, (const uint16_t *)input,
+                          (const uint32_t *)row_ids, row_count, row_size);
 }
 
 extern "C" bool k3_rocm_weighted_sum_bf16_batch(void *output, const void *vectors,
@@ -355,10 +417,12 @@ extern "C" bool k3_rocm_weighted_sum_bf16_batch(void *output, const void *vector
     }
     const size_t smem = (size_t)vector_count * sizeof(float);
     if (smem > 48 * 1024) return false;
-    weighted_sum_kernel<<<grid_for(token_count, 1), kThreads, smem, (cudaStream_t)stream>>>(
-        (uint16_t *)output, (const uint16_t *)vectors, (const float *)weights, token_count,
-        vector_count, hidden_size);
-    return launch_ok();
+    // few tokens: the columns of a token over several small blocks
+    const bool few = token_count < 128u;
+    const uint32_t threads = few ? 64u : kThreads;
+    const dim3 grid(grid_for(token_count, 1), few ? (hidden_size / 8u + threads - 1u) / threads + 1u : 1u);
+    return launch_chained(weighted_sum_kernel, grid, threads, smem, (cudaStream_t)stream, (uint16_t *)output,
+                          (const uint16_t *)vectors, (const float *)weights, token_count, vector_count, hidden_size);
 }
 
 extern "C" bool k3_rocm_weighted_sum_bf16(void *output, const void *vectors, const void *weights,
@@ -375,10 +439,9 @@ extern "C" bool k3_rocm_rms_norm_bf16(void *output, const void *input, const voi
         epsilon <= 0.0f) {
         return false;
     }
-    rms_norm_kernel<<<grid_for(vector_count, 1), kThreads, 0, (cudaStream_t)stream>>>(
-        (uint16_t *)output, (const uint16_t *)input, (const uint16_t *)weight, vector_count,
-        hidden_size, epsilon);
-    return launch_ok();
+    return launch_chained(rms_norm_kernel, grid_for(vector_count, 1), kThreads, 0, (cudaStream_t)stream,
+                          (uint16_t *)output, (const uint16_t *)input, (const uint16_t *)weight, vector_count,
+                          hidden_size, epsilon);
 }
 
 extern "C" bool k3_rocm_router_topk_f32_batch(void *expert_ids, void *expert_weights,
@@ -391,10 +454,9 @@ extern "C" bool k3_rocm_router_topk_f32_batch(void *expert_ids, void *expert_wei
         expert_count > 1024u || top_k > 32u || scaling_factor <= 0.0f) {
         return false;
     }
-    router_topk_kernel<<<grid_for(vector_count, 1), kThreads, 0, (cudaStream_t)stream>>>(
-        (uint32_t *)expert_ids, (float *)expert_weights, (const float *)logits,
-        (const float *)correction_bias, vector_count, expert_count, top_k, scaling_factor);
-    return launch_ok();
+    return launch_chained(router_topk_kernel, grid_for(vector_count, 1), kThreads, 0, (cudaStream_t)stream,
+                          (uint32_t *)expert_ids, (float *)expert_weights, (const float *)logits,
+                          (const float *)correction_bias, vector_count, expert_count, top_k, scaling_factor);
 }
 
 extern "C" bool k3_rocm_router_topk_f32(void *expert_ids, void *expert_weights,
@@ -413,11 +475,8 @@ extern "C" bool k3_moe_q8_quantize(void *quantized, void *scales, const void *we
         return false;
     }
     const uint64_t blocks = (uint64_t)rows * (columns / block);
-    q8_quantize_kernel<<<grid_for(blocks, kThreads / kWarp), kThreads, 0,
-                         (cudaStream_t)stream>>>((int8_t *)quantized, scales,
-                                                 (const uint16_t *)weights, blocks, block,
-                                                 scale_type);
-    return launch_ok();
+    return launch_chained(q8_quantize_kernel, grid_for(blocks, kThreads / kWarp), kThreads, 0, (cudaStream_t)stream,
+                          (int8_t *)quantized, scales, (const uint16_t *)weights, blocks, block, scale_type);
 }
 
 extern "C" bool k3_rocm_bf16_quantize_q8_128(void *quantized, void *scales, const void *weights,
@@ -434,7 +493,6 @@ extern "C" bool k3_rocm_q8_128_dequantize_bf16(void *weights, const void *quanti
         return false;
     }
     const uint64_t count = (uint64_t)rows * columns;
-    q8_dequantize_kernel<<<grid_for(count, kThreads), kThreads, 0, (cudaStream_t)stream>>>(
-        (uint16_t *)weights, (const int8_t *)quantized, scales, count, 128u, 0);
-    return launch_ok();
+    return launch_chained(q8_dequantize_kernel, grid_for(count, kThreads), kThreads, 0, (cudaStream_t)stream,
+                          (uint16_t *)weights, (const int8_t *)quantized, scales, count, 128u, 0);
 }

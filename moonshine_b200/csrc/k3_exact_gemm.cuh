@@ -29,7 +29,8 @@ K3_DEVINL void fma_bf16(float &acc, uint16_t a, uint16_t b) {
 
 // ------------------------------------------------------------------------ Q8
 // Warp i owns tree slot i: lanes 32 i .. 32 i + 31, i.e. octets 32 i + lane + 256 j.
-template <int kR, int kV>
+// kDeep steps' loads are in flight at once (one or two input rows: the weights come from HBM).
+template <int kR, int kV, int kDeep>
 __global__ void __launch_bounds__(256)
 exact_q8_kernel(uint16_t *__restrict__ out, const int8_t *__restrict__ q, const void *__restrict__ scales,
                 const uint16_t *__restrict__ x, uint32_t vectors, uint32_t rows, uint32_t columns, uint32_t block,
@@ -41,6 +42,9 @@ exact_q8_kernel(uint16_t *__restrict__ out, const int8_t *__restrict__ q, const 
     const uint32_t slot = threadIdx.x / kWarp;
     const uint32_t octets = columns / 8u, per_row = columns / block;
     const uint32_t row0 = blockIdx.x * kR, v0 = blockIdx.y * kV;
+    if (blockIdx.y == 0 && threadIdx.x == 0 && row0 < rows)
+        prefetch_l2(q + (uint64_t)row0 * columns, (uint64_t)min((uint32_t)kR, rows - row0) * columns);
+    pdl_wait();
     // rows and vectors past the end read the last one; their sums are not stored
     const int8_t *qr[kR];
     uint32_t sr[kR];
@@ -59,40 +63,50 @@ exact_q8_kernel(uint16_t *__restrict__ out, const int8_t *__restrict__ q, const 
 #pragma unroll
         for (int v = 0; v < kV; v++) acc[r][v] = 0.f;
 
-    for (uint32_t octet = 32u * slot + lane; octet < octets; octet += 256u) {
-        uint2 wq[kR];
-        float s[kR];
-        uint4 xq[kV];
-        const uint32_t sidx = octet * 8u / block;
+    for (uint32_t first = 32u * slot + lane; first < octets; first += 256u * kDeep) {
+        uint2 wq[kDeep][kR];
+        float s[kDeep][kR];
+        uint4 xq[kDeep][kV];
 #pragma unroll
-        for (int r = 0; r < kR; r++) wq[r] = *reinterpret_cast<const uint2 *>(qr[r] + (uint64_t)octet * 8u);
+        for (int j = 0; j < kDeep; j++) {
+            const uint32_t octet = min(first + 256u * j, octets - 1u);     // past the end: loaded, not used
+            const uint32_t sidx = octet * 8u / block;
 #pragma unroll
-        for (int v = 0; v < kV; v++) xq[v] = *reinterpret_cast<const uint4 *>(xr[v] + (uint64_t)octet * 8u);
+            for (int r = 0; r < kR; r++) wq[j][r] = *reinterpret_cast<const uint2 *>(qr[r] + (uint64_t)octet * 8u);
 #pragma unroll
-        for (int r = 0; r < kR; r++) {
-            const uint64_t at = (uint64_t)sr[r] * per_row + sidx;
-            s[r] = scale_f16 ? __half2float(reinterpret_cast<const __half *>(scales)[at])
-                             : reinterpret_cast<const float *>(scales)[at];
-        }
-#pragma unroll
-        for (int b = 0; b < 8; b++) {
-            float wf[kR];
+            for (int v = 0; v < kV; v++) xq[j][v] = *reinterpret_cast<const uint4 *>(xr[v] + (uint64_t)octet * 8u);
 #pragma unroll
             for (int r = 0; r < kR; r++) {
-                // byte + 128 spliced under the exponent of 2^23, minus (2^23 + 128): exact
-                const uint32_t word = (b < 4 ? wq[r].x : wq[r].y) ^ 0x80808080u;
-                const float f = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7650u + (b & 3))) - 8388736.0f;
-                wf[r] = __fmul_rn(f, s[r]);
+                const uint64_t at = (uint64_t)sr[r] * per_row + sidx;
+                s[j][r] = scale_f16 ? __half2float(reinterpret_cast<const __half *>(scales)[at])
+                                    : reinterpret_cast<const float *>(scales)[at];
             }
+        }
 #pragma unroll
-            for (int v = 0; v < kV; v++) {
-                const uint32_t pair = (b >> 1) == 0 ? xq[v].x : (b >> 1) == 1 ? xq[v].y : (b >> 1) == 2 ? xq[v].z : xq[v].w;
-                const float xf = (b & 1) ? bf16_hi(pair) : bf16_lo(pair);
+        for (int j = 0; j < kDeep; j++) {
+            if (first + 256u * j >= octets) break;
 #pragma unroll
-                for (int r = 0; r < kR; r++) acc[r][v] = fmaf(wf[r], xf, acc[r][v]);
+            for (int b = 0; b < 8; b++) {
+                float wf[kR];
+#pragma unroll
+                for (int r = 0; r < kR; r++) {
+                    // byte + 128 spliced under the exponent of 2^23, minus (2^23 + 128): exact
+                    const uint32_t word = (b < 4 ? wq[j][r].x : wq[j][r].y) ^ 0x80808080u;
+                    const float f = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7650u + (b & 3))) - 8388736.0f;
+                    wf[r] = __fmul_rn(f, s[j][r]);
+                }
+#pragma unroll
+                for (int v = 0; v < kV; v++) {
+                    const uint4 &xv = xq[j][v];
+                    const uint32_t pair = (b >> 1) == 0 ? xv.x : (b >> 1) == 1 ? xv.y : (b >> 1) == 2 ? xv.z : xv.w;
+                    const float xf = (b & 1) ? bf16_hi(pair) : bf16_lo(pair);
+#pragma unroll
+                    for (int r = 0; r < kR; r++) acc[r][v] = fmaf(wf[r], xf, acc[r][v]);
+                }
             }
         }
     }
+    pdl_trigger();
     // tree: widths 128, 64, 32 join slots, 16 .. 1 join lanes
 #pragma unroll
     for (int p = 0; p < kV; p += kPhase) {
@@ -130,6 +144,9 @@ exact_bf16_kernel(Out *__restrict__ out, const uint16_t *__restrict__ w, const u
     const uint32_t lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
     const uint32_t h = warp & 1u, pair = warp >> 1;
     const uint32_t row0 = (blockIdx.x * kSR + pair % kSR) * kR, v0 = (blockIdx.y * kSV + pair / kSR) * kV;
+    if (blockIdx.y == 0 && lane == 0 && h == 0 && row0 < rows)
+        prefetch_l2(w + (uint64_t)row0 * columns, (uint64_t)min((uint32_t)kR, rows - row0) * columns * 2u);
+    pdl_wait();
     const uint16_t *wr[kR];
     const uint16_t *xr[kV];
 #pragma unroll
@@ -162,6 +179,7 @@ exact_bf16_kernel(Out *__restrict__ out, const uint16_t *__restrict__ w, const u
                 fma_bf16(acc[r][v][3], (uint16_t)(wq[r].y >> 16), (uint16_t)(xq[v].y >> 16));
             }
     }
+    pdl_trigger();
     // tree: width 128 joins the two warps, 64 .. 4 join lanes (16 .. 1), 2 and 1 the four columns
 #pragma unroll
     for (int p = 0; p < kR * kV; p += kPhase) {

@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(256)
 bf16_gemm_kernel(Out *__restrict__ out, const uint16_t *__restrict__ w,
                  const uint16_t *__restrict__ x, uint32_t vectors, uint32_t rows,
                  uint32_t columns) {
+    pdl_wait();
     const uint32_t lane = threadIdx.x % kWarp;
     const uint32_t warps = (gridDim.x * blockDim.x) / kWarp;
     const bool wide = (columns % 8u == 0) && ((((uintptr_t)w) | ((uintptr_t)x)) & 15u) == 0;
@@ -101,11 +102,11 @@ bf16_gemm_kernel(Out *__restrict__ out, const uint16_t *__restrict__ w,
 }
 
 template <typename Out, int kR, int kV, int kSR, int kSV>
-void launch_exact_bf16(void *output, const void *weights, const void *input, uint32_t vectors, uint32_t rows,
+bool launch_exact_bf16(void *output, const void *weights, const void *input, uint32_t vectors, uint32_t rows,
                        uint32_t columns, cudaStream_t stream) {
     const dim3 grid((rows + kR * kSR - 1u) / (kR * kSR), (vectors + kV * kSV - 1u) / (kV * kSV));
-    exact_bf16_kernel<Out, kR, kV, kSR, kSV><<<grid, 64 * kSR * kSV, 0, stream>>>(
-        (Out *)output, (const uint16_t *)weights, (const uint16_t *)input, vectors, rows, columns);
+    return launch_chained(exact_bf16_kernel<Out, kR, kV, kSR, kSV>, grid, 64 * kSR * kSV, 0, stream, (Out *)output,
+                          (const uint16_t *)weights, (const uint16_t *)input, vectors, rows, columns);
 }
 
 template <typename Out>
@@ -115,20 +116,14 @@ bool launch_bf16(void *output, const void *weights, const void *input, uint32_t 
         // ragged columns or odd bases: one warp per weight row, element by element where it must
         const uint32_t blocks = (uint32_t)std::min<uint64_t>(((uint64_t)rows + 7) / 8, (uint64_t)sm_count() * 8);
         auto kernel = vectors == 1u ? bf16_gemm_kernel<Out, 1> : bf16_gemm_kernel<Out, 4>;
-        kernel<<<blocks, 256, 0, stream>>>((Out *)output, (const uint16_t *)weights, (const uint16_t *)input, vectors,
-                                           rows, columns);
-    } else if (vectors == 1u) {
-        launch_exact_bf16<Out, 1, 1, 4, 1>(output, weights, input, vectors, rows, columns, stream);
-    } else if (vectors == 2u) {
-        launch_exact_bf16<Out, 1, 2, 4, 1>(output, weights, input, vectors, rows, columns, stream);
-    } else if (vectors <= 4u) {
-        launch_exact_bf16<Out, 2, 4, 4, 1>(output, weights, input, vectors, rows, columns, stream);
-    } else if (vectors <= 16u) {
-        launch_exact_bf16<Out, 2, 4, 2, 2>(output, weights, input, vectors, rows, columns, stream);
-    } else {
-        launch_exact_bf16<Out, 4, 4, 4, 2>(output, weights, input, vectors, rows, columns, stream);
+        return launch_chained(kernel, blocks, 256, 0, stream, (Out *)output, (const uint16_t *)weights,
+                              (const uint16_t *)input, vectors, rows, columns);
     }
-    return launch_ok();
+    if (vectors == 1u) return launch_exact_bf16<Out, 1, 1, 4, 1>(output, weights, input, vectors, rows, columns, stream);
+    if (vectors == 2u) return launch_exact_bf16<Out, 1, 2, 4, 1>(output, weights, input, vectors, rows, columns, stream);
+    if (vectors <= 4u) return launch_exact_bf16<Out, 2, 4, 4, 1>(output, weights, input, vectors, rows, columns, stream);
+    if (vectors <= 16u) return launch_exact_bf16<Out, 2, 4, 2, 2>(output, weights, input, vectors, rows, columns, stream);
+    return launch_exact_bf16<Out, 4, 4, 4, 2>(output, weights, input, vectors, rows, columns, stream);
 }
 
 template <int kTiles, int kBlocks, int kTeams>
@@ -138,19 +133,17 @@ bool launch_mxfp4(void *output, const void *packed, const void *scales, const vo
     auto kernel = mxfp4_tile_kernel<kTiles, kBlocks, kTeams>;
     if (!set_max_dynamic_smem((const void *)kernel, smem)) return false;
     const dim3 grid((rows + 16u * kBlocks - 1u) / (16u * kBlocks), (vectors + 8u * kTiles - 1u) / (8u * kTiles));
-    kernel<<<grid, 32 * kBlocks * kTeams, smem, stream>>>((uint16_t *)output, (const uint8_t *)packed,
-                                                          (const uint8_t *)scales, (const uint16_t *)input, vectors,
-                                                          rows, columns);
-    return launch_ok();
+    return launch_chained(kernel, grid, 32 * kBlocks * kTeams, smem, stream, (uint16_t *)output,
+                          (const uint8_t *)packed, (const uint8_t *)scales, (const uint16_t *)input, vectors, rows,
+                          columns);
 }
 
-template <int kR, int kV>
-void launch_exact_q8(void *output, const void *quantized, const void *scales, const void *input, uint32_t vectors,
+template <int kR, int kV, int kDeep>
+bool launch_exact_q8(void *output, const void *quantized, const void *scales, const void *input, uint32_t vectors,
                      uint32_t rows, uint32_t columns, uint32_t block, int scale_type, cudaStream_t stream) {
     const dim3 grid((rows + kR - 1u) / kR, (vectors + kV - 1u) / kV);
-    exact_q8_kernel<kR, kV><<<grid, 256, 0, stream>>>(
-        (uint16_t *)output, (const int8_t *)quantized, scales, (const uint16_t *)input, vectors, rows, columns, block,
-        scale_type);
+    return launch_chained(exact_q8_kernel<kR, kV, kDeep>, grid, 256, 0, stream, (uint16_t *)output, (const int8_t *)quantized,
+                          scales, (const uint16_t *)input, vectors, rows, columns, block, scale_type);
 }
 
 }  // namespace
@@ -216,16 +209,14 @@ extern "C" bool k3_moe_q8_gemm_bf16(void *output, const void *quantized, const v
     }
     if ((((uintptr_t)quantized) & 7u) != 0 || (((uintptr_t)input) & 15u) != 0) return false;
     cudaStream_t st = (cudaStream_t)stream;
-    if (vector_count == 1u) {
-        launch_exact_q8<4, 1>(output, quantized, scales, input, vector_count, rows, columns, block, scale_type, st);
-    } else if (vector_count <= 2u) {
-        launch_exact_q8<4, 2>(output, quantized, scales, input, vector_count, rows, columns, block, scale_type, st);
-    } else if (vector_count <= 4u) {
-        launch_exact_q8<4, 4>(output, quantized, scales, input, vector_count, rows, columns, block, scale_type, st);
-    } else {
-        launch_exact_q8<4, 8>(output, quantized, scales, input, vector_count, rows, columns, block, scale_type, st);
-    }
-    return launch_ok();
+    const uint32_t steps = (columns / 8u + 255u) / 256u;
+    auto launch = vector_count > 4u    ? launch_exact_q8<4, 8, 1>
+                  : vector_count > 2u  ? launch_exact_q8<4, 4, 1>
+                  : vector_count == 2u ? (steps == 1u ? launch_exact_q8<4, 2, 1> : launch_exact_q8<4, 2, 4>)
+                  : steps == 1u        ? launch_exact_q8<4, 1, 1>
+                  : steps == 2u        ? launch_exact_q8<4, 1, 2>
+                                       : launch_exact_q8<4, 1, 4>;
+    return launch(output, quantized, scales, input, vector_count, rows, columns, block, scale_type, st);
 }
 
 extern "C" bool k3_rocm_q8_128_gemm_tiled_bf16(void *output, const void *quantized,
@@ -268,10 +259,9 @@ extern "C" bool k3_rocm_mxfp4_gemm_tiled_bf16(void *output, const void *packed,
     const bool wide = (((uintptr_t)input) & 15u) == 0;
     if (tiles == 1u || !wide) {
         auto kernel = wide ? mxfp4_rows_kernel<true> : mxfp4_rows_kernel<false>;
-        kernel<<<dim3((rows + 15u) / 16u, tiles), 32 * kMxSplits, 0, st>>>(
-            (uint16_t *)output, (const uint8_t *)packed, (const uint8_t *)scales, (const uint16_t *)input, vector_count,
-            rows, columns);
-        return launch_ok();
+        return launch_chained(kernel, dim3((rows + 15u) / 16u, tiles), 32 * kMxSplits, 0, st, (uint16_t *)output,
+                              (const uint8_t *)packed, (const uint8_t *)scales, (const uint16_t *)input,
+                              vector_count, rows, columns);
     }
     // Vectors in passes of equal width, at most seven tiles of accumulators: a block's time is
     // about tiles + 3 (the dequantisation), and what counts is that of the waves it takes.

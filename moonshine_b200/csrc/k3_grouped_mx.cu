@@ -235,6 +235,11 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         }
         fence_barrier_init();
     }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, kTmemCols);
+        tmem_relinquish();
+    }
+    pdl_wait();
     {   // exclusive prefix of ceil(rows_g / BN) over the groups (<= 1024)
         __shared__ uint32_t warp_tot[kThreads / kWarp];
         uint32_t v[2], incl[2], run = 0;
@@ -265,10 +270,6 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                 *total_items_s = (excl + incl[j]) * a.m_items;
             }
         }
-    }
-    if (warp == 1) {
-        tmem_alloc(tmem_slot, kTmemCols);
-        tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
@@ -583,7 +584,9 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
 // columns (8 each); a warp converts 256 columns per pass.
 __global__ void __launch_bounds__(256)
 split_rows_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t *__restrict__ sf,
-                  const uint16_t *__restrict__ x, uint32_t rows, uint32_t k) {
+                  const uint16_t *__restrict__ x, uint32_t *__restrict__ counters, uint32_t rows, uint32_t k) {
+    pdl_wait();
+    if (blockIdx.x == 0 && threadIdx.x < 64u) counters[threadIdx.x] = 0u;      // of the two product launches
     const uint32_t lane = threadIdx.x % kWarp;
     const uint32_t warps = (gridDim.x * blockDim.x) / kWarp;
     const uint32_t blocks = k / 32u;
@@ -623,6 +626,7 @@ split_rows_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t *_
 __global__ void __launch_bounds__(256)
 gather_units_kernel(uint4 *__restrict__ dst, const uint4 *__restrict__ src, const uint32_t *__restrict__ index,
                     uint32_t rows, uint32_t units) {
+    pdl_wait();
     const uint32_t lane = threadIdx.x % kWarp;
     const uint32_t warps = (gridDim.x * blockDim.x) / kWarp;
     for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp; r < rows; r += warps) {
@@ -719,8 +723,7 @@ bool launch(const Operands &op, const GmxArgs &args, cudaStream_t stream) {
         }
     }
     if (!set_max_dynamic_smem((const void *)grouped_mx_kernel<kE>, kSmemBytes)) return false;
-    grouped_mx_kernel<kE><<<sm_count(), kThreads, kSmemBytes, stream>>>(maps, args);
-    return launch_ok();
+    return launch_chained(grouped_mx_kernel<kE>, sm_count(), kThreads, kSmemBytes, stream, maps, args);
 }
 
 inline size_t up256(size_t v) { return (v + 255u) & ~(size_t)255u; }
@@ -795,23 +798,22 @@ bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act
     const Scratch s = carve_scratch(d, rows, index ? source_rows : 0u, workspace);
     const uint32_t conv_rows = index ? source_rows : rows;
     const uint32_t cap = (uint32_t)sm_count() * 16u;
-    split_rows_kernel<<<std::min<uint32_t>((conv_rows + 7u) / 8u, cap), 256, 0, stream>>>(
-        index ? s.t_hi : s.x_hi, index ? s.t_lo : s.x_lo, index ? s.t_sf : s.x_sf, (const uint16_t *)rows_in,
-        conv_rows, H);
-    if (!launch_ok()) return false;
+    if (!launch_chained(split_rows_kernel, std::min<uint32_t>((conv_rows + 7u) / 8u, cap), 256, 0, stream,
+                        index ? s.t_hi : s.x_hi, index ? s.t_lo : s.x_lo, index ? s.t_sf : s.x_sf,
+                        (const uint16_t *)rows_in, s.counters, conv_rows, H)) {
+        return false;
+    }
     if (index) {
         const uint32_t blocks = std::min<uint32_t>((rows + 7u) / 8u, cap);
-        gather_units_kernel<<<blocks, 256, 0, stream>>>((uint4 *)s.x_hi, (const uint4 *)s.t_hi,
-                                                       (const uint32_t *)index, rows, H / 16u);
-        gather_units_kernel<<<blocks, 256, 0, stream>>>((uint4 *)s.x_lo, (const uint4 *)s.t_lo,
-                                                       (const uint32_t *)index, rows, H / 16u);
-        gather_units_kernel<<<blocks, 256, 0, stream>>>((uint4 *)s.x_sf, (const uint4 *)s.t_sf,
-                                                       (const uint32_t *)index, rows, H / 512u);
-        if (!launch_ok()) return false;
-    }
-    if (cudaMemsetAsync(s.counters, 0, 256, stream) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
+        const uint32_t *map = (const uint32_t *)index;
+        if (!launch_chained(gather_units_kernel, blocks, 256, 0, stream, (uint4 *)s.x_hi, (const uint4 *)s.t_hi, map,
+                            rows, H / 16u) ||
+            !launch_chained(gather_units_kernel, blocks, 256, 0, stream, (uint4 *)s.x_lo, (const uint4 *)s.t_lo, map,
+                            rows, H / 16u) ||
+            !launch_chained(gather_units_kernel, blocks, 256, 0, stream, (uint4 *)s.x_sf, (const uint4 *)s.t_sf, map,
+                            rows, H / 512u)) {
+            return false;
+        }
     }
     GmxArgs a{};
     a.offsets = (const uint32_t *)offsets;

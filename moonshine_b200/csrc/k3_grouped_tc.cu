@@ -201,6 +201,11 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a0,
         }
         fence_barrier_init();
     }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, kTmemCols);
+        tmem_relinquish();
+    }
+    pdl_wait();
     if (a.offsets != nullptr) {
         // exclusive prefix of ceil(rows_g / BN); groups <= 1024, two elements per thread
         __shared__ uint32_t warp_tot[kThreads / kWarp];
@@ -235,10 +240,6 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a0,
         }
     } else if (threadIdx.x == 0) {
         *total_items_s = ((a.rows + BN - 1u) / BN) * a.m_items;
-    }
-    if (warp == 1) {
-        tmem_alloc(tmem_slot, kTmemCols);
-        tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
@@ -559,8 +560,7 @@ bool launch_tc(const void *a0, const void *a1, const TcArgs &args, const void *b
     if (!ok) return false;
     auto kernel = grouped_tc_kernel<kA, kE>;
     if (!set_max_dynamic_smem((const void *)kernel, C::kSmemBytes)) return false;
-    kernel<<<sm_count(), kThreads, C::kSmemBytes, stream>>>(ma0, ma1, mb, args);
-    return launch_ok();
+    return launch_chained(kernel, sm_count(), kThreads, C::kSmemBytes, stream, ma0, ma1, mb, args);
 }
 
 // Q8 weights -> bf16 (each product q * scale rounded once, as the in-kernel
@@ -568,6 +568,7 @@ bool launch_tc(const void *a0, const void *a1, const TcArgs &args, const void *b
 __global__ void __launch_bounds__(256)
 q8_to_bf16_kernel(uint4 *__restrict__ w, const uint4 *__restrict__ q, const void *__restrict__ scales,
                   uint64_t units, uint32_t block, int scale_f16) {
+    pdl_wait();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < units; i += stride) {
         const uint64_t b = i * 16u / block;
@@ -701,9 +702,10 @@ bool k3_grouped_q8_dense_bf16(void *out, const void *q, const void *scales, cons
     }
     const uint64_t units = (uint64_t)rows * cols / 16u;
     const uint32_t blocks = (uint32_t)std::min<uint64_t>((units + 255u) / 256u, (uint64_t)sm_count() * 16u);
-    q8_to_bf16_kernel<<<blocks, 256, 0, stream>>>((uint4 *)weight_scratch, (const uint4 *)q, scales, units, block,
-                                                  scale_type);
-    if (!launch_ok()) return false;
+    if (!launch_chained(q8_to_bf16_kernel, blocks, 256, 0, stream, (uint4 *)weight_scratch, (const uint4 *)q, scales,
+                        units, block, scale_type)) {
+        return false;
+    }
     TcArgs a{};
     a.out = out;
     a.groups = 1;
@@ -738,10 +740,11 @@ bool k3_grouped_shared_expert(const k3_moe_layer_desc *d, void *out, void *act, 
     const uint32_t blocks = (uint32_t)std::min<uint64_t>((units + 255u) / 256u, (uint64_t)sm_count() * 16u);
     for (int t = 0; t < 3; t++) {
         if ((((uintptr_t)q[t]) & 15u) != 0) return false;
-        q8_to_bf16_kernel<<<blocks, 256, 0, stream>>>((uint4 *)dst[t], (const uint4 *)q[t], sc[t], units,
-                                                      d->q8_block, d->q8_scale_type);
+        if (!launch_chained(q8_to_bf16_kernel, blocks, 256, 0, stream, (uint4 *)dst[t], (const uint4 *)q[t], sc[t],
+                            units, d->q8_block, d->q8_scale_type)) {
+            return false;
+        }
     }
-    if (!launch_ok()) return false;
     TcArgs a{};
     a.groups = 1;
     a.rows = tokens;

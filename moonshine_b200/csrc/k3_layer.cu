@@ -38,6 +38,7 @@ struct GroupedArgs {
 template <bool kFuseAct>
 __global__ void __launch_bounds__(kGemvThreads)
 grouped_rows_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ in, GroupedArgs a) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const GemvSmem sm = carve_gemv_smem(smem_raw, a.k_pad);
     uint32_t expert, row_begin, n;
@@ -101,6 +102,7 @@ combine_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ rows,
                const uint32_t *__restrict__ index, const float *__restrict__ weights,
                const uint16_t *__restrict__ shared, const uint16_t *__restrict__ residual,
                uint32_t tokens, uint32_t top_k, uint32_t hidden) {
+    pdl_wait();
     __shared__ float w_s[32];
     __shared__ uint32_t idx_s[32];
     for (uint32_t token = blockIdx.x; token < tokens; token += gridDim.x) {
@@ -427,10 +429,9 @@ extern "C" bool k3_moe_combine_residual(void *out, const void *rows, const void 
     const uint32_t threads = few ? 64u : 256u;
     const dim3 grid(std::min<uint32_t>(tokens, (uint32_t)sm_count() * 8u),
                     few ? (hidden / 8u + threads - 1u) / threads : 1u);
-    combine_kernel<<<grid, threads, 0, (cudaStream_t)stream>>>(
-        (uint16_t *)out, (const uint16_t *)rows, (const uint32_t *)index, (const float *)weights,
-        (const uint16_t *)shared, (const uint16_t *)residual, tokens, top_k, hidden);
-    return launch_ok();
+    return launch_chained(combine_kernel, grid, threads, 0, (cudaStream_t)stream, (uint16_t *)out,
+                          (const uint16_t *)rows, (const uint32_t *)index, (const float *)weights,
+                          (const uint16_t *)shared, (const uint16_t *)residual, tokens, top_k, hidden);
 }
 
 extern "C" bool k3_moe_combine(void *out, const void *rows, const void *index, const void *weights,

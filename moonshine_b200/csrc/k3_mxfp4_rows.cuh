@@ -100,7 +100,8 @@ K3_DEVINL void mx_finish(uint16_t *out, const float *red, uint32_t row_base, uin
 
 // Up to eight vectors: a block owns 16 rows, a warp one of the eight splits, everything straight
 // from global memory.  Bound by launch and memory latency (a 3072 x 3584 matrix is 5.8 MB: 0.9 us
-// of HBM time).  kWide: the vectors are 16-byte aligned.
+// of HBM time; 5.1 us in a chain of them, 8.2 before chained launches).  Through shared memory by
+// asynchronous copies it is slower (6.2 us).  kWide: the vectors are 16-byte aligned.
 template <bool kWide>
 __global__ void __launch_bounds__(32 * kMxSplits)
 mxfp4_rows_kernel(uint16_t *__restrict__ out, const uint8_t *__restrict__ packed, const uint8_t *__restrict__ scales,
@@ -110,6 +111,12 @@ mxfp4_rows_kernel(uint16_t *__restrict__ out, const uint8_t *__restrict__ packed
     const uint32_t g = lane >> 2, t = lane & 3u;
     const uint32_t groups = k / 32u, per = (groups + kMxSplits - 1u) / kMxSplits;
     const uint32_t row0 = blockIdx.x * 16u, v0 = blockIdx.y * 8u;
+    if (blockIdx.y == 0 && threadIdx.x == 0) {
+        const uint64_t n = min(16u, rows - row0);
+        prefetch_l2(packed + (uint64_t)row0 * (k / 2u), n * (k / 2u));
+        prefetch_l2(scales + (uint64_t)row0 * groups, n * groups);
+    }
+    pdl_wait();
     const MxRowPointers p = mx_row_pointers(packed, scales, row0, rows, k);
     const uint16_t *xv = x + (uint64_t)min(v0 + g, vectors - 1u) * k + 8u * t;
     const uint32_t begin = min(groups, split * per), end = min(groups, begin + per);
@@ -127,6 +134,7 @@ mxfp4_rows_kernel(uint16_t *__restrict__ out, const uint8_t *__restrict__ packed
         dequant_word_bf16(wb, fb);
         mx_group(acc, fa, fb, xq, s_a, s_b);
     }
+    pdl_trigger();
     mx_put(red + (size_t)split * 8u * 16u, acc);
     __syncthreads();
     mx_finish<8, 1, 32 * kMxSplits>(out, red, row0, v0, rows, vectors);
@@ -152,6 +160,11 @@ mxfp4_tile_kernel(uint16_t *__restrict__ out, const uint8_t *__restrict__ packed
     const uint32_t team = warp / kBlocks, rb = warp % kBlocks, tid = threadIdx.x % kTeamThreads;
     const uint32_t groups = k / 32u, per = (groups + kMxSplits - 1u) / kMxSplits;
     const uint32_t row_base = blockIdx.x * kBlocks * 16u, v0 = blockIdx.y * kCols;
+    if (blockIdx.y == 0 && team == 0 && lane == 0 && row_base + rb * 16u < rows) {
+        const uint64_t first = row_base + rb * 16u, n = min(16u, rows - (uint32_t)first);
+        prefetch_l2(packed + first * (k / 2u), n * (k / 2u));
+    }
+    pdl_wait();
     const MxRowPointers p = mx_row_pointers(packed, scales, row_base + rb * 16u, rows, k);
     unsigned char *ring = smem_mx + team * 3u * kStage;
     // this thread's 16-byte chunks of a stage: chunk tid % 8 of vectors tid / 8 + kTeamThreads / 8 * m
@@ -244,6 +257,7 @@ mxfp4_tile_kernel(uint16_t *__restrict__ out, const uint8_t *__restrict__ packed
         for (int n = 0; n < kTiles; n++)
             mx_put(red + ((size_t)(rb * kMxSplits + split) * kCols + 8u * n) * 16u, acc[n]);
     }
+    pdl_trigger();
     __syncthreads();
     mx_finish<kCols, kBlocks, 32 * kBlocks * kTeams>(out, red, row_base, v0, rows, vectors);
 }
