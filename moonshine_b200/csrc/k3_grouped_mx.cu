@@ -21,8 +21,8 @@
 // are numbered with the row tiles of one (expert, weight tile) adjacent: CTAs that take
 // neighbouring items stream the same weights at the same time and the second reader
 // finds them in L2.  Warps: 0 TMA producer (weights), 2 TMA producer (token terms),
-// 3 TMA producer (block scales), 1 and 16 MMA issuers (one per weight tile), 4-7
-// scale writers (shared memory -> tensor memory, one lane quadrant each), 8-15
+// 3 TMA producer (block scales), 1 and 24 MMA issuers (one per weight tile), 4-7
+// scale writers (shared memory -> tensor memory, one lane quadrant each), 8-23
 // epilogue.  All barrier waits are bounded.
 #include "k3_grouped.h"
 #include "k3_moe_ops.h"
@@ -33,10 +33,10 @@
 #include <cuda_fp8.h>
 
 #include <algorithm>
-#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 using namespace k3;
 using namespace k3::tc;
@@ -44,13 +44,15 @@ using namespace k3::tc;
 namespace {
 
 constexpr uint32_t BM = 128, BN = 128, KS = 128;          // K per pipeline stage
-constexpr uint32_t kStages = 3;
 constexpr uint32_t kATile = BM * 128u;                    // bytes in shared memory (8-bit containers)
 constexpr uint32_t kATx = BM * 64u;                       // bytes the TMA transaction counts (packed)
 constexpr uint32_t kBTile = BN * 128u;
 constexpr uint32_t kBBox = 32u;                           // token rows per TMA box
-constexpr uint32_t kStageBytes = 2u * kATile + 2u * kBTile;        // A0 | A1 | Bhi | Blo
-constexpr uint32_t kThreads = 544;                        // 17 warps
+constexpr uint32_t kRingBytes = 192u * 1024u;             // stages of A0 | A1 | token terms: three of 64 KB, or four of
+                                                          //   48 KB where no tile has more than 64 rows
+constexpr uint32_t kEpilogueWarps = 16;
+constexpr uint32_t kIssuer1 = 8u + kEpilogueWarps;        // warp of the second MMA issuer
+constexpr uint32_t kThreads = (kIssuer1 + 1u) * 32u;      // 25 warps
 constexpr uint32_t kSfBatches = 3;                        // scale ring in tensor memory: batches of 4 stages
 constexpr uint32_t kSfSlots = 4;                          // scale ring in shared memory
 constexpr uint32_t kSfKind = BM * 16u;                    // one table's 128 rows x 16 scale bytes
@@ -62,11 +64,11 @@ constexpr uint32_t kSfa1Col = kSfa0Col + 16u * kSfBatches;
 constexpr uint32_t kSfbCol = kSfa1Col + 16u * kSfBatches;
 constexpr uint32_t kMaxGroups = 1024;
 constexpr uint32_t kItemSlots = 4;                        // mailbox of item numbers, producer -> other roles
-constexpr uint32_t kItemReaders = 16;                     // term + scale producers, 2 issuers, 4 writers, 8 epilogue warps
+constexpr uint32_t kItemReaders = 8u + kEpilogueWarps;    // term + scale producers, 2 issuers, 4 writers, epilogue warps
 constexpr uint32_t kNoItem = 0xffffffffu;
 constexpr uint32_t kBarBytes = 512;
 constexpr uint32_t kSmemBytes =
-    kStages * kStageBytes + kSfSlots * kSfSlotBytes + 1024u + kBarBytes + (kMaxGroups + 1u) * 4u;
+    kRingBytes + kSfSlots * kSfSlotBytes + 1024u + kBarBytes + (kMaxGroups + 1u) * 4u;
 
 enum EMode : int { kEAct = 0, kEBf16 = 1 };
 
@@ -79,6 +81,12 @@ K3_DEVINL void tmem_st_32x16(uint32_t taddr, const uint32_t (&v)[16]) {
         "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
         "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
+}
+K3_DEVINL void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
 }
 K3_DEVINL void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -122,12 +130,20 @@ K3_DEVINL uint32_t split_pair(float a, float b) {
     return (uint32_t)hi | ((uint32_t)lo << 16);
 }
 
+// bf16 of lo in the low half, of hi in the high half (round to nearest even)
+K3_DEVINL uint32_t pack_bf16x2(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+
 struct GmxArgs {
     const uint32_t *offsets;             // [groups+1]
     uint16_t *out;                       // bf16 [rows, out_width] (may be null in gate/up mode)
     uint8_t *act_hi, *act_lo, *act_sf;   // gate/up mode: E4M3 terms and block scales of the activation
-    uint32_t groups, rows, w_rows, k, out_width, m_items;
+    uint32_t groups, rows, row_floor, row_ceil, w_rows, k, out_width, m_items;   // groups of row_floor < rows <= row_ceil
     uint32_t *item_counter;              // zero before the launch; items are drawn from it
+    bool behind_wait;                    // the kernel in front of this one in the stream already waited for its inputs
     int activation;
     float beta, linear_beta;
 };
@@ -135,6 +151,25 @@ struct GmxArgs {
 struct Item {
     uint32_t group, row_start, rows_valid, m_item;
 };
+
+// How a row tile's terms lie in shared memory.  Up to 64 rows the hi rows and the lo rows are ONE
+// N operand (lo from row `block` on), so that a K block of 32 is one MMA per weight tile: the
+// 8-bit weight containers are read from shared memory once instead of twice, and shared memory
+// is what bounds short tiles (88 KB per stage of 32 rows instead of 120 KB; 24 rows per
+// expert: 1.15 -> 1.01 ms together with the fourth stage).  A larger tile does not fit its accumulators that way (2 x 256
+// columns): its hi and lo MMAs add into the same columns.
+struct TermLayout {
+    uint32_t block, n;
+    bool stacked;
+};
+K3_DEVINL TermLayout term_layout(uint32_t rows_valid) {
+    TermLayout t;
+    const uint32_t n16 = (rows_valid + 15u) & ~15u;
+    t.block = rows_valid <= 32u ? 32u : rows_valid <= 64u ? 64u : BN;
+    t.stacked = t.block < BN;
+    t.n = t.stacked ? t.block + n16 : n16;
+    return t;
+}
 
 // Item w -> (group, weight tile, row tile).  prefix[g] = row tiles of the groups before
 // g; group g owns items [prefix[g] * m_items, prefix[g + 1] * m_items), numbered with
@@ -157,16 +192,16 @@ K3_DEVINL Item decode_item(uint32_t w, const uint32_t *prefix, const GmxArgs &a)
     return it;
 }
 
-// Accumulator columns [0, 256) as two buffers of 128: a row tile of at most 64 rows takes
-// one buffer (tile 0 in its first 64 columns, tile 1 in the other 64), so that its MMAs run
-// while the epilogue still reads the item before; a larger tile takes both (tile 0 in
+// Accumulator columns [0, 256) as two buffers of 128: a row tile of at most 32 rows (N <= 64)
+// takes one buffer (tile 0 in its first 64 columns, tile 1 in the other 64), so that its MMAs
+// run while the epilogue still reads the item before; a larger tile takes both (tile 0 in
 // [0, 128), tile 1 in [128, 256)).  Issuers and epilogue warps walk the items in the same
 // order and keep the same books: uses per buffer (the barriers' phase) and whose turn it is.
 struct AccBuffers {
     uint32_t use0 = 0u, use1 = 0u;
     uint32_t turn = 0u;
     __device__ uint32_t uses(uint32_t b) const { return b == 0u ? use0 : use1; }
-    __device__ bool small(uint32_t rows_valid) const { return rows_valid <= 64u; }
+    __device__ bool small(uint32_t rows_valid) const { return rows_valid <= 32u; }
     __device__ uint32_t first(bool is_small) const { return is_small ? turn : 0u; }
     __device__ uint32_t column(bool is_small, uint32_t b0, uint32_t tile) const {
         return is_small ? b0 * 128u + tile * 64u : tile * BN;
@@ -190,12 +225,17 @@ struct GmxMaps {
     CUtensorMap sfb;           // token block scales  [rows, K/32]
 };
 
-template <int kE>
+// kStages stages in flight: four where every group has at most 64 rows (the weight stream bounds
+// those), else three.  Weights and terms of a stage share their barriers: an issuer's commits
+// cost about 0.1 us each, and with separate rings (two commits per stage) 128 rows per expert
+// took 2.07 ms instead of 1.89.
+template <int kE, uint32_t kStages>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    unsigned char *sf_smem = base + kStages * kStageBytes;
+    constexpr uint32_t kStageBytes = kRingBytes / kStages;
+    unsigned char *sf_smem = base + kRingBytes;
     uint64_t *bars = reinterpret_cast<uint64_t *>(sf_smem + kSfSlots * kSfSlotBytes);
     uint64_t *full = bars, *empty = full + kStages;
     uint64_t *sf_full = empty + kStages, *sf_empty = sf_full + kSfBatches;
@@ -227,7 +267,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         }
         for (uint32_t b = 0; b < 2u; b++) {
             mbar_init(&acc_full[b], 2);
-            mbar_init(&acc_empty[b], 8);
+            mbar_init(&acc_empty[b], kEpilogueWarps);
         }
         for (uint32_t b = 0; b < kItemSlots; b++) {
             mbar_init(&item_full[b], 1);
@@ -239,14 +279,18 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         tmem_alloc(tmem_slot, kTmemCols);
         tmem_relinquish();
     }
-    pdl_wait();
+    // Two such kernels in a row (few and many rows per group) do not depend on each other: the
+    // second one's blocks start as the first one's leave, and wait for it only before they end.
+    if (!a.behind_wait) pdl_wait();
+    pdl_trigger();
     {   // exclusive prefix of ceil(rows_g / BN) over the groups (<= 1024)
         __shared__ uint32_t warp_tot[kThreads / kWarp];
         uint32_t v[2], incl[2], run = 0;
 #pragma unroll
         for (int j = 0; j < 2; j++) {
             const uint32_t g = threadIdx.x * 2u + j;
-            v[j] = g < a.groups ? (a.offsets[g + 1u] - a.offsets[g] + BN - 1u) / BN : 0u;
+            const uint32_t n = g < a.groups ? a.offsets[g + 1u] - a.offsets[g] : 0u;
+            v[j] = n > a.row_floor && n <= a.row_ceil ? (n + BN - 1u) / BN : 0u;
             run += v[j];
             incl[j] = run;
         }
@@ -334,13 +378,13 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             for (uint32_t w = next_item(); ok && w != kNoItem; w = next_item()) {
                 const Item it = decode_item(w, prefix, a);
                 const uint32_t boxes = (it.rows_valid + kBBox - 1u) / kBBox;
+                const TermLayout t = term_layout(it.rows_valid);
                 for (uint32_t st = 0; st < steps; st++) {
                     if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag)) { ok = false; break; }
-                    unsigned char *dst = base + s * kStageBytes;
                     const int32_t x = (int32_t)(st * KS);
                     // only as many 32-row boxes as the tile has rows
                     mbar_arrive_expect_tx(&full[s], 2u * boxes * kBBox * 128u);
-                    unsigned char *bh = dst + 2u * kATile, *bl = bh + kBTile;
+                    unsigned char *bh = base + s * kStageBytes + 2u * kATile, *bl = bh + t.block * 128u;
                     for (uint32_t b = 0; b < boxes; b++) {
                         const int32_t y = (int32_t)(it.row_start + b * kBBox);
                         tma_load_2d(bh + b * kBBox * 128u, &maps.bhi, &full[s], x, y);
@@ -374,10 +418,10 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                 }
             }
         }
-    } else if (warp == 1 || warp == 16) {
+    } else if (warp == 1 || warp == kIssuer1) {
         // ==================================================== MMA issuers
         // One thread's issue loop cannot keep the tensor pipe fed with K = 32 MMAs, so
-        // warp 1 issues the MMAs of weight tile 0 and warp 16 those of tile 1.  Both
+        // warp 1 issues the MMAs of weight tile 0 and warp kIssuer1 those of tile 1.  Both
         // commit to the same stage / scale / accumulator barriers (count 2).
         if (lane == 0) {
             const uint32_t q = warp == 1 ? 0u : 1u;
@@ -386,10 +430,10 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             bool ok = true;
             for (uint32_t w = next_item(); ok && w != kNoItem; w = next_item()) {
                 const Item it = decode_item(w, prefix, a);
-                const uint32_t n_eff = max(16u, (it.rows_valid + 15u) & ~15u);
+                const TermLayout t = term_layout(it.rows_valid);
                 uint32_t idesc[4];
 #pragma unroll
-                for (uint32_t j = 0; j < 4u; j++) idesc[j] = make_idesc_mx(n_eff, j);
+                for (uint32_t j = 0; j < 4u; j++) idesc[j] = make_idesc_mx(t.n, j);
                 const bool small = acc.small(it.rows_valid);
                 const uint32_t b0 = acc.first(small);
                 if (!mbar_wait(&acc_empty[b0], (acc.uses(b0) & 1u) ^ 1u, abort_flag) ||
@@ -406,16 +450,24 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                         break;
                     }
                     tc_fence_after();
-                    unsigned char *src = base + s * kStageBytes;
+                    const unsigned char *src = base + s * kStageBytes;
                     const uint64_t da = make_desc_sw128(smem_u32(src + q * kATile));
                     const uint64_t dbh = make_desc_sw128(smem_u32(src + 2u * kATile));
-                    const uint64_t dbl = make_desc_sw128(smem_u32(src + 2u * kATile + kBTile));
                     const uint32_t sfs = sb * 16u + (st & 3u) * 4u;
+                    if (t.stacked) {
 #pragma unroll
-                    for (uint32_t j = 0; j < 4u; j++) {          // K blocks of 32 inside the stage
-                        mma_mx(d, da + 2u * j, dbh + 2u * j, idesc[j], sfa_col + sfs, tmem + kSfbCol + sfs,
-                               (st | j) != 0u ? 1u : 0u);
-                        mma_mx(d, da + 2u * j, dbl + 2u * j, idesc[j], sfa_col + sfs, tmem + kSfbCol + sfs, 1u);
+                        for (uint32_t j = 0; j < 4u; j++) {          // K blocks of 32 inside the stage
+                            mma_mx(d, da + 2u * j, dbh + 2u * j, idesc[j], sfa_col + sfs, tmem + kSfbCol + sfs,
+                                   (st | j) != 0u ? 1u : 0u);
+                        }
+                    } else {
+                        const uint64_t dbl = make_desc_sw128(smem_u32(src + 2u * kATile + kBTile));
+#pragma unroll
+                        for (uint32_t j = 0; j < 4u; j++) {
+                            mma_mx(d, da + 2u * j, dbh + 2u * j, idesc[j], sfa_col + sfs, tmem + kSfbCol + sfs,
+                                   (st | j) != 0u ? 1u : 0u);
+                            mma_mx(d, da + 2u * j, dbl + 2u * j, idesc[j], sfa_col + sfs, tmem + kSfbCol + sfs, 1u);
+                        }
                     }
                     mma_commit(&empty[s]);
                     if (++s == kStages) { s = 0; ph ^= 1u; }
@@ -441,6 +493,8 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         bool ok = true;
         for (uint32_t w = __shfl_sync(0xffffffffu, next_item(), 0); ok && w != kNoItem;
              w = __shfl_sync(0xffffffffu, next_item(), 0)) {
+            // a stacked operand's lo rows have the scales of its hi rows
+            const uint32_t repeat = term_layout(decode_item(w, prefix, a).rows_valid).block / 32u - 1u;
             for (uint32_t st = 0; st < steps; st += 4u) {
                 if (!mbar_wait(&sfs_full[ss], ssph, abort_flag)) { ok = false; break; }
                 const unsigned char *src = sf_smem + ss * kSfSlotBytes;
@@ -449,7 +503,8 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                 for (uint32_t t = 0; t < 3u; t++)
 #pragma unroll
                     for (uint32_t c = 0; c < 4u; c++)
-                        v[t][c] = *reinterpret_cast<const uint4 *>(src + t * kSfKind + (32u * c + lane) * 16u);
+                        v[t][c] = *reinterpret_cast<const uint4 *>(
+                            src + t * kSfKind + (32u * (t == 2u ? c & repeat : c) + lane) * 16u);
                 if (!mbar_wait(&sf_empty[sb], sph ^ 1u, abort_flag)) { ok = false; break; }
                 tc_fence_after();
 #pragma unroll
@@ -476,11 +531,13 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         }
     } else {
         // ======================================================== epilogue
-        // Eight warps: quadrant = warp % 4 (tensor-memory lanes), column chunks of 32
-        // token rows alternate between the two warps of a quadrant.  A warp signals
-        // the accumulators free right after its last tensor-memory load.
+        // Sixteen warps: quadrant = warp % 4 (tensor-memory lanes), the tile's token rows in
+        // four parts.  A warp takes its part of both accumulators out of tensor memory at once,
+        // rounded to bf16 (which both modes do anyway) and packed in pairs, and frees the
+        // accumulators before it computes anything: a tile of more than 32 rows has no second
+        // buffer, so the MMAs of the next item wait for exactly this.
         const uint32_t quad = warp & 3u;
-        const uint32_t half = (warp - 8u) >> 2;
+        const uint32_t part = (warp - 8u) >> 2;
         const uint32_t m = 32u * quad + lane;            // weight row inside the tile
         AccBuffers acc;
         for (uint32_t w = __shfl_sync(0xffffffffu, next_item(), 0); w != kNoItem;
@@ -499,73 +556,76 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             const uint32_t col0 = it.m_item * tile_rows + m;
             const uint32_t col1 = kE == kEAct ? col0 : col0 + BM;
             const bool in0 = col0 < a.w_rows, in1 = col1 < a.w_rows;
-            bool released = false;
-#pragma unroll 1
-            for (uint32_t c = 32u * half; c < BN; c += 64u) {
-                const bool mine = c < it.rows_valid;
-                uint32_t r0[32], r1[32];
-                if (mine) {
-                    tmem_ld_32x32(t0 + c, r0);
-                    tmem_ld_32x32(t0 + tile1 + c, r1);
+            const TermLayout t = term_layout(it.rows_valid);
+            const uint32_t span = t.block / 4u, c = span * part;         // this warp's token rows
+            uint32_t pair[32];                                           // bf16 of tile 0 | tile 1 << 16
+#pragma unroll
+            for (uint32_t i = 0; i < 32u; i += 8u) {
+                if (i >= span || c + i >= it.rows_valid) break;
+                uint32_t r0[8], r1[8];
+                tmem_ld_32x8(t0 + c + i, r0);
+                tmem_ld_32x8(t0 + tile1 + c + i, r1);
+                if (t.stacked) {
+                    uint32_t lo[8];
+                    tmem_ld_32x8(t0 + t.block + c + i, lo);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (uint32_t j = 0; j < 8u; j++)
+                        r0[j] = __float_as_uint(__uint_as_float(r0[j]) + __uint_as_float(lo[j]));
+                    tmem_ld_32x8(t0 + tile1 + t.block + c + i, lo);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (uint32_t j = 0; j < 8u; j++)
+                        r1[j] = __float_as_uint(__uint_as_float(r1[j]) + __uint_as_float(lo[j]));
+                } else {
                     tmem_ld_wait();
                 }
-                if (!released && (!mine || c + 64u >= it.rows_valid)) {
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) {
-                        mbar_arrive(&acc_empty[b0]);
-                        if (!small) mbar_arrive(&acc_empty[1]);
-                    }
-                    released = true;
-                }
-                if (!mine) break;
-                const uint32_t n_here = min(32u, it.rows_valid - c);
-                if (kE == kEAct) {
 #pragma unroll
-                    for (uint32_t j = 0; j < 32u; j += 2u) {
-                        if (j >= n_here) break;                          // uniform across the warp
-                        const uint64_t row = (uint64_t)(it.row_start + c + j);
-                        float av[2];
-#pragma unroll
-                        for (uint32_t q = 0; q < 2u; q++) {
-                            const float g = bf16_bits_to_float(float_to_bf16_bits(__uint_as_float(r0[j + q])));
-                            const float u = bf16_bits_to_float(float_to_bf16_bits(__uint_as_float(r1[j + q])));
-                            const uint16_t bits =
-                                float_to_bf16_bits(activation(g, u, a.activation, a.beta, a.linear_beta));
-                            av[q] = in0 ? bf16_bits_to_float(bits) : 0.f;
-                            if (a.out != nullptr && in0 && j + q < n_here)
-                                a.out[(row + q) * a.out_width + col0] = bits;
-                        }
-                        const SplitScale s0 = block_scale(av[0]), s1 = block_scale(av[1]);
-                        const uint32_t packed = split_pair(av[0] * s0.mult, av[1] * s1.mult);
-                        if (in0) {
-                            a.act_hi[row * a.w_rows + col0] = (uint8_t)packed;
-                            a.act_lo[row * a.w_rows + col0] = (uint8_t)(packed >> 16);
-                            if (lane == 0) a.act_sf[row * (a.w_rows / 32u) + col0 / 32u] = (uint8_t)s0.scale_byte;
-                            if (j + 1u < n_here) {
-                                a.act_hi[(row + 1u) * a.w_rows + col0] = (uint8_t)(packed >> 8);
-                                a.act_lo[(row + 1u) * a.w_rows + col0] = (uint8_t)(packed >> 24);
-                                if (lane == 0)
-                                    a.act_sf[(row + 1u) * (a.w_rows / 32u) + col0 / 32u] = (uint8_t)s1.scale_byte;
-                            }
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (uint32_t j = 0; j < 32u; j++) {
-                        if (j >= n_here) break;
-                        const uint64_t row = (uint64_t)(it.row_start + c + j);
-                        if (in0) a.out[row * a.out_width + col0] = float_to_bf16_bits(__uint_as_float(r0[j]));
-                        if (in1) a.out[row * a.out_width + col1] = float_to_bf16_bits(__uint_as_float(r1[j]));
-                    }
-                }
+                for (uint32_t j = 0; j < 8u; j++)
+                    pair[i + j] = pack_bf16x2(__uint_as_float(r0[j]), __uint_as_float(r1[j]));
             }
-            if (!released) {
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&acc_empty[b0]);
-                    if (!small) mbar_arrive(&acc_empty[1]);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&acc_empty[b0]);
+                if (!small) mbar_arrive(&acc_empty[1]);
+            }
+            if (c >= it.rows_valid) continue;
+            const uint32_t n_here = min(span, it.rows_valid - c);
+            if (kE == kEAct) {
+#pragma unroll
+                for (uint32_t j = 0; j < 32u; j += 2u) {
+                    if (j >= n_here) break;                              // uniform across the warp
+                    const uint64_t row = (uint64_t)(it.row_start + c + j);
+                    float av[2];
+#pragma unroll
+                    for (uint32_t q = 0; q < 2u; q++) {
+                        const uint16_t bits = float_to_bf16_bits(
+                            activation(bf16_lo(pair[j + q]), bf16_hi(pair[j + q]), a.activation, a.beta, a.linear_beta));
+                        av[q] = in0 ? bf16_bits_to_float(bits) : 0.f;
+                        if (a.out != nullptr && in0 && j + q < n_here) a.out[(row + q) * a.out_width + col0] = bits;
+                    }
+                    const SplitScale s0 = block_scale(av[0]), s1 = block_scale(av[1]);
+                    const uint32_t packed = split_pair(av[0] * s0.mult, av[1] * s1.mult);
+                    if (in0) {
+                        a.act_hi[row * a.w_rows + col0] = (uint8_t)packed;
+                        a.act_lo[row * a.w_rows + col0] = (uint8_t)(packed >> 16);
+                        if (lane == 0) a.act_sf[row * (a.w_rows / 32u) + col0 / 32u] = (uint8_t)s0.scale_byte;
+                        if (j + 1u < n_here) {
+                            a.act_hi[(row + 1u) * a.w_rows + col0] = (uint8_t)(packed >> 8);
+                            a.act_lo[(row + 1u) * a.w_rows + col0] = (uint8_t)(packed >> 24);
+                            if (lane == 0)
+                                a.act_sf[(row + 1u) * (a.w_rows / 32u) + col0 / 32u] = (uint8_t)s1.scale_byte;
+                        }
+                    }
+                }
+            } else {
+#pragma unroll
+                for (uint32_t j = 0; j < 32u; j++) {
+                    if (j >= n_here) break;
+                    const uint64_t row = (uint64_t)(it.row_start + c + j);
+                    if (in0) a.out[row * a.out_width + col0] = (uint16_t)pair[j];
+                    if (in1) a.out[row * a.out_width + col1] = (uint16_t)(pair[j] >> 16);
                 }
             }
         }
@@ -578,20 +638,30 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         tc_fence_after();
         tmem_dealloc(tmem, kTmemCols);
     }
+    if (a.behind_wait) pdl_wait();
 }
 
-// bf16 rows -> E4M3 terms + block scales.  Four lanes share a block of 32
-// columns (8 each); a warp converts 256 columns per pass.
+// Product rows' E4M3 terms and block scales straight from the bf16 source rows (row r reads
+// x[index[r]], or x[r]).  Four lanes share a block of 32 columns (8 each); a warp converts 256
+// columns per pass.  Rows of groups this path leaves to the other kernel are skipped.  Writing
+// the terms bounds it (14 KB per row at 7168 columns); converting each token once and gathering
+// the terms moved another 14 KB per row and took four launches.
 __global__ void __launch_bounds__(256)
 split_rows_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t *__restrict__ sf,
-                  const uint16_t *__restrict__ x, uint32_t *__restrict__ counters, uint32_t rows, uint32_t k) {
-    pdl_wait();
-    if (blockIdx.x == 0 && threadIdx.x < 64u) counters[threadIdx.x] = 0u;      // of the two product launches
+                  const uint16_t *__restrict__ x, const uint32_t *__restrict__ index,
+                  const uint32_t *__restrict__ offsets, uint32_t groups, uint32_t row_floor, uint32_t rows, uint32_t k) {
+    // launched behind a kernel that waited for the dispatch and shares nothing else with this one
     const uint32_t lane = threadIdx.x % kWarp;
     const uint32_t warps = (gridDim.x * blockDim.x) / kWarp;
     const uint32_t blocks = k / 32u;
     for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp; r < rows; r += warps) {
-        const uint16_t *src = x + (uint64_t)r * k;
+        uint32_t g = 0, end = groups;                      // group of row r
+        while (end - g > 1u) {
+            const uint32_t mid = (g + end) >> 1;
+            if (offsets[mid] <= r) g = mid; else end = mid;
+        }
+        if (offsets[g + 1u] - offsets[g] <= row_floor) continue;
+        const uint16_t *src = x + (uint64_t)(index ? index[r] : r) * k;
         for (uint32_t c = lane * 8u; c < k; c += 256u) {
             const uint4 raw = *reinterpret_cast<const uint4 *>(src + c);
             const uint32_t wv[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -620,20 +690,7 @@ split_rows_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t *_
             if ((lane & 3u) == 0u) sf[(uint64_t)r * blocks + c / 32u] = (uint8_t)(be - 7u);
         }
     }
-}
-
-// rows of 16-byte units gathered through an index: dst[r] = src[index[r]]
-__global__ void __launch_bounds__(256)
-gather_units_kernel(uint4 *__restrict__ dst, const uint4 *__restrict__ src, const uint32_t *__restrict__ index,
-                    uint32_t rows, uint32_t units) {
     pdl_wait();
-    const uint32_t lane = threadIdx.x % kWarp;
-    const uint32_t warps = (gridDim.x * blockDim.x) / kWarp;
-    for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp; r < rows; r += warps) {
-        const uint4 *s = src + (uint64_t)index[r] * units;
-        uint4 *d = dst + (uint64_t)r * units;
-        for (uint32_t u = lane; u < units; u += kWarp) d[u] = s[u];
-    }
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -687,7 +744,7 @@ struct MapKey {
 };
 
 template <int kE>
-bool launch(const Operands &op, const GmxArgs &args, cudaStream_t stream) {
+bool launch(const Operands &op, GmxArgs args, bool few, cudaStream_t stream) {
     constexpr size_t kCachedSets = 256;
     static std::mutex map_lock;
     static std::map<MapKey, GmxMaps> cached;
@@ -722,22 +779,23 @@ bool launch(const Operands &op, const GmxArgs &args, cudaStream_t stream) {
             maps = it->second;
         }
     }
-    if (!set_max_dynamic_smem((const void *)grouped_mx_kernel<kE>, kSmemBytes)) return false;
-    return launch_chained(grouped_mx_kernel<kE>, sm_count(), kThreads, kSmemBytes, stream, maps, args);
+    auto kernel = few ? grouped_mx_kernel<kE, 4> : grouped_mx_kernel<kE, 3>;
+    if (!set_max_dynamic_smem((const void *)kernel, kSmemBytes)) return false;
+    return launch_chained(kernel, sm_count(), kThreads, kSmemBytes, stream, maps, args);
 }
 
 inline size_t up256(size_t v) { return (v + 255u) & ~(size_t)255u; }
 
 struct Scratch {
-    uint8_t *t_hi, *t_lo, *t_sf;       // per source row (only with an index)
     uint8_t *x_hi, *x_lo, *x_sf;       // per product row
     uint8_t *a_hi, *a_lo, *a_sf;       // activation, per product row
-    uint32_t *counters;                // item counters of the two launches (zeroed per call)
+    uint32_t *counters;                // item counters of the six launches (zeroed per call)
+    void *few;                         // scratch of the kernel for few rows per group
     size_t total;
 };
 
 Scratch carve_scratch(const k3_moe_layer_desc *d, uint32_t rows, uint32_t source_rows, void *workspace) {
-    const size_t H = d->hidden, I = d->expert_hidden, R = rows, S = source_rows;
+    const size_t H = d->hidden, I = d->expert_hidden, R = rows;
     uint8_t *p = (uint8_t *)(((uintptr_t)workspace + 255u) & ~(uintptr_t)255u);
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -746,9 +804,6 @@ Scratch carve_scratch(const k3_moe_layer_desc *d, uint32_t rows, uint32_t source
         return q;
     };
     Scratch s{};
-    s.t_hi = take(S * H);
-    s.t_lo = take(S * H);
-    s.t_sf = take(S * (H / 32u));
     s.x_hi = take(R * H);
     s.x_lo = take(R * H);
     s.x_sf = take(R * (H / 32u));
@@ -756,6 +811,7 @@ Scratch carve_scratch(const k3_moe_layer_desc *d, uint32_t rows, uint32_t source
     s.a_lo = take(R * I);
     s.a_sf = take(R * (I / 32u));
     s.counters = (uint32_t *)take(256);
+    s.few = take(k3_grouped_mx4_workspace_bytes(d, rows, source_rows ? source_rows : rows));
     s.total = off + 256u;
     return s;
 }
@@ -788,41 +844,50 @@ bool k3_grouped_mx_supported(const k3_moe_layer_desc *d, uint32_t rows) {
            ((((uintptr_t)d->w1_scales) | ((uintptr_t)d->w3_scales) | ((uintptr_t)d->w2_scales)) & 15u) == 0;
 }
 
+// Which kernel a group goes to, by its rows (device time of both projections of 192 experts at
+// 7168 x 2048; the weights alone are 0.69 ms of HBM time):
+//   rows                   1     8     16    24    32    48    64    96    128
+//   packed                 0.70  0.73  0.81  1.28  1.38  1.94
+//   two-term, four stages  0.97  0.99  1.00  1.01  1.03  1.21  1.28
+//   two-term, three        1.10        1.14  1.15  1.17  1.27  1.37  1.70  1.95
+constexpr uint32_t kFewRows = k3_mx4_rows, kSomeRows = 64;
+
 // rows_in bf16 [source_rows, H]; product row r reads rows_in[index[r]] (or row r
 // when index == nullptr, source_rows == 0).  `act` bf16 [rows, I] is written when
 // not null; rows_out bf16 [rows, H].
 bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act, const void *rows_in,
                            const void *index, uint32_t source_rows, const void *offsets, uint32_t rows,
-                           void *workspace, cudaStream_t stream) {
+                           void *workspace, cudaStream_t stream, uint32_t max_group_rows) {
     const uint32_t H = d->hidden, I = d->expert_hidden;
     const Scratch s = carve_scratch(d, rows, index ? source_rows : 0u, workspace);
     const uint32_t conv_rows = index ? source_rows : rows;
-    const uint32_t cap = (uint32_t)sm_count() * 16u;
-    if (!launch_chained(split_rows_kernel, std::min<uint32_t>((conv_rows + 7u) / 8u, cap), 256, 0, stream,
-                        index ? s.t_hi : s.x_hi, index ? s.t_lo : s.x_lo, index ? s.t_sf : s.x_sf,
-                        (const uint16_t *)rows_in, s.counters, conv_rows, H)) {
+    const bool few = max_group_rows > kFewRows, many = max_group_rows > kSomeRows;   // launches beyond the packed one
+    if (!k3_grouped_mx4_terms(d, rows_in, conv_rows, rows, s.few, s.counters, stream)) return false;
+    if (few && !launch_chained(split_rows_kernel, std::min<uint32_t>((rows + 7u) / 8u, (uint32_t)sm_count() * 16u), 256, 0,
+                               stream, s.x_hi, s.x_lo, s.x_sf, (const uint16_t *)rows_in, (const uint32_t *)index,
+                               (const uint32_t *)offsets, d->local_expert_count, kFewRows, rows, H)) {
         return false;
-    }
-    if (index) {
-        const uint32_t blocks = std::min<uint32_t>((rows + 7u) / 8u, cap);
-        const uint32_t *map = (const uint32_t *)index;
-        if (!launch_chained(gather_units_kernel, blocks, 256, 0, stream, (uint4 *)s.x_hi, (const uint4 *)s.t_hi, map,
-                            rows, H / 16u) ||
-            !launch_chained(gather_units_kernel, blocks, 256, 0, stream, (uint4 *)s.x_lo, (const uint4 *)s.t_lo, map,
-                            rows, H / 16u) ||
-            !launch_chained(gather_units_kernel, blocks, 256, 0, stream, (uint4 *)s.x_sf, (const uint4 *)s.t_sf, map,
-                            rows, H / 512u)) {
-            return false;
-        }
     }
     GmxArgs a{};
     a.offsets = (const uint32_t *)offsets;
-    a.item_counter = s.counters;
     a.groups = d->local_expert_count;
     a.rows = rows;
     a.activation = d->activation;
     a.beta = d->beta;
     a.linear_beta = d->linear_beta;
+    a.behind_wait = true;
+    auto launches = [&](auto mode, const Operands &op, uint32_t *counters) {
+        constexpr int kE = decltype(mode)::value;
+        GmxArgs b = a;
+        b.row_floor = kFewRows;
+        b.row_ceil = kSomeRows;
+        b.item_counter = counters;
+        if (few && !launch<kE>(op, b, true, stream)) return false;
+        b.row_floor = kSomeRows;
+        b.row_ceil = 0xffffffffu;
+        b.item_counter = counters + 8;
+        return !many || launch<kE>(op, b, false, stream);
+    };
     // gate/up + activation
     a.out = (uint16_t *)act;
     a.act_hi = s.a_hi;
@@ -833,9 +898,11 @@ bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act
     a.out_width = I;
     a.m_items = (I + BM - 1u) / BM;
     const Operands gu{d->w1_packed, d->w3_packed, d->w1_scales, d->w3_scales, s.x_hi, s.x_lo, s.x_sf};
-    if (!launch<kEAct>(gu, a, stream)) return false;
+    if (!k3_grouped_mx4_gateup(d, act, index, conv_rows, offsets, rows, s.few, s.counters, stream) ||
+        !launches(std::integral_constant<int, kEAct>{}, gu, s.counters + 8)) {
+        return false;
+    }
     // down
-    a.item_counter = s.counters + 32;
     a.out = (uint16_t *)rows_out;
     a.act_hi = a.act_lo = a.act_sf = nullptr;
     a.w_rows = H;
@@ -843,5 +910,6 @@ bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act
     a.out_width = H;
     a.m_items = (H + 2u * BM - 1u) / (2u * BM);
     const Operands dn{d->w2_packed, d->w2_packed, d->w2_scales, d->w2_scales, s.a_hi, s.a_lo, s.a_sf};
-    return launch<kEBf16>(dn, a, stream);
+    return k3_grouped_mx4_down(d, rows_out, offsets, rows, conv_rows, s.few, s.counters + 24, stream) &&
+           launches(std::integral_constant<int, kEBf16>{}, dn, s.counters + 32);
 }

@@ -601,7 +601,7 @@ extern "C" uint32_t k3_moe_device_status(void) {
     uint32_t v = 0xffffffffu;
     if (cudaMemcpyFromSymbol(&v, g_tc_status, sizeof(v)) != cudaSuccess) (void)cudaGetLastError();
     return v | k3_decode_mx_status() | k3_decode_status() | k3_decode_shared_status() | k3_grouped_mx_status() |
-           k3_dispatch_status();
+           k3_grouped_mx4_status() | k3_dispatch_status();
 }
 
 bool k3_status_words_clear() {
@@ -613,6 +613,7 @@ bool k3_status_words_clear() {
     ok = k3_decode_shared_status_clear() && ok;
     ok = k3_dispatch_status_clear() && ok;
     ok = k3_grouped_mx_status_clear() && ok;
+    ok = k3_grouped_mx4_status_clear() && ok;
     return ok;
 }
 

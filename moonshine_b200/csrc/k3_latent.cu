@@ -155,7 +155,7 @@ extern "C" bool k3_moe_latent_layer_forward(const k3_moe_latent_desc *d, void *o
         // rows_out already holds the expert rows
     } else if (w.mx_bytes != 0) {
         if (!k3_grouped_mx_experts(&e, w.rows_out, nullptr, w.latent, w.sorted_token, tokens, w.offsets, routes,
-                                   w.mx_ws, stream)) {
+                                   w.mx_ws, stream, tokens)) {
             return false;
         }
     } else {

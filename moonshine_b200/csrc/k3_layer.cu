@@ -498,7 +498,7 @@ bool layer_forward_impl(const k3_moe_layer_desc *d, void *out, const void *x, ui
                 // block-scaled path: tokens are converted once, then gathered as bytes
                 if (!mark(events, 3, stream)) return false;
                 if (!k3_grouped_mx_experts(d, w.rows_out, nullptr, x, w.sorted_token, tokens, w.offsets,
-                                           routes, w.mx_ws, stream)) {
+                                           routes, w.mx_ws, stream, tokens)) {
                     return false;
                 }
             } else {
