@@ -50,6 +50,98 @@ route_hist_kernel(uint32_t *__restrict__ hist, const uint32_t *__restrict__ ids,
     }
 }
 
+// Few routes (a decode batch, a short prompt): the three passes in one block.  Warp w owns the
+// routes [w * per, (w + 1) * per); counts per warp and expert live in shared memory.  Three
+// launches of one or two blocks took 17 us for 80 routes and 27 us for 384: a chunk's 16 steps
+// are a serial chain, and so are the launches.
+constexpr uint32_t kSmallRoutes = 4096;
+constexpr uint32_t kSmallWarps = 32;
+
+__global__ void __launch_bounds__(kSmallWarps * 32)
+route_small_kernel(uint32_t *__restrict__ offsets, uint32_t *__restrict__ sorted_route,
+                   uint32_t *__restrict__ sorted_token, uint32_t *__restrict__ inv_perm,
+                   const uint32_t *__restrict__ ids, uint32_t routes, uint32_t experts, uint32_t top_k) {
+    extern __shared__ uint16_t small_counts[];             // [kSmallWarps][experts], then cursors
+    __shared__ uint32_t warp_sums[kSmallWarps];
+    const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    uint32_t *words = reinterpret_cast<uint32_t *>(small_counts);
+    for (uint32_t i = threadIdx.x; i < (kSmallWarps * experts + 1u) / 2u; i += blockDim.x) words[i] = 0u;
+    pdl_wait();
+    const uint32_t per = (routes + kSmallWarps - 1u) / kSmallWarps;
+    const uint32_t begin = min(routes, warp * per), end = min(routes, begin + per);
+    uint16_t *mine = small_counts + warp * experts;
+    __syncthreads();
+    // all steps' ids in flight at once (at most 128 routes per warp)
+    uint32_t id[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; j++) {
+        const uint32_t r = begin + j * kWarp + lane;
+        id[j] = r < end ? ids[r] : 0xffffffffu;
+        if (r < end && id[j] >= experts) g_dispatch_status = 2u;       // invalid route id
+    }
+    uint32_t rank[4];                                      // among this warp's routes to the same expert
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; j++) {
+        const bool usable = id[j] < experts;
+        const uint32_t active = __ballot_sync(0xffffffffu, usable);
+        rank[j] = 0u;
+        if (usable) {
+            const uint32_t peers = __match_any_sync(active, id[j]);
+            const uint32_t before = __popc(peers & ((1u << lane) - 1u)), base = mine[id[j]];
+            __syncwarp(active);
+            if (before == 0u) mine[id[j]] = (uint16_t)(base + __popc(peers));
+            rank[j] = base + before;
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    uint32_t running = 0u;                                 // expert threadIdx.x: exclusive scan over the warps
+    if (threadIdx.x < experts) {
+#pragma unroll 8
+        for (uint32_t w = 0; w < kSmallWarps; w++) {
+            const uint32_t v = small_counts[w * experts + threadIdx.x];
+            small_counts[w * experts + threadIdx.x] = (uint16_t)running;
+            running += v;
+        }
+    }
+    uint32_t incl = running;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += n;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t w = warp_sums[lane], wi = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t n = __shfl_up_sync(0xffffffffu, wi, o);
+            if (lane >= (uint32_t)o) wi += n;
+        }
+        warp_sums[lane] = wi - w;
+    }
+    __syncthreads();
+    const uint32_t excl = warp_sums[warp] + incl - running;
+    if (threadIdx.x < experts) {
+        offsets[threadIdx.x] = excl;
+        if (threadIdx.x == experts - 1u) offsets[experts] = excl + running;
+#pragma unroll 8
+        for (uint32_t w = 0; w < kSmallWarps; w++) small_counts[w * experts + threadIdx.x] += (uint16_t)excl;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; j++) {
+        const uint32_t r = begin + j * kWarp + lane;
+        if (id[j] < experts) {
+            const uint32_t pos = mine[id[j]] + rank[j];
+            sorted_route[pos] = r;
+            sorted_token[pos] = r / top_k;
+            inv_perm[r] = pos;
+        }
+    }
+}
+
 // One block, one thread per expert.
 __global__ void __launch_bounds__(kMaxExperts)
 route_scan_kernel(uint32_t *__restrict__ hist, uint32_t *__restrict__ offsets,
@@ -59,11 +151,15 @@ route_scan_kernel(uint32_t *__restrict__ hist, uint32_t *__restrict__ offsets,
     const uint32_t e = threadIdx.x;
     uint32_t running = 0u;
     if (e < experts) {
-        for (uint32_t c = 0; c < chunks; c++) {
-            const uint64_t i = (uint64_t)c * experts + e;
-            const uint32_t v = hist[i];
-            hist[i] = running;
-            running += v;
+        for (uint32_t c0 = 0; c0 < chunks; c0 += 16u) {    // sixteen loads in flight
+            uint32_t v[16];
+#pragma unroll
+            for (uint32_t j = 0; j < 16u; j++) v[j] = c0 + j < chunks ? hist[(uint64_t)(c0 + j) * experts + e] : 0u;
+#pragma unroll
+            for (uint32_t j = 0; j < 16u; j++) {
+                if (c0 + j < chunks) hist[(uint64_t)(c0 + j) * experts + e] = running;
+                running += v[j];
+            }
         }
     }
     // exclusive scan over experts
@@ -132,6 +228,13 @@ route_place_kernel(uint32_t *__restrict__ sorted_route, uint32_t *__restrict__ s
 
 bool launch_dispatch(uint32_t *hist, void *offsets, void *sorted_route, void *sorted_token, void *inv_perm,
                      const void *expert_ids, uint32_t routes, uint32_t experts, uint32_t top_k, cudaStream_t stream) {
+    if (routes <= kSmallRoutes) {
+        const size_t counts = (size_t)kSmallWarps * experts * sizeof(uint16_t) + 4u;
+        return set_max_dynamic_smem((const void *)route_small_kernel, counts) &&
+               launch_chained(route_small_kernel, 1, kSmallWarps * 32, counts, stream, (uint32_t *)offsets,
+                              (uint32_t *)sorted_route, (uint32_t *)sorted_token, (uint32_t *)inv_perm,
+                              (const uint32_t *)expert_ids, routes, experts, top_k);
+    }
     const uint32_t chunks = (routes + kChunk - 1) / kChunk;
     const uint32_t blocks = (chunks + kWarpsPerBlock - 1) / kWarpsPerBlock;
     const size_t smem = (size_t)kWarpsPerBlock * experts * sizeof(uint32_t);

@@ -113,15 +113,19 @@ bool k3_status_words_clear();   // all of the above and the dense kernels' word 
 
 // Block-scaled tensor-core grouped expert products for many rows
 // (k3_grouped_mx.cu).  `index` (u32 per row, or null) gathers rows_in, which then
-// has source_rows rows; `act` may be null.  max_group_rows: a bound on the rows of one group
-// that the caller knows (tokens, where a token selects an expert at most once).
+// has source_rows rows; `act` may be null.  routes: what a caller whose source rows are tokens
+// with top_k routes each knows besides the index.
+struct k3_token_routes {
+    const void *ids;           // u32 [tokens, top_k] expert ids, all of this table
+    const void *inv_perm;      // u32 [tokens, top_k] product row of a route
+};
 bool k3_grouped_mx_supported(const k3_moe_layer_desc *desc, uint32_t rows);
 size_t k3_grouped_mx_workspace_bytes(const k3_moe_layer_desc *desc, uint32_t rows,
                                      uint32_t source_rows);
 bool k3_grouped_mx_experts(const k3_moe_layer_desc *desc, void *rows_out, void *act,
                            const void *rows_in, const void *index, uint32_t source_rows,
                            const void *offsets, uint32_t rows, void *workspace,
-                           cudaStream_t stream, uint32_t max_group_rows = 0xffffffffu);
+                           cudaStream_t stream, const k3_token_routes *routes = nullptr);
 uint32_t k3_grouped_mx_status();
 constexpr uint32_t k3_mx4_rows = 16;
 // The same for groups of at most k3_mx4_rows rows (k3_grouped_mx4.cu) in three steps; larger groups
@@ -129,7 +133,7 @@ constexpr uint32_t k3_mx4_rows = 16;
 // product launch takes one.
 size_t k3_grouped_mx4_workspace_bytes(const k3_moe_layer_desc *desc, uint32_t rows, uint32_t source_rows);
 bool k3_grouped_mx4_terms(const k3_moe_layer_desc *desc, const void *rows_in, uint32_t source_rows, uint32_t rows,
-                          void *workspace, uint32_t *counters, cudaStream_t stream);
+                          const void *ids, const void *offsets, void *workspace, uint32_t *counters, cudaStream_t stream);
 bool k3_grouped_mx4_gateup(const k3_moe_layer_desc *desc, void *act, const void *index, uint32_t source_rows,
                            const void *offsets, uint32_t rows, void *workspace, uint32_t *counter,
                            cudaStream_t stream);

@@ -20,8 +20,8 @@
 // shared memory, so a CTA that drew short row tiles simply takes more of them.  Items
 // are numbered with the row tiles of one (expert, weight tile) adjacent: CTAs that take
 // neighbouring items stream the same weights at the same time and the second reader
-// finds them in L2.  Warps: 0 TMA producer (weights), 2 TMA producer (token terms),
-// 3 TMA producer (block scales), 1 and 24 MMA issuers (one per weight tile), 4-7
+// finds them in L2.  Warps: 0 TMA producer (weights, all block scales), 2 TMA producer
+// (token terms), 1 and 3 MMA issuers (one per weight tile), 4-7
 // scale writers (shared memory -> tensor memory, one lane quadrant each), 8-23
 // epilogue.  All barrier waits are bounded.
 #include "k3_grouped.h"
@@ -51,8 +51,7 @@ constexpr uint32_t kBBox = 32u;                           // token rows per TMA 
 constexpr uint32_t kRingBytes = 192u * 1024u;             // stages of A0 | A1 | token terms: three of 64 KB, or four of
                                                           //   48 KB where no tile has more than 64 rows
 constexpr uint32_t kEpilogueWarps = 16;
-constexpr uint32_t kIssuer1 = 8u + kEpilogueWarps;        // warp of the second MMA issuer
-constexpr uint32_t kThreads = (kIssuer1 + 1u) * 32u;      // 25 warps
+constexpr uint32_t kThreads = (8u + kEpilogueWarps) * 32u;   // 24 warps
 constexpr uint32_t kSfBatches = 3;                        // scale ring in tensor memory: batches of 4 stages
 constexpr uint32_t kSfSlots = 4;                          // scale ring in shared memory
 constexpr uint32_t kSfKind = BM * 16u;                    // one table's 128 rows x 16 scale bytes
@@ -64,7 +63,7 @@ constexpr uint32_t kSfa1Col = kSfa0Col + 16u * kSfBatches;
 constexpr uint32_t kSfbCol = kSfa1Col + 16u * kSfBatches;
 constexpr uint32_t kMaxGroups = 1024;
 constexpr uint32_t kItemSlots = 4;                        // mailbox of item numbers, producer -> other roles
-constexpr uint32_t kItemReaders = 8u + kEpilogueWarps;    // term + scale producers, 2 issuers, 4 writers, epilogue warps
+constexpr uint32_t kItemReaders = 7u + kEpilogueWarps;    // term producer, 2 issuers, 4 writers, epilogue warps
 constexpr uint32_t kNoItem = 0xffffffffu;
 constexpr uint32_t kBarBytes = 512;
 constexpr uint32_t kSmemBytes =
@@ -338,11 +337,14 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
     };
 
     if (warp == 0) {
-        // ================================ TMA producer: weights; draws the items
+        // ================================ TMA producer: weights and block scales; draws the items
         if (lane == 0) {
             prefetch_tensormap(&maps.a0);
             prefetch_tensormap(&maps.a1);
-            uint32_t s = 0, ph = 0, seq = 0;
+            prefetch_tensormap(&maps.sfa0);
+            prefetch_tensormap(&maps.sfa1);
+            prefetch_tensormap(&maps.sfb);
+            uint32_t s = 0, ph = 0, ss = 0, ssph = 0, seq = 0;
             bool ok = true;
             uint32_t w = atomicAdd(a.item_counter, 1u);
             while (ok) {
@@ -358,6 +360,15 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                 const int32_t y0 = (int32_t)(it.group * a.w_rows + it.m_item * tile_rows);
                 const int32_t y1 = kE == kEAct ? y0 : y0 + (int32_t)BM;
                 for (uint32_t st = 0; st < steps; st++) {
+                    if ((st & 3u) == 0u) {                 // scales, four stages at a time
+                        if (!mbar_wait(&sfs_empty[ss], ssph ^ 1u, abort_flag)) { ok = false; break; }
+                        unsigned char *sf = sf_smem + ss * kSfSlotBytes;
+                        mbar_arrive_expect_tx(&sfs_full[ss], kSfSlotBytes);
+                        tma_load_2d(sf, &maps.sfa0, &sfs_full[ss], (int32_t)(st * 4u), y0);
+                        tma_load_2d(sf + kSfKind, &maps.sfa1, &sfs_full[ss], (int32_t)(st * 4u), y1);
+                        tma_load_2d(sf + 2u * kSfKind, &maps.sfb, &sfs_full[ss], (int32_t)(st * 4u), (int32_t)it.row_start);
+                        if (++ss == kSfSlots) { ss = 0; ssph ^= 1u; }
+                    }
                     if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag)) { ok = false; break; }
                     unsigned char *dst = base + s * kStageBytes;
                     const int32_t x = (int32_t)(st * KS);
@@ -394,34 +405,10 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                 }
             }
         }
-    } else if (warp == 3) {
-        // ====================== TMA producer: block scales, 4 stages at a time
-        if (lane == 0) {
-            prefetch_tensormap(&maps.sfa0);
-            prefetch_tensormap(&maps.sfa1);
-            prefetch_tensormap(&maps.sfb);
-            uint32_t s = 0, ph = 0;
-            bool ok = true;
-            for (uint32_t w = next_item(); ok && w != kNoItem; w = next_item()) {
-                const Item it = decode_item(w, prefix, a);
-                const int32_t y0 = (int32_t)(it.group * a.w_rows + it.m_item * tile_rows);
-                const int32_t y1 = kE == kEAct ? y0 : y0 + (int32_t)BM;
-                for (uint32_t st = 0; st < steps; st += 4u) {
-                    if (!mbar_wait(&sfs_empty[s], ph ^ 1u, abort_flag)) { ok = false; break; }
-                    unsigned char *dst = sf_smem + s * kSfSlotBytes;
-                    mbar_arrive_expect_tx(&sfs_full[s], kSfSlotBytes);
-                    tma_load_2d(dst, &maps.sfa0, &sfs_full[s], (int32_t)(st * 4u), y0);
-                    tma_load_2d(dst + kSfKind, &maps.sfa1, &sfs_full[s], (int32_t)(st * 4u), y1);
-                    tma_load_2d(dst + 2u * kSfKind, &maps.sfb, &sfs_full[s], (int32_t)(st * 4u),
-                                (int32_t)it.row_start);
-                    if (++s == kSfSlots) { s = 0; ph ^= 1u; }
-                }
-            }
-        }
-    } else if (warp == 1 || warp == kIssuer1) {
+    } else if (warp == 1 || warp == 3) {
         // ==================================================== MMA issuers
         // One thread's issue loop cannot keep the tensor pipe fed with K = 32 MMAs, so
-        // warp 1 issues the MMAs of weight tile 0 and warp kIssuer1 those of tile 1.  Both
+        // warp 1 issues the MMAs of weight tile 0 and warp 3 those of tile 1.  Both
         // commit to the same stage / scale / accumulator barriers (count 2).
         if (lane == 0) {
             const uint32_t q = warp == 1 ? 0u : 1u;
@@ -641,53 +628,84 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
     if (a.behind_wait) pdl_wait();
 }
 
-// Product rows' E4M3 terms and block scales straight from the bf16 source rows (row r reads
-// x[index[r]], or x[r]).  Four lanes share a block of 32 columns (8 each); a warp converts 256
-// columns per pass.  Rows of groups this path leaves to the other kernel are skipped.  Writing
-// the terms bounds it (14 KB per row at 7168 columns); converting each token once and gathering
-// the terms moved another 14 KB per row and took four launches.
+// 16 bf16 columns of one lane (two lanes share a block of 32) -> E4M3 terms and the block's scale.
+struct SplitColumns {
+    uint4 hi, lo;
+    uint32_t scale_byte;
+};
+K3_DEVINL SplitColumns split_columns(const uint16_t *p) {
+    const uint4 q0 = reinterpret_cast<const uint4 *>(p)[0], q1 = reinterpret_cast<const uint4 *>(p)[1];
+    const uint32_t wv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+    uint32_t mx = 0;
+#pragma unroll
+    for (int q = 0; q < 8; q++) mx = max(mx, max(wv[q] & 0x7fffu, (wv[q] >> 16) & 0x7fffu));   // bf16 magnitudes
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    const uint32_t be = min(max(mx >> 7, 8u), 254u);
+    const float mult = __uint_as_float((261u - be) << 23);
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint32_t p0 = split_pair(bf16_lo(wv[2 * q]) * mult, bf16_hi(wv[2 * q]) * mult);
+        const uint32_t p1 = split_pair(bf16_lo(wv[2 * q + 1]) * mult, bf16_hi(wv[2 * q + 1]) * mult);
+        h[q] = (p0 & 0xffffu) | (p1 << 16);
+        l[q] = (p0 >> 16) | (p1 & 0xffff0000u);
+    }
+    return {make_uint4(h[0], h[1], h[2], h[3]), make_uint4(l[0], l[1], l[2], l[3]), be - 7u};
+}
+
+// Product rows' E4M3 terms and block scales from the bf16 source rows (row r reads x[index[r]],
+// or x[r]); a warp converts 512 columns per pass.  Rows of groups this path leaves to the other
+// kernel are skipped.
 __global__ void __launch_bounds__(256)
 split_rows_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t *__restrict__ sf,
                   const uint16_t *__restrict__ x, const uint32_t *__restrict__ index,
-                  const uint32_t *__restrict__ offsets, uint32_t groups, uint32_t row_floor, uint32_t rows, uint32_t k) {
+                  const uint32_t *__restrict__ offsets, uint32_t groups, uint32_t rows, uint32_t k) {
     // launched behind a kernel that waited for the dispatch and shares nothing else with this one
     const uint32_t lane = threadIdx.x % kWarp;
     const uint32_t warps = (gridDim.x * blockDim.x) / kWarp;
-    const uint32_t blocks = k / 32u;
     for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp; r < rows; r += warps) {
         uint32_t g = 0, end = groups;                      // group of row r
         while (end - g > 1u) {
             const uint32_t mid = (g + end) >> 1;
             if (offsets[mid] <= r) g = mid; else end = mid;
         }
-        if (offsets[g + 1u] - offsets[g] <= row_floor) continue;
+        if (offsets[g + 1u] - offsets[g] <= k3_mx4_rows) continue;
         const uint16_t *src = x + (uint64_t)(index ? index[r] : r) * k;
-        for (uint32_t c = lane * 8u; c < k; c += 256u) {
-            const uint4 raw = *reinterpret_cast<const uint4 *>(src + c);
-            const uint32_t wv[4] = {raw.x, raw.y, raw.z, raw.w};
-            float v[8];
-            uint32_t mx = 0;
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                v[2 * q] = bf16_lo(wv[q]);
-                v[2 * q + 1] = bf16_hi(wv[q]);
-                mx = max(mx, max(__float_as_uint(fabsf(v[2 * q])), __float_as_uint(fabsf(v[2 * q + 1]))));
-            }
-            mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-            mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-            uint32_t be = min(max((mx >> 23) & 0xffu, 8u), 254u);
-            const float mult = __uint_as_float((261u - be) << 23);
-            uint32_t h[2], l[2];
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const uint32_t p0 = split_pair(v[4 * q] * mult, v[4 * q + 1] * mult);
-                const uint32_t p1 = split_pair(v[4 * q + 2] * mult, v[4 * q + 3] * mult);
-                h[q] = (p0 & 0xffffu) | (p1 << 16);
-                l[q] = (p0 >> 16) | (p1 & 0xffff0000u);
-            }
-            *reinterpret_cast<uint2 *>(hi + (uint64_t)r * k + c) = make_uint2(h[0], h[1]);
-            *reinterpret_cast<uint2 *>(lo + (uint64_t)r * k + c) = make_uint2(l[0], l[1]);
-            if ((lane & 3u) == 0u) sf[(uint64_t)r * blocks + c / 32u] = (uint8_t)(be - 7u);
+        for (uint32_t c = lane * 16u; c < k; c += 512u) {
+            const SplitColumns t = split_columns(src + c);
+            *reinterpret_cast<uint4 *>(hi + (uint64_t)r * k + c) = t.hi;
+            *reinterpret_cast<uint4 *>(lo + (uint64_t)r * k + c) = t.lo;
+            if ((lane & 1u) == 0u) sf[(uint64_t)r * (k / 32u) + c / 32u] = (uint8_t)t.scale_byte;
+        }
+    }
+    pdl_wait();
+}
+
+// The same for tokens whose routes are known: a warp converts 512 columns of a token once and
+// stores them to each of its product rows.  Bound by those stores (14 KB per row at 7168
+// columns): 8192 tokens took 649 us when every product row was converted on its own.
+__global__ void __launch_bounds__(256)
+split_tokens_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t *__restrict__ sf,
+                    const uint16_t *__restrict__ x, const uint32_t *__restrict__ ids,
+                    const uint32_t *__restrict__ inv_perm, const uint32_t *__restrict__ offsets, uint32_t top_k,
+                    uint32_t tokens, uint32_t k) {
+    const uint32_t lane = threadIdx.x % kWarp, passes = k / 512u;
+    const uint64_t warps = (uint64_t)(gridDim.x * blockDim.x) / kWarp, jobs = (uint64_t)tokens * passes;
+    for (uint64_t job = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp; job < jobs; job += warps) {
+        const uint32_t token = (uint32_t)(job / passes), c = (uint32_t)(job % passes) * 512u + lane * 16u;
+        uint32_t row = 0u;
+        bool mine = false;
+        if (lane < top_k) {
+            const uint32_t e = ids[(uint64_t)token * top_k + lane];
+            row = inv_perm[(uint64_t)token * top_k + lane];
+            mine = offsets[e + 1u] - offsets[e] > k3_mx4_rows;
+        }
+        const SplitColumns t = split_columns(x + (uint64_t)token * k + c);
+        for (uint32_t todo = __ballot_sync(0xffffffffu, mine); todo != 0u; todo &= todo - 1u) {
+            const uint64_t r = __shfl_sync(0xffffffffu, row, __ffs((int)todo) - 1);
+            *reinterpret_cast<uint4 *>(hi + r * k + c) = t.hi;
+            *reinterpret_cast<uint4 *>(lo + r * k + c) = t.lo;
+            if ((lane & 1u) == 0u) sf[r * (k / 32u) + c / 32u] = (uint8_t)t.scale_byte;
         }
     }
     pdl_wait();
@@ -857,15 +875,29 @@ constexpr uint32_t kFewRows = k3_mx4_rows, kSomeRows = 64;
 // not null; rows_out bf16 [rows, H].
 bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act, const void *rows_in,
                            const void *index, uint32_t source_rows, const void *offsets, uint32_t rows,
-                           void *workspace, cudaStream_t stream, uint32_t max_group_rows) {
+                           void *workspace, cudaStream_t stream, const k3_token_routes *routes) {
+    // a token selects an expert at most once, so no group has more rows than there are tokens
+    const uint32_t max_group_rows = routes ? source_rows : 0xffffffffu;
     const uint32_t H = d->hidden, I = d->expert_hidden;
     const Scratch s = carve_scratch(d, rows, index ? source_rows : 0u, workspace);
     const uint32_t conv_rows = index ? source_rows : rows;
     const bool few = max_group_rows > kFewRows, many = max_group_rows > kSomeRows;   // launches beyond the packed one
-    if (!k3_grouped_mx4_terms(d, rows_in, conv_rows, rows, s.few, s.counters, stream)) return false;
-    if (few && !launch_chained(split_rows_kernel, std::min<uint32_t>((rows + 7u) / 8u, (uint32_t)sm_count() * 16u), 256, 0,
-                               stream, s.x_hi, s.x_lo, s.x_sf, (const uint16_t *)rows_in, (const uint32_t *)index,
-                               (const uint32_t *)offsets, d->local_expert_count, kFewRows, rows, H)) {
+    if (!k3_grouped_mx4_terms(d, rows_in, conv_rows, rows, routes ? routes->ids : nullptr, offsets, s.few, s.counters,
+                              stream)) {
+        return false;
+    }
+    if (few && routes) {
+        const uint64_t jobs = (uint64_t)source_rows * (H / 512u);
+        if (!launch_chained(split_tokens_kernel, (uint32_t)std::min<uint64_t>((jobs + 7u) / 8u, (uint64_t)sm_count() * 16u),
+                            256, 0, stream, s.x_hi, s.x_lo, s.x_sf, (const uint16_t *)rows_in,
+                            (const uint32_t *)routes->ids, (const uint32_t *)routes->inv_perm, (const uint32_t *)offsets,
+                            d->top_k, source_rows, H)) {
+            return false;
+        }
+    } else if (few && !launch_chained(split_rows_kernel, std::min<uint32_t>((rows + 7u) / 8u, (uint32_t)sm_count() * 16u),
+                                      256, 0, stream, s.x_hi, s.x_lo, s.x_sf, (const uint16_t *)rows_in,
+                                      (const uint32_t *)index, (const uint32_t *)offsets, d->local_expert_count, rows,
+                                      H)) {
         return false;
     }
     GmxArgs a{};

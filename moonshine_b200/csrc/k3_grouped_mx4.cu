@@ -17,10 +17,10 @@
 // items from a global counter.  Groups of more than 16 rows are left to the other kernel: the
 // terms of a row are 4 bytes per column and cross from L2 once per weight tile, so from two row
 // tiles on L2 bounds this form (24 rows per expert 1.28 ms, two-term form 1.01).  Warps: 0
-// weight producer, 2 term producer (one box of 8 term rows x 2 stages per token row, straight
-// from the token's terms: no gather pass), 3 weight-scale producer, 1 and 16 MMA issuers (one
-// per weight tile), 4-7 scale writers (weight scales from shared memory, term scales from global
-// memory -> tensor memory), 8-15 epilogue.  192 experts at 7168 x 2048 (4.5 GB) with 1, 8, 16
+// producer of weights and their scales, 2 term producer (one box of 8 term rows x 2 stages per
+// token row, straight from the token's terms: no gather pass), 1 and 3 MMA issuers (one per
+// weight tile), 4-7 scale writers (weight scales from shared memory, term scales from global
+// memory -> tensor memory), 8-23 epilogue.  192 experts at 7168 x 2048 (4.5 GB) with 1, 8, 16
 // rows each: 0.70, 0.73, 0.81 ms = 6.5, 6.2, 5.6 TB/s (the two-term kernel took 1.10, 1.11,
 // 1.14).  All barrier waits are bounded.
 #include "k3_e2m1_terms.cuh"
@@ -47,7 +47,8 @@ constexpr uint32_t kBAtom = kTerms * 128u;                 // one token row: 8 t
 constexpr uint32_t kStageBytes = 2u * kATile;              // weights; the terms have a ring of their own:
 constexpr uint32_t kBSlots = 2;                            // slots of two stages (512 K) of up to 16 token rows
 constexpr uint32_t kBSlotBytes = 2u * kTileRows * kBAtom;
-constexpr uint32_t kThreads = 544;                         // 17 warps
+constexpr uint32_t kEpilogueWarps = 16;
+constexpr uint32_t kThreads = (8u + kEpilogueWarps) * 32u; // 24 warps
 constexpr uint32_t kSfBatches = 4;                         // scale ring in tensor memory: batches of 2 stages
 constexpr uint32_t kSfSlots = 4;                           // scale ring in shared memory
 constexpr uint32_t kSfKind = BM * 16u;                     // 128 rows x 16 scale bytes (512 K)
@@ -58,7 +59,7 @@ constexpr uint32_t kSfa1Col = kSfa0Col + 16u * kSfBatches;
 constexpr uint32_t kSfbCol = kSfa1Col + 16u * kSfBatches;
 constexpr uint32_t kMaxGroups = 1024;
 constexpr uint32_t kItemSlots = 4;                         // mailbox of item numbers, producer -> other roles
-constexpr uint32_t kItemReaders = 16;
+constexpr uint32_t kItemReaders = 7u + kEpilogueWarps;     // term producer, 2 issuers, 4 writers, epilogue warps
 constexpr uint32_t kNoItem = 0xffffffffu;
 constexpr uint32_t kBarBytes = 512;
 constexpr uint32_t kSmemBytes =
@@ -73,6 +74,15 @@ K3_DEVINL void tmem_st_32x16(uint32_t taddr, const uint32_t (&v)[16]) {
         "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
         "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
         "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+}
+K3_DEVINL void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
         : "memory");
 }
 K3_DEVINL void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -211,7 +221,7 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
         }
         for (uint32_t b = 0; b < 2u; b++) {
             mbar_init(&acc_full[b], 2);
-            mbar_init(&acc_empty[b], 8);
+            mbar_init(&acc_empty[b], kEpilogueWarps);
         }
         for (uint32_t b = 0; b < kItemSlots; b++) {
             mbar_init(&item_full[b], 1);
@@ -279,12 +289,14 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
     };
 
     if (warp == 0) {
-        // ================================ TMA producer: weights; draws the items
+        // ================================ TMA producer: weights and their scales; draws the items
         if (lane == 0) {
             prefetch_tensormap(&maps.a0);
             prefetch_tensormap(&maps.a1);
+            prefetch_tensormap(&maps.sfa0);
+            prefetch_tensormap(&maps.sfa1);
             const uint64_t stream_once = l2_policy_evict_first();
-            uint32_t s = 0, ph = 0, seq = 0;
+            uint32_t s = 0, ph = 0, ss = 0, ssph = 0, seq = 0;
             bool ok = true;
             uint32_t w = atomicAdd(a.item_counter, 1u);
             while (ok) {
@@ -300,6 +312,14 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
                 const int32_t y0 = (int32_t)(it.group * a.w_rows + it.m_item * tile_rows);
                 const int32_t y1 = kAct ? y0 : y0 + (int32_t)BM;
                 for (uint32_t st = 0; st < steps; st++) {
+                    if ((st & 1u) == 0u) {                 // scales, two stages at a time
+                        if (!mbar_wait(&sfs_empty[ss], ssph ^ 1u, abort_flag)) { ok = false; break; }
+                        unsigned char *sf = sf_smem + ss * kSfSlotBytes;
+                        mbar_arrive_expect_tx(&sfs_full[ss], 2u * kSfKind);
+                        tma_load_2d(sf, &maps.sfa0, &sfs_full[ss], (int32_t)(st * 8u), y0);
+                        tma_load_2d(sf + kSfKind, &maps.sfa1, &sfs_full[ss], (int32_t)(st * 8u), y1);
+                        if (++ss == kSfSlots) { ss = 0; ssph ^= 1u; }
+                    }
                     if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag)) { ok = false; break; }
                     unsigned char *dst = base + s * kStageBytes;
                     const int32_t x = (int32_t)(st * 128u);
@@ -333,28 +353,7 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
                 if (++s == kBSlots) { s = 0; ph ^= 1u; }
             }
         }
-    } else if (warp == 3) {
-        // ================================ TMA producer: weight scales, two stages at a time
-        if (lane == 0) {
-            prefetch_tensormap(&maps.sfa0);
-            prefetch_tensormap(&maps.sfa1);
-            uint32_t s = 0, ph = 0;
-            bool ok = true;
-            for (uint32_t w = next_item(); ok && w != kNoItem; w = next_item()) {
-                const Item it = decode_item(w, prefix, a);
-                const int32_t y0 = (int32_t)(it.group * a.w_rows + it.m_item * tile_rows);
-                const int32_t y1 = kAct ? y0 : y0 + (int32_t)BM;
-                for (uint32_t st = 0; st < steps; st += 2u) {
-                    if (!mbar_wait(&sfs_empty[s], ph ^ 1u, abort_flag)) { ok = false; break; }
-                    unsigned char *dst = sf_smem + s * kSfSlotBytes;
-                    mbar_arrive_expect_tx(&sfs_full[s], 2u * kSfKind);
-                    tma_load_2d(dst, &maps.sfa0, &sfs_full[s], (int32_t)(st * 8u), y0);
-                    tma_load_2d(dst + kSfKind, &maps.sfa1, &sfs_full[s], (int32_t)(st * 8u), y1);
-                    if (++s == kSfSlots) { s = 0; ph ^= 1u; }
-                }
-            }
-        }
-    } else if (warp == 1 || warp == 16) {
+    } else if (warp == 1 || warp == 3) {
         // ==================================================== MMA issuers, one per weight tile
         if (lane == 0) {
             const uint32_t q = warp == 1 ? 0u : 1u;
@@ -466,9 +465,11 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
         }
     } else {
         // ======================================================== epilogue
-        // Quadrant = warp % 4 (tensor-memory lanes); chunks of four token rows (32 columns)
-        // alternate between the two warps of a quadrant.
-        const uint32_t quad = warp & 3u, half = (warp - 8u) >> 2;
+        // Quadrant = warp % 4 (tensor-memory lanes); four token rows (32 columns) per warp, their
+        // activations and term splits interleaved: one row after the other in eight warps, the
+        // epilogue and not the stream bounded the gate/up launch at the latent shape (SiTU, K = 3584:
+        // a 1021-token prompt 4.47 -> 4.2 ms).
+        const uint32_t quad = warp & 3u, r0 = 4u * ((warp - 8u) >> 2);
         const uint32_t m = 32u * quad + lane;              // weight row inside the tile
         AccBuffers acc;
         for (uint32_t w = __shfl_sync(0xffffffffu, next_item(), 0); w != kNoItem;
@@ -485,18 +486,18 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
             const uint32_t t1 = tmem + ((32u * quad) << 16) + acc.column(small, b0, 1u);
             acc.advance(small, b0);
             const uint32_t col0 = it.m_item * tile_rows + m, col1 = kAct ? col0 : col0 + BM;
-            float v0[8], v1[8];                            // this warp's rows: 4 * half + 8 * (i / 4) + i % 4
+            float v0[4], v1[4];
+            if (r0 < it.rows_valid) {
 #pragma unroll
-            for (uint32_t c = 0; c < 2u; c++) {
-                if (8u * c + 4u * half < it.rows_valid) {
-                    uint32_t r0[32], r1[32];
-                    tmem_ld_32x32(t0 + 64u * c + 32u * half, r0);
-                    tmem_ld_32x32(t1 + 64u * c + 32u * half, r1);
+                for (uint32_t c = 0; c < 2u; c++) {
+                    uint32_t q0[16], q1[16];
+                    tmem_ld_32x16(t0 + 8u * r0 + 16u * c, q0);
+                    tmem_ld_32x16(t1 + 8u * r0 + 16u * c, q1);
                     tmem_ld_wait();
 #pragma unroll
-                    for (uint32_t i = 0; i < 4u; i++) {
-                        v0[4u * c + i] = sum8(r0 + 8u * i);
-                        v1[4u * c + i] = sum8(r1 + 8u * i);
+                    for (uint32_t i = 0; i < 2u; i++) {
+                        v0[2u * c + i] = sum8(q0 + 8u * i);
+                        v1[2u * c + i] = sum8(q1 + 8u * i);
                     }
                 }
             }
@@ -506,25 +507,62 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
                 mbar_arrive(&acc_empty[b0]);
                 if (!small) mbar_arrive(&acc_empty[1]);
             }
+            if (r0 >= it.rows_valid) continue;
+            const uint32_t n = min(4u, it.rows_valid - r0);
+            const uint64_t row = it.row_start + r0;
+            if (!kAct) {
 #pragma unroll
-            for (uint32_t i = 0; i < 8u; i++) {
-                const uint32_t r = 8u * (i / 4u) + 4u * half + i % 4u;
-                if (r >= it.rows_valid) continue;          // uniform across the warp
-                const uint64_t row = it.row_start + r;
-                if (kAct) {
-                    // gate and up are rounded to bf16 before the activation
-                    const float g = bf16_bits_to_float(float_to_bf16_bits(v0[i]));
-                    const float u = bf16_bits_to_float(float_to_bf16_bits(v1[i]));
-                    const uint16_t bits = float_to_bf16_bits(activation(g, u, a.activation, a.beta, a.linear_beta));
-                    if (a.out != nullptr) a.out[row * a.out_width + col0] = bits;
-                    uint32_t code[kTerms], sbyte[kTerms];
-                    split_block_e2m1(bf16_bits_to_float(bits), code, sbyte);
-                    store_block_e2m1(a.act_terms + row * kTerms * (a.w_rows / 2u), a.act_sf + row * kTerms * (a.w_rows / 32u),
-                                     a.w_rows / 2u, a.w_rows / 32u, col0 / 32u, code, sbyte, lane);
-                } else {
-                    a.out[row * a.out_width + col0] = float_to_bf16_bits(v0[i]);
-                    a.out[row * a.out_width + col1] = float_to_bf16_bits(v1[i]);
+                for (uint32_t i = 0; i < 4u; i++) {
+                    if (i >= n) break;
+                    a.out[(row + i) * a.out_width + col0] = float_to_bf16_bits(v0[i]);
+                    a.out[(row + i) * a.out_width + col1] = float_to_bf16_bits(v1[i]);
                 }
+                continue;
+            }
+            float rest[4];                                 // what the terms so far leave of the activation
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; i++) {
+                // gate and up are rounded to bf16 before the activation
+                const float g = bf16_bits_to_float(float_to_bf16_bits(v0[i]));
+                const float u = bf16_bits_to_float(float_to_bf16_bits(v1[i]));
+                const uint16_t bits = float_to_bf16_bits(activation(g, u, a.activation, a.beta, a.linear_beta));
+                if (a.out != nullptr && i < n) a.out[(row + i) * a.out_width + col0] = bits;
+                rest[i] = i < n ? bf16_bits_to_float(bits) : 0.f;
+            }
+            // eight E2M1 terms of the four rows' 32-column blocks (split_block_e2m1); a lane keeps the
+            // packed word it stores: lane 8 w + j the columns 8 w .. 8 w + 7 of term j
+            uint32_t word[4] = {0u, 0u, 0u, 0u}, scale[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (uint32_t j = 0; j < kTerms; j++) {
+#pragma unroll
+                for (uint32_t i = 0; i < 4u; i++) {
+                    const uint32_t mx = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(rest[i])));
+                    const uint32_t be = mx >> 23;
+                    const bool none = be < 4u || be == 0xffu;
+                    const uint32_t sb = none ? 127u : be - 2u;
+                    uint32_t code = 0u;
+                    if (!none) {                           // uniform across the warp
+                        const float scaled = rest[i] * __uint_as_float((254u - sb) << 23);
+                        code = (uint32_t)__nv_cvt_float_to_fp4(scaled, __NV_E2M1, cudaRoundNearest) & 0xfu;
+                        const float back =
+                            __half2float(__half(__nv_cvt_fp4_to_halfraw((__nv_fp4_storage_t)code, __NV_E2M1)));
+                        rest[i] -= back * __uint_as_float(sb << 23);
+                    }
+                    uint32_t v = code << (4u * (lane & 7u));
+                    v |= __shfl_xor_sync(0xffffffffu, v, 1);
+                    v |= __shfl_xor_sync(0xffffffffu, v, 2);
+                    v |= __shfl_xor_sync(0xffffffffu, v, 4);
+                    if ((lane & 7u) == j) word[i] = v;
+                    if (lane == j) scale[i] = sb;
+                }
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; i++) {
+                if (i >= n) break;
+                const uint64_t term = (row + i) * kTerms;
+                *reinterpret_cast<uint32_t *>(a.act_terms + (term + (lane & 7u)) * (a.w_rows / 2u) + (col0 & ~31u) / 2u +
+                                              4u * (lane >> 3)) = word[i];
+                if (lane < kTerms) a.act_sf[(term + lane) * (a.w_rows / 32u) + col0 / 32u] = (uint8_t)scale[i];
             }
         }
     }
@@ -538,19 +576,31 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
     }
 }
 
+// (`ids` given: the experts of row r are ids[r * top_k ..], and a row none of whose experts is a
+// group of this kernel is skipped.)
 // bf16 rows -> E2M1 terms and block scales: four lanes share a block of 32 columns (8 each), a
 // warp converts 256 columns per pass and stores each term as 128 contiguous bytes.  The same
 // values as split_block_e2m1 (one element per lane), a sixth of its instructions.
 __global__ void __launch_bounds__(256)
 term_rows_kernel(uint8_t *__restrict__ terms, uint8_t *__restrict__ sf, const uint16_t *__restrict__ x,
-                 uint32_t *__restrict__ counters, uint32_t rows, uint32_t k) {
+                 uint32_t *__restrict__ counters, const uint32_t *__restrict__ ids,
+                 const uint32_t *__restrict__ offsets, uint32_t top_k, uint32_t rows, uint32_t k) {
     pdl_wait();
     pdl_trigger();
     if (blockIdx.x == 0 && threadIdx.x < 64u) counters[threadIdx.x] = 0u;      // of the product launches
     const uint32_t lane = threadIdx.x % kWarp, passes = k / 256u;
     const uint64_t warps = (uint64_t)(gridDim.x * blockDim.x) / kWarp, jobs = (uint64_t)rows * passes;
     for (uint64_t job = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp; job < jobs; job += warps) {
-        const uint32_t r = (uint32_t)(job / passes), c = (uint32_t)(job % passes) * 256u + lane * 8u;
+        const uint32_t r = (uint32_t)(job / passes);
+        if (ids != nullptr) {
+            bool mine = false;
+            if (lane < top_k) {
+                const uint32_t e = ids[(uint64_t)r * top_k + lane];
+                mine = offsets[e + 1u] - offsets[e] <= kTileRows;
+            }
+            if (!__any_sync(0xffffffffu, mine)) continue;
+        }
+        const uint32_t c = (uint32_t)(job % passes) * 256u + lane * 8u;
         const uint4 raw = *reinterpret_cast<const uint4 *>(x + (uint64_t)r * k + c);
         const uint32_t wv[4] = {raw.x, raw.y, raw.z, raw.w};
         float v[8];
@@ -732,11 +782,13 @@ size_t k3_grouped_mx4_workspace_bytes(const k3_moe_layer_desc *d, uint32_t rows,
 }
 
 bool k3_grouped_mx4_terms(const k3_moe_layer_desc *d, const void *rows_in, uint32_t source_rows, uint32_t rows,
-                          void *workspace, uint32_t *counters, cudaStream_t stream) {
+                          const void *ids, const void *offsets, void *workspace, uint32_t *counters,
+                          cudaStream_t stream) {
     const Scratch s = carve_scratch(d, rows, source_rows, workspace);
     const uint64_t jobs = (uint64_t)source_rows * (d->hidden / 256u);
     return launch_chained(term_rows_kernel, (uint32_t)std::min<uint64_t>((jobs + 7u) / 8u, (uint64_t)sm_count() * 16u), 256, 0,
-                          stream, s.x_terms, s.x_sf, (const uint16_t *)rows_in, counters, source_rows, d->hidden);
+                          stream, s.x_terms, s.x_sf, (const uint16_t *)rows_in, counters, (const uint32_t *)ids, (const uint32_t *)offsets,
+                          d->top_k, source_rows, d->hidden);
 }
 
 bool k3_grouped_mx4_gateup(const k3_moe_layer_desc *d, void *act, const void *index, uint32_t source_rows,

@@ -154,8 +154,9 @@ extern "C" bool k3_moe_latent_layer_forward(const k3_moe_latent_desc *d, void *o
     if (token_path) {
         // rows_out already holds the expert rows
     } else if (w.mx_bytes != 0) {
+        const k3_token_routes by_token{w.ids, w.inv_perm};
         if (!k3_grouped_mx_experts(&e, w.rows_out, nullptr, w.latent, w.sorted_token, tokens, w.offsets, routes,
-                                   w.mx_ws, stream, tokens)) {
+                                   w.mx_ws, stream, &by_token)) {
             return false;
         }
     } else {

@@ -116,7 +116,7 @@ combine_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ rows,
         for (uint32_t c = blockIdx.y * blockDim.x + threadIdx.x; c < hidden / 8u;
              c += gridDim.y * blockDim.x) {
             float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
+#pragma unroll 8
             for (uint32_t r = 0; r < top_k; r++) {
                 const uint4 q = reinterpret_cast<const uint4 *>(rows + (uint64_t)idx_s[r] * hidden)[c];
                 const float w = w_s[r];
@@ -497,8 +497,9 @@ bool layer_forward_impl(const k3_moe_layer_desc *d, void *out, const void *x, ui
             if (w.mx_bytes != 0) {
                 // block-scaled path: tokens are converted once, then gathered as bytes
                 if (!mark(events, 3, stream)) return false;
+                const k3_token_routes by_token{w.ids, w.inv_perm};
                 if (!k3_grouped_mx_experts(d, w.rows_out, nullptr, x, w.sorted_token, tokens, w.offsets,
-                                           routes, w.mx_ws, stream, tokens)) {
+                                           routes, w.mx_ws, stream, &by_token)) {
                     return false;
                 }
             } else {
