@@ -10,7 +10,7 @@
 // scale per 32 columns, x = 2^s (hi + lo); bf16 carries 8 significant bits and
 // each term 4, so every element within 2^10 of its block maximum is exact and
 // the rest is held to 2^-17 of the block maximum.  Each K block of 32 issues two
-// MMAs per weight tile (hi and lo against the same weight tile and scales).
+// MMAs (hi and lo against the same weights and scales).
 //
 // Work item = two 128-row weight tiles x up to 128 token rows of one group over
 // the whole K extent (gate+up with fused activation, or 256 rows of the down
@@ -58,9 +58,8 @@ constexpr uint32_t kSfKind = BM * 16u;                    // one table's 128 row
 constexpr uint32_t kSfSlotBytes = 3u * kSfKind;           // SFA0 | SFA1 | SFB
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kAccCol = 0;                           // tile 0: [0,128), tile 1: [128,256)
-constexpr uint32_t kSfa0Col = 256;                        // kSfBatches x 16 columns each
-constexpr uint32_t kSfa1Col = kSfa0Col + 16u * kSfBatches;
-constexpr uint32_t kSfbCol = kSfa1Col + 16u * kSfBatches;
+constexpr uint32_t kSfwCol = 256;                         // weight scales: kSfBatches x 4 stages x (tile 0 | tile 1)
+constexpr uint32_t kSftCol = kSfwCol + 32u * kSfBatches;  // token scales: kSfBatches x 4 stages x 4 columns
 constexpr uint32_t kMaxGroups = 1024;
 constexpr uint32_t kItemSlots = 4;                        // mailbox of item numbers, producer -> other roles
 constexpr uint32_t kItemReaders = 7u + kEpilogueWarps;    // term producer, 2 issuers, 4 writers, epilogue warps
@@ -98,9 +97,12 @@ K3_DEVINL void mma_mx(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32
         : "memory");
 }
 
-// A = E2M1 (5), B = E4M3 (0), UE8M0 scales, M = 128, K-major; sf = byte of the scale column
-K3_DEVINL uint32_t make_idesc_mx(uint32_t n, uint32_t sf) {
-    return (5u << 7) | (0u << 10) | ((n >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24) | (sf << 29) | (sf << 4);
+// UE8M0 scales, M = 128, K-major; sf = byte of the scale column (kNextScaleByte: one further).
+// A = weights (E2M1, 5) and B = token terms (E4M3, 0), or the other way round.
+constexpr uint32_t kNextScaleByte = (1u << 29) | (1u << 4);
+K3_DEVINL uint32_t make_idesc_mx(uint32_t n, uint32_t sf, bool tokens_are_a) {
+    return ((tokens_are_a ? 0u : 5u) << 7) | ((tokens_are_a ? 5u : 0u) << 10) | ((n >> 3) << 17) | (1u << 23) |
+           ((128u >> 4) << 24) | (sf << 29) | (sf << 4);
 }
 
 // Two-term E4M3 form of a block of 32 values held one per lane:
@@ -155,18 +157,24 @@ struct Item {
 // N operand (lo from row `block` on), so that a K block of 32 is one MMA per weight tile: the
 // 8-bit weight containers are read from shared memory once instead of twice, and shared memory
 // is what bounds short tiles (88 KB per stage of 32 rows instead of 120 KB; 24 rows per
-// expert: 1.15 -> 1.01 ms together with the fourth stage).  A larger tile does not fit its accumulators that way (2 x 256
-// columns): its hi and lo MMAs add into the same columns.
+// expert: 1.15 -> 1.01 ms together with the fourth stage).  A larger tile does not fit its
+// accumulators that way (2 x 256 columns): there the terms are the A operand and both weight
+// tiles together the N = 256 operand, and the hi and the lo MMA add into the same columns.  A K
+// block of 32 then takes two MMAs of N = 256 (92 ns each, 12 KB of operands) where the weights
+// as A take four of N = 128 (55 ns, 8 KB), and a result row is stored in whole sectors.  192
+// experts of 128 rows, back to back: 2.72 -> 2.65 ms (first pass of the 8192-token layer 13.03
+// -> 12.96 ms; the power cap hides the rest of it).
 struct TermLayout {
     uint32_t block, n;
     bool stacked;
 };
+template <uint32_t kStages>
 K3_DEVINL TermLayout term_layout(uint32_t rows_valid) {
     TermLayout t;
     const uint32_t n16 = (rows_valid + 15u) & ~15u;
-    t.block = rows_valid <= 32u ? 32u : rows_valid <= 64u ? 64u : BN;
+    t.block = rows_valid <= 32u ? 32u : kStages > 3u || rows_valid <= 64u ? 64u : BN;
     t.stacked = t.block < BN;
-    t.n = t.stacked ? t.block + n16 : n16;
+    t.n = t.stacked ? t.block + n16 : 2u * BM;
     return t;
 }
 
@@ -223,6 +231,75 @@ struct GmxMaps {
     CUtensorMap sfa0, sfa1;    // weight block scales [rows, K/32]
     CUtensorMap sfb;           // token block scales  [rows, K/32]
 };
+
+// 32 bytes of one thread in one store where the address allows it (whole sectors)
+K3_DEVINL void store_32_bytes(void *p, const uint32_t (&v)[8], bool aligned) {
+    if (aligned) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]),
+                     "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                     : "memory");
+    } else {
+#pragma unroll
+        for (uint32_t j = 0; j < 8u; j++) {
+            reinterpret_cast<uint16_t *>(p)[2u * j] = (uint16_t)v[j];
+            reinterpret_cast<uint16_t *>(p)[2u * j + 1u] = (uint16_t)(v[j] >> 16);
+        }
+    }
+}
+// 16 bf16 values to out[at ...]
+K3_DEVINL void store_16_values(uint16_t *out, uint64_t at, const uint32_t (&v)[8]) {
+    store_32_bytes(out + at, v, (reinterpret_cast<uintptr_t>(out) & 31u) == 0);     // rows are multiples of 512 columns
+}
+
+// One result row's columns c .. c + 31 (tile 0, low halves of `pair`) and the same of tile 1
+// (high halves): activation, two-term split and stores, or plain stores.
+template <int kE>
+K3_DEVINL void store_row(const GmxArgs &a, uint64_t row, uint32_t c, uint32_t (&pair)[32]) {
+    uint32_t v[8];
+    if (kE == kEAct) {
+        uint32_t mx = 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < 16u; j++) {              // two bf16 results in one register
+            const uint32_t p0 = pair[2u * j], p1 = pair[2u * j + 1u];
+            const uint32_t b0 =
+                float_to_bf16_bits(activation(bf16_lo(p0), bf16_hi(p0), a.activation, a.beta, a.linear_beta));
+            const uint32_t b1 =
+                float_to_bf16_bits(activation(bf16_lo(p1), bf16_hi(p1), a.activation, a.beta, a.linear_beta));
+            mx = max(mx, max(b0 & 0x7fffu, b1 & 0x7fffu));
+            pair[j] = b0 | (b1 << 16);
+        }
+        if (a.out != nullptr) {
+#pragma unroll
+            for (uint32_t h = 0; h < 2u; h++) {
+#pragma unroll
+                for (uint32_t j = 0; j < 8u; j++) v[j] = pair[8u * h + j];
+                store_16_values(a.out, row * a.out_width + c + 16u * h, v);
+            }
+        }
+        const uint32_t be = min(max(mx >> 7, 8u), 254u);  // as block_scale()
+        const float mult = __uint_as_float((261u - be) << 23);
+        uint32_t lo[8];
+#pragma unroll
+        for (uint32_t j = 0; j < 8u; j++) {
+            const uint32_t p0 = split_pair(bf16_lo(pair[2u * j]) * mult, bf16_hi(pair[2u * j]) * mult);
+            const uint32_t p1 = split_pair(bf16_lo(pair[2u * j + 1u]) * mult, bf16_hi(pair[2u * j + 1u]) * mult);
+            v[j] = (p0 & 0xffffu) | (p1 << 16);
+            lo[j] = (p0 >> 16) | (p1 & 0xffff0000u);
+        }
+        store_32_bytes(a.act_hi + row * a.w_rows + c, v, true);      // buffers of the workspace: aligned
+        store_32_bytes(a.act_lo + row * a.w_rows + c, lo, true);
+        a.act_sf[row * (a.w_rows / 32u) + c / 32u] = (uint8_t)(be - 7u);
+    } else {
+#pragma unroll
+        for (uint32_t h = 0; h < 4u; h++) {               // tile 0's columns, then tile 1's
+#pragma unroll
+            for (uint32_t j = 0; j < 8u; j++)
+                v[j] = __byte_perm(pair[16u * (h & 1u) + 2u * j], pair[16u * (h & 1u) + 2u * j + 1u],
+                                   h < 2u ? 0x5410 : 0x7632);
+            store_16_values(a.out, row * a.out_width + c + (h >> 1) * BM + 16u * (h & 1u), v);
+        }
+    }
+}
 
 // kStages stages in flight: four where every group has at most 64 rows (the weight stream bounds
 // those), else three.  Weights and terms of a stage share their barriers: an issuer's commits
@@ -389,7 +466,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             for (uint32_t w = next_item(); ok && w != kNoItem; w = next_item()) {
                 const Item it = decode_item(w, prefix, a);
                 const uint32_t boxes = (it.rows_valid + kBBox - 1u) / kBBox;
-                const TermLayout t = term_layout(it.rows_valid);
+                const TermLayout t = term_layout<kStages>(it.rows_valid);
                 for (uint32_t st = 0; st < steps; st++) {
                     if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag)) { ok = false; break; }
                     const int32_t x = (int32_t)(st * KS);
@@ -407,20 +484,23 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         }
     } else if (warp == 1 || warp == 3) {
         // ==================================================== MMA issuers
-        // One thread's issue loop cannot keep the tensor pipe fed with K = 32 MMAs, so
-        // warp 1 issues the MMAs of weight tile 0 and warp 3 those of tile 1.  Both
-        // commit to the same stage / scale / accumulator barriers (count 2).
+        // One thread's issue loop cannot keep the tensor pipe fed with K = 32 MMAs of N <= 128,
+        // so warp 1 issues the MMAs of weight tile 0 and warp 3 those of tile 1.  Both
+        // commit to the same stage / scale / accumulator barriers (count 2).  The MMAs of a
+        // larger tile all add into one accumulator: warp 1 issues them, warp 3 only arrives.
         if (lane == 0) {
             const uint32_t q = warp == 1 ? 0u : 1u;
             uint32_t s = 0, ph = 0, sb = 0, sph = 0;
             AccBuffers acc;
+            auto release = [](uint64_t *bar, bool bystander) {
+                if (bystander) mbar_arrive(bar); else mma_commit(bar);
+            };
             bool ok = true;
             for (uint32_t w = next_item(); ok && w != kNoItem; w = next_item()) {
                 const Item it = decode_item(w, prefix, a);
-                const TermLayout t = term_layout(it.rows_valid);
-                uint32_t idesc[4];
-#pragma unroll
-                for (uint32_t j = 0; j < 4u; j++) idesc[j] = make_idesc_mx(t.n, j);
+                const TermLayout t = term_layout<kStages>(it.rows_valid);
+                const uint32_t idesc = make_idesc_mx(t.n, 0u, !t.stacked);
+                const bool bystander = !t.stacked && q == 1u;
                 const bool small = acc.small(it.rows_valid);
                 const uint32_t b0 = acc.first(small);
                 if (!mbar_wait(&acc_empty[b0], (acc.uses(b0) & 1u) ^ 1u, abort_flag) ||
@@ -429,7 +509,6 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                 }
                 tc_fence_after();
                 const uint32_t d = tmem + kAccCol + acc.column(small, b0, q);
-                const uint32_t sfa_col = tmem + (q == 0u ? kSfa0Col : kSfa1Col);
                 for (uint32_t st = 0; st < steps; st++) {
                     if (!mbar_wait(&full[s], ph, abort_flag) ||
                         ((st & 3u) == 0u && !mbar_wait(&sf_full[sb], sph, abort_flag))) {
@@ -438,34 +517,36 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                     }
                     tc_fence_after();
                     const unsigned char *src = base + s * kStageBytes;
-                    const uint64_t da = make_desc_sw128(smem_u32(src + q * kATile));
-                    const uint64_t dbh = make_desc_sw128(smem_u32(src + 2u * kATile));
-                    const uint32_t sfs = sb * 16u + (st & 3u) * 4u;
+                    const uint64_t dw = make_desc_sw128(smem_u32(src + q * kATile));
+                    const uint64_t dhi = make_desc_sw128(smem_u32(src + 2u * kATile));
+                    const uint32_t sfw = tmem + kSfwCol + sb * 32u + (st & 3u) * 8u;
+                    const uint32_t sft = tmem + kSftCol + sb * 16u + (st & 3u) * 4u;
                     if (t.stacked) {
 #pragma unroll
                         for (uint32_t j = 0; j < 4u; j++) {          // K blocks of 32 inside the stage
-                            mma_mx(d, da + 2u * j, dbh + 2u * j, idesc[j], sfa_col + sfs, tmem + kSfbCol + sfs,
+                            mma_mx(d, dw + 2u * j, dhi + 2u * j, idesc + j * kNextScaleByte, sfw + 4u * q, sft,
                                    (st | j) != 0u ? 1u : 0u);
                         }
-                    } else {
-                        const uint64_t dbl = make_desc_sw128(smem_u32(src + 2u * kATile + kBTile));
+                    } else if (!bystander) {
+                        // weight tiles 0 and 1 lie one behind the other: 256 rows of one operand
+                        const uint64_t dlo = make_desc_sw128(smem_u32(src + 2u * kATile + kBTile));
 #pragma unroll
                         for (uint32_t j = 0; j < 4u; j++) {
-                            mma_mx(d, da + 2u * j, dbh + 2u * j, idesc[j], sfa_col + sfs, tmem + kSfbCol + sfs,
+                            mma_mx(d, dhi + 2u * j, dw + 2u * j, idesc + j * kNextScaleByte, sft, sfw,
                                    (st | j) != 0u ? 1u : 0u);
-                            mma_mx(d, da + 2u * j, dbl + 2u * j, idesc[j], sfa_col + sfs, tmem + kSfbCol + sfs, 1u);
+                            mma_mx(d, dlo + 2u * j, dw + 2u * j, idesc + j * kNextScaleByte, sft, sfw, 1u);
                         }
                     }
-                    mma_commit(&empty[s]);
+                    release(&empty[s], bystander);
                     if (++s == kStages) { s = 0; ph ^= 1u; }
                     if ((st & 3u) == 3u) {
-                        mma_commit(&sf_empty[sb]);
+                        release(&sf_empty[sb], bystander);
                         if (++sb == kSfBatches) { sb = 0; sph ^= 1u; }
                     }
                 }
                 if (!ok) break;
-                mma_commit(&acc_full[b0]);
-                if (!small) mma_commit(&acc_full[1]);
+                release(&acc_full[b0], bystander);
+                if (!small) release(&acc_full[1], bystander);
                 acc.advance(small, b0);
             }
         }
@@ -481,7 +562,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         for (uint32_t w = __shfl_sync(0xffffffffu, next_item(), 0); ok && w != kNoItem;
              w = __shfl_sync(0xffffffffu, next_item(), 0)) {
             // a stacked operand's lo rows have the scales of its hi rows
-            const uint32_t repeat = term_layout(decode_item(w, prefix, a).rows_valid).block / 32u - 1u;
+            const uint32_t repeat = term_layout<kStages>(decode_item(w, prefix, a).rows_valid).block / 32u - 1u;
             for (uint32_t st = 0; st < steps; st += 4u) {
                 if (!mbar_wait(&sfs_full[ss], ssph, abort_flag)) { ok = false; break; }
                 const unsigned char *src = sf_smem + ss * kSfSlotBytes;
@@ -494,15 +575,22 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                             src + t * kSfKind + (32u * (t == 2u ? c & repeat : c) + lane) * 16u);
                 if (!mbar_wait(&sf_empty[sb], sph ^ 1u, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-#pragma unroll
-                for (uint32_t t = 0; t < 3u; t++) {
-                    const uint32_t cols[16] = {v[t][0].x, v[t][1].x, v[t][2].x, v[t][3].x,
-                                               v[t][0].y, v[t][1].y, v[t][2].y, v[t][3].y,
-                                               v[t][0].z, v[t][1].z, v[t][2].z, v[t][3].z,
-                                               v[t][0].w, v[t][1].w, v[t][2].w, v[t][3].w};
-                    const uint32_t col = (t == 0 ? kSfa0Col : t == 1 ? kSfa1Col : kSfbCol) + sb * 16u;
-                    tmem_st_32x16(tmem + lane_base + col, cols);
-                }
+                // a stage's columns: tile 0 | tile 1 side by side (rows 0..255 of one operand)
+                const uint32_t w01[16] = {v[0][0].x, v[0][1].x, v[0][2].x, v[0][3].x,
+                                          v[1][0].x, v[1][1].x, v[1][2].x, v[1][3].x,
+                                          v[0][0].y, v[0][1].y, v[0][2].y, v[0][3].y,
+                                          v[1][0].y, v[1][1].y, v[1][2].y, v[1][3].y};
+                tmem_st_32x16(tmem + lane_base + kSfwCol + sb * 32u, w01);
+                const uint32_t w23[16] = {v[0][0].z, v[0][1].z, v[0][2].z, v[0][3].z,
+                                          v[1][0].z, v[1][1].z, v[1][2].z, v[1][3].z,
+                                          v[0][0].w, v[0][1].w, v[0][2].w, v[0][3].w,
+                                          v[1][0].w, v[1][1].w, v[1][2].w, v[1][3].w};
+                tmem_st_32x16(tmem + lane_base + kSfwCol + sb * 32u + 16u, w23);
+                const uint32_t tok[16] = {v[2][0].x, v[2][1].x, v[2][2].x, v[2][3].x,
+                                          v[2][0].y, v[2][1].y, v[2][2].y, v[2][3].y,
+                                          v[2][0].z, v[2][1].z, v[2][2].z, v[2][3].z,
+                                          v[2][0].w, v[2][1].w, v[2][2].w, v[2][3].w};
+                tmem_st_32x16(tmem + lane_base + kSftCol + sb * 16u, tok);
                 // The shared-memory slot goes back to the TMA producer only now: the
                 // stores above consumed every loaded register, so the loads have
                 // completed (an arrive right after issuing them would not wait for that).
@@ -518,14 +606,17 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         }
     } else {
         // ======================================================== epilogue
-        // Sixteen warps: quadrant = warp % 4 (tensor-memory lanes), the tile's token rows in
+        // Sixteen warps: quadrant = warp % 4 (tensor-memory lanes), the accumulators' columns in
         // four parts.  A warp takes its part of both accumulators out of tensor memory at once,
         // rounded to bf16 (which both modes do anyway) and packed in pairs, and frees the
         // accumulators before it computes anything: a tile of more than 32 rows has no second
-        // buffer, so the MMAs of the next item wait for exactly this.
+        // buffer, so the MMAs of the next item wait for exactly this.  Lanes are weight rows
+        // and columns token rows, or, in a tile of more than 64 rows, the other way round: a
+        // thread then holds 32 neighbouring columns of one result row (a whole scale block)
+        // and stores them in 32-byte pieces.
         const uint32_t quad = warp & 3u;
         const uint32_t part = (warp - 8u) >> 2;
-        const uint32_t m = 32u * quad + lane;            // weight row inside the tile
+        const uint32_t m = 32u * quad + lane;            // tensor-memory lane: weight row, or token row
         AccBuffers acc;
         for (uint32_t w = __shfl_sync(0xffffffffu, next_item(), 0); w != kNoItem;
              w = __shfl_sync(0xffffffffu, next_item(), 0)) {
@@ -543,12 +634,12 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             const uint32_t col0 = it.m_item * tile_rows + m;
             const uint32_t col1 = kE == kEAct ? col0 : col0 + BM;
             const bool in0 = col0 < a.w_rows, in1 = col1 < a.w_rows;
-            const TermLayout t = term_layout(it.rows_valid);
+            const TermLayout t = term_layout<kStages>(it.rows_valid);
             const uint32_t span = t.block / 4u, c = span * part;         // this warp's token rows
             uint32_t pair[32];                                           // bf16 of tile 0 | tile 1 << 16
 #pragma unroll
             for (uint32_t i = 0; i < 32u; i += 8u) {
-                if (i >= span || c + i >= it.rows_valid) break;
+                if (t.stacked && (i >= span || c + i >= it.rows_valid)) break;
                 uint32_t r0[8], r1[8];
                 tmem_ld_32x8(t0 + c + i, r0);
                 tmem_ld_32x8(t0 + tile1 + c + i, r1);
@@ -576,6 +667,11 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             if (lane == 0) {
                 mbar_arrive(&acc_empty[b0]);
                 if (!small) mbar_arrive(&acc_empty[1]);
+            }
+            if (!t.stacked) {
+                if (m < it.rows_valid) store_row<kE>(a, (uint64_t)(it.row_start + m), it.m_item * tile_rows + c, pair);
+                __syncwarp();
+                continue;
             }
             if (c >= it.rows_valid) continue;
             const uint32_t n_here = min(span, it.rows_valid - c);
