@@ -124,7 +124,8 @@ struct Mx4Args {
     const uint32_t *index;               // term row block of product row r (null: r itself)
     const uint8_t *sfb;                  // term scales [term rows, K/32]
     uint16_t *out;                       // bf16 [rows, out_width] (may be null in gate/up mode)
-    uint8_t *act_terms, *act_sf;         // gate/up mode: E2M1 terms [rows * 8, w_rows / 2] and scales [rows * 8, w_rows / 32]
+    uint8_t *act_terms, *act_sf;         // gate/up mode: E2M1 terms [act rows * 8, w_rows / 2] and scales [.., w_rows / 32]
+    bool act_by_group;                   // an activation row's place: 16 per group of this kernel, or the product row
     uint32_t groups, w_rows, k, out_width, m_items;
     uint32_t *item_counter;              // zero before the launch
     int activation;
@@ -139,6 +140,7 @@ struct Mx4Maps {
 
 struct Item {
     uint32_t group, row_start, rows_valid, m_item;
+    uint32_t act_row;                    // where the activation rows start
 };
 
 // Item w -> (group, weight tile); prefix[g] = groups this kernel takes before group g.
@@ -154,6 +156,7 @@ K3_DEVINL Item decode_item(uint32_t w, const uint32_t *prefix, const Mx4Args &a)
     it.m_item = w - n * a.m_items;
     it.row_start = a.offsets[lo];
     it.rows_valid = a.offsets[lo + 1u] - it.row_start;
+    it.act_row = a.act_by_group ? n * kTileRows : it.row_start;
     return it;
 }
 
@@ -339,8 +342,8 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
              w = __shfl_sync(0xffffffffu, next_item(), 0)) {
             const Item it = decode_item(w, prefix, a);
             const bool mine = lane < it.rows_valid;
-            const uint32_t row = it.row_start + lane;
-            const int32_t y = mine ? (int32_t)(kTerms * (a.index ? a.index[row] : row)) : 0;
+            const uint32_t row = (kAct ? it.row_start : it.act_row) + lane;
+            const int32_t y = mine ? (int32_t)(kTerms * (kAct && a.index ? a.index[row] : row)) : 0;
             for (uint32_t st = 0; st < steps; st += 2u) {
                 if (lane == 0) {
                     ok = mbar_wait(&b_empty[s], ph ^ 1u, abort_flag);
@@ -422,8 +425,9 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
             uint4 vb[4];
 #pragma unroll
             for (uint32_t c = 0; c < 4u; c++) {
-                const uint32_t i = 4u * c + lane / 8u, row = it.row_start + (i < it.rows_valid ? i : 0u);
-                const uint64_t term = (uint64_t)kTerms * (a.index ? a.index[row] : row) + lane % 8u;
+                const uint32_t i = 4u * c + lane / 8u;
+                const uint32_t row = (kAct ? it.row_start : it.act_row) + (i < it.rows_valid ? i : 0u);
+                const uint64_t term = (uint64_t)kTerms * (kAct && a.index ? a.index[row] : row) + lane % 8u;
                 term_sf[c] = reinterpret_cast<const uint4 *>(a.sfb + term * (a.k / 32u));
             }
 #pragma unroll
@@ -559,7 +563,7 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
 #pragma unroll
             for (uint32_t i = 0; i < 4u; i++) {
                 if (i >= n) break;
-                const uint64_t term = (row + i) * kTerms;
+                const uint64_t term = (uint64_t)(it.act_row + r0 + i) * kTerms;
                 *reinterpret_cast<uint32_t *>(a.act_terms + (term + (lane & 7u)) * (a.w_rows / 2u) + (col0 & ~31u) / 2u +
                                               4u * (lane >> 3)) = word[i];
                 if (lane < kTerms) a.act_sf[(term + lane) * (a.w_rows / 32u) + col0 / 32u] = (uint8_t)scale[i];
@@ -738,7 +742,9 @@ bool launch(const Operands &op, Mx4Args args, cudaStream_t stream) {
 
 struct Scratch {
     uint8_t *x_terms, *x_sf;             // per source row
-    uint8_t *a_terms, *a_sf;             // activation, per product row
+    uint8_t *a_terms, *a_sf;             // activation, per activation row
+    uint32_t act_rows;
+    bool act_by_group;
     size_t total;
 };
 
@@ -754,8 +760,13 @@ Scratch carve_scratch(const k3_moe_layer_desc *d, uint32_t rows, uint32_t source
     Scratch s{};
     s.x_terms = take((size_t)source_rows * kTerms * (H / 2u));
     s.x_sf = take((size_t)source_rows * kTerms * (H / 32u));
-    s.a_terms = take((size_t)rows * kTerms * (I / 2u));
-    s.a_sf = take((size_t)rows * kTerms * (I / 32u));
+    // A row's terms are 4.25 bytes per column and at most kTileRows rows of a group come here, so
+    // with many rows the activation is laid out by group: 125 MB instead of 2.3 GB for the
+    // 262144 rows of 16384 tokens at 896 experts.  With few rows the product rows take less.
+    s.act_by_group = (uint64_t)d->local_expert_count * kTileRows < rows;
+    s.act_rows = s.act_by_group ? d->local_expert_count * kTileRows : rows;
+    s.a_terms = take((size_t)s.act_rows * kTerms * (I / 2u));
+    s.a_sf = take((size_t)s.act_rows * kTerms * (I / 32u));
     s.total = off + 256u;
     return s;
 }
@@ -806,6 +817,7 @@ bool k3_grouped_mx4_gateup(const k3_moe_layer_desc *d, void *act, const void *in
     a.out = (uint16_t *)act;
     a.act_terms = s.a_terms;
     a.act_sf = s.a_sf;
+    a.act_by_group = s.act_by_group;
     a.w_rows = d->expert_hidden;
     a.k = d->hidden;
     a.out_width = d->expert_hidden;
@@ -827,6 +839,7 @@ bool k3_grouped_mx4_down(const k3_moe_layer_desc *d, void *rows_out, const void 
     a.k = d->expert_hidden;
     a.out_width = d->hidden;
     a.m_items = d->hidden / (2u * BM);
-    const Operands op{d->w2_packed, d->w2_packed, d->w2_scales, d->w2_scales, s.a_terms, s.a_sf, rows * kTerms};
+    a.act_by_group = s.act_by_group;
+    const Operands op{d->w2_packed, d->w2_packed, d->w2_scales, d->w2_scales, s.a_terms, s.a_sf, s.act_rows * kTerms};
     return launch<false>(op, a, stream);
 }
