@@ -543,7 +543,7 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
                     const uint32_t mx = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(rest[i])));
                     const uint32_t be = mx >> 23;
                     const bool none = be < 4u || be == 0xffu;
-                    const uint32_t sb = none ? 127u : be - 2u;
+                    const uint32_t sb = be == 0xffu ? 255u : none ? 127u : be - 2u;     // 255: E8M0's NaN
                     uint32_t code = 0u;
                     if (!none) {                           // uniform across the warp
                         const float scaled = rest[i] * __uint_as_float((254u - sb) << 23);
@@ -621,8 +621,10 @@ term_rows_kernel(uint8_t *__restrict__ terms, uint8_t *__restrict__ sf, const ui
             mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
             mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
             const uint32_t be = mx >> 23;
-            const bool none = be < 4u || be == 0xffu;      // nothing (finite) left in this block
-            const uint32_t sb = none ? 127u : be - 2u;     // largest magnitude / 2^(sb - 127) in [4, 8)
+            const bool none = be < 4u || be == 0xffu;      // nothing left in this block, or nothing finite
+            // largest magnitude / 2^(sb - 127) in [4, 8); a block with an infinity or NaN gets the
+            // scale 255, E8M0's NaN, so that its row's results are NaN
+            const uint32_t sb = be == 0xffu ? 255u : none ? 127u : be - 2u;
             const float down = none ? 0.f : __uint_as_float((254u - sb) << 23), up = __uint_as_float(sb << 23);
             uint32_t word = 0;
 #pragma unroll

@@ -54,3 +54,26 @@ def test_result_rows_of_any_alignment():
         tc.status_ok()
         results.append((G.host(out).tobytes(), G.host(act).tobytes()))
     assert results[0] == results[1] == results[2]
+
+
+@pytest.mark.parametrize("counts", [[3, 16, 20, 1], [3, 16, 200, 1]])
+def test_a_nan_reaches_its_own_row_only(counts):
+    """One NaN in a row makes this row's results NaN and no other's, in every kernel."""
+    d, i, e, rows = 1024, 512, 4, sum(counts)
+    cfg = synth.baseline_config(hidden=d, expert_hidden=i, experts=e, top_k=2, shared_hidden=0)
+    w = synth.make_layer(cfg, seed=31)
+    x, offsets = synth.activations(31, rows, d), np.concatenate([[0], np.cumsum(counts)]).astype(np.uint32)
+    hit = [0, 4, 25, rows - 1]
+    x[hit, 77] = 0x7FC0
+    desc = _native.LayerDesc(hidden=d, expert_hidden=i, expert_count=e, top_k=2, shared_hidden=0,
+                             activation=cfg["activation"], route_scale=1.0, local_expert_count=e)
+    keep = {k: G.dev(w[k]) for k in w if k.startswith("w")}
+    for k, v in keep.items():
+        setattr(desc, k, v.data_ptr())
+    need = ops.k3_moe_experts_workspace_bytes(desc, rows, 0)
+    ws, out = torch.empty(need, dtype=torch.uint8, device="cuda"), G.empty((rows, d), np.uint16)
+    assert ops.k3_moe_experts_grouped_ws(desc, out, None, G.dev(x), None, 0, G.dev(offsets), rows, ws, need)
+    tc.status_ok()
+    nan = np.isnan(G.bf16_f32(G.host(out, np.uint16)))
+    assert nan[hit].all()
+    assert not np.delete(nan, hit, axis=0).any()
