@@ -5,15 +5,16 @@
 // per term, then the binary tree 128, 64, ... 1.  So the work is fp32 FMAs on the vector
 // pipes (72 TFLOP/s, measured) and what is left to choose is how little else is issued and
 // moved around them.  A block computes a tile of weight rows x input rows out of register
-// tiles (8 x 8 outputs per thread for Q8, 4 x 4 outputs x 4 columns for BF16): a weight is
-// converted once per 8 input rows and an input once per 8 weight rows, where the one-row
+// tiles (4 x 8 outputs per thread for Q8, 2 x 4 or 4 x 4 outputs x 4 columns for BF16): a weight is
+// converted once per 8 input rows and an input once per 4 weight rows, where the one-row
 // kernel these replace converted both again for every output and re-read each weight row
 // from L2 for every four input rows.
 //
 // Bound: the issue rate.  Per 512 FMAs of a Q8 octet step about 300 other instructions go
 // out (byte -> float and the rounded scale product of the weights, bf16 -> float of the
-// inputs, loads); a BF16 step has none of these, since the mixed-precision FMA takes bf16
-// operands.
+// inputs, loads), so two input rows share one packed FMA: 200 rows of 3584 x 7168 517 -> 443
+// us, of 7168 x 3584 653 -> 541, 8 rows 26 -> 22 and 29 -> 25.  A BF16 step has no conversions,
+// since the mixed-precision FMA takes bf16 operands.
 #pragma once
 
 #include "k3_common.cuh"
@@ -21,6 +22,14 @@
 #include <cuda_fp16.h>
 
 namespace k3 {
+
+// Two fp32 fused multiply-adds in one instruction (each rounds as fmaf does).
+K3_DEVINL void fma_pair(float2 &acc, float a, float2 b) {
+    asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %2};\n\tmov.b64 b, {%3, %4};\n\tmov.b64 c, {%0, %1};\n\t"
+        "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+        : "+f"(acc.x), "+f"(acc.y)
+        : "f"(a), "f"(b.x), "f"(b.y));
+}
 
 // acc + a * b for bf16 a, b: the product is exact in fp32, so this is fmaf(float(a), float(b), acc)
 K3_DEVINL void fma_bf16(float &acc, uint16_t a, uint16_t b) {
@@ -57,11 +66,12 @@ exact_q8_kernel(uint16_t *__restrict__ out, const int8_t *__restrict__ q, const 
     const uint16_t *xr[kV];
 #pragma unroll
     for (int v = 0; v < kV; v++) xr[v] = x + (uint64_t)min(v0 + (uint32_t)v, vectors - 1u) * columns;
-    float acc[kR][kV];
+    constexpr int kPairs = (kV + 1) / 2;                   // input rows go in pairs through the packed FMA
+    float2 acc[kR][kPairs];
 #pragma unroll
     for (int r = 0; r < kR; r++)
 #pragma unroll
-        for (int v = 0; v < kV; v++) acc[r][v] = 0.f;
+        for (int v = 0; v < kPairs; v++) acc[r][v] = make_float2(0.f, 0.f);
 
     for (uint32_t first = 32u * slot + lane; first < octets; first += 256u * kDeep) {
         uint2 wq[kDeep][kR];
@@ -95,13 +105,21 @@ exact_q8_kernel(uint16_t *__restrict__ out, const int8_t *__restrict__ q, const 
                     const float f = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7650u + (b & 3))) - 8388736.0f;
                     wf[r] = __fmul_rn(f, s[j][r]);
                 }
-#pragma unroll
-                for (int v = 0; v < kV; v++) {
+                auto input = [&](int v) {
                     const uint4 &xv = xq[j][v];
                     const uint32_t pair = (b >> 1) == 0 ? xv.x : (b >> 1) == 1 ? xv.y : (b >> 1) == 2 ? xv.z : xv.w;
-                    const float xf = (b & 1) ? bf16_hi(pair) : bf16_lo(pair);
+                    return (b & 1) ? bf16_hi(pair) : bf16_lo(pair);
+                };
 #pragma unroll
-                    for (int r = 0; r < kR; r++) acc[r][v] = fmaf(wf[r], xf, acc[r][v]);
+                for (int v = 0; v + 1 < kV; v += 2) {
+                    const float2 xf = make_float2(input(v), input(v + 1));
+#pragma unroll
+                    for (int r = 0; r < kR; r++) fma_pair(acc[r][v / 2], wf[r], xf);
+                }
+                if constexpr (kV % 2 != 0) {
+                    const float xf = input(kV - 1);
+#pragma unroll
+                    for (int r = 0; r < kR; r++) acc[r][kPairs - 1].x = fmaf(wf[r], xf, acc[r][kPairs - 1].x);
                 }
             }
         }
@@ -114,7 +132,7 @@ exact_q8_kernel(uint16_t *__restrict__ out, const int8_t *__restrict__ q, const 
 #pragma unroll
         for (int r = 0; r < kR; r++)
 #pragma unroll
-            for (int v = 0; v < kPhase; v++) red[r * kPhase + v][slot][lane] = acc[r][p + v];
+            for (int v = 0; v < kPhase; v++) red[r * kPhase + v][slot][lane] = (p + v) % 2 ? acc[r][(p + v) / 2].y : acc[r][(p + v) / 2].x;
         __syncthreads();
         for (int o = (int)slot; o < kOut; o += 8) {
             const float(*a)[32] = red[o];

@@ -120,10 +120,17 @@ bool launch_bf16(void *output, const void *weights, const void *input, uint32_t 
                               (const uint16_t *)input, vectors, rows, columns);
     }
     if (vectors == 1u) return launch_exact_bf16<Out, 1, 1, 4, 1>(output, weights, input, vectors, rows, columns, stream);
-    if (vectors == 2u) return launch_exact_bf16<Out, 1, 2, 4, 1>(output, weights, input, vectors, rows, columns, stream);
-    if (vectors <= 4u) return launch_exact_bf16<Out, 2, 4, 4, 1>(output, weights, input, vectors, rows, columns, stream);
-    if (vectors <= 16u) return launch_exact_bf16<Out, 2, 4, 2, 2>(output, weights, input, vectors, rows, columns, stream);
-    return launch_exact_bf16<Out, 4, 4, 4, 2>(output, weights, input, vectors, rows, columns, stream);
+    if (vectors <= 6u) return launch_exact_bf16<Out, 1, 2, 4, 1>(output, weights, input, vectors, rows, columns, stream);
+    // 2 x 4 outputs per thread fill the chip best with many blocks; between one wave of those (six
+    // blocks of 128 threads per SM) and one wave of 4 x 4 (four per SM) the larger tile saves the
+    // second wave.  896 x 7168, 2 x 4 against 4 x 4: 12 rows 8.2 / 11.6 us, 16 rows 14 / 12.5, 20 rows
+    // 14.2 / 12.5, 24 rows 14.7 / 20, 200 rows 104 / 108 (blocks of 256 and 512 threads, as before:
+    // 14.6, 14.7, 25.1, 25.2 and 123); six rows and fewer 1 x 2: 6.0 (8.0).
+    const uint64_t sms = (uint64_t)sm_count(), passes = (vectors + 3u) / 4u;
+    const bool one_wave_2x4 = (rows + 3u) / 4u * passes <= 6u * sms, one_wave_4x4 = (rows + 7u) / 8u * passes <= 4u * sms;
+    if (!one_wave_2x4 && one_wave_4x4)
+        return launch_exact_bf16<Out, 4, 4, 2, 1>(output, weights, input, vectors, rows, columns, stream);
+    return launch_exact_bf16<Out, 2, 4, 2, 1>(output, weights, input, vectors, rows, columns, stream);
 }
 
 template <int kTiles, int kBlocks, int kTeams>
