@@ -18,6 +18,14 @@ bool k3_grouped_q8_bf16(void *out, const void *q, const void *scales, const void
                         uint32_t tokens, uint32_t rows, uint32_t cols, uint32_t block,
                         int scale_type, void *stream);
 
+// Q8 products of at most 32 rows on mma.sync (k3_q8_few.cu), whole scale steps of 32 columns; gate/up
+// writes both products and the activation, bf16 [vectors, shared_hidden] each.
+bool k3_q8_few_supported(const void *q, const void *x, uint32_t vectors, uint32_t columns, uint32_t block);
+bool k3_q8_few_product(void *out, const void *q, const void *scales, const void *x, uint32_t vectors, uint32_t rows,
+                       uint32_t columns, uint32_t block, int scale_type, cudaStream_t stream);
+bool k3_q8_few_gateup(const k3_moe_layer_desc *desc, void *act, void *gate, void *up, const void *x, uint32_t vectors,
+                      cudaStream_t stream);
+
 // One Q8 projection as a plain bf16 tensor-core GEMM: the table is converted to bf16
 // once into weight_scratch (rows * cols * 2 bytes).  False when the shape or the
 // token count does not suit the path (the caller then uses k3_grouped_q8_bf16).

@@ -392,6 +392,14 @@ extern "C" bool k3_moe_shared_expert(const k3_moe_layer_desc *d, void *out, void
         return false;
     }
     const uint32_t S = d->shared_hidden;
+    if (tokens < 32u && d->shared_gate_q && d->shared_gate_s && d->shared_up_q && d->shared_up_s &&
+        (d->q8_scale_type == K3_MOE_Q8_SCALE_F32 || d->q8_scale_type == K3_MOE_Q8_SCALE_F16) &&
+        k3_q8_few_supported(d->shared_gate_q, x, tokens, d->hidden, d->q8_block) &&
+        k3_q8_few_supported(d->shared_up_q, x, tokens, d->hidden, d->q8_block)) {
+        return k3_q8_few_gateup(d, act, gate, up, x, tokens, (cudaStream_t)stream) &&
+               k3_grouped_q8_bf16(out, d->shared_down_q, d->shared_down_s, act, tokens, d->hidden, S, d->q8_block,
+                                  d->q8_scale_type, stream);
+    }
     return k3_grouped_q8_bf16(gate, d->shared_gate_q, d->shared_gate_s, x, tokens, S, d->hidden,
                               d->q8_block, d->q8_scale_type, stream) &&
            k3_grouped_q8_bf16(up, d->shared_up_q, d->shared_up_s, x, tokens, S, d->hidden,
