@@ -21,7 +21,7 @@
 // are numbered with the row tiles of one (expert, weight tile) adjacent: CTAs that take
 // neighbouring items stream the same weights at the same time and the second reader
 // finds them in L2.  Warps: 0 TMA producer (weights, all block scales), 2 TMA producer
-// (token terms), 1 and 3 MMA issuers (one per weight tile), 4-7
+// (token terms), 1 and 3 MMA issuers (one per weight tile; 1 alone for a tile of more than 64 rows), 4-7
 // scale writers (shared memory -> tensor memory, one lane quadrant each), 8-23
 // epilogue.  All barrier waits are bounded.
 #include "k3_grouped.h"
@@ -155,9 +155,9 @@ struct Item {
 
 // How a row tile's terms lie in shared memory.  Up to 64 rows the hi rows and the lo rows are ONE
 // N operand (lo from row `block` on), so that a K block of 32 is one MMA per weight tile: the
-// 8-bit weight containers are read from shared memory once instead of twice, and shared memory
-// is what bounds short tiles (88 KB per stage of 32 rows instead of 120 KB; 24 rows per
-// expert: 1.15 -> 1.01 ms together with the fourth stage).  A larger tile does not fit its
+// 8-bit weight containers are read from shared memory once instead of twice (24 rows per expert:
+// 1.15 -> 1.01 ms together with the fourth stage; without any MMA 0.98, the TMA unit's expansion
+// of the weights at 16 packed bytes per clock and SM).  A larger tile does not fit its
 // accumulators that way (2 x 256 columns): there the terms are the A operand and both weight
 // tiles together the N = 256 operand, and the hi and the lo MMA add into the same columns.  A K
 // block of 32 then takes two MMAs of N = 256 (92 ns each, 12 KB of operands) where the weights
