@@ -157,22 +157,30 @@ inline int sm_count() {
 }
 
 // cudaFuncAttributeMaxDynamicSharedMemorySize for `kernel` on the current device,
-// remembered per (device, kernel) so that the call is made once each (it costs
-// microseconds of host time).  Requests of 48 KB or less need no attribute.
+// remembered per (device, kernel) so that the calls are made once each (they cost
+// microseconds of host time).  Without the attribute a block has 48 KB for its static and
+// dynamic shared memory together, so the kernel's static part counts against the default.
 inline bool set_max_dynamic_smem(const void *kernel, size_t bytes) {
-    if (bytes <= 48u * 1024u) return true;
     static std::mutex lock;
-    static std::map<std::pair<int, const void *>, size_t> done;
+    static std::map<std::pair<int, const void *>, size_t> limits;
     const int dev = current_device();
     std::lock_guard<std::mutex> guard(lock);
     const auto key = std::make_pair(dev, kernel);
-    auto it = done.find(key);
-    if (it != done.end() && it->second >= bytes) return true;
+    auto it = limits.find(key);
+    if (it == limits.end()) {
+        cudaFuncAttributes attributes{};
+        if (cudaFuncGetAttributes(&attributes, kernel) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        it = limits.emplace(key, 48u * 1024u - attributes.sharedSizeBytes).first;
+    }
+    if (it->second >= bytes) return true;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
-    done[key] = bytes;
+    it->second = bytes;
     return true;
 }
 
