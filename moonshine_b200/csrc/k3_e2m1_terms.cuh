@@ -30,9 +30,9 @@ K3_DEVINL void split_block_e2m1(float value, uint32_t (&code)[kTerms], uint32_t 
         // non-negative floats order like their bit patterns
         const uint32_t mx = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(residual)) & 0x7fffffffu);
         const uint32_t be = (mx >> 23) & 0xffu;               // biased exponent of the largest residual
-        if (be < 4u || be == 0xffu) {                          // nothing (finite) left in this block
+        if (be < 4u || be == 0xffu) {                          // nothing left in this block, or nothing finite
             code[j] = 0u;
-            scale_byte[j] = 127u;
+            scale_byte[j] = be == 0xffu ? 255u : 127u;         // 255: E8M0's NaN, so the results are NaN
             continue;
         }
         const uint32_t sb = be - 2u;                           // largest magnitude / 2^(sb-127) in [4, 8)

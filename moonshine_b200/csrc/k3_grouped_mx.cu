@@ -107,18 +107,22 @@ K3_DEVINL uint32_t make_idesc_mx(uint32_t n, uint32_t sf, bool tokens_are_a) {
 
 // Two-term E4M3 form of a block of 32 values held one per lane:
 // v = 2^(scale_byte - 127) * (hi + lo).  The block exponent puts the largest
-// magnitude in [128, 256), inside E4M3's finite range (448).
+// magnitude in [128, 256), inside E4M3's finite range (448).  The terms saturate, so a block
+// that holds an infinity or NaN gets E8M0's NaN as its scale: its row's results are NaN.
+K3_DEVINL uint32_t block_scale_byte(uint32_t max_exponent) {
+    return max_exponent == 0xffu ? 255u : min(max(max_exponent, 8u), 254u) - 7u;
+}
 struct SplitScale {
     float mult;             // 2^-(block exponent)
     uint32_t scale_byte;    // E8M0
 };
 K3_DEVINL SplitScale block_scale(float v) {
     const uint32_t mx = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(v)));
-    uint32_t be = (mx >> 23) & 0xffu;                 // biased exponent of the block maximum
-    be = min(max(be, 8u), 254u);
+    const uint32_t max_exponent = mx >> 23;           // biased, of the block maximum
+    const uint32_t be = min(max(max_exponent, 8u), 254u);
     SplitScale s;
     s.mult = __uint_as_float((261u - be) << 23);      // 2^(7 - (be - 127))
-    s.scale_byte = be - 7u;
+    s.scale_byte = block_scale_byte(max_exponent);
     return s;
 }
 // (hi0, hi1) in the low 16 bits, (lo0, lo1) in the high 16 bits
@@ -288,7 +292,7 @@ K3_DEVINL void store_row(const GmxArgs &a, uint64_t row, uint32_t c, uint32_t (&
         }
         store_32_bytes(a.act_hi + row * a.w_rows + c, v, true);      // buffers of the workspace: aligned
         store_32_bytes(a.act_lo + row * a.w_rows + c, lo, true);
-        a.act_sf[row * (a.w_rows / 32u) + c / 32u] = (uint8_t)(be - 7u);
+        a.act_sf[row * (a.w_rows / 32u) + c / 32u] = (uint8_t)block_scale_byte(mx >> 7);
     } else {
 #pragma unroll
         for (uint32_t h = 0; h < 4u; h++) {               // tile 0's columns, then tile 1's
@@ -746,7 +750,7 @@ K3_DEVINL SplitColumns split_columns(const uint16_t *p) {
         h[q] = (p0 & 0xffffu) | (p1 << 16);
         l[q] = (p0 >> 16) | (p1 & 0xffff0000u);
     }
-    return {make_uint4(h[0], h[1], h[2], h[3]), make_uint4(l[0], l[1], l[2], l[3]), be - 7u};
+    return {make_uint4(h[0], h[1], h[2], h[3]), make_uint4(l[0], l[1], l[2], l[3]), block_scale_byte(mx >> 7)};
 }
 
 // Product rows' E4M3 terms and block scales from the bf16 source rows (row r reads x[index[r]],
