@@ -145,6 +145,22 @@ bool k3_moe_experts_grouped_ws(const k3_moe_layer_desc *desc, void *rows_out,
                                uint32_t rows, void *workspace,
                                size_t workspace_bytes, void *stream);
 
+/* The same for a part of a larger pass (no counterpart in the reference): the
+ * rows get the bits they have when the whole pass is one call.  The order in
+ * which a row's sums are added depends on how many rows its group has and, above
+ * 64, on its place among them, so a part that is computed by itself differs from
+ * the whole pass in the last bits.  group_rows: u32 [local_expert_count] on the
+ * device, rows of each group in the whole pass; place: u32 [rows], place of each
+ * row in its group there, ascending within a group.  Fails where
+ * k3_moe_experts_workspace_bytes is 0 (fewer than 32 rows, or a shape that does
+ * not suit the path) or the workspace is smaller. */
+bool k3_moe_experts_grouped_part(const k3_moe_layer_desc *desc, void *rows_out,
+                                 void *act, const void *rows_in, const void *index,
+                                 uint32_t source_rows, const void *offsets,
+                                 const void *group_rows, const void *place,
+                                 uint32_t rows, void *workspace,
+                                 size_t workspace_bytes, void *stream);
+
 /* One token whose routing the host brings (the partially resident store plans
  * on the host, k3_engine.cu:1580-1590): ids u32 [top_k] on the device index the
  * descriptor's expert tables (slot numbers for a slot table), weights f32

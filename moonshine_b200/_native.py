@@ -130,6 +130,7 @@ SIGNATURES = {
     "k3_moe_experts_token_workspace_bytes": (sz, [_DP]),
     "k3_moe_experts_token": (C.c_bool, [_DP, vp, vp, vp, vp, vp, sz, vp]),
     "k3_moe_experts_grouped_ws": (C.c_bool, [_DP, vp, vp, vp, vp, u32, vp, u32, vp, sz, vp]),
+    "k3_moe_experts_grouped_part": (C.c_bool, [_DP, vp, vp, vp, vp, u32, vp, vp, vp, u32, vp, sz, vp]),
     "k3_moe_shared_workspace_bytes": (sz, [_DP, u32]),
     "k3_moe_shared_expert_ws": (C.c_bool, [_DP, vp, vp, vp, u32, vp, sz, vp]),
     "k3_moe_shared_expert": (C.c_bool, [_DP, vp, vp, vp, vp, vp, u32, vp]),

@@ -127,15 +127,27 @@ struct k3_token_routes {
     const void *ids;           // u32 [tokens, top_k] expert ids, all of this table
     const void *inv_perm;      // u32 [tokens, top_k] product row of a route
 };
+// pass: the rows of the call are a part of a larger pass and get the bits they have there.
+struct k3_part_of_pass {
+    const void *group_rows;    // u32 [groups] rows of a group in the whole pass
+    const void *place;         // u32 [rows] place of a row in its group there, ascending within a group
+};
 bool k3_grouped_mx_supported(const k3_moe_layer_desc *desc, uint32_t rows);
 size_t k3_grouped_mx_workspace_bytes(const k3_moe_layer_desc *desc, uint32_t rows,
                                      uint32_t source_rows);
 bool k3_grouped_mx_experts(const k3_moe_layer_desc *desc, void *rows_out, void *act,
                            const void *rows_in, const void *index, uint32_t source_rows,
                            const void *offsets, uint32_t rows, void *workspace,
-                           cudaStream_t stream, const k3_token_routes *routes = nullptr);
+                           cudaStream_t stream, const k3_token_routes *routes = nullptr,
+                           const k3_part_of_pass *pass = nullptr);
 uint32_t k3_grouped_mx_status();
 constexpr uint32_t k3_mx4_rows = 16;
+// What decides a group's kernel and operand layout when its rows here are a part of a pass: u32
+// [groups][2], its rows in the whole pass and how many of the rows here lie in the pass's stacked
+// tile (k3_grouped_mx.cu).  A null table: the call is the whole pass.
+struct k3_group_parts {
+    const uint32_t *table;
+};
 // The same for groups of at most k3_mx4_rows rows (k3_grouped_mx4.cu) in three steps; larger groups
 // are left alone.  The first step also zeroes the 64 words at `counters`, from which each
 // product launch takes one.
@@ -144,9 +156,9 @@ bool k3_grouped_mx4_terms(const k3_moe_layer_desc *desc, const void *rows_in, ui
                           const void *ids, const void *offsets, void *workspace, uint32_t *counters, cudaStream_t stream);
 bool k3_grouped_mx4_gateup(const k3_moe_layer_desc *desc, void *act, const void *index, uint32_t source_rows,
                            const void *offsets, uint32_t rows, void *workspace, uint32_t *counter,
-                           cudaStream_t stream);
+                           k3_group_parts parts, cudaStream_t stream);
 bool k3_grouped_mx4_down(const k3_moe_layer_desc *desc, void *rows_out, const void *offsets, uint32_t rows,
                          uint32_t source_rows, void *workspace, uint32_t *counter,
-                         cudaStream_t stream);
+                         k3_group_parts parts, cudaStream_t stream);
 uint32_t k3_grouped_mx4_status();
 bool k3_grouped_mx4_status_clear();

@@ -144,6 +144,7 @@ K3_DEVINL uint32_t pack_bf16x2(float lo, float hi) {
 
 struct GmxArgs {
     const uint32_t *offsets;             // [groups+1]
+    k3_group_parts parts;
     uint16_t *out;                       // bf16 [rows, out_width] (may be null in gate/up mode)
     uint8_t *act_hi, *act_lo, *act_sf;   // gate/up mode: E4M3 terms and block scales of the activation
     uint32_t groups, rows, row_floor, row_ceil, w_rows, k, out_width, m_items;   // groups of row_floor < rows <= row_ceil
@@ -155,7 +156,20 @@ struct GmxArgs {
 
 struct Item {
     uint32_t group, row_start, rows_valid, m_item;
+    bool stacked;
 };
+
+// A group's rows are cut into tiles of BN rows; a last tile of at most 64 rows (kSomeRows) is
+// stacked, which adds a row's sums in another order than the larger tiles do.
+constexpr uint32_t kStackedRows = 64;
+K3_DEVINL uint32_t stacked_rows(uint32_t rows) { return rows % BN <= kStackedRows ? rows % BN : 0u; }
+struct GroupShape {
+    uint32_t whole, stacked;             // rows in the pass, rows here that lie in its stacked tile
+};
+K3_DEVINL GroupShape group_shape(const k3_group_parts &parts, uint32_t group, uint32_t rows) {
+    if (parts.table == nullptr) return {rows, stacked_rows(rows)};
+    return {parts.table[2u * group], parts.table[2u * group + 1u]};
+}
 
 // How a row tile's terms lie in shared memory.  Up to 64 rows the hi rows and the lo rows are ONE
 // N operand (lo from row `block` on), so that a K block of 32 is one MMA per weight tile: the
@@ -173,11 +187,11 @@ struct TermLayout {
     bool stacked;
 };
 template <uint32_t kStages>
-K3_DEVINL TermLayout term_layout(uint32_t rows_valid) {
+K3_DEVINL TermLayout term_layout(const Item &it) {
     TermLayout t;
-    const uint32_t n16 = (rows_valid + 15u) & ~15u;
-    t.block = rows_valid <= 32u ? 32u : kStages > 3u || rows_valid <= 64u ? 64u : BN;
-    t.stacked = t.block < BN;
+    const uint32_t n16 = (it.rows_valid + 15u) & ~15u;
+    t.stacked = kStages > 3u || it.stacked;
+    t.block = !t.stacked ? BN : it.rows_valid <= 32u ? 32u : kStackedRows;
     t.n = t.stacked ? t.block + n16 : 2u * BM;
     return t;
 }
@@ -197,9 +211,11 @@ K3_DEVINL Item decode_item(uint32_t w, const uint32_t *prefix, const GmxArgs &a)
     const uint32_t tiles = prefix[lo + 1u] - prefix[lo];
     const uint32_t j = w - prefix[lo] * a.m_items;
     it.m_item = j / tiles;
-    const uint32_t begin = a.offsets[lo], end = a.offsets[lo + 1u];
-    it.row_start = begin + (j % tiles) * BN;
-    it.rows_valid = min(BN, end - it.row_start);
+    const uint32_t begin = a.offsets[lo], rows = a.offsets[lo + 1u] - begin, tile = j % tiles;
+    const uint32_t stacked = group_shape(a.parts, lo, rows).stacked, large = rows - stacked;
+    it.stacked = tile * BN >= large;
+    it.row_start = begin + (it.stacked ? large : tile * BN);
+    it.rows_valid = it.stacked ? stacked : min(BN, large - tile * BN);
     return it;
 }
 
@@ -212,7 +228,7 @@ struct AccBuffers {
     uint32_t use0 = 0u, use1 = 0u;
     uint32_t turn = 0u;
     __device__ uint32_t uses(uint32_t b) const { return b == 0u ? use0 : use1; }
-    __device__ bool small(uint32_t rows_valid) const { return rows_valid <= 32u; }
+    __device__ bool small(const Item &it) const { return it.stacked && it.rows_valid <= 32u; }
     __device__ uint32_t first(bool is_small) const { return is_small ? turn : 0u; }
     __device__ uint32_t column(bool is_small, uint32_t b0, uint32_t tile) const {
         return is_small ? b0 * 128u + tile * 64u : tile * BN;
@@ -370,7 +386,9 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         for (int j = 0; j < 2; j++) {
             const uint32_t g = threadIdx.x * 2u + j;
             const uint32_t n = g < a.groups ? a.offsets[g + 1u] - a.offsets[g] : 0u;
-            v[j] = n > a.row_floor && n <= a.row_ceil ? (n + BN - 1u) / BN : 0u;
+            const GroupShape shape = n != 0u ? group_shape(a.parts, g, n) : GroupShape{0u, 0u};
+            v[j] = shape.whole > a.row_floor && shape.whole <= a.row_ceil
+                       ? (n - shape.stacked + BN - 1u) / BN + (shape.stacked != 0u ? 1u : 0u) : 0u;
             run += v[j];
             incl[j] = run;
         }
@@ -470,7 +488,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             for (uint32_t w = next_item(); ok && w != kNoItem; w = next_item()) {
                 const Item it = decode_item(w, prefix, a);
                 const uint32_t boxes = (it.rows_valid + kBBox - 1u) / kBBox;
-                const TermLayout t = term_layout<kStages>(it.rows_valid);
+                const TermLayout t = term_layout<kStages>(it);
                 for (uint32_t st = 0; st < steps; st++) {
                     if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag)) { ok = false; break; }
                     const int32_t x = (int32_t)(st * KS);
@@ -502,10 +520,10 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             bool ok = true;
             for (uint32_t w = next_item(); ok && w != kNoItem; w = next_item()) {
                 const Item it = decode_item(w, prefix, a);
-                const TermLayout t = term_layout<kStages>(it.rows_valid);
+                const TermLayout t = term_layout<kStages>(it);
                 const uint32_t idesc = make_idesc_mx(t.n, 0u, !t.stacked);
                 const bool bystander = !t.stacked && q == 1u;
-                const bool small = acc.small(it.rows_valid);
+                const bool small = acc.small(it);
                 const uint32_t b0 = acc.first(small);
                 if (!mbar_wait(&acc_empty[b0], (acc.uses(b0) & 1u) ^ 1u, abort_flag) ||
                     (!small && !mbar_wait(&acc_empty[1], (acc.use1 & 1u) ^ 1u, abort_flag))) {
@@ -566,7 +584,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         for (uint32_t w = __shfl_sync(0xffffffffu, next_item(), 0); ok && w != kNoItem;
              w = __shfl_sync(0xffffffffu, next_item(), 0)) {
             // a stacked operand's lo rows have the scales of its hi rows
-            const uint32_t repeat = term_layout<kStages>(decode_item(w, prefix, a).rows_valid).block / 32u - 1u;
+            const uint32_t repeat = term_layout<kStages>(decode_item(w, prefix, a)).block / 32u - 1u;
             for (uint32_t st = 0; st < steps; st += 4u) {
                 if (!mbar_wait(&sfs_full[ss], ssph, abort_flag)) { ok = false; break; }
                 const unsigned char *src = sf_smem + ss * kSfSlotBytes;
@@ -625,7 +643,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         for (uint32_t w = __shfl_sync(0xffffffffu, next_item(), 0); w != kNoItem;
              w = __shfl_sync(0xffffffffu, next_item(), 0)) {
             const Item it = decode_item(w, prefix, a);
-            const bool small = acc.small(it.rows_valid);
+            const bool small = acc.small(it);
             const uint32_t b0 = acc.first(small);
             if (!mbar_wait(&acc_full[b0], acc.uses(b0) & 1u, abort_flag) ||
                 (!small && !mbar_wait(&acc_full[1], acc.use1 & 1u, abort_flag))) {
@@ -638,7 +656,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             const uint32_t col0 = it.m_item * tile_rows + m;
             const uint32_t col1 = kE == kEAct ? col0 : col0 + BM;
             const bool in0 = col0 < a.w_rows, in1 = col1 < a.w_rows;
-            const TermLayout t = term_layout<kStages>(it.rows_valid);
+            const TermLayout t = term_layout<kStages>(it);
             const uint32_t span = t.block / 4u, c = span * part;         // this warp's token rows
             uint32_t pair[32];                                           // bf16 of tile 0 | tile 1 << 16
 #pragma unroll
@@ -759,7 +777,8 @@ K3_DEVINL SplitColumns split_columns(const uint16_t *p) {
 __global__ void __launch_bounds__(256)
 split_rows_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t *__restrict__ sf,
                   const uint16_t *__restrict__ x, const uint32_t *__restrict__ index,
-                  const uint32_t *__restrict__ offsets, uint32_t groups, uint32_t rows, uint32_t k) {
+                  const uint32_t *__restrict__ offsets, k3_group_parts parts, uint32_t groups, uint32_t rows,
+                  uint32_t k) {
     // launched behind a kernel that waited for the dispatch and shares nothing else with this one
     const uint32_t lane = threadIdx.x % kWarp;
     const uint32_t warps = (gridDim.x * blockDim.x) / kWarp;
@@ -769,7 +788,7 @@ split_rows_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t *_
             const uint32_t mid = (g + end) >> 1;
             if (offsets[mid] <= r) g = mid; else end = mid;
         }
-        if (offsets[g + 1u] - offsets[g] <= k3_mx4_rows) continue;
+        if (group_shape(parts, g, offsets[g + 1u] - offsets[g]).whole <= k3_mx4_rows) continue;
         const uint16_t *src = x + (uint64_t)(index ? index[r] : r) * k;
         for (uint32_t c = lane * 16u; c < k; c += 512u) {
             const SplitColumns t = split_columns(src + c);
@@ -809,6 +828,25 @@ split_tokens_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t 
         }
     }
     pdl_wait();
+}
+
+// One thread per group: the group's line of k3_group_parts.  The places of a group's rows ascend,
+// so its rows in the pass's stacked tile are its last ones.
+__global__ void __launch_bounds__(256)
+group_parts_kernel(uint32_t *table, const uint32_t *group_rows, const uint32_t *place, const uint32_t *offsets,
+                   uint32_t groups) {
+    pdl_wait();
+    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= groups) return;
+    const uint32_t begin = offsets[g], rows = offsets[g + 1u] - begin;
+    const uint32_t whole = max(group_rows[g], rows), large = whole - stacked_rows(whole);
+    uint32_t lo = 0u, hi = rows;                           // first row whose place is in the stacked tile
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (place[begin + mid] < large) lo = mid + 1u; else hi = mid;
+    }
+    table[2u * g] = whole;
+    table[2u * g + 1u] = min(rows - lo, kStackedRows);     // the limit holds for any places
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -908,6 +946,7 @@ struct Scratch {
     uint8_t *x_hi, *x_lo, *x_sf;       // per product row
     uint8_t *a_hi, *a_lo, *a_sf;       // activation, per product row
     uint32_t *counters;                // item counters of the six launches (zeroed per call)
+    uint32_t *parts;                   // k3_group_parts of a call that is a part of a pass
     void *few;                         // scratch of the kernel for few rows per group
     size_t total;
 };
@@ -929,6 +968,7 @@ Scratch carve_scratch(const k3_moe_layer_desc *d, uint32_t rows, uint32_t source
     s.a_lo = take(R * I);
     s.a_sf = take(R * (I / 32u));
     s.counters = (uint32_t *)take(256);
+    s.parts = (uint32_t *)take(2u * sizeof(uint32_t) * d->local_expert_count);
     s.few = take(k3_grouped_mx4_workspace_bytes(d, rows, source_rows ? source_rows : rows));
     s.total = off + 256u;
     return s;
@@ -968,20 +1008,31 @@ bool k3_grouped_mx_supported(const k3_moe_layer_desc *d, uint32_t rows) {
 //   packed                 0.70  0.73  0.81  1.28  1.38  1.94
 //   two-term, four stages  0.97  0.99  1.00  1.01  1.03  1.21  1.28
 //   two-term, three        1.10        1.14  1.15  1.17  1.27  1.37  1.70  1.95
-constexpr uint32_t kFewRows = k3_mx4_rows, kSomeRows = 64;
+constexpr uint32_t kFewRows = k3_mx4_rows, kSomeRows = kStackedRows;
 
 // rows_in bf16 [source_rows, H]; product row r reads rows_in[index[r]] (or row r
 // when index == nullptr, source_rows == 0).  `act` bf16 [rows, I] is written when
 // not null; rows_out bf16 [rows, H].
+//
+// A group's kernel and, above 64 rows, the tile a row lies in decide the order in which the row's
+// sums are added.  A caller that cuts a pass into parts and wants the pass's bits says with `pass`
+// what the groups are in the whole pass.
 bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act, const void *rows_in,
                            const void *index, uint32_t source_rows, const void *offsets, uint32_t rows,
-                           void *workspace, cudaStream_t stream, const k3_token_routes *routes) {
+                           void *workspace, cudaStream_t stream, const k3_token_routes *routes,
+                           const k3_part_of_pass *pass) {
     // a token selects an expert at most once, so no group has more rows than there are tokens
     const uint32_t max_group_rows = routes ? source_rows : 0xffffffffu;
     const uint32_t H = d->hidden, I = d->expert_hidden;
     const Scratch s = carve_scratch(d, rows, index ? source_rows : 0u, workspace);
     const uint32_t conv_rows = index ? source_rows : rows;
     const bool few = max_group_rows > kFewRows, many = max_group_rows > kSomeRows;   // launches beyond the packed one
+    const k3_group_parts parts{pass ? s.parts : nullptr};
+    if (pass && !launch_chained(group_parts_kernel, (d->local_expert_count + 255u) / 256u, 256, 0, stream, s.parts,
+                                (const uint32_t *)pass->group_rows, (const uint32_t *)pass->place,
+                                (const uint32_t *)offsets, d->local_expert_count)) {
+        return false;
+    }
     if (!k3_grouped_mx4_terms(d, rows_in, conv_rows, rows, routes ? routes->ids : nullptr, offsets, s.few, s.counters,
                               stream)) {
         return false;
@@ -996,12 +1047,13 @@ bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act
         }
     } else if (few && !launch_chained(split_rows_kernel, std::min<uint32_t>((rows + 7u) / 8u, (uint32_t)sm_count() * 16u),
                                       256, 0, stream, s.x_hi, s.x_lo, s.x_sf, (const uint16_t *)rows_in,
-                                      (const uint32_t *)index, (const uint32_t *)offsets, d->local_expert_count, rows,
-                                      H)) {
+                                      (const uint32_t *)index, (const uint32_t *)offsets, parts, d->local_expert_count,
+                                      rows, H)) {
         return false;
     }
     GmxArgs a{};
     a.offsets = (const uint32_t *)offsets;
+    a.parts = parts;
     a.groups = d->local_expert_count;
     a.rows = rows;
     a.activation = d->activation;
@@ -1030,7 +1082,7 @@ bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act
     a.out_width = I;
     a.m_items = (I + BM - 1u) / BM;
     const Operands gu{d->w1_packed, d->w3_packed, d->w1_scales, d->w3_scales, s.x_hi, s.x_lo, s.x_sf};
-    if (!k3_grouped_mx4_gateup(d, act, index, conv_rows, offsets, rows, s.few, s.counters, stream) ||
+    if (!k3_grouped_mx4_gateup(d, act, index, conv_rows, offsets, rows, s.few, s.counters, parts, stream) ||
         !launches(std::integral_constant<int, kEAct>{}, gu, s.counters + 8)) {
         return false;
     }
@@ -1042,6 +1094,6 @@ bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act
     a.out_width = H;
     a.m_items = (H + 2u * BM - 1u) / (2u * BM);
     const Operands dn{d->w2_packed, d->w2_packed, d->w2_scales, d->w2_scales, s.a_hi, s.a_lo, s.a_sf};
-    return k3_grouped_mx4_down(d, rows_out, offsets, rows, conv_rows, s.few, s.counters + 24, stream) &&
+    return k3_grouped_mx4_down(d, rows_out, offsets, rows, conv_rows, s.few, s.counters + 24, parts, stream) &&
            launches(std::integral_constant<int, kEBf16>{}, dn, s.counters + 32);
 }

@@ -121,6 +121,7 @@ K3_DEVINL float sum8(const uint32_t *r) {
 
 struct Mx4Args {
     const uint32_t *offsets;             // [groups+1]
+    k3_group_parts parts;
     const uint32_t *index;               // term row block of product row r (null: r itself)
     const uint8_t *sfb;                  // term scales [term rows, K/32]
     uint16_t *out;                       // bf16 [rows, out_width] (may be null in gate/up mode)
@@ -245,7 +246,8 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
         for (int j = 0; j < 2; j++) {
             const uint32_t g = threadIdx.x * 2u + j;
             const uint32_t n = g < a.groups ? a.offsets[g + 1u] - a.offsets[g] : 0u;
-            v[j] = n != 0u && n <= kTileRows ? 1u : 0u;
+            const uint32_t whole = a.parts.table != nullptr && g < a.groups ? a.parts.table[2u * g] : n;
+            v[j] = n != 0u && whole <= kTileRows ? 1u : 0u;
             run += v[j];
             incl[j] = run;
         }
@@ -806,10 +808,11 @@ bool k3_grouped_mx4_terms(const k3_moe_layer_desc *d, const void *rows_in, uint3
 
 bool k3_grouped_mx4_gateup(const k3_moe_layer_desc *d, void *act, const void *index, uint32_t source_rows,
                            const void *offsets, uint32_t rows, void *workspace, uint32_t *counter,
-                           cudaStream_t stream) {
+                           k3_group_parts parts, cudaStream_t stream) {
     const Scratch s = carve_scratch(d, rows, source_rows, workspace);
     Mx4Args a{};
     a.offsets = (const uint32_t *)offsets;
+    a.parts = parts;
     a.index = (const uint32_t *)index;
     a.groups = d->local_expert_count;
     a.activation = d->activation;
@@ -830,10 +833,11 @@ bool k3_grouped_mx4_gateup(const k3_moe_layer_desc *d, void *act, const void *in
 
 bool k3_grouped_mx4_down(const k3_moe_layer_desc *d, void *rows_out, const void *offsets, uint32_t rows,
                          uint32_t source_rows, void *workspace, uint32_t *counter,
-                         cudaStream_t stream) {
+                         k3_group_parts parts, cudaStream_t stream) {
     const Scratch s = carve_scratch(d, rows, source_rows, workspace);
     Mx4Args a{};
     a.offsets = (const uint32_t *)offsets;
+    a.parts = parts;
     a.groups = d->local_expert_count;
     a.item_counter = counter;
     a.out = (uint16_t *)rows_out;

@@ -385,6 +385,21 @@ extern "C" bool k3_moe_experts_grouped_ws(const k3_moe_layer_desc *d, void *rows
     return k3_moe_experts_grouped(d, rows_out, act, rows_in, offsets, rows, stream);
 }
 
+extern "C" bool k3_moe_experts_grouped_part(const k3_moe_layer_desc *d, void *rows_out, void *act,
+                                            const void *rows_in, const void *index, uint32_t source_rows,
+                                            const void *offsets, const void *group_rows, const void *place,
+                                            uint32_t rows, void *workspace, size_t workspace_bytes, void *stream) {
+    if (!desc_ok(d) || !rows_out || !rows_in || !offsets || !group_rows || !place || rows == 0 ||
+        !slot_pointers_aligned(d) || (index != nullptr && source_rows == 0) || !workspace) {
+        return false;
+    }
+    const size_t need = k3_moe_experts_workspace_bytes(d, rows, index ? source_rows : 0u);
+    if (need == 0 || workspace_bytes < need) return false;
+    const k3_part_of_pass pass{group_rows, place};
+    return k3_grouped_mx_experts(d, rows_out, act, rows_in, index, source_rows, offsets, rows, workspace,
+                                 (cudaStream_t)stream, nullptr, &pass);
+}
+
 extern "C" bool k3_moe_shared_expert(const k3_moe_layer_desc *d, void *out, void *gate, void *up,
                                      void *act, const void *x, uint32_t tokens, void *stream) {
     if (!desc_ok(d) || d->shared_hidden == 0 || !out || !gate || !up || !act || !x ||

@@ -106,8 +106,12 @@ class NativeBackend:
             raise RuntimeError("k3_rocm_gather_rows_bf16 failed")
         return out
 
-    def experts(self, rows, offsets_local, index):
-        """Expert products of rows[index] (grouped by local expert as offsets_local says)."""
+    takes_parts = True
+
+    def experts(self, rows, offsets_local, index, whole=None):
+        """Expert products of rows[index] (grouped by local expert as offsets_local says).
+        ``whole`` = (group_rows, place) of ``k3_moe_experts_grouped_part`` when the rows are a
+        part of a pass."""
         n, d, i = index.numel(), self.cfg["hidden"], self.cfg["expert_hidden"]
         out = self._buf("eo", (n, d), rows.dtype)
         act = self._buf("ea", (n, i), rows.dtype)
@@ -117,8 +121,12 @@ class NativeBackend:
         need = ops.k3_moe_experts_workspace_bytes(self.layer.desc, n, rows.shape[0])
         if need:
             ws = self._buf("ews", (need,), torch.uint8)
-            ok = ops.k3_moe_experts_grouped_ws(self.layer.desc, out, None, rows, index, rows.shape[0],
-                                               offsets_local, n, ws, need)
+            if whole is None:
+                ok = ops.k3_moe_experts_grouped_ws(self.layer.desc, out, None, rows, index, rows.shape[0],
+                                                   offsets_local, n, ws, need)
+            else:
+                ok = ops.k3_moe_experts_grouped_part(self.layer.desc, out, None, rows, index, rows.shape[0],
+                                                     offsets_local, *whole, n, ws, need)
         else:
             ok = ops.k3_moe_experts_grouped(self.layer.desc, out, act, self.gather(rows, index, "rows_in"),
                                             offsets_local, n)
@@ -170,6 +178,19 @@ def exchange_plan(all_counts: torch.Tensor, rank: int, first: int, per: int):
     return send, recv, starts, lengths, offsets_local
 
 
+def part_of_pass(counts, piece: int, first: int, per: int):
+    """Where one piece's received rows lie in the whole pass.  ``counts``: per piece the
+    [world, E] matrix of rows each rank routes to each expert (host tensors).  The whole
+    pass groups its rows by (expert asc, source asc, piece asc, route asc).  Returns the
+    rows of each local expert in the whole pass [per] and, per (expert, source) block of
+    this piece, the place of its first row in the expert's group [per * world]."""
+    mine = torch.stack([c[:, first:first + per] for c in counts])    # [piece, source, local expert]
+    blocks = mine.transpose(0, 1).reshape(-1, per)                   # (source asc, piece asc)
+    before = torch.cumsum(blocks, 0) - blocks
+    places = before.reshape(mine.shape[1], mine.shape[0], per)[:, piece]         # [source, local expert]
+    return blocks.sum(dim=0), places.t().reshape(-1)
+
+
 def rows_once_per_destination(world: int, top_k: int) -> bool:
     """Whether a pass sends each token row once per destination (plus a slot index per
     route) instead of once per route.  A token's top_k routes reach about
@@ -180,11 +201,15 @@ def rows_once_per_destination(world: int, top_k: int) -> bool:
     return 3.0 * distinct <= top_k
 
 
-def _ep_steps(backend, x, cfg: dict, group, once_per_destination=None):
+def _ep_steps(backend, x, cfg: dict, group, once_per_destination=None, pieces=None, piece=0):
     """One expert-parallel pass for the rows ``x`` as a generator: it yields after
     every point where the host has queued all it can without waiting, so that a
     driver can advance another pass (on another stream) in the meantime.  The
-    value of the generator (StopIteration.value) is (out, ids, weights)."""
+    value of the generator (StopIteration.value) is (out, ids, weights).
+
+    ``pieces``: a list with a place for each pass that is one piece of a larger one
+    (``piece`` is this one's index).  Every piece leaves its counts there before its first
+    yield, so with the pieces in lock step all of them are there after it."""
     world = dist.get_world_size(group)
     rank = dist.get_rank(group)
     e, k = cfg["experts"], cfg["top_k"]
@@ -227,6 +252,8 @@ def _ep_steps(backend, x, cfg: dict, group, once_per_destination=None):
             dist.all_gather(gathered, counts, group=group)
             pinned.copy_(torch.stack(gathered), non_blocking=True)
             done.record(side)
+        if pieces is not None:
+            pieces[piece] = (done, pinned)
         shared = backend.shared(x)
         # every (destination, token) candidate row is gathered before the host knows how
         # many are members (members come first): the copy of the few surplus rows costs
@@ -239,6 +266,8 @@ def _ep_steps(backend, x, cfg: dict, group, once_per_destination=None):
         gathered = [torch.empty_like(counts) for _ in range(world)]
         dist.all_gather(gathered, counts, group=group)
         all_counts = torch.stack(gathered).cpu()
+        if pieces is not None:
+            pieces[piece] = (None, all_counts)
         shared = backend.shared(x)
         rows_send = backend.gather(x, token_of_unique, "rows_send")
         yield
@@ -246,6 +275,12 @@ def _ep_steps(backend, x, cfg: dict, group, once_per_destination=None):
     send_unique = [int(v) for v in all_counts[rank, e:]] if dedup else send
     recv_unique = [int(v) for v in all_counts[:, e + rank]] if dedup else recv
     n_recv, n_unique = sum(recv), sum(recv_unique)
+    whole = None
+    if pieces is not None and getattr(backend, "takes_parts", False):
+        for counted, _ in pieces:
+            if counted is not None:
+                counted.synchronize()
+        group_rows, block_place = part_of_pass([c[:, :e] for _, c in pieces], piece, first, per)
 
     rows_send = rows_send[:sum(send_unique)]
     rows_recv = torch.empty((n_unique, x.shape[1]), dtype=x.dtype, device=dev)
@@ -271,6 +306,11 @@ def _ep_steps(backend, x, cfg: dict, group, once_per_destination=None):
                  + torch.arange(n_recv, device=dev)).to(torch.int32)
         inverse = torch.empty_like(order)
         inverse[order.long()] = torch.arange(n_recv, device=dev, dtype=torch.int32)
+        if pieces is not None and getattr(backend, "takes_parts", False):
+            passed = torch.cat([group_rows, block_place]).to(dev)
+            place = (torch.repeat_interleave(passed[per:] - dest_base, lengths_d, output_size=n_recv)
+                     + torch.arange(n_recv, device=dev)).to(torch.int32)
+            whole = (passed[:per].to(torch.int32), place)
         # first received row of each source, repeated for each of its routes
         if dedup:
             base_of_route = torch.repeat_interleave(base_of_source, recv_d, output_size=n_recv)
@@ -281,7 +321,8 @@ def _ep_steps(backend, x, cfg: dict, group, once_per_destination=None):
     if n_recv:
         # grouped position -> received route (-> row of its token among the received rows)
         row_of_route = (base_of_route + slots_recv.long())[order.long()].to(torch.int32) if dedup else order
-        rows_out = backend.experts(rows_recv, offsets_d, row_of_route)
+        rows_out = (backend.experts(rows_recv, offsets_d, row_of_route) if whole is None
+                    else backend.experts(rows_recv, offsets_d, row_of_route, whole))
         rows_back = backend.gather(rows_out, inverse, "rows_back")   # received order again
     else:
         rows_back = torch.empty((0, x.shape[1]), dtype=x.dtype, device=dev)
@@ -319,14 +360,19 @@ def ep_forward_pipelined(backends, x, cfg: dict, group=None, streams=None):
     advance in lock step, each with a backend (scratch buffers) of its own and, on
     a GPU, a stream of its own: while one piece's rows cross the links, another
     piece's kernels run.  Every rank must use the same number of pieces (the
-    collectives pair up in issue order).  Rows are independent in every kernel of
-    the pass, so the result equals ``ep_forward`` bit for bit."""
+    collectives pair up in issue order).  An expert's kernel, and with it the order of a
+    row's sums, depends on how many rows the expert has; the pieces take it from the whole
+    pass, so the result equals ``ep_forward`` bit for bit as long as every piece has at
+    least 32 rows of its own and 32 rows arrive for it on every rank (fewer take the
+    kernels for few rows, in the whole pass as well)."""
     pieces = len(backends)
     t = x.shape[0]
     bounds = [t * p // pieces for p in range(pieces + 1)]
     parts = [x[bounds[p]:bounds[p + 1]] for p in range(pieces)]
+    counts = [None] * pieces
     if not x.is_cuda:
-        results = _drive([_ep_steps(b, part, cfg, group) for b, part in zip(backends, parts)])
+        results = _drive([_ep_steps(b, part, cfg, group, None, counts, p)
+                          for p, (b, part) in enumerate(zip(backends, parts))])
     else:
         main = torch.cuda.current_stream(x.device)
 
@@ -342,8 +388,8 @@ def ep_forward_pipelined(backends, x, cfg: dict, group=None, streams=None):
 
         for s in streams:
             s.wait_stream(main)
-        results = _drive([on_stream(_ep_steps(b, part, cfg, group), s)
-                          for b, part, s in zip(backends, parts, streams)])
+        results = _drive([on_stream(_ep_steps(b, part, cfg, group, None, counts, p), s)
+                          for p, (b, part, s) in enumerate(zip(backends, parts, streams))])
         for s, r in zip(streams, results):
             main.wait_stream(s)
             for tensor in r:
