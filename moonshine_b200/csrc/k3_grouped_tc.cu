@@ -688,7 +688,7 @@ bool k3_grouped_q8_bf16(void *out, const void *q, const void *scales, const void
         a.q8_scale_f16 = scale_type;
         return launch_tc<kAQ8, kEBf16>(q, q, a, x, (cudaStream_t)stream);
     }
-    if (tokens >= 2u && out && q && scales && x && rows != 0u && (scale_type == 0 || scale_type == 1) &&
+    if (out && q && scales && x && rows != 0u && (scale_type == 0 || scale_type == 1) &&
         k3_q8_few_supported(q, x, tokens, cols, block)) {
         return k3_q8_few_product(out, q, scales, x, tokens, rows, cols, block, scale_type, (cudaStream_t)stream);
     }

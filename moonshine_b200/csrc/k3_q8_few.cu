@@ -10,15 +10,15 @@
 // step applies the scale - the arithmetic of the one-token kernels.  That rounds less than the
 // exact-order kernel, which rounds every scaled weight.
 //
-// A block takes 16 weight rows; its warps share the columns step by step (8 or 16 splits, added in
-// ascending order).  Gate and up go together: half of the warps each, and the block applies the
-// activation (one launch instead of three).  A block's table rows are requested into L2 before
-// the wait for the kernel in front.  Tables from HBM, 5 / 24 / 31 rows: 2048 x 7168 9.6 / 14.6 /
-// 15.5 us (exact order 15.3 / 40 / 50), 7168 x 2048 8.3 / 13.0 / 13.8 (20 / 56 / 73), 7168 x 3584
-// 11.9 / 17.0 / 19.2 (30 / 83 / 109).  One row is the exact-order kernel's (6.8 to 12.7 us against
-// 8.1 to 11.9) except for the pair.  Against 64-bit results the error is that of the final
-// rounding to bf16, as in the exact-order kernel: rel-L2 equal to six digits, and as many results
-// on the wrong side of a rounding line (one in 5000).
+// A block takes 16 weight rows; its warps share the columns step by step (8 splits, 16 from 4096
+// columns on, added in ascending order).  The splits do not depend on the number of rows: a row has
+// the same bits in any batch of 1 to 31.  Gate and up go together: half of the warps each, and the
+// block applies the activation (one launch instead of three).  A block's table rows are requested
+// into L2 before the wait for the kernel in front.  Tables from HBM: 2048 x 7168 with 5 / 24 / 31
+// rows 9.6 / 14.6 / 15.5 us (exact order 15.3 / 40 / 50), 7168 x 2048 8.3 / 13.0 / 13.8 (20 / 56 /
+// 73), 7168 x 3584 11.9 / 17.0 / 19.2 (30 / 83 / 109); one row 8.1 to 11.9 (6.8 to 12.7).  Against
+// 64-bit results the error is that of the final rounding to bf16, as in the exact-order kernel:
+// rel-L2 equal to six digits, and as many results on the wrong side of a rounding line (one in 5000).
 #include "k3_grouped.h"
 #include "k3_mxfp4_rows.cuh"
 
@@ -57,8 +57,10 @@ K3_DEVINL void int8_to_bf16(uint2 w, uint32_t (&out)[4]) {
     out[3] = int8_pair_to_bf16(w.y, 0x4342u);
 }
 
-// kTiles tiles of eight token rows; kDeep column steps' loads in flight; kSplits warps per table.
-template <int kTiles, bool kPair, int kSplits, int kDeep>
+// kTiles tiles of eight token rows; kDeep column steps' loads in flight; kSplits warps per table,
+// each with kTurns of the kSplits * kTurns splits (step s belongs to split s mod that), so that a
+// row's sum has the same order whatever the number of warps.
+template <int kTiles, bool kPair, uint32_t kSplits, uint32_t kDeep, uint32_t kTurns>
 __global__ void __launch_bounds__(32 * kSplits * (kPair ? 2 : 1))
 q8_few_kernel(Q8FewArgs a) {
     constexpr uint32_t kTables = kPair ? 2u : 1u;
@@ -82,50 +84,66 @@ q8_few_kernel(Q8FewArgs a) {
 #pragma unroll
     for (int n = 0; n < kTiles; n++)
         x[n] = a.x + (uint64_t)min(8u * n + g, a.vectors - 1u) * a.columns + 8u * t;
-    float acc[kTiles][4];
+    // the splits' sums in ascending order: first turn of every warp, then the second
+    constexpr uint32_t kThreads = 32u * kSplits * kTables, kMine = (kTiles * 8u * kRows + kThreads - 1u) / kThreads;
+    constexpr uint32_t kAll = kSplits * kTurns;
+    float sums[kMine][kTables];
 #pragma unroll
-    for (int n = 0; n < kTiles; n++)
+    for (uint32_t turn = 0; turn < kTurns; turn++) {
+        float acc[kTiles][4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) acc[n][i] = 0.f;
-    for (uint32_t first = split; first < steps; first += (uint32_t)(kSplits * kDeep)) {
-        uint2 wa[kDeep], wb[kDeep];
-        float fa[kDeep], fb[kDeep];
-        uint4 xq[kDeep][kTiles];
+        for (int n = 0; n < kTiles; n++)
 #pragma unroll
-        for (int j = 0; j < kDeep; j++) {
-            const uint32_t step = first + kSplits * j, c = 32u * step;
-            if (step >= steps) break;                                          // uniform across the warp
-            wa[j] = *reinterpret_cast<const uint2 *>(qa + c);
-            wb[j] = *reinterpret_cast<const uint2 *>(qb + c);
-            const uint32_t at = a.per_block == 1u ? step : __umulhi(step, a.reciprocal);
-            fa[j] = scale(sa + at);
-            fb[j] = scale(sb + at);
+            for (int i = 0; i < 4; i++) acc[n][i] = 0.f;
+        for (uint32_t first = split + turn * kSplits; first < steps; first += kAll * kDeep) {
+            uint2 wa[kDeep], wb[kDeep];
+            float fa[kDeep], fb[kDeep];
+            uint4 xq[kDeep][kTiles];
 #pragma unroll
-            for (int n = 0; n < kTiles; n++) xq[j][n] = *reinterpret_cast<const uint4 *>(x[n] + c);
+            for (uint32_t j = 0; j < kDeep; j++) {
+                const uint32_t step = first + kAll * j, c = 32u * step;
+                if (step >= steps) break;                                      // uniform across the warp
+                wa[j] = *reinterpret_cast<const uint2 *>(qa + c);
+                wb[j] = *reinterpret_cast<const uint2 *>(qb + c);
+                const uint32_t at = a.per_block == 1u ? step : __umulhi(step, a.reciprocal);
+                fa[j] = scale(sa + at);
+                fb[j] = scale(sb + at);
+#pragma unroll
+                for (int n = 0; n < kTiles; n++) xq[j][n] = *reinterpret_cast<const uint4 *>(x[n] + c);
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < kDeep; j++) {
+                if (first + kAll * j >= steps) break;
+                uint32_t va[4], vb[4];
+                int8_to_bf16(wa[j], va);
+                int8_to_bf16(wb[j], vb);
+#pragma unroll
+                for (int n = 0; n < kTiles; n++) mx_group(acc[n], va, vb, xq[j][n], fa[j], fb[j]);
+            }
         }
+        if (turn + 1u == kTurns) pdl_trigger();
+        if (turn != 0u) __syncthreads();
 #pragma unroll
-        for (int j = 0; j < kDeep; j++) {
-            if (first + kSplits * j >= steps) break;
-            uint32_t va[4], vb[4];
-            int8_to_bf16(wa[j], va);
-            int8_to_bf16(wb[j], vb);
+        for (int n = 0; n < kTiles; n++) mx_put(&red[warp][8 * n][0], acc[n]);
+        __syncthreads();
 #pragma unroll
-            for (int n = 0; n < kTiles; n++) mx_group(acc[n], va, vb, xq[j][n], fa[j], fb[j]);
+        for (uint32_t j = 0; j < kMine; j++) {
+            const uint32_t i = threadIdx.x + j * kThreads, r = i % kRows, v = i / kRows;
+            if (i >= kTiles * 8u * kRows) break;
+#pragma unroll
+            for (uint32_t m = 0; m < kTables; m++) {
+                float sum = turn != 0u ? sums[j][m] : red[m * kSplits][v][r];
+#pragma unroll
+                for (uint32_t s = turn != 0u ? 0u : 1u; s < kSplits; s++) sum += red[m * kSplits + s][v][r];
+                sums[j][m] = sum;
+            }
         }
     }
-    pdl_trigger();
 #pragma unroll
-    for (int n = 0; n < kTiles; n++) mx_put(&red[warp][8 * n][0], acc[n]);
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < kTiles * 8u * kRows; i += blockDim.x) {
-        const uint32_t r = i % kRows, v = i / kRows;
-        float sum[kTables];
-#pragma unroll
-        for (uint32_t m = 0; m < kTables; m++) {
-            sum[m] = red[m * kSplits][v][r];
-#pragma unroll
-            for (uint32_t s = 1; s < kSplits; s++) sum[m] += red[m * kSplits + s][v][r];
-        }
+    for (uint32_t j = 0; j < kMine; j++) {
+        const uint32_t i = threadIdx.x + j * kThreads, r = i % kRows, v = i / kRows;
+        if (i >= kTiles * 8u * kRows) break;
+        const float(&sum)[kTables] = sums[j];
         if (row0 + r >= a.rows || v >= a.vectors) continue;
         const uint64_t at = (uint64_t)v * a.rows + row0 + r;
         uint16_t bits = float_to_bf16_bits(sum[0]);
@@ -154,11 +172,15 @@ bool launch(const Q8FewArgs &a, cudaStream_t stream) {
     // from 9 rows on eight splits of four (25 and more rows: three) steps are best or within 1 us
     // nearly everywhere (7168 x 2048 with 24 rows: 10.9 with four splits, 13.0).
     const bool deep = a.columns >= 4096u;
+    // A row's order of sums must not depend on the rows beside it, so where up to 8 rows take sixteen
+    // warps, more rows take sixteen splits as well, two per warp one after the other (sixteen warps would
+    // run out of registers).  Shared expert of 7168 x 2048, all three products: 9 / 16 / 24 / 31 rows
+    // 32.4 / 33.4 / 37.0 / 39.8 us; with eight splits there 31.7 / 32.8 / 36.6 / 37.5.
     const uint32_t warps = (tiles == 1u && deep ? 16u : 8u) * (kPair ? 2u : 1u);
-    auto kernel = tiles == 1u   ? (deep ? q8_few_kernel<1, kPair, 16, 2> : q8_few_kernel<1, kPair, 8, 2>)
-                  : tiles == 2u ? q8_few_kernel<2, kPair, 8, 4>
-                  : tiles == 3u ? q8_few_kernel<3, kPair, 8, 4>
-                                : q8_few_kernel<4, kPair, 8, 3>;
+    auto kernel = tiles == 1u   ? (deep ? q8_few_kernel<1, kPair, 16, 2, 1> : q8_few_kernel<1, kPair, 8, 2, 1>)
+                  : tiles == 2u ? (deep ? q8_few_kernel<2, kPair, 8, 4, 2> : q8_few_kernel<2, kPair, 8, 4, 1>)
+                  : tiles == 3u ? (deep ? q8_few_kernel<3, kPair, 8, 4, 2> : q8_few_kernel<3, kPair, 8, 4, 1>)
+                                : (deep ? q8_few_kernel<4, kPair, 8, 2, 2> : q8_few_kernel<4, kPair, 8, 3, 1>);
     return launch_chained(kernel, (a.rows + kRows - 1u) / kRows, 32u * warps, 0, stream, a);
 }
 
