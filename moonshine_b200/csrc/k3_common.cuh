@@ -91,8 +91,10 @@ K3_DEVINL uint2 ld_stream_8(const void *p) {
 // has called pdl_trigger() or left, set themselves up and then wait in pdl_wait() until
 // everything in front has completed and its memory is visible.  Nothing may be read or written
 // before that wait; the one thing that may go first is a prefetch into L2 (prefetch_l2), which
-// is coherent.  This takes the launch latency and the drain of the kernel in front off a chain
-// of short kernels: a 3072 x 3584 MXFP4 row product in such a chain went from 8.2 to 5.1 us.
+// is coherent.  Inputs are read with ordinary loads (no __ldg, no const __restrict__): read-only
+// loads want the data unchanged from the kernel's start on, and the wait does not order them.
+// This takes the launch latency and the drain of the kernel in front off a chain of short
+// kernels: a 3072 x 3584 MXFP4 row product in such a chain went from 8.2 to 5.1 us.
 // The trigger belongs behind a block's loads: called at its start, the blocks of the next two
 // or three kernels crowd the SMs and the same product takes 10.3 us.
 K3_DEVINL void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

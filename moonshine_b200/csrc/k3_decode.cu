@@ -422,7 +422,7 @@ decode_router_kernel(DecodeArgs a) {
 // The token's E2M1 terms alone (and the expert kernel's control words cleared), for a
 // caller that brings its own routing: 32-column blocks, one per warp.
 __global__ void __launch_bounds__(256)
-decode_terms_kernel(const uint16_t *__restrict__ x, uint8_t *x_terms, uint8_t *x_sf, uint32_t *control,
+decode_terms_kernel(const uint16_t *x, uint8_t *x_terms, uint8_t *x_sf, uint32_t *control,
                     uint32_t hidden) {
     pdl_wait();
     const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;

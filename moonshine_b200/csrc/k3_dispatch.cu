@@ -26,7 +26,7 @@ constexpr uint32_t kMaxExperts = 1024;
 __device__ uint32_t g_dispatch_status = 0;
 
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-route_hist_kernel(uint32_t *__restrict__ hist, const uint32_t *__restrict__ ids,
+route_hist_kernel(uint32_t *__restrict__ hist, const uint32_t *ids,
                   uint32_t routes, uint32_t experts, uint32_t chunks) {
     pdl_wait();
     extern __shared__ uint32_t smem_hist[];   // [kWarpsPerBlock][experts]
@@ -60,7 +60,7 @@ constexpr uint32_t kSmallWarps = 32;
 __global__ void __launch_bounds__(kSmallWarps * 32)
 route_small_kernel(uint32_t *__restrict__ offsets, uint32_t *__restrict__ sorted_route,
                    uint32_t *__restrict__ sorted_token, uint32_t *__restrict__ inv_perm,
-                   const uint32_t *__restrict__ ids, uint32_t routes, uint32_t experts, uint32_t top_k) {
+                   const uint32_t *ids, uint32_t routes, uint32_t experts, uint32_t top_k) {
     extern __shared__ uint16_t small_counts[];             // [kSmallWarps][experts], then cursors
     __shared__ uint32_t warp_sums[kSmallWarps];
     const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
@@ -190,8 +190,8 @@ route_scan_kernel(uint32_t *__restrict__ hist, uint32_t *__restrict__ offsets,
 
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 route_place_kernel(uint32_t *__restrict__ sorted_route, uint32_t *__restrict__ sorted_token,
-                   uint32_t *__restrict__ inv_perm, const uint32_t *__restrict__ hist,
-                   const uint32_t *__restrict__ offsets, const uint32_t *__restrict__ ids,
+                   uint32_t *__restrict__ inv_perm, const uint32_t *hist,
+                   const uint32_t *offsets, const uint32_t *ids,
                    uint32_t routes, uint32_t experts, uint32_t chunks, uint32_t top_k) {
     pdl_wait();
     extern __shared__ uint32_t smem_cursor[];   // [kWarpsPerBlock][experts]

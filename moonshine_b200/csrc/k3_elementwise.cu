@@ -23,8 +23,8 @@ inline uint32_t grid_for(uint64_t items, uint32_t per_block) {
 
 // ---------------------------------------------------------------- activation
 __global__ void __launch_bounds__(kThreads)
-activation_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ gate,
-                  const uint16_t *__restrict__ up, uint64_t count, int kind, float beta,
+activation_kernel(uint16_t *__restrict__ out, const uint16_t *gate,
+                  const uint16_t *up, uint64_t count, int kind, float beta,
                   float linear_beta) {
     pdl_wait();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -66,7 +66,7 @@ activation_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ gate,
 // The same for a row or a few: two elements per thread, so that a row of 3072 spreads over a
 // dozen blocks instead of queueing eight expf / tanhf chains in each of 384 threads.
 __global__ void __launch_bounds__(128)
-activation_pairs_kernel(uint32_t *__restrict__ out, const uint32_t *__restrict__ gate, const uint32_t *__restrict__ up,
+activation_pairs_kernel(uint32_t *__restrict__ out, const uint32_t *gate, const uint32_t *up,
                         uint32_t pairs, int kind, float beta, float linear_beta) {
     pdl_wait();
     const uint32_t i = blockIdx.x * 128u + threadIdx.x;
@@ -79,8 +79,8 @@ activation_pairs_kernel(uint32_t *__restrict__ out, const uint32_t *__restrict__
 
 // ----------------------------------------------------------------------- add
 __global__ void __launch_bounds__(kThreads)
-add_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ a,
-           const uint16_t *__restrict__ b, uint64_t count) {
+add_kernel(uint16_t *__restrict__ out, const uint16_t *a,
+           const uint16_t *b, uint64_t count) {
     pdl_wait();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -112,8 +112,8 @@ add_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ a,
 // ------------------------------------------------------------ gather/scatter
 template <bool Scatter>
 __global__ void __launch_bounds__(kThreads)
-copy_rows_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ in,
-                 const uint32_t *__restrict__ ids, uint32_t rows, uint32_t row_size) {
+copy_rows_kernel(uint16_t *__restrict__ out, const uint16_t *in,
+                 const uint32_t *ids, uint32_t rows, uint32_t row_size) {
     pdl_wait();
     // one warp per row; 16-byte copies when both sides allow it
     const uint32_t warps_per_block = blockDim.x / kWarp;
@@ -140,8 +140,8 @@ copy_rows_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ in,
 // out[t,d] = bf16( sum_r w[t,r] * v[t,r,d] ), r ascending, one fused
 // multiply-add per term (k3_rocm_ops.cu:1452-1474 of the reference).
 __global__ void __launch_bounds__(kThreads)
-weighted_sum_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ vectors,
-                    const float *__restrict__ weights, uint32_t tokens, uint32_t count,
+weighted_sum_kernel(uint16_t *__restrict__ out, const uint16_t *vectors,
+                    const float *weights, uint32_t tokens, uint32_t count,
                     uint32_t hidden) {
     pdl_wait();
     extern __shared__ float w_s[];
@@ -203,8 +203,8 @@ weighted_sum_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ vec
 constexpr uint32_t kNormHeld = 32;
 
 __global__ void __launch_bounds__(kThreads)
-rms_norm_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ in,
-                const uint16_t *__restrict__ weight, uint32_t vectors, uint32_t hidden,
+rms_norm_kernel(uint16_t *__restrict__ out, const uint16_t *in,
+                const uint16_t *weight, uint32_t vectors, uint32_t hidden,
                 float epsilon) {
     pdl_wait();
     __shared__ float red[2][kThreads];
@@ -273,7 +273,7 @@ rms_norm_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ in,
 // above it take under 7 us and 47 us.
 __global__ void __launch_bounds__(kThreads)
 router_topk_kernel(uint32_t *__restrict__ ids_out, float *__restrict__ weights_out,
-                   const float *__restrict__ logits, const float *__restrict__ bias,
+                   const float *logits, const float *bias,
                    uint32_t vectors, uint32_t experts, uint32_t top_k, float scale) {
     pdl_wait();
     __shared__ RouteScratch rs;
@@ -310,7 +310,7 @@ router_topk_kernel(uint32_t *__restrict__ ids_out, float *__restrict__ weights_o
 
 // ------------------------------------------------------------ Q8 quantiser
 __global__ void q8_quantize_kernel(int8_t *__restrict__ q, void *__restrict__ scales,
-                                   const uint16_t *__restrict__ w, uint64_t blocks,
+                                   const uint16_t *w, uint64_t blocks,
                                    uint32_t block, int scale_f16) {
     pdl_wait();
     // one warp per block of `block` elements
@@ -340,8 +340,8 @@ __global__ void q8_quantize_kernel(int8_t *__restrict__ q, void *__restrict__ sc
     }
 }
 
-__global__ void q8_dequantize_kernel(uint16_t *__restrict__ w, const int8_t *__restrict__ q,
-                                     const void *__restrict__ scales, uint64_t count,
+__global__ void q8_dequantize_kernel(uint16_t *__restrict__ w, const int8_t *q,
+                                     const void *scales, uint64_t count,
                                      uint32_t block, int scale_f16) {
     pdl_wait();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;

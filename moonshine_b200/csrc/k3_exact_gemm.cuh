@@ -41,8 +41,8 @@ K3_DEVINL void fma_bf16(float &acc, uint16_t a, uint16_t b) {
 // kDeep steps' loads are in flight at once (one or two input rows: the weights come from HBM).
 template <int kR, int kV, int kDeep>
 __global__ void __launch_bounds__(256)
-exact_q8_kernel(uint16_t *__restrict__ out, const int8_t *__restrict__ q, const void *__restrict__ scales,
-                const uint16_t *__restrict__ x, uint32_t vectors, uint32_t rows, uint32_t columns, uint32_t block,
+exact_q8_kernel(uint16_t *__restrict__ out, const int8_t *q, const void *scales,
+                const uint16_t *x, uint32_t vectors, uint32_t rows, uint32_t columns, uint32_t block,
                 int scale_f16) {
     constexpr int kPhase = kV < 2 ? kV : 2;                // input rows reduced per pass over shared memory
     constexpr int kOut = kR * kPhase;
@@ -155,7 +155,7 @@ exact_q8_kernel(uint16_t *__restrict__ out, const int8_t *__restrict__ q, const 
 // its own kR weight rows and kV input rows.
 template <typename Out, int kR, int kV, int kSR, int kSV>
 __global__ void __launch_bounds__(64 * kSR * kSV)
-exact_bf16_kernel(Out *__restrict__ out, const uint16_t *__restrict__ w, const uint16_t *__restrict__ x,
+exact_bf16_kernel(Out *__restrict__ out, const uint16_t *w, const uint16_t *x,
                   uint32_t vectors, uint32_t rows, uint32_t columns) {
     constexpr int kPhase = kR * kV < 8 ? kR * kV : 8;      // outputs whose halves meet per pass over shared memory
     __shared__ float half_sum[kSR * kSV][kPhase][4][32];

@@ -25,8 +25,8 @@ namespace {
 // 8u..8u+7 (columns 256j + 8u + i).
 template <typename Out, int VT>
 __global__ void __launch_bounds__(256)
-bf16_gemm_kernel(Out *__restrict__ out, const uint16_t *__restrict__ w,
-                 const uint16_t *__restrict__ x, uint32_t vectors, uint32_t rows,
+bf16_gemm_kernel(Out *__restrict__ out, const uint16_t *w,
+                 const uint16_t *x, uint32_t vectors, uint32_t rows,
                  uint32_t columns) {
     pdl_wait();
     const uint32_t lane = threadIdx.x % kWarp;

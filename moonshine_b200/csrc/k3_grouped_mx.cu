@@ -776,8 +776,8 @@ K3_DEVINL SplitColumns split_columns(const uint16_t *p) {
 // kernel are skipped.
 __global__ void __launch_bounds__(256)
 split_rows_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t *__restrict__ sf,
-                  const uint16_t *__restrict__ x, const uint32_t *__restrict__ index,
-                  const uint32_t *__restrict__ offsets, k3_group_parts parts, uint32_t groups, uint32_t rows,
+                  const uint16_t *x, const uint32_t *index,
+                  const uint32_t *offsets, k3_group_parts parts, uint32_t groups, uint32_t rows,
                   uint32_t k) {
     // launched behind a kernel that waited for the dispatch and shares nothing else with this one
     const uint32_t lane = threadIdx.x % kWarp;
@@ -805,8 +805,8 @@ split_rows_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t *_
 // columns): 8192 tokens took 649 us when every product row was converted on its own.
 __global__ void __launch_bounds__(256)
 split_tokens_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t *__restrict__ sf,
-                    const uint16_t *__restrict__ x, const uint32_t *__restrict__ ids,
-                    const uint32_t *__restrict__ inv_perm, const uint32_t *__restrict__ offsets, uint32_t top_k,
+                    const uint16_t *x, const uint32_t *ids,
+                    const uint32_t *inv_perm, const uint32_t *offsets, uint32_t top_k,
                     uint32_t tokens, uint32_t k) {
     const uint32_t lane = threadIdx.x % kWarp, passes = k / 512u;
     const uint64_t warps = (uint64_t)(gridDim.x * blockDim.x) / kWarp, jobs = (uint64_t)tokens * passes;

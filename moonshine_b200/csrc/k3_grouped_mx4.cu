@@ -588,9 +588,9 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
 // warp converts 256 columns per pass and stores each term as 128 contiguous bytes.  The same
 // values as split_block_e2m1 (one element per lane), a sixth of its instructions.
 __global__ void __launch_bounds__(256)
-term_rows_kernel(uint8_t *__restrict__ terms, uint8_t *__restrict__ sf, const uint16_t *__restrict__ x,
-                 uint32_t *__restrict__ counters, const uint32_t *__restrict__ ids,
-                 const uint32_t *__restrict__ offsets, uint32_t top_k, uint32_t rows, uint32_t k) {
+term_rows_kernel(uint8_t *__restrict__ terms, uint8_t *__restrict__ sf, const uint16_t *x,
+                 uint32_t *__restrict__ counters, const uint32_t *ids,
+                 const uint32_t *offsets, uint32_t top_k, uint32_t rows, uint32_t k) {
     pdl_wait();
     pdl_trigger();
     if (blockIdx.x == 0 && threadIdx.x < 64u) counters[threadIdx.x] = 0u;      // of the product launches

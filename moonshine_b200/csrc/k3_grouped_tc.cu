@@ -566,7 +566,7 @@ bool launch_tc(const void *a0, const void *a1, const TcArgs &args, const void *b
 // Q8 weights -> bf16 (each product q * scale rounded once, as the in-kernel
 // conversion of the Q8 mode does); 16 elements per thread, block % 16 == 0.
 __global__ void __launch_bounds__(256)
-q8_to_bf16_kernel(uint4 *__restrict__ w, const uint4 *__restrict__ q, const void *__restrict__ scales,
+q8_to_bf16_kernel(uint4 *__restrict__ w, const uint4 *q, const void *scales,
                   uint64_t units, uint32_t block, int scale_f16) {
     pdl_wait();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;

@@ -38,7 +38,6 @@ struct GroupedArgs {
 template <bool kFuseAct>
 __global__ void __launch_bounds__(kGemvThreads)
 grouped_rows_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ in, GroupedArgs a) {
-    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const GemvSmem sm = carve_gemv_smem(smem_raw, a.k_pad);
     uint32_t expert, row_begin, n;
@@ -98,9 +97,9 @@ grouped_rows_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ in,
 // out[t] = bf16( bf16( bf16(sum_r w[t,r] * rows[idx[t,r]]) + shared[t] ) + residual[t] )
 // (shared and residual optional)
 __global__ void __launch_bounds__(256)
-combine_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ rows,
-               const uint32_t *__restrict__ index, const float *__restrict__ weights,
-               const uint16_t *__restrict__ shared, const uint16_t *__restrict__ residual,
+combine_kernel(uint16_t *__restrict__ out, const uint16_t *rows,
+               const uint32_t *index, const float *weights,
+               const uint16_t *shared, const uint16_t *residual,
                uint32_t tokens, uint32_t top_k, uint32_t hidden) {
     pdl_wait();
     __shared__ float w_s[32];

@@ -104,8 +104,8 @@ K3_DEVINL void mx_finish(uint16_t *out, const float *red, uint32_t row_base, uin
 // asynchronous copies it is slower (6.2 us).  kWide: the vectors are 16-byte aligned.
 template <bool kWide>
 __global__ void __launch_bounds__(32 * kMxSplits)
-mxfp4_rows_kernel(uint16_t *__restrict__ out, const uint8_t *__restrict__ packed, const uint8_t *__restrict__ scales,
-                  const uint16_t *__restrict__ x, uint32_t vectors, uint32_t rows, uint32_t k) {
+mxfp4_rows_kernel(uint16_t *__restrict__ out, const uint8_t *packed, const uint8_t *scales,
+                  const uint16_t *x, uint32_t vectors, uint32_t rows, uint32_t k) {
     __shared__ float red[kMxSplits * 8u * 16u];
     const uint32_t lane = threadIdx.x % kWarp, split = threadIdx.x / kWarp;
     const uint32_t g = lane >> 2, t = lane & 3u;
@@ -123,10 +123,10 @@ mxfp4_rows_kernel(uint16_t *__restrict__ out, const uint8_t *__restrict__ packed
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 7
     for (uint32_t grp = begin; grp < end; grp++) {
-        const uint32_t wa = __ldg(p.pa + 4u * grp), wb = __ldg(p.pb + 4u * grp);
-        const float s_a = e8m0_to_float(__ldg(p.sa + grp)), s_b = e8m0_to_float(__ldg(p.sb + grp));
+        const uint32_t wa = p.pa[4u * grp], wb = p.pb[4u * grp];
+        const float s_a = e8m0_to_float(p.sa[grp]), s_b = e8m0_to_float(p.sb[grp]);
         const uint16_t *xp = xv + 32u * grp;
-        const uint4 xq = kWide ? __ldg(reinterpret_cast<const uint4 *>(xp))
+        const uint4 xq = kWide ? *reinterpret_cast<const uint4 *>(xp)
                                : make_uint4(xp[0] | (uint32_t)xp[1] << 16, xp[2] | (uint32_t)xp[3] << 16,
                                             xp[4] | (uint32_t)xp[5] << 16, xp[6] | (uint32_t)xp[7] << 16);
         uint32_t fa[4], fb[4];
@@ -149,8 +149,8 @@ mxfp4_rows_kernel(uint16_t *__restrict__ out, const uint8_t *__restrict__ packed
 // Bound by issue: per scale group 34 instructions dequantise, 7 per tile multiply and scale.
 template <int kTiles, int kBlocks, int kTeams>
 __global__ void __launch_bounds__(32 * kBlocks * kTeams)
-mxfp4_tile_kernel(uint16_t *__restrict__ out, const uint8_t *__restrict__ packed, const uint8_t *__restrict__ scales,
-                  const uint16_t *__restrict__ x, uint32_t vectors, uint32_t rows, uint32_t k) {
+mxfp4_tile_kernel(uint16_t *__restrict__ out, const uint8_t *packed, const uint8_t *scales,
+                  const uint16_t *x, uint32_t vectors, uint32_t rows, uint32_t k) {
     constexpr uint32_t kCols = 8 * kTiles, kTeamThreads = 32 * kBlocks;
     constexpr uint32_t kStage = kCols * 128u;              // bytes: 64 columns of every vector
     extern __shared__ __align__(128) unsigned char smem_mx[];
@@ -215,10 +215,10 @@ mxfp4_tile_kernel(uint16_t *__restrict__ out, const uint8_t *__restrict__ packed
             for (uint32_t j = 0; j < 2u; j++) {
                 // zero weights and a finite scale where a split ends in half a stage
                 const bool there = j < left;
-                wa[j] = there ? __ldg(qa + 4u * j) : 0u;
-                wb[j] = there ? __ldg(qb + 4u * j) : 0u;
-                ea[j] = there ? __ldg(ca + j) : 0u;
-                eb[j] = there ? __ldg(cb + j) : 0u;
+                wa[j] = there ? qa[4u * j] : 0u;
+                wb[j] = there ? qb[4u * j] : 0u;
+                ea[j] = there ? ca[j] : 0u;
+                eb[j] = there ? cb[j] : 0u;
             }
             qa += 8;
             qb += 8;
