@@ -7,6 +7,8 @@
 
 #include <math.h>
 
+#include <algorithm>
+
 using namespace k3;
 
 namespace {
@@ -417,10 +419,11 @@ extern "C" bool k3_rocm_weighted_sum_bf16_batch(void *output, const void *vector
     }
     const size_t smem = (size_t)vector_count * sizeof(float);
     if (smem > 48 * 1024) return false;
-    // few tokens: the columns of a token over several small blocks
+    // few tokens: the columns of a token over several small blocks (at most 65535 fit the grid; the
+    // kernel goes on from there)
     const bool few = token_count < 128u;
     const uint32_t threads = few ? 64u : kThreads;
-    const dim3 grid(grid_for(token_count, 1), few ? (hidden_size / 8u + threads - 1u) / threads + 1u : 1u);
+    const dim3 grid(grid_for(token_count, 1), few ? std::min((hidden_size / 8u + threads - 1u) / threads + 1u, 65535u) : 1u);
     return launch_chained(weighted_sum_kernel, grid, threads, smem, (cudaStream_t)stream, (uint16_t *)output,
                           (const uint16_t *)vectors, (const float *)weights, token_count, vector_count, hidden_size);
 }

@@ -450,7 +450,7 @@ extern "C" bool k3_moe_combine_residual(void *out, const void *rows, const void 
     const bool few = tokens < 128u;
     const uint32_t threads = few ? 64u : 256u;
     const dim3 grid(std::min<uint32_t>(tokens, (uint32_t)sm_count() * 8u),
-                    few ? (hidden / 8u + threads - 1u) / threads : 1u);
+                    few ? std::min((hidden / 8u + threads - 1u) / threads, 65535u) : 1u);
     return launch_chained(combine_kernel, grid, threads, 0, (cudaStream_t)stream, (uint16_t *)out,
                           (const uint16_t *)rows, (const uint32_t *)index, (const float *)weights,
                           (const uint16_t *)shared, (const uint16_t *)residual, tokens, top_k, hidden);
