@@ -2,7 +2,8 @@
 
 ``python -m moonshine_b200.build`` compiles every ``csrc/*.cu`` into
 ``moonshine_b200/libk3moe.so`` and ``csrc/k3_pyops.cpp``, the CPython bindings of
-its entry points, into ``moonshine_b200/_k3ops.so``.  Object files are cached
+its entry points, into ``moonshine_b200/_k3ops.so`` (without a C++ compiler or Python's
+headers that step is left out with a warning: the calls then go through ctypes).  Object files are cached
 under ``moonshine_b200/_build`` and rebuilt when a source or header is newer.
 """
 from __future__ import annotations
@@ -76,9 +77,14 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False) 
             raise RuntimeError("link failed")
     src = os.path.join(CSRC, "k3_pyops.cpp")
     if force or not os.path.exists(BINDINGS) or os.path.getmtime(BINDINGS) < max(os.path.getmtime(src), hdr_time):
-        run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall",
-             "-I", os.path.join(ROOT, "include"), "-I", sysconfig.get_paths()["include"], "-o", BINDINGS, src,
-             "-L", HERE, "-l:libk3moe.so", "-Wl,-rpath,$ORIGIN"])
+        try:
+            run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall",
+                 "-I", os.path.join(ROOT, "include"), "-I", sysconfig.get_paths()["include"], "-o", BINDINGS, src,
+                 "-L", HERE, "-l:libk3moe.so", "-Wl,-rpath,$ORIGIN"])
+        except (OSError, RuntimeError) as e:
+            if os.path.exists(BINDINGS):               # one built for other headers must not stay
+                os.remove(BINDINGS)
+            sys.stderr.write(f"warning: no CPython bindings, operator calls go through ctypes ({e})\n")
     return LIB
 
 

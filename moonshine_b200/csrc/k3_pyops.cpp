@@ -18,7 +18,7 @@
 
 namespace {
 
-PyObject *g_tensor_type, *g_get_stream, *g_get_device, *g_is_contiguous, *g_data_ptr, *g_stream_kw;
+PyObject *g_tensor_type, *g_layer_desc_type, *g_latent_desc_type, *g_get_stream, *g_get_device, *g_is_contiguous, *g_data_ptr, *g_stream_kw;
 
 enum class Got { kYes, kFallback, kError };
 
@@ -79,11 +79,12 @@ template <>
 struct Arg<const void *> {
     static Got get(PyObject *o, const void **out) { return pointer_of(o, (void **)out); }
 };
-template <typename T>
-struct Structure {                                         // a ctypes structure of exactly this size
+template <typename T, PyObject **kType>
+struct Structure {                                         // the ctypes structure that mirrors T
     static Got get(PyObject *o, const T **out) {
         Py_buffer view;
-        if (!PyObject_CheckBuffer(o) || PyObject_GetBuffer(o, &view, PyBUF_SIMPLE) != 0) {
+        if (!PyObject_TypeCheck(o, (PyTypeObject *)*kType)) return Got::kFallback;
+        if (PyObject_GetBuffer(o, &view, PyBUF_SIMPLE) != 0) {
             PyErr_Clear();
             return Got::kFallback;
         }
@@ -93,8 +94,8 @@ struct Structure {                                         // a ctypes structure
         return fits ? Got::kYes : Got::kFallback;
     }
 };
-template <> struct Arg<const k3_moe_layer_desc *> : Structure<k3_moe_layer_desc> {};
-template <> struct Arg<const k3_moe_latent_desc *> : Structure<k3_moe_latent_desc> {};
+template <> struct Arg<const k3_moe_layer_desc *> : Structure<k3_moe_layer_desc, &g_layer_desc_type> {};
+template <> struct Arg<const k3_moe_latent_desc *> : Structure<k3_moe_latent_desc, &g_latent_desc_type> {};
 
 Got current_stream(void **out) {
     PyObject *device = PyObject_CallNoArgs(g_get_device);
@@ -108,7 +109,6 @@ Got current_stream(void **out) {
 }
 
 inline PyObject *to_python(bool v) { return PyBool_FromLong(v); }
-inline PyObject *to_python(size_t v) { return PyLong_FromSize_t(v); }
 
 template <typename A, typename... Rest>
 struct Last { using type = typename Last<Rest...>::type; };
@@ -209,15 +209,19 @@ PyMethodDef kBound[] = {
     {nullptr, nullptr, 0, nullptr},
 };
 
-// bind(fallbacks, tensor type, raw stream getter, device getter) -> {name: function}
+// bind(fallbacks, tensor type, layer and latent description types, raw stream getter, device
+// getter) -> {name: function}
 PyObject *bind(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
-    if (nargs != 4 || !PyDict_Check(args[0])) {
-        PyErr_SetString(PyExc_TypeError, "bind(dict, tensor type, stream getter, device getter)");
+    if (nargs != 6 || !PyDict_Check(args[0]) || !PyType_Check(args[1]) || !PyType_Check(args[2]) ||
+        !PyType_Check(args[3])) {
+        PyErr_SetString(PyExc_TypeError, "bind(dict, tensor type, layer type, latent type, stream getter, device getter)");
         return nullptr;
     }
     g_tensor_type = Py_NewRef(args[1]);
-    g_get_stream = Py_NewRef(args[2]);
-    g_get_device = Py_NewRef(args[3]);
+    g_layer_desc_type = Py_NewRef(args[2]);
+    g_latent_desc_type = Py_NewRef(args[3]);
+    g_get_stream = Py_NewRef(args[4]);
+    g_get_device = Py_NewRef(args[5]);
     PyObject *out = PyDict_New();
     for (PyMethodDef *d = kBound; out && d->ml_name; d++) {
         PyObject *fallback = PyDict_GetItemString(args[0], d->ml_name);

@@ -13,6 +13,7 @@ Example (compare tests of the reference, tests/test_k3_rocm_components.cu):
 from __future__ import annotations
 
 import ctypes as C
+import os
 
 import torch
 
@@ -65,13 +66,14 @@ def _make(name, restype, argtypes):
 
 
 _CALLS = {_name: _make(_name, _res, _args) for _name, (_res, _args) in _native.SIGNATURES.items()}
-try:
-    # the same functions with their arguments converted in C (csrc/k3_pyops.cpp): a ctypes call
-    # takes longer than most operators run
+# The same functions with their arguments converted in C (csrc/k3_pyops.cpp): a ctypes call takes
+# longer than most operators run.  Without the file, or with a torch that lacks these two getters,
+# the ctypes forms stay; a file that does not load is an error.
+if (os.path.exists(os.path.join(os.path.dirname(__file__), "_k3ops.so"))
+        and hasattr(torch._C, "_cuda_getCurrentRawStream") and hasattr(torch._C, "_cuda_getDevice")):
     from . import _k3ops
-    _CALLS.update(_k3ops.bind(_CALLS, torch.Tensor, torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice))
-except (ImportError, AttributeError):        # not built, or a torch without these: the ctypes forms stay
-    pass
+    _CALLS.update(_k3ops.bind(_CALLS, torch.Tensor, _native.LayerDesc, _native.LatentDesc,
+                              torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice))
 globals().update(_CALLS)
 
 ACT_SITU, ACT_SWIGLU = 0, 1
