@@ -10,11 +10,12 @@
 // kernel these replace converted both again for every output and re-read each weight row
 // from L2 for every four input rows.
 //
-// Bound: the issue rate.  Per 512 FMAs of a Q8 octet step about 300 other instructions go
-// out (byte -> float and the rounded scale product of the weights, bf16 -> float of the
-// inputs, loads), so two input rows share one packed FMA: 200 rows of 3584 x 7168 517 -> 443
-// us, of 7168 x 3584 653 -> 541, 8 rows 26 -> 22 and 29 -> 25.  A BF16 step has no conversions,
-// since the mixed-precision FMA takes bf16 operands.
+// Bound: the issue rate.  Of the roughly 300 instructions of a 4 x 8 tile's Q8 octet step (256
+// multiply-adds) 128 are packed FMAs, each for two input rows, 96 convert and scale the weights
+// (byte -> float, the rounded scale product), 64 convert the inputs and about 20 load.  Before and
+// after the packed FMAs: 200 rows of 3584 x 7168 517 -> 443 us, of 7168 x 3584 653 -> 541, 8 rows
+// 26 -> 22 and 29 -> 25.  A BF16 step has no conversions, since the mixed-precision FMA takes bf16
+// operands.
 #pragma once
 
 #include "k3_common.cuh"

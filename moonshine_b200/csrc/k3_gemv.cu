@@ -21,7 +21,8 @@ using namespace k3;
 namespace {
 
 // ------------------------------------------------------------------- BF16
-// One warp per weight row.  Thread u keeps the partial sums of virtual lanes
+// Columns or bases that the register tiles (k3_exact_gemm.cuh) do not take, element by element: one
+// warp per weight row.  Thread u keeps the partial sums of virtual lanes
 // 8u..8u+7 (columns 256j + 8u + i).
 template <typename Out, int VT>
 __global__ void __launch_bounds__(256)
@@ -31,7 +32,6 @@ bf16_gemm_kernel(Out *__restrict__ out, const uint16_t *w,
     pdl_wait();
     const uint32_t lane = threadIdx.x % kWarp;
     const uint32_t warps = (gridDim.x * blockDim.x) / kWarp;
-    const bool wide = (columns % 8u == 0) && ((((uintptr_t)w) | ((uintptr_t)x)) & 15u) == 0;
     for (uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp; row < rows;
          row += warps) {
         const uint16_t *wr = w + (uint64_t)row * columns;
@@ -44,31 +44,17 @@ bf16_gemm_kernel(Out *__restrict__ out, const uint16_t *w,
             for (uint32_t c0 = lane * 8u; c0 < columns; c0 += 256u) {
                 float wf[8];
                 uint32_t valid = min(8u, columns - c0);
-                if (wide) {
-                    const uint4 q = *reinterpret_cast<const uint4 *>(wr + c0);
-                    wf[0] = bf16_lo(q.x); wf[1] = bf16_hi(q.x); wf[2] = bf16_lo(q.y);
-                    wf[3] = bf16_hi(q.y); wf[4] = bf16_lo(q.z); wf[5] = bf16_hi(q.z);
-                    wf[6] = bf16_lo(q.w); wf[7] = bf16_hi(q.w);
-                } else {
 #pragma unroll
-                    for (int i = 0; i < 8; i++)
-                        wf[i] = (uint32_t)i < valid ? bf16_bits_to_float(wr[c0 + i]) : 0.f;
-                }
+                for (int i = 0; i < 8; i++)
+                    wf[i] = (uint32_t)i < valid ? bf16_bits_to_float(wr[c0 + i]) : 0.f;
 #pragma unroll
                 for (int v = 0; v < VT; v++) {
                     if (v0 + v >= vectors) break;
                     const uint16_t *xr = x + (uint64_t)(v0 + v) * columns + c0;
                     float xf[8];
-                    if (wide) {
-                        const uint4 q = *reinterpret_cast<const uint4 *>(xr);
-                        xf[0] = bf16_lo(q.x); xf[1] = bf16_hi(q.x); xf[2] = bf16_lo(q.y);
-                        xf[3] = bf16_hi(q.y); xf[4] = bf16_lo(q.z); xf[5] = bf16_hi(q.z);
-                        xf[6] = bf16_lo(q.w); xf[7] = bf16_hi(q.w);
-                    } else {
 #pragma unroll
-                        for (int i = 0; i < 8; i++)
-                            xf[i] = (uint32_t)i < valid ? bf16_bits_to_float(xr[i]) : 0.f;
-                    }
+                    for (int i = 0; i < 8; i++)
+                        xf[i] = (uint32_t)i < valid ? bf16_bits_to_float(xr[i]) : 0.f;
 #pragma unroll
                     for (int i = 0; i < 8; i++) {
                         if ((uint32_t)i < valid) acc[v][i] = fmaf(wf[i], xf[i], acc[v][i]);

@@ -427,16 +427,6 @@ K3_DEVINL void mxfp4_item_2x16(float *out_s /* [2][32] */, float *red, const Row
     __syncthreads();
 }
 
-template <bool kAligned16>
-K3_DEVINL void mxfp4_item_32rows(float *out_s, float *red, const uint8_t *packed,
-                                 const uint8_t *scales, uint32_t row0, uint32_t rows_end,
-                                 uint32_t k, const __half *xs, uint32_t k_pad, uint32_t nvec,
-                                 const float *inv_scale) {
-    const RowBlock b0{packed, scales, row0, rows_end};
-    const RowBlock b1{packed, scales, row0 + 16u, rows_end};
-    mxfp4_item_2x16<kAligned16>(out_s, red, b0, b1, k, xs, k_pad, nvec, inv_scale);
-}
-
 // Shared-memory layout used by every kernel built on the item routine.
 struct GemvSmem {
     __half *xs;        // [2][k_pad]

@@ -1,7 +1,8 @@
 // Internal interface between the layer composition and the tensor-core
 // (tcgen05) GEMM kernels.  Each function picks the tensor-core kernel when the
-// shape, alignment and row count suit it and otherwise runs the exact-order
-// SIMT kernel behind the legacy entry points.
+// shape, alignment and row count suit it.  Otherwise Q8 products of up to 32 rows
+// go to k3_q8_few.cu (mma.sync, an order of sums of its own) where their shape
+// allows, and the rest to the exact-order kernels behind the legacy entry points.
 #pragma once
 
 #include "k3_moe_layer.h"

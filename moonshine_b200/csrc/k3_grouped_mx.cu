@@ -149,7 +149,6 @@ struct GmxArgs {
     uint8_t *act_hi, *act_lo, *act_sf;   // gate/up mode: E4M3 terms and block scales of the activation
     uint32_t groups, rows, row_floor, row_ceil, w_rows, k, out_width, m_items;   // groups of row_floor < rows <= row_ceil
     uint32_t *item_counter;              // zero before the launch; items are drawn from it
-    bool behind_wait;                    // the kernel in front of this one in the stream already waited for its inputs
     int activation;
     float beta, linear_beta;
 };
@@ -375,9 +374,9 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         tmem_alloc(tmem_slot, kTmemCols);
         tmem_relinquish();
     }
-    // Two such kernels in a row (few and many rows per group) do not depend on each other: the
-    // second one's blocks start as the first one's leave, and wait for it only before they end.
-    if (!a.behind_wait) pdl_wait();
+    // The kernel in front is the packed one or the other instance of this one.  It has waited for
+    // everything before it, and nothing it writes is read here, so this kernel's blocks start as its
+    // blocks leave and wait for it only before they end (so that who waits for this one waits for both).
     pdl_trigger();
     {   // exclusive prefix of ceil(rows_g / BN) over the groups (<= 1024)
         __shared__ uint32_t warp_tot[kThreads / kWarp];
@@ -743,7 +742,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         tc_fence_after();
         tmem_dealloc(tmem, kTmemCols);
     }
-    if (a.behind_wait) pdl_wait();
+    pdl_wait();
 }
 
 // 16 bf16 columns of one lane (two lanes share a block of 32) -> E4M3 terms and the block's scale.
@@ -1059,7 +1058,6 @@ bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act
     a.activation = d->activation;
     a.beta = d->beta;
     a.linear_beta = d->linear_beta;
-    a.behind_wait = true;
     auto launches = [&](auto mode, const Operands &op, uint32_t *counters) {
         constexpr int kE = decltype(mode)::value;
         GmxArgs b = a;

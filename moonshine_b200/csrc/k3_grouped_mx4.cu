@@ -582,11 +582,11 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
     }
 }
 
-// (`ids` given: the experts of row r are ids[r * top_k ..], and a row none of whose experts is a
-// group of this kernel is skipped.)
 // bf16 rows -> E2M1 terms and block scales: four lanes share a block of 32 columns (8 each), a
 // warp converts 256 columns per pass and stores each term as 128 contiguous bytes.  The same
-// values as split_block_e2m1 (one element per lane), a sixth of its instructions.
+// values as split_block_e2m1 (one element per lane), a sixth of its instructions.  With `ids`, the
+// experts of row r are ids[r * top_k ..], and a row none of whose experts is a group of this kernel
+// is skipped.
 __global__ void __launch_bounds__(256)
 term_rows_kernel(uint8_t *__restrict__ terms, uint8_t *__restrict__ sf, const uint16_t *x,
                  uint32_t *__restrict__ counters, const uint32_t *ids,

@@ -517,7 +517,7 @@ bool layer_forward_impl(const k3_moe_layer_desc *d, void *out, const void *x, ui
                 return false;
             }
             if (w.mx_bytes != 0) {
-                // block-scaled path: tokens are converted once, then gathered as bytes
+                // block-scaled path: a token is converted once and its terms stored to its product rows
                 if (!mark(events, 3, stream)) return false;
                 const k3_token_routes by_token{w.ids, w.inv_perm};
                 if (!k3_grouped_mx_experts(d, w.rows_out, nullptr, x, w.sorted_token, tokens, w.offsets,

@@ -1,6 +1,7 @@
-// Top-k routing of one token by a whole thread block from its per-expert scores: choice = sigmoid(logit) + bias decides (larger first,
-// lower expert id on ties, k3_rocm_ops.cu:1385-1450 / tests/test_k3_moe_smoke.cu:215-253),
-// weight = score / (1e-20 + sum of the selected scores in rank order) * scale.
+// Top-k routing of one token by a whole thread block from its per-expert scores: choice =
+// sigmoid(logit) + bias decides (larger first, lower expert id on ties,
+// k3_rocm_ops.cu:1385-1450 / tests/test_k3_moe_smoke.cu:215-253), weight = score / (1e-20 + sum
+// of the selected scores in rank order) * scale.
 //
 // Warps 0..7 each own 128 experts, four per lane, as order keys (0 = none).  A few arg-max
 // rounds per warp give a threshold: with W fully populated warps and r = ceil(top_k / W), the
