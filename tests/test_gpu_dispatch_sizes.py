@@ -48,6 +48,41 @@ def test_expert_counts_around_the_default_shared_memory():
     assert res.returncode == 0, res.stdout[-2000:] + res.stderr[-2000:]
 
 
+@pytest.mark.parametrize("tokens,top_k,experts", [(64, 4, 32), (512, 8, 32), (513, 8, 32), (700, 8, 896)])
+def test_out_of_range_ids_on_both_sides_of_the_route_limit(tokens, top_k, experts):
+    """They are left out of the order, the status word says so, and all other routes are placed."""
+    assert ops.k3_moe_device_status_clear()
+    rng = np.random.default_rng(tokens)
+    ids = rng.integers(0, experts, tokens * top_k).astype(np.uint32)
+    build(ids, tokens, top_k, experts)
+    assert ops.k3_moe_device_status() == 0
+    bad = rng.choice(ids.size, 7, replace=False)
+    ids[bad] = [experts, experts + 1, 0xFFFFFFFF, 0x80000000, 1 << 20, experts + 31, 0xFFFFFFFE]
+    offsets, sorted_route, sorted_token, inv = build(ids, tokens, top_k, experts)
+    assert ops.k3_moe_device_status() & 2
+    assert ops.k3_moe_device_status_clear() and ops.k3_moe_device_status() == 0
+    good = np.flatnonzero(ids < experts)
+    order = good[np.argsort(ids[good], kind="stable")].astype(np.uint32)
+    assert np.array_equal(offsets, np.concatenate([[0], np.cumsum(np.bincount(ids[good], minlength=experts))]))
+    n = good.size
+    assert np.array_equal(sorted_route[:n], order) and np.array_equal(sorted_token[:n], order // top_k)
+    assert np.array_equal(inv[order], np.arange(n))
+    assert (sorted_route[n:] == 0xFFFFFFFF).all() and (inv[bad] == 0xFFFFFFFF).all()       # untouched
+
+
+def test_the_shared_histograms_of_a_larger_call_do_not_leak():
+    """Of the calls without a workspace only those above 4096 routes use the shared array: a large
+    one, a smaller one with another expert count, and the large one again."""
+    import ctypes as C
+    for tokens, top_k, experts in ((8192, 16, 896), (700, 8, 64), (8192, 16, 896)):
+        ids = np.random.default_rng(tokens).integers(0, experts, tokens * top_k).astype(np.uint32)
+        got = [G.empty((experts + 1,), np.uint32)] + [G.empty((ids.size,), np.uint32) for _ in range(3)]
+        err = C.create_string_buffer(256)
+        assert ops.k3_moe_dispatch_build_noalloc(*got, G.dev(ids), tokens, top_k, experts, err, 256), err.value
+        for a, b in zip(got, build(ids, tokens, top_k, experts)):
+            assert np.array_equal(G.host(a, np.uint32), b)
+
+
 if __name__ == "__main__":
     for e in (1, 765, 766, 767, 768, 1024):
         for n in (1, 4096, 4097):
