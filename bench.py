@@ -278,9 +278,10 @@ def run_config(args, cfg, tokens, world):
 
 
 # DRAM bytes per launch measured with ncu on these workloads (one-pass metrics,
-# summary kept under profiles/): prefill = gate/up (16.70 GB) + down (9.39 GB)
-# launches of the grouped expert phase; decode = the four kernels of one token.
-PREFILL_TRAFFIC_BYTES = 26.09e9
+# summary kept under profiles/): prefill = the six grouped expert launches (gate/up 17.22 GB,
+# down 9.41 GB, the launches for groups that this load does not have nothing); decode = the
+# four kernels of one token.
+PREFILL_TRAFFIC_BYTES = 26.63e9
 DECODE_TRAFFIC_BYTES = 434.9e6
 
 
@@ -289,8 +290,12 @@ def launches_per_step(tokens: int, shared: bool) -> int:
     """Kernels of this library one layer pass launches (baseline shapes)."""
     if tokens == 1:
         return 4                                   # shared-expert ring kernel, router rows, experts, tail
-    route, shared_k, dispatch, combine = 2, (5 if shared else 0), 3, 1
-    experts = 1 + 3 + 2                            # row split, 3 gathers, gate/up and down GEMMs
+    route, combine = 2, 1
+    shared_k = 0 if not shared else 5 if tokens >= 32 else 2      # 3 conversions and 2 GEMMs; gate/up and down
+    dispatch = 1 if tokens * 16 <= 4096 else 3
+    # row terms, gate/up and down of the packed kernel; two-term rows and the two-term kernel's
+    # launches where an expert can have more than 16 rows; those for more than 64
+    experts = 3 + (3 if tokens > 16 else 0) + (2 if tokens > 64 else 0)
     return route + shared_k + dispatch + experts + combine
 
 
@@ -872,7 +877,7 @@ def run_layer(args, device, peaks, torch, dist, world, rank, local_rank, MoELaye
                         "unit": "TFLOP/s", "frac": achieved / peaks["bf16_tflops_sustained"],
                         "frac_of_burst": achieved / peaks["bf16_tflops"],
                         "traffic": PREFILL_TRAFFIC_BYTES if args.workload == "prefill8k" and world == 1 else None,
-                        "traffic_note": "DRAM read+write of the two grouped GEMM launches, ncu one-pass capture "
+                        "traffic_note": "DRAM read+write of the six grouped GEMM launches, ncu one-pass capture "
                                         "of this workload (summary under profiles/); algorithmic 26.2 GB",
                         "peak_source": peaks["source"] + " bf16 sustained",
                         "launch_ms": experts_ms,

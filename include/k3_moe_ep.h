@@ -17,7 +17,7 @@
  *            order (expert asc, source asc, route asc) - with contiguous token
  *            blocks that is the single-GPU grouping order
  *            (k3_engine_prefill.inc:1175-1194), so results equal the one-GPU
- *            layer bit for bit
+ *            layer bit for bit where both take the same kernels (below)
  *   dispatch sends each token row once per destination rank (however many of its
  *            routes go there) plus a 4-byte slot per route
  *   return   the reverse grouped send/recv, then the weighted combine in rank
@@ -27,6 +27,15 @@
  * the selected experts it holds, and one all-reduce merges the rows (integer
  * sum of the bf16 bit patterns: every row is produced by exactly one rank, all
  * others contribute zero bits, so the merge is exact).
+ *
+ * Same kernels: an expert's rows are the same ones in the same order as on one
+ * GPU, so its kernel is the same too, as long as at least 32 rows arrive on every
+ * rank (or fewer than 32 on each and in the one-GPU pass).  Router, shared expert
+ * and projections go by the rank's own token count: 1 to 31 tokens and 32 and more
+ * have different orders of sums, so the rank's tokens and the one-GPU batch must
+ * lie on the same side of 32 (a one-GPU batch of one token takes the one-token
+ * kernels).  Elsewhere results differ in the last bits of bf16 intermediates
+ * (rel-L2 about 1e-3, inside the layer tolerance of 1e-2).
  *
  * Conventions are those of k3_moe_layer.h: caller-owned device pointers, the
  * stream as void *, bool results, messages through `error`.  NCCL is loaded
@@ -56,7 +65,7 @@ bool k3_moe_ep_create(k3_moe_ep **out, const void *id_bytes, int rank, int world
 void k3_moe_ep_destroy(k3_moe_ep *ep);
 /* Return direction of k3_moe_ep_layer_forward.  Default (false): every expert row comes
  * back and the token's own rank sums the top_k rows in rank order - results equal the
- * one-GPU layer bit for bit.  Reduced (true): the expert rank forms, per token it
+ * one-GPU layer bit for bit where both take the same kernels (above).  Reduced (true): the expert rank forms, per token it
  * served, the weighted sum of that token's rows in rank order (fp32, rounded to bf16
  * once) and returns ONE row per (token, rank); the token's rank adds the partial sums
  * in rank-of-GPU order.  top_k / (distinct ranks per token) times fewer bytes come back
