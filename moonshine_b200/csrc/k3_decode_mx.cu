@@ -207,7 +207,7 @@ decode_experts_kernel(const __grid_constant__ MxMaps maps, MxArgs a) {
     volatile uint32_t *item_box = tmem_slot + 2;       // [kItemSlots]
     uint32_t *ids_s = tmem_slot + 8;                   // [32]
     float *weights_s = reinterpret_cast<float *>(tmem_slot + 40);   // [32]
-    const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    const uint32_t warp = warp_index(), lane = threadIdx.x % kWarp;
     const uint32_t tiles_g = a.expert_hidden / 128u, tiles_d = a.hidden / 128u;
     const uint32_t items_g = a.ranks * tiles_g, items = items_g + a.ranks * tiles_d;
 
@@ -355,7 +355,7 @@ decode_experts_kernel(const __grid_constant__ MxMaps maps, MxArgs a) {
             if (cur == kNoItem) break;
             const Item it = decode(cur);
             if (!it.local) continue;
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t w_rows = it.down ? a.hidden : a.expert_hidden;
                 const int32_t y = (int32_t)(it.expert * w_rows + it.tile * 128u);
                 const uint32_t phases = it.down ? 1u : 2u, steps = it.down ? steps_d : steps_g;
@@ -370,12 +370,12 @@ decode_experts_kernel(const __grid_constant__ MxMaps maps, MxArgs a) {
                     }
                 }
             }
-            ok = __shfl_sync(0xffffffffu, ok ? 1u : 0u, 0) != 0u;
+            ok = __all_sync(0xffffffffu, ok);
         }
     } else if (warp == 12) {
         // ===================================== term producer
         bool ok = true;
-        if (lane == 0) {
+        if (elect_one()) {
             prefetch_tensormap(&maps.x_terms);
             prefetch_tensormap(&maps.x_sf);
             prefetch_tensormap(&maps.a_terms);
@@ -393,7 +393,7 @@ decode_experts_kernel(const __grid_constant__ MxMaps maps, MxArgs a) {
             if (!it.local || !it.down) continue;
             const uint32_t buf = dcount & 1u, par = (dcount >> 1) & 1u;
             dcount++;
-            if (lane == 0) {
+            if (elect_one()) {
                 // the rank's activation is complete when all its G epilogue warps have arrived
                 const uint32_t need = 4u * tiles_g;
                 const uint32_t *word = a.control + 16u + it.rank;
@@ -419,7 +419,7 @@ decode_experts_kernel(const __grid_constant__ MxMaps maps, MxArgs a) {
                                     &bd_full[buf], (int32_t)(bt * 16u), y);
                 }
             }
-            ok = __shfl_sync(0xffffffffu, ok ? 1u : 0u, 0) != 0u;
+            ok = __all_sync(0xffffffffu, ok);
         }
     } else if (warp == 10) {
         // ===================================== weight-scale producer: 512 K per box
@@ -434,7 +434,7 @@ decode_experts_kernel(const __grid_constant__ MxMaps maps, MxArgs a) {
         for (uint32_t w = next_item(); ok && w != kNoItem; w = next_item()) {
             const Item it = decode(w);
             if (!it.local) continue;
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t w_rows = it.down ? a.hidden : a.expert_hidden;
                 const int32_t y = (int32_t)(it.expert * w_rows + it.tile * 128u);
                 const uint32_t phases = it.down ? 1u : 2u, steps = it.down ? steps_d : steps_g;
@@ -450,7 +450,7 @@ decode_experts_kernel(const __grid_constant__ MxMaps maps, MxArgs a) {
                     }
                 }
             }
-            ok = __shfl_sync(0xffffffffu, ok ? 1u : 0u, 0) != 0u;
+            ok = __all_sync(0xffffffffu, ok);
         }
     } else if (warp == 1 || warp == 11) {
         // ===================================== MMA issuers
@@ -469,7 +469,7 @@ decode_experts_kernel(const __grid_constant__ MxMaps maps, MxArgs a) {
                 dbuf = dcount & 1u;
                 dcount++;
             }
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t dpar = ((dcount - 1u) >> 1) & 1u;
                 const uint32_t phases = it.down ? 1u : 2u, steps = it.down ? steps_d : steps_g;
                 const uint32_t b_base = smem_u32(base + (it.down ? lay.bd + dbuf * steps_d * kBAtom : lay.bg));
@@ -510,7 +510,7 @@ decode_experts_kernel(const __grid_constant__ MxMaps maps, MxArgs a) {
                 }
             }
             if (++buf == 2u) { buf = 0; pacc ^= 1u; }
-            ok = __shfl_sync(0xffffffffu, ok ? 1u : 0u, 0) != 0u;
+            ok = __all_sync(0xffffffffu, ok);
         }
     } else if (warp < 6) {
         // ===================================== scale writers: shared memory -> tensor memory,

@@ -104,7 +104,7 @@ decode_shared_ring_kernel(const __grid_constant__ RingMaps maps, RingArgs a) {
     __shared__ float inv_scale_s[2], warp_max_s[kGroups * kWarps];
     __shared__ uint32_t abort_word;
     volatile uint32_t *abort_flag = &abort_word;
-    const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    const uint32_t warp = warp_index(), lane = threadIdx.x % kWarp;
     const uint32_t H = a.H, S = a.S, n = gridDim.x;
     const uint32_t tasks_gu = 2u * S / 16u, tasks_dn = H / 16u;
     const uint32_t per_gu = H / 1024u, per_dn = S / 1024u;
@@ -141,7 +141,7 @@ decode_shared_ring_kernel(const __grid_constant__ RingMaps maps, RingArgs a) {
 
     if (warp == kProducerWarp) {
         // ===================================================== producer
-        if (lane == 0) {
+        if (elect_one()) {
             prefetch_tensormap(&maps.gate);
             prefetch_tensormap(&maps.up);
             prefetch_tensormap(&maps.down);

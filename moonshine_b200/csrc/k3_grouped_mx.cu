@@ -342,7 +342,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
     uint32_t *total_items_s = tmem_slot + 2;
     volatile uint32_t *item_box = tmem_slot + 3;          // [kItemSlots]
     uint32_t *prefix = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(bars) + kBarBytes);
-    const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    const uint32_t warp = warp_index(), lane = threadIdx.x % kWarp;
     const uint32_t steps = a.k / KS;
     const uint32_t tile_rows = kE == kEAct ? BM : 2u * BM;     // weight rows one item advances
 
@@ -418,25 +418,28 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
     const uint32_t tmem = *tmem_slot;
     const uint32_t total_items = *total_items_s;
 
-    // Reader side of the item mailbox (whole warp, or one thread with lane_count 1):
-    // the n-th call returns the n-th item this CTA drew, kNoItem when there are no more.
+    // Reader side of the item mailbox: the n-th call (of one thread, or of a warp) returns the n-th
+    // item this CTA drew, kNoItem when there are no more.
     uint32_t item_seq = 0;
     auto next_item = [&]() -> uint32_t {
         const uint32_t slot = item_seq % kItemSlots, parity = (item_seq / kItemSlots) & 1u;
         item_seq++;
         uint32_t w = kNoItem;
-        if (lane == 0) {
-            if (mbar_wait(&item_full[slot], parity, abort_flag)) {
-                w = item_box[slot];
-                mbar_arrive(&item_empty[slot]);
-            }
+        if (mbar_wait(&item_full[slot], parity, abort_flag)) {
+            w = item_box[slot];
+            mbar_arrive(&item_empty[slot]);
         }
         return w;
+    };
+    auto next_item_warp = [&]() -> uint32_t {
+        uint32_t w = kNoItem;
+        if (lane == 0) w = next_item();
+        return __shfl_sync(0xffffffffu, w, 0);
     };
 
     if (warp == 0) {
         // ================================ TMA producer: weights and block scales; draws the items
-        if (lane == 0) {
+        if (elect_one()) {
             prefetch_tensormap(&maps.a0);
             prefetch_tensormap(&maps.a1);
             prefetch_tensormap(&maps.sfa0);
@@ -479,7 +482,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         }
     } else if (warp == 2) {
         // ================================ TMA producer: token terms
-        if (lane == 0) {
+        if (elect_one()) {
             prefetch_tensormap(&maps.bhi);
             prefetch_tensormap(&maps.blo);
             uint32_t s = 0, ph = 0;
@@ -509,7 +512,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         // so warp 1 issues the MMAs of weight tile 0 and warp 3 those of tile 1.  Both
         // commit to the same stage / scale / accumulator barriers (count 2).  The MMAs of a
         // larger tile all add into one accumulator: warp 1 issues them, warp 3 only arrives.
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t q = warp == 1 ? 0u : 1u;
             uint32_t s = 0, ph = 0, sb = 0, sph = 0;
             AccBuffers acc;
@@ -580,8 +583,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         const uint32_t lane_base = (32u * quad) << 16;
         uint32_t sb = 0, sph = 0, ss = 0, ssph = 0;
         bool ok = true;
-        for (uint32_t w = __shfl_sync(0xffffffffu, next_item(), 0); ok && w != kNoItem;
-             w = __shfl_sync(0xffffffffu, next_item(), 0)) {
+        for (uint32_t w = next_item_warp(); ok && w != kNoItem; w = next_item_warp()) {
             // a stacked operand's lo rows have the scales of its hi rows
             const uint32_t repeat = term_layout<kStages>(decode_item(w, prefix, a)).block / 32u - 1u;
             for (uint32_t st = 0; st < steps; st += 4u) {
@@ -639,8 +641,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         const uint32_t part = (warp - 8u) >> 2;
         const uint32_t m = 32u * quad + lane;            // tensor-memory lane: weight row, or token row
         AccBuffers acc;
-        for (uint32_t w = __shfl_sync(0xffffffffu, next_item(), 0); w != kNoItem;
-             w = __shfl_sync(0xffffffffu, next_item(), 0)) {
+        for (uint32_t w = next_item_warp(); w != kNoItem; w = next_item_warp()) {
             const Item it = decode_item(w, prefix, a);
             const bool small = acc.small(it);
             const uint32_t b0 = acc.first(small);

@@ -201,7 +201,7 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
     uint32_t *total_items_s = tmem_slot + 2;
     volatile uint32_t *item_box = tmem_slot + 3;           // [kItemSlots]
     uint32_t *prefix = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(bars) + kBarBytes);
-    const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    const uint32_t warp = warp_index(), lane = threadIdx.x % kWarp;
     const uint32_t steps = a.k / KS;                       // even: K is a multiple of 512
     const uint32_t tile_rows = kAct ? BM : 2u * BM;        // weight rows one item advances
 
@@ -278,24 +278,28 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
     const uint32_t tmem = *tmem_slot;
     const uint32_t total_items = *total_items_s;
 
-    // Reader side of the item mailbox: the n-th call returns the n-th item this CTA drew.
+    // Reader side of the item mailbox: the n-th call (of one thread, or of a warp) returns
+    // the n-th item this CTA drew.
     uint32_t item_seq = 0;
     auto next_item = [&]() -> uint32_t {
         const uint32_t slot = item_seq % kItemSlots, parity = (item_seq / kItemSlots) & 1u;
         item_seq++;
         uint32_t w = kNoItem;
-        if (lane == 0) {
-            if (mbar_wait(&item_full[slot], parity, abort_flag)) {
-                w = item_box[slot];
-                mbar_arrive(&item_empty[slot]);
-            }
+        if (mbar_wait(&item_full[slot], parity, abort_flag)) {
+            w = item_box[slot];
+            mbar_arrive(&item_empty[slot]);
         }
         return w;
+    };
+    auto next_item_warp = [&]() -> uint32_t {
+        uint32_t w = kNoItem;
+        if (lane == 0) w = next_item();
+        return __shfl_sync(0xffffffffu, w, 0);
     };
 
     if (warp == 0) {
         // ================================ TMA producer: weights and their scales; draws the items
-        if (lane == 0) {
+        if (elect_one()) {
             prefetch_tensormap(&maps.a0);
             prefetch_tensormap(&maps.a1);
             prefetch_tensormap(&maps.sfa0);
@@ -336,12 +340,11 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
             }
         }
     } else if (warp == 2) {
-        // ================================ TMA producer: token terms; lane i brings row i of the tile
+        // ================================ TMA producer: token terms; lane i knows row i of the tile
         if (lane == 0) prefetch_tensormap(&maps.b);
         uint32_t s = 0, ph = 0;
         bool ok = true;
-        for (uint32_t w = __shfl_sync(0xffffffffu, next_item(), 0); ok && w != kNoItem;
-             w = __shfl_sync(0xffffffffu, next_item(), 0)) {
+        for (uint32_t w = next_item_warp(); ok && w != kNoItem; w = next_item_warp()) {
             const Item it = decode_item(w, prefix, a);
             const bool mine = lane < it.rows_valid;
             const uint32_t row = (kAct ? it.row_start : it.act_row) + lane;
@@ -353,14 +356,17 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1u : 0u, 0) != 0u;
                 if (!ok) break;
-                if (mine)
-                    tma_load_3d(b_smem + s * kBSlotBytes + lane * 2u * kBAtom, &maps.b, &b_full[s], 0, y, (int32_t)st);
+                for (uint32_t i = 0; i < it.rows_valid; i++) {
+                    const int32_t row_y = __shfl_sync(0xffffffffu, y, (int)i);
+                    if (elect_one())
+                        tma_load_3d(b_smem + s * kBSlotBytes + i * 2u * kBAtom, &maps.b, &b_full[s], 0, row_y, (int32_t)st);
+                }
                 if (++s == kBSlots) { s = 0; ph ^= 1u; }
             }
         }
     } else if (warp == 1 || warp == 3) {
         // ==================================================== MMA issuers, one per weight tile
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t q = warp == 1 ? 0u : 1u;
             uint32_t s = 0, ph = 0, bs = 0, bph = 0, sb = 0, sph = 0;
             AccBuffers acc;
@@ -418,8 +424,7 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
         const uint32_t lane_base = (32u * quad) << 16;
         uint32_t sb = 0, sph = 0, ss = 0, ssph = 0;
         bool ok = true;
-        for (uint32_t w = __shfl_sync(0xffffffffu, next_item(), 0); ok && w != kNoItem;
-             w = __shfl_sync(0xffffffffu, next_item(), 0)) {
+        for (uint32_t w = next_item_warp(); ok && w != kNoItem; w = next_item_warp()) {
             const Item it = decode_item(w, prefix, a);
             // this lane's term rows 32 c + lane: term lane % 8 of token row 4 c + lane / 8 (a row past
             // the tile's end repeats row 0: those accumulator columns are not read)
@@ -478,8 +483,7 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
         const uint32_t quad = warp & 3u, r0 = 4u * ((warp - 8u) >> 2);
         const uint32_t m = 32u * quad + lane;              // weight row inside the tile
         AccBuffers acc;
-        for (uint32_t w = __shfl_sync(0xffffffffu, next_item(), 0); w != kNoItem;
-             w = __shfl_sync(0xffffffffu, next_item(), 0)) {
+        for (uint32_t w = next_item_warp(); w != kNoItem; w = next_item_warp()) {
             const Item it = decode_item(w, prefix, a);
             const bool small = it.rows_valid <= 8u;
             const uint32_t b0 = acc.first(small);

@@ -177,7 +177,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a0,
     uint32_t *total_items_s = tmem_slot + 2;
     uint32_t *prefix = reinterpret_cast<uint32_t *>(base + C::kRingBytes + 512);
 
-    const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    const uint32_t warp = warp_index(), lane = threadIdx.x % kWarp;
     const uint32_t ksteps = a.k / BK;
 
     // ---- prologue: n-tile prefix of the groups, barriers, tensor memory
@@ -249,7 +249,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a0,
 
     if (warp == 0) {
         // ===================================================== TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             prefetch_tensormap(&map_a0);
             prefetch_tensormap(&map_a1);
             prefetch_tensormap(&map_b);
@@ -286,7 +286,7 @@ grouped_tc_kernel(const __grid_constant__ CUtensorMap map_a0,
         }
     } else if (warp == 1) {
         // ======================================================= MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t s = 0, ph = 0, sa = 0, pha = 0, buf = 0, pacc = 0;
             bool ok = true;
             for (uint32_t w = blockIdx.x; ok && w < total_items; w += gridDim.x) {

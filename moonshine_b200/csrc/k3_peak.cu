@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(kPeakThreads, 1) peak_kernel(int kind, uint32_
     uint64_t *done = reinterpret_cast<uint64_t *>(base + kATile + kBTile);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
     volatile uint32_t *abort_flag = tmem_slot + 1;
-    const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    const uint32_t warp = warp_index(), lane = threadIdx.x % kWarp;
     // operand bytes: small finite values in every format used (E4M3 / E2M1 pairs / bf16 halves)
     for (uint32_t i = threadIdx.x; i < (kATile + kBTile) / 4u; i += blockDim.x) {
         const uint32_t h = (i * 2654435761u) ^ (blockIdx.x * 40503u);
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kPeakThreads, 1) peak_kernel(int kind, uint32_
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     tc_fence_before();
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp == 0 && elect_one()) {
         tc_fence_after();
         const uint64_t da = make_desc_sw128(smem_u32(base));
         const uint64_t db = make_desc_sw128(smem_u32(base + kATile));

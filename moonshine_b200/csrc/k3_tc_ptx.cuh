@@ -11,6 +11,23 @@ K3_DEVINL uint32_t smem_u32(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// ---------------------------------------------------------------- one thread of a warp
+// TMA, MMA and commit instructions take their operands from uniform registers.  A branch on
+// lane == 0 does not tell the compiler that one thread runs it, so every operand goes through a
+// loop over the values that the active lanes might hold; behind elect.sync, in a warp whose index
+// is the same in all lanes for the compiler too (warp_index), it moves them directly.  Measured,
+// one thread issuing back to back: a block-scaled MMA of N = 128 every 36 ns instead of 57 (its
+// operand fetch: N = 64 28 ns instead of 54), a bf16 MMA of N = 32 with A in tensor memory 11 instead
+// of 51, a TMA box every 14 instead of 32 to 60.
+K3_DEVINL uint32_t warp_index() { return __shfl_sync(0xffffffffu, threadIdx.x / kWarp, 0); }
+
+// true in one lane of a converged warp, the same lane each time
+K3_DEVINL bool elect_one() {
+    uint32_t elected;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+    return elected != 0u;
+}
+
 // ------------------------------------------------------------------ mbarrier
 K3_DEVINL void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
