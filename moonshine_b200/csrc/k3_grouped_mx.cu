@@ -20,9 +20,9 @@
 // shared memory, so a CTA that drew short row tiles simply takes more of them.  Items
 // are numbered with the row tiles of one (expert, weight tile) adjacent: CTAs that take
 // neighbouring items stream the same weights at the same time and the second reader
-// finds them in L2.  Warps: 0 TMA producer (weights, all block scales), 2 TMA producer
+// finds them in L2.  Warps: 0 TMA producer (weights), 2 TMA producer
 // (token terms), 1 and 3 MMA issuers (one per weight tile; 1 alone for a tile of more than 64 rows), 4-7
-// scale writers (shared memory -> tensor memory, one lane quadrant each), 8-23
+// scale writers (global -> shared -> tensor memory, one lane quadrant each), 8-23
 // epilogue.  All barrier waits are bounded.
 #include "k3_grouped.h"
 #include "k3_moe_ops.h"
@@ -62,6 +62,7 @@ constexpr uint32_t kSfwCol = 256;                         // weight scales: kSfB
 constexpr uint32_t kSftCol = kSfwCol + 32u * kSfBatches;  // token scales: kSfBatches x 4 stages x 4 columns
 constexpr uint32_t kMaxGroups = 1024;
 constexpr uint32_t kItemSlots = 4;                        // mailbox of item numbers, producer -> other roles
+constexpr uint32_t kItemLead = 16;                        // stages by which an item is published ahead of its stream
 constexpr uint32_t kItemReaders = 7u + kEpilogueWarps;    // term producer, 2 issuers, 4 writers, epilogue warps
 constexpr uint32_t kNoItem = 0xffffffffu;
 constexpr uint32_t kBarBytes = 512;
@@ -145,6 +146,8 @@ K3_DEVINL uint32_t pack_bf16x2(float lo, float hi) {
 struct GmxArgs {
     const uint32_t *offsets;             // [groups+1]
     k3_group_parts parts;
+    const uint8_t *sfa0, *sfa1;          // weight block scales [groups * w_rows, k / 32], tile 0 / tile 1
+    const uint8_t *sfb;                  // token block scales [rows, k / 32]
     uint16_t *out;                       // bf16 [rows, out_width] (may be null in gate/up mode)
     uint8_t *act_hi, *act_lo, *act_sf;   // gate/up mode: E4M3 terms and block scales of the activation
     uint32_t groups, rows, row_floor, row_ceil, w_rows, k, out_width, m_items;   // groups of row_floor < rows <= row_ceil
@@ -247,8 +250,6 @@ struct AccBuffers {
 struct GmxMaps {
     CUtensorMap a0, a1;        // packed E2M1 weights (4-bit elements, expanded by the copy)
     CUtensorMap bhi, blo;      // token terms, E4M3 bytes
-    CUtensorMap sfa0, sfa1;    // weight block scales [rows, K/32]
-    CUtensorMap sfb;           // token block scales  [rows, K/32]
 };
 
 // 32 bytes of one thread in one store where the address allows it (whole sectors)
@@ -357,7 +358,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             mbar_init(&sf_empty[b], 2);
         }
         for (uint32_t b = 0; b < kSfSlots; b++) {
-            mbar_init(&sfs_full[b], 1);
+            mbar_init(&sfs_full[b], 4u * kWarp);     // every thread of the scale writers
             mbar_init(&sfs_empty[b], 4);
         }
         for (uint32_t b = 0; b < 2u; b++) {
@@ -431,6 +432,10 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         }
         return w;
     };
+    auto item_published = [&]() -> bool {                 // would next_item_warp() return at once?
+        const bool ready = lane == 0 && mbar_test(&item_full[item_seq % kItemSlots], (item_seq / kItemSlots) & 1u);
+        return __any_sync(0xffffffffu, ready);
+    };
     auto next_item_warp = [&]() -> uint32_t {
         uint32_t w = kNoItem;
         if (lane == 0) w = next_item();
@@ -438,38 +443,31 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
     };
 
     if (warp == 0) {
-        // ================================ TMA producer: weights and block scales; draws the items
+        // ================================ TMA producer: weights; draws the items
+        // The next item is published kItemLead stages before this one's stream ends, so that the scale
+        // writers can ask for its first scales while this one's last stages are multiplied.
         if (elect_one()) {
             prefetch_tensormap(&maps.a0);
             prefetch_tensormap(&maps.a1);
-            prefetch_tensormap(&maps.sfa0);
-            prefetch_tensormap(&maps.sfa1);
-            prefetch_tensormap(&maps.sfb);
-            uint32_t s = 0, ph = 0, ss = 0, ssph = 0, seq = 0;
-            bool ok = true;
-            uint32_t w = atomicAdd(a.item_counter, 1u);
-            while (ok) {
+            uint32_t s = 0, ph = 0, seq = 0;
+            auto publish = [&](uint32_t w) -> bool {
                 const uint32_t slot = seq % kItemSlots, parity = (seq / kItemSlots) & 1u;
                 seq++;
-                if (!mbar_wait(&item_empty[slot], parity ^ 1u, abort_flag)) break;
-                const bool valid = w < total_items;
-                item_box[slot] = valid ? w : kNoItem;
+                if (!mbar_wait(&item_empty[slot], parity ^ 1u, abort_flag)) return false;
+                item_box[slot] = w < total_items ? w : kNoItem;
                 mbar_arrive(&item_full[slot]);
-                if (!valid) break;
+                return true;
+            };
+            const uint32_t draw_at = steps > kItemLead + 1u ? steps - kItemLead - 1u : 0u;
+            uint32_t w = atomicAdd(a.item_counter, 1u);
+            bool ok = publish(w);
+            while (ok && w < total_items) {
                 const Item it = decode_item(w, prefix, a);
-                w = atomicAdd(a.item_counter, 1u);                 // the next draw travels while this item streams
                 const int32_t y0 = (int32_t)(it.group * a.w_rows + it.m_item * tile_rows);
                 const int32_t y1 = kE == kEAct ? y0 : y0 + (int32_t)BM;
                 for (uint32_t st = 0; st < steps; st++) {
-                    if ((st & 3u) == 0u) {                 // scales, four stages at a time
-                        if (!mbar_wait(&sfs_empty[ss], ssph ^ 1u, abort_flag)) { ok = false; break; }
-                        unsigned char *sf = sf_smem + ss * kSfSlotBytes;
-                        mbar_arrive_expect_tx(&sfs_full[ss], kSfSlotBytes);
-                        tma_load_2d(sf, &maps.sfa0, &sfs_full[ss], (int32_t)(st * 4u), y0);
-                        tma_load_2d(sf + kSfKind, &maps.sfa1, &sfs_full[ss], (int32_t)(st * 4u), y1);
-                        tma_load_2d(sf + 2u * kSfKind, &maps.sfb, &sfs_full[ss], (int32_t)(st * 4u), (int32_t)it.row_start);
-                        if (++ss == kSfSlots) { ss = 0; ssph ^= 1u; }
-                    }
+                    if (st == draw_at) w = atomicAdd(a.item_counter, 1u);      // travels during this stage
+                    if (st == draw_at + 1u && !publish(w)) { ok = false; break; }
                     if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag)) { ok = false; break; }
                     unsigned char *dst = base + s * kStageBytes;
                     const int32_t x = (int32_t)(st * KS);
@@ -575,58 +573,92 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             }
         }
     } else if (warp < 8) {
-        // ================== scale writers: shared memory -> tensor memory
+        // ================== scale writers: global -> shared -> tensor memory
         // A scale column holds rows 32c .. 32c+31 (lane = row % 32), the same in every
         // lane quadrant; each warp fills its own quadrant.  One batch = 4 stages =
-        // 16 columns per table.
+        // 16 columns per table.  A thread fetches the 16 scale bytes of one row of each table, three
+        // batches before they are stored: by TMA boxes of 128 x 16 bytes, issued with the
+        // weights of the batch's first stage, they came late (the batch has three stages to get here)
+        // and took a sixth of the copy unit's rows (256 rows per expert: gate/up and down 2.81 ms,
+        // 2.21 without any scales).
         const uint32_t quad = warp & 3u;
         const uint32_t lane_base = (32u * quad) << 16;
+        const uint32_t row = 32u * quad + lane, kb = a.k / 32u;
         uint32_t sb = 0, sph = 0, ss = 0, ssph = 0;
-        bool ok = true;
-        for (uint32_t w = next_item_warp(); ok && w != kNoItem; w = next_item_warp()) {
-            // a stacked operand's lo rows have the scales of its hi rows
-            const uint32_t repeat = term_layout<kStages>(decode_item(w, prefix, a)).block / 32u - 1u;
-            for (uint32_t st = 0; st < steps; st += 4u) {
-                if (!mbar_wait(&sfs_full[ss], ssph, abort_flag)) { ok = false; break; }
-                const unsigned char *src = sf_smem + ss * kSfSlotBytes;
-                uint4 v[3][4];
-#pragma unroll
-                for (uint32_t t = 0; t < 3u; t++)
-#pragma unroll
-                    for (uint32_t c = 0; c < 4u; c++)
-                        v[t][c] = *reinterpret_cast<const uint4 *>(
-                            src + t * kSfKind + (32u * (t == 2u ? c & repeat : c) + lane) * 16u);
-                if (!mbar_wait(&sf_empty[sb], sph ^ 1u, abort_flag)) { ok = false; break; }
-                tc_fence_after();
-                // a stage's columns: tile 0 | tile 1 side by side (rows 0..255 of one operand)
-                const uint32_t w01[16] = {v[0][0].x, v[0][1].x, v[0][2].x, v[0][3].x,
-                                          v[1][0].x, v[1][1].x, v[1][2].x, v[1][3].x,
-                                          v[0][0].y, v[0][1].y, v[0][2].y, v[0][3].y,
-                                          v[1][0].y, v[1][1].y, v[1][2].y, v[1][3].y};
-                tmem_st_32x16(tmem + lane_base + kSfwCol + sb * 32u, w01);
-                const uint32_t w23[16] = {v[0][0].z, v[0][1].z, v[0][2].z, v[0][3].z,
-                                          v[1][0].z, v[1][1].z, v[1][2].z, v[1][3].z,
-                                          v[0][0].w, v[0][1].w, v[0][2].w, v[0][3].w,
-                                          v[1][0].w, v[1][1].w, v[1][2].w, v[1][3].w};
-                tmem_st_32x16(tmem + lane_base + kSfwCol + sb * 32u + 16u, w23);
-                const uint32_t tok[16] = {v[2][0].x, v[2][1].x, v[2][2].x, v[2][3].x,
-                                          v[2][0].y, v[2][1].y, v[2][2].y, v[2][3].y,
-                                          v[2][0].z, v[2][1].z, v[2][2].z, v[2][3].z,
-                                          v[2][0].w, v[2][1].w, v[2][2].w, v[2][3].w};
-                tmem_st_32x16(tmem + lane_base + kSftCol + sb * 16u, tok);
-                // The shared-memory slot goes back to the TMA producer only now: the
-                // stores above consumed every loaded register, so the loads have
-                // completed (an arrive right after issuing them would not wait for that).
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sfs_empty[ss]);
-                if (++ss == kSfSlots) { ss = 0; ssph ^= 1u; }
-                tmem_st_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sf_full[sb]);
-                if (++sb == kSfBatches) { sb = 0; sph ^= 1u; }
+        uint32_t fs = 0, fph = 0, left = 0, pending = 0;       // fetching side: slot, batches left in its item
+        const uint8_t *p0 = nullptr, *p1 = nullptr, *pt = nullptr;
+        bool ok = true, more = true;
+        // One batch's copies.  While batches are pending it does not wait for an item that is not
+        // published yet: the items in front would then wait for scales that this warp holds back.
+        auto fetch = [&]() -> bool {
+            if (left == 0u) {
+                if (pending != 0u && !item_published()) return false;
+                const uint32_t w = next_item_warp();
+                if (w == kNoItem) { more = false; return false; }
+                const Item it = decode_item(w, prefix, a);
+                const uint64_t y0 = (uint64_t)it.group * a.w_rows + it.m_item * tile_rows + row;
+                p0 = a.sfa0 + y0 * kb;
+                p1 = a.sfa1 + (kE == kEAct ? y0 : y0 + BM) * kb;
+                // a stacked operand's lo rows have the scales of its hi rows; rows past the end repeat the last
+                const uint32_t r = min(row & (term_layout<kStages>(it).block - 1u), it.rows_valid - 1u);
+                pt = a.sfb + (uint64_t)(it.row_start + r) * kb;
+                left = steps / 4u;
             }
+            if (!mbar_wait(&sfs_empty[fs], fph ^ 1u, abort_flag)) { ok = false; return false; }
+            unsigned char *dst = sf_smem + fs * kSfSlotBytes + row * 16u;
+            cp_async_16(dst, p0);
+            cp_async_16(dst + kSfKind, p1);
+            cp_async_16(dst + 2u * kSfKind, pt);
+            cp_async_arrive(&sfs_full[fs]);
+            p0 += 16;
+            p1 += 16;
+            pt += 16;
+            left--;
+            pending++;
+            if (++fs == kSfSlots) { fs = 0; fph ^= 1u; }
+            return true;
+        };
+        while (true) {
+            while (ok && more && pending + 1u < kSfSlots && fetch()) {
+            }
+            if (!ok || pending == 0u) break;
+            if (!mbar_wait(&sfs_full[ss], ssph, abort_flag)) break;
+            const unsigned char *src = sf_smem + ss * kSfSlotBytes;
+            auto rows_of = [&](uint32_t t, uint4 (&v)[4]) {
+#pragma unroll
+                for (uint32_t c = 0; c < 4u; c++)
+                    v[c] = *reinterpret_cast<const uint4 *>(src + t * kSfKind + (32u * c + lane) * 16u);
+            };
+            uint4 v0[4], v1[4];
+            rows_of(0u, v0);
+            rows_of(1u, v1);
+            if (!mbar_wait(&sf_empty[sb], sph ^ 1u, abort_flag)) break;
+            tc_fence_after();
+            // a stage's columns: tile 0 | tile 1 side by side (rows 0..255 of one operand)
+            const uint32_t w01[16] = {v0[0].x, v0[1].x, v0[2].x, v0[3].x, v1[0].x, v1[1].x, v1[2].x, v1[3].x,
+                                      v0[0].y, v0[1].y, v0[2].y, v0[3].y, v1[0].y, v1[1].y, v1[2].y, v1[3].y};
+            tmem_st_32x16(tmem + lane_base + kSfwCol + sb * 32u, w01);
+            const uint32_t w23[16] = {v0[0].z, v0[1].z, v0[2].z, v0[3].z, v1[0].z, v1[1].z, v1[2].z, v1[3].z,
+                                      v0[0].w, v0[1].w, v0[2].w, v0[3].w, v1[0].w, v1[1].w, v1[2].w, v1[3].w};
+            tmem_st_32x16(tmem + lane_base + kSfwCol + sb * 32u + 16u, w23);
+            rows_of(2u, v0);
+            const uint32_t tok[16] = {v0[0].x, v0[1].x, v0[2].x, v0[3].x, v0[0].y, v0[1].y, v0[2].y, v0[3].y,
+                                      v0[0].z, v0[1].z, v0[2].z, v0[3].z, v0[0].w, v0[1].w, v0[2].w, v0[3].w};
+            tmem_st_32x16(tmem + lane_base + kSftCol + sb * 16u, tok);
+            // The shared-memory slot is given back only now: the stores above consumed every
+            // loaded register, so the loads have completed (an arrive right after issuing
+            // them would not wait for that).
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sfs_empty[ss]);
+            if (++ss == kSfSlots) { ss = 0; ssph ^= 1u; }
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sf_full[sb]);
+            if (++sb == kSfBatches) { sb = 0; sph ^= 1u; }
+            pending--;
         }
+        cp_async_wait_all();
     } else {
         // ======================================================== epilogue
         // Sixteen warps: quadrant = warp % 4 (tensor-memory lanes), the accumulators' columns in
@@ -889,7 +921,7 @@ struct Operands {
 // so a steady-state pass encodes nothing; when the table is full it starts over.
 struct MapKey {
     int device, mode;
-    const void *p[7];
+    const void *p[4];
     uint32_t dims[4];
     bool operator<(const MapKey &o) const {
         if (device != o.device) return device < o.device;
@@ -907,8 +939,11 @@ bool launch(const Operands &op, GmxArgs args, bool few, cudaStream_t stream) {
     MapKey key{};
     key.device = current_device();
     key.mode = kE;
-    const void *ptrs[7] = {op.a0, op.a1, op.sfa0, op.sfa1, op.bhi, op.blo, op.sfb};
+    const void *ptrs[4] = {op.a0, op.a1, op.bhi, op.blo};
     memcpy(key.p, ptrs, sizeof(ptrs));
+    args.sfa0 = (const uint8_t *)op.sfa0;
+    args.sfa1 = (const uint8_t *)op.sfa1;
+    args.sfb = op.sfb;
     key.dims[0] = args.groups; key.dims[1] = args.w_rows; key.dims[2] = args.k; key.dims[3] = args.rows;
     GmxMaps maps;
     {
@@ -916,17 +951,13 @@ bool launch(const Operands &op, GmxArgs args, bool few, cudaStream_t stream) {
         auto it = cached.find(key);
         if (it == cached.end()) {
             const uint64_t w_total = (uint64_t)args.groups * args.w_rows;
-            const uint64_t kb = args.k / 32u;
             const auto u4 = CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B;
             const auto u8 = CU_TENSOR_MAP_DATA_TYPE_UINT8;
-            const auto sw = CU_TENSOR_MAP_SWIZZLE_128B, none = CU_TENSOR_MAP_SWIZZLE_NONE;
+            const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
             if (!map_2d(&maps.a0, op.a0, u4, w_total, args.k, args.k / 2u, 128, BM, sw, 32u) ||
                 !map_2d(&maps.a1, op.a1, u4, w_total, args.k, args.k / 2u, 128, BM, sw, 32u) ||
                 !map_2d(&maps.bhi, op.bhi, u8, args.rows, args.k, args.k, 128, kBBox, sw, 16u) ||
-                !map_2d(&maps.blo, op.blo, u8, args.rows, args.k, args.k, 128, kBBox, sw, 16u) ||
-                !map_2d(&maps.sfa0, op.sfa0, u8, w_total, kb, kb, 16, BM, none, 16u) ||
-                !map_2d(&maps.sfa1, op.sfa1, u8, w_total, kb, kb, 16, BM, none, 16u) ||
-                !map_2d(&maps.sfb, op.sfb, u8, args.rows, kb, kb, 16, BN, none, 16u)) {
+                !map_2d(&maps.blo, op.blo, u8, args.rows, args.k, args.k, 128, kBBox, sw, 16u)) {
                 return false;
             }
             if (cached.size() >= kCachedSets) cached.clear();

@@ -340,7 +340,7 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
             }
         }
     } else if (warp == 2) {
-        // ================================ TMA producer: token terms; lane i knows row i of the tile
+        // ================================ TMA producer: token terms; lane i brings row i of the tile
         if (lane == 0) prefetch_tensormap(&maps.b);
         uint32_t s = 0, ph = 0;
         bool ok = true;
@@ -356,11 +356,8 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
                 }
                 ok = __shfl_sync(0xffffffffu, ok ? 1u : 0u, 0) != 0u;
                 if (!ok) break;
-                for (uint32_t i = 0; i < it.rows_valid; i++) {
-                    const int32_t row_y = __shfl_sync(0xffffffffu, y, (int)i);
-                    if (elect_one())
-                        tma_load_3d(b_smem + s * kBSlotBytes + i * 2u * kBAtom, &maps.b, &b_full[s], 0, row_y, (int32_t)st);
-                }
+                if (mine)
+                    tma_load_3d(b_smem + s * kBSlotBytes + lane * 2u * kBAtom, &maps.b, &b_full[s], 0, y, (int32_t)st);
                 if (++s == kBSlots) { s = 0; ph ^= 1u; }
             }
         }

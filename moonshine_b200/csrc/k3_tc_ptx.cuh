@@ -55,6 +55,19 @@ K3_DEVINL bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     return ok != 0;
 }
 
+// has the phase of this parity completed? (does not wait)
+K3_DEVINL bool mbar_test(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait: gives up two seconds after it started (wall clock of the
 // device) or as soon as another thread of the CTA gave up (abort_flag in shared
 // memory).  Returns false on give-up.
@@ -127,6 +140,17 @@ K3_DEVINL void tma_prefetch_2d(const void *map, int32_t x, int32_t y) {
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y)
                  : "memory");
 }
+
+// ------------------------------------------------------------- asynchronous copies
+// 16 bytes global -> shared memory of one thread (both 16-byte aligned)
+K3_DEVINL void cp_async_16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+// one arrival of this thread on `bar` (counted in its initial value) when its copies so far are done
+K3_DEVINL void cp_async_arrive(uint64_t *bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+K3_DEVINL void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // -------------------------------------------------------------- tensor memory
 K3_DEVINL void tmem_alloc(uint32_t *dst_smem, uint32_t columns) {
