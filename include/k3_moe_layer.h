@@ -147,11 +147,12 @@ bool k3_moe_experts_grouped_ws(const k3_moe_layer_desc *desc, void *rows_out,
 
 /* The same for a part of a larger pass (no counterpart in the reference): the
  * rows get the bits they have when the whole pass is one call.  The order in
- * which a row's sums are added depends on how many rows its group has and, above
- * 64, on its place among them, so a part that is computed by itself differs from
- * the whole pass in the last bits.  group_rows: u32 [local_expert_count] on the
- * device, rows of each group in the whole pass; place: u32 [rows], place of each
- * row in its group there, ascending within a group.  Fails where
+ * which a row's sums are added depends on how many rows its group has (up to 16,
+ * up to 64, more), so a part that is computed by itself differs from the whole
+ * pass in the last bits.  group_rows: u32 [local_expert_count] on the device,
+ * rows of each group in the whole pass; place: u32 [rows], place of each row in
+ * its group there, ascending within a group (no longer read: all row tiles of a
+ * group add a row's sums in one order).  Fails where
  * k3_moe_experts_workspace_bytes is 0 (fewer than 32 rows, or a shape that does
  * not suit the path) or the workspace is smaller. */
 bool k3_moe_experts_grouped_part(const k3_moe_layer_desc *desc, void *rows_out,

@@ -131,7 +131,6 @@ struct k3_token_routes {
 // pass: the rows of the call are a part of a larger pass and get the bits they have there.
 struct k3_part_of_pass {
     const void *group_rows;    // u32 [groups] rows of a group in the whole pass
-    const void *place;         // u32 [rows] place of a row in its group there, ascending within a group
 };
 bool k3_grouped_mx_supported(const k3_moe_layer_desc *desc, uint32_t rows);
 size_t k3_grouped_mx_workspace_bytes(const k3_moe_layer_desc *desc, uint32_t rows,
@@ -143,9 +142,8 @@ bool k3_grouped_mx_experts(const k3_moe_layer_desc *desc, void *rows_out, void *
                            const k3_part_of_pass *pass = nullptr);
 uint32_t k3_grouped_mx_status();
 constexpr uint32_t k3_mx4_rows = 16;
-// What decides a group's kernel and operand layout when its rows here are a part of a pass: u32
-// [groups][2], its rows in the whole pass and how many of the rows here lie in the pass's stacked
-// tile (k3_grouped_mx.cu).  A null table: the call is the whole pass.
+// What decides a group's kernel when its rows here are a part of a pass: u32 [groups], its rows in
+// the whole pass.  A null table: the call is the whole pass.
 struct k3_group_parts {
     const uint32_t *table;
 };

@@ -12,7 +12,7 @@
 // the rest is held to 2^-17 of the block maximum.  Each K block of 32 issues two
 // MMAs (hi and lo against the same weights and scales).
 //
-// Work item = two 128-row weight tiles x up to 128 token rows of one group over
+// Work item = two 128-row weight tiles x up to 160 token rows of one group over
 // the whole K extent (gate+up with fused activation, or 256 rows of the down
 // projection).  One CTA per SM, persistent; the item list is derived in-kernel from the
 // group offsets and handed out by a global counter: the weight producer takes the next
@@ -21,7 +21,7 @@
 // are numbered with the row tiles of one (expert, weight tile) adjacent: CTAs that take
 // neighbouring items stream the same weights at the same time and the second reader
 // finds them in L2.  Warps: 0 TMA producer (weights), 2 TMA producer
-// (token terms), 1 and 3 MMA issuers (one per weight tile; 1 alone for a tile of more than 64 rows), 4-7
+// (token terms), 1 and 3 MMA issuers (one per weight tile), 4-7
 // scale writers (global -> shared -> tensor memory, one lane quadrant each), 8-23
 // epilogue.  All barrier waits are bounded.
 #include "k3_grouped.h"
@@ -43,31 +43,54 @@ using namespace k3::tc;
 
 namespace {
 
-constexpr uint32_t BM = 128, BN = 128, KS = 128;          // K per pipeline stage
+constexpr uint32_t BM = 128, KS = 128;                    // weight rows per tile, K per pipeline stage
 constexpr uint32_t kATile = BM * 128u;                    // bytes in shared memory (8-bit containers)
 constexpr uint32_t kATx = BM * 64u;                       // bytes the TMA transaction counts (packed)
-constexpr uint32_t kBTile = BN * 128u;
 constexpr uint32_t kBBox = 32u;                           // token rows per TMA box
-constexpr uint32_t kRingBytes = 192u * 1024u;             // stages of A0 | A1 | token terms: three of 64 KB, or four of
-                                                          //   48 KB where no tile has more than 64 rows
 constexpr uint32_t kEpilogueWarps = 16;
 constexpr uint32_t kThreads = (8u + kEpilogueWarps) * 32u;   // 24 warps
-constexpr uint32_t kSfBatches = 3;                        // scale ring in tensor memory: batches of 4 stages
-constexpr uint32_t kSfSlots = 4;                          // scale ring in shared memory
-constexpr uint32_t kSfKind = BM * 16u;                    // one table's 128 rows x 16 scale bytes
-constexpr uint32_t kSfSlotBytes = 3u * kSfKind;           // SFA0 | SFA1 | SFB
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kAccCol = 0;                           // tile 0: [0,128), tile 1: [128,256)
-constexpr uint32_t kSfwCol = 256;                         // weight scales: kSfBatches x 4 stages x (tile 0 | tile 1)
-constexpr uint32_t kSftCol = kSfwCol + 32u * kSfBatches;  // token scales: kSfBatches x 4 stages x 4 columns
 constexpr uint32_t kMaxGroups = 1024;
 constexpr uint32_t kItemSlots = 4;                        // mailbox of item numbers, producer -> other roles
 constexpr uint32_t kItemLead = 16;                        // stages by which an item is published ahead of its stream
 constexpr uint32_t kItemReaders = 7u + kEpilogueWarps;    // term producer, 2 issuers, 4 writers, epilogue warps
 constexpr uint32_t kNoItem = 0xffffffffu;
-constexpr uint32_t kBarBytes = 512;
-constexpr uint32_t kSmemBytes =
-    kRingBytes + kSfSlots * kSfSlotBytes + 1024u + kBarBytes + (kMaxGroups + 1u) * 4u;
+constexpr uint32_t kBarBytes = 448;                       // barriers, then a few words, then the scan's warp totals
+constexpr uint32_t kStackedRows = 64;
+
+// The two instances.  Groups of up to 64 rows (kMany false): one row tile per group, the hi and the
+// lo rows ONE N operand (lo from row `block` on) with accumulator columns of their own, so that a K
+// block of 32 is one MMA per weight tile and the 8-bit weight containers are read from shared
+// memory once.  Larger groups: row tiles of up to 160 rows, the hi and the lo MMA adding into the
+// same columns.  A tile of 160 rows takes the weights through the copy unit once where a tile
+// of 128 and a remainder took them twice: with 8192 tokens most experts have 129 to 160 rows, and
+// their remainders of a few rows were 29 % of the expert phase.  160 is what fits: three
+// stages of 72 KB, two accumulators of 160 columns beside the scales (192 rows in two stages of
+// 80 KB ran at 1250 useful TFLOP/s, 160 in three at 1300; both operand orders alike).
+template <bool kMany>
+struct Cfg {
+    static constexpr uint32_t kTileRows = kMany ? 160u : kStackedRows;
+    static constexpr uint32_t kTermRows = kMany ? 160u : 2u * kStackedRows;      // rows of the N operand, at most
+    static constexpr uint32_t kStages = kMany ? 3u : 4u;
+    static constexpr uint32_t kStageBytes = 2u * kATile + 2u * kTileRows * 128u; // A0 | A1 | token terms
+    static constexpr uint32_t kSfStages = kMany ? 2u : 4u;                       // stages per scale batch
+    static constexpr uint32_t kSfSlots = kMany ? 2u : 4u;                        // scale ring in shared memory
+    static constexpr uint32_t kSfAhead = kMany ? 2u : 3u;                        // batches under way to it
+    static constexpr uint32_t kSfRow = 4u * kSfStages;                           // scale bytes of a row per batch
+    static constexpr uint32_t kSfSlotBytes = (2u * BM + kTermRows) * kSfRow;     // SFA0 | SFA1 | SFB
+    static constexpr uint32_t kSfBatches = kMany ? 6u : 3u;                      // scale ring in tensor memory
+    static constexpr uint32_t kAccStride = kMany ? 160u : 128u;                  // tile 0 | tile 1
+    static constexpr uint32_t kSftStage = kMany ? 8u : 4u;                       // token scale columns per stage
+    static constexpr uint32_t kSfwCol = 2u * kAccStride;                         // weight scales: 8 columns per stage
+    static constexpr uint32_t kSftCol = kSfwCol + 8u * kSfStages * kSfBatches;
+    static constexpr uint32_t kSpan = kTileRows / 4u;                            // token rows of an epilogue warp, at most
+    static constexpr uint32_t kSmemBytes =
+        kStages * kStageBytes + kSfSlots * kSfSlotBytes + kBarBytes + (kMaxGroups + 1u) * 4u;
+    static_assert(kSftCol + kSftStage * kSfStages * kSfBatches <= kTmemCols, "tensor memory");
+    static_assert(kSmemBytes <= 227u * 1024u, "one CTA's shared memory");
+    static_assert((2u * (kStages + kSfBatches + kSfSlots + 2u + kItemSlots)) * 8u + (3u + kItemSlots + kThreads / 32u) * 4u <= kBarBytes,
+                  "barriers and words");
+};
 
 enum EMode : int { kEAct = 0, kEBf16 = 1 };
 
@@ -98,12 +121,11 @@ K3_DEVINL void mma_mx(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32
         : "memory");
 }
 
-// UE8M0 scales, M = 128, K-major; sf = byte of the scale column (kNextScaleByte: one further).
-// A = weights (E2M1, 5) and B = token terms (E4M3, 0), or the other way round.
+// UE8M0 scales, M = 128, K-major, byte 0 of the scale columns (kNextScaleByte: one further).
+// A = weights (E2M1, 5), B = token terms (E4M3, 0).
 constexpr uint32_t kNextScaleByte = (1u << 29) | (1u << 4);
-K3_DEVINL uint32_t make_idesc_mx(uint32_t n, uint32_t sf, bool tokens_are_a) {
-    return ((tokens_are_a ? 0u : 5u) << 7) | ((tokens_are_a ? 5u : 0u) << 10) | ((n >> 3) << 17) | (1u << 23) |
-           ((128u >> 4) << 24) | (sf << 29) | (sf << 4);
+K3_DEVINL uint32_t make_idesc_mx(uint32_t n) {
+    return (5u << 7) | (0u << 10) | ((n >> 3) << 17) | (1u << 23) | ((128u >> 4) << 24);
 }
 
 // Two-term E4M3 form of a block of 32 values held one per lane:
@@ -158,49 +180,31 @@ struct GmxArgs {
 
 struct Item {
     uint32_t group, row_start, rows_valid, m_item;
-    bool stacked;
 };
 
-// A group's rows are cut into tiles of BN rows; a last tile of at most 64 rows (kSomeRows) is
-// stacked, which adds a row's sums in another order than the larger tiles do.
-constexpr uint32_t kStackedRows = 64;
-K3_DEVINL uint32_t stacked_rows(uint32_t rows) { return rows % BN <= kStackedRows ? rows % BN : 0u; }
-struct GroupShape {
-    uint32_t whole, stacked;             // rows in the pass, rows here that lie in its stacked tile
-};
-K3_DEVINL GroupShape group_shape(const k3_group_parts &parts, uint32_t group, uint32_t rows) {
-    if (parts.table == nullptr) return {rows, stacked_rows(rows)};
-    return {parts.table[2u * group], parts.table[2u * group + 1u]};
+// rows of the group in the whole pass
+K3_DEVINL uint32_t pass_rows(const k3_group_parts &parts, uint32_t group, uint32_t rows) {
+    return parts.table == nullptr ? rows : max(parts.table[group], rows);
 }
 
-// How a row tile's terms lie in shared memory.  Up to 64 rows the hi rows and the lo rows are ONE
-// N operand (lo from row `block` on), so that a K block of 32 is one MMA per weight tile: the
-// 8-bit weight containers are read from shared memory once instead of twice (24 rows per expert:
-// 1.15 -> 1.01 ms together with the fourth stage; without any MMA 0.98, the TMA unit's expansion
-// of the weights at 16 packed bytes per clock and SM).  A larger tile does not fit its
-// accumulators that way (2 x 256 columns): there the terms are the A operand and both weight
-// tiles together the N = 256 operand, and the hi and the lo MMA add into the same columns.  A K
-// block of 32 then takes two MMAs of N = 256 (92 ns each, 12 KB of operands) where the weights
-// as A take four of N = 128 (55 ns, 8 KB), and a result row is stored in whole sectors.  192
-// experts of 128 rows, back to back: 2.72 -> 2.65 ms (first pass of the 8192-token layer 13.03
-// -> 12.96 ms; the power cap hides the rest of it).
+// How a row tile's terms lie in shared memory: hi rows from row 0, lo rows from row `block` on; n
+// rows of the N operand per MMA (hi and lo together where they are stacked).
 struct TermLayout {
     uint32_t block, n;
-    bool stacked;
 };
-template <uint32_t kStages>
+template <bool kMany>
 K3_DEVINL TermLayout term_layout(const Item &it) {
-    TermLayout t;
     const uint32_t n16 = (it.rows_valid + 15u) & ~15u;
-    t.stacked = kStages > 3u || it.stacked;
-    t.block = !t.stacked ? BN : it.rows_valid <= 32u ? 32u : kStackedRows;
-    t.n = t.stacked ? t.block + n16 : 2u * BM;
-    return t;
+    if (kMany) return {Cfg<true>::kTileRows, n16};
+    const uint32_t block = it.rows_valid <= 32u ? 32u : kStackedRows;
+    return {block, block + n16};
 }
 
 // Item w -> (group, weight tile, row tile).  prefix[g] = row tiles of the groups before
 // g; group g owns items [prefix[g] * m_items, prefix[g + 1] * m_items), numbered with
-// the row tile fastest.
+// the row tile fastest.  A group's tiles are as even as multiples of 16 rows allow; none is
+// empty, since their size is at most kTileRows and their number rows / kTileRows rounded up.
+template <bool kMany>
 K3_DEVINL Item decode_item(uint32_t w, const uint32_t *prefix, const GmxArgs &a) {
     Item it;
     const uint32_t nt = w / a.m_items;             // prefix[group] <= nt < prefix[group + 1]
@@ -213,27 +217,28 @@ K3_DEVINL Item decode_item(uint32_t w, const uint32_t *prefix, const GmxArgs &a)
     const uint32_t tiles = prefix[lo + 1u] - prefix[lo];
     const uint32_t j = w - prefix[lo] * a.m_items;
     it.m_item = j / tiles;
-    const uint32_t begin = a.offsets[lo], rows = a.offsets[lo + 1u] - begin, tile = j % tiles;
-    const uint32_t stacked = group_shape(a.parts, lo, rows).stacked, large = rows - stacked;
-    it.stacked = tile * BN >= large;
-    it.row_start = begin + (it.stacked ? large : tile * BN);
-    it.rows_valid = it.stacked ? stacked : min(BN, large - tile * BN);
+    const uint32_t begin = a.offsets[lo], rows = a.offsets[lo + 1u] - begin, first = j % tiles *
+        (kMany ? ((rows + tiles - 1u) / tiles + 15u) & ~15u : kStackedRows);
+    it.row_start = begin + first;
+    it.rows_valid = min(kMany ? ((rows + tiles - 1u) / tiles + 15u) & ~15u : kStackedRows, rows - first);
     return it;
 }
 
-// Accumulator columns [0, 256) as two buffers of 128: a row tile of at most 32 rows (N <= 64)
-// takes one buffer (tile 0 in its first 64 columns, tile 1 in the other 64), so that its MMAs
-// run while the epilogue still reads the item before; a larger tile takes both (tile 0 in
-// [0, 128), tile 1 in [128, 256)).  Issuers and epilogue warps walk the items in the same
-// order and keep the same books: uses per buffer (the barriers' phase) and whose turn it is.
+// Accumulator columns [0, 256) of the instance for smaller groups as two buffers of 128: a row
+// tile of at most 32 rows (N <= 64) takes one buffer (tile 0 in its first 64 columns, tile 1 in
+// the other 64), so that its MMAs run while the epilogue still reads the item before; a larger
+// tile takes both (tile 0 in [0, 128), tile 1 in [128, 256)), and so does every tile of the other
+// instance.  Issuers and epilogue warps walk the items in the same order and keep the same books:
+// uses per buffer (the barriers' phase) and whose turn it is.
+template <bool kMany>
 struct AccBuffers {
     uint32_t use0 = 0u, use1 = 0u;
     uint32_t turn = 0u;
     __device__ uint32_t uses(uint32_t b) const { return b == 0u ? use0 : use1; }
-    __device__ bool small(const Item &it) const { return it.stacked && it.rows_valid <= 32u; }
+    __device__ bool small(const Item &it) const { return !kMany && it.rows_valid <= 32u; }
     __device__ uint32_t first(bool is_small) const { return is_small ? turn : 0u; }
     __device__ uint32_t column(bool is_small, uint32_t b0, uint32_t tile) const {
-        return is_small ? b0 * 128u + tile * 64u : tile * BN;
+        return is_small ? b0 * 128u + tile * 64u : tile * Cfg<kMany>::kAccStride;
     }
     __device__ void advance(bool is_small, uint32_t b0) {
         if (is_small) {
@@ -252,87 +257,16 @@ struct GmxMaps {
     CUtensorMap bhi, blo;      // token terms, E4M3 bytes
 };
 
-// 32 bytes of one thread in one store where the address allows it (whole sectors)
-K3_DEVINL void store_32_bytes(void *p, const uint32_t (&v)[8], bool aligned) {
-    if (aligned) {
-        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]),
-                     "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-                     : "memory");
-    } else {
-#pragma unroll
-        for (uint32_t j = 0; j < 8u; j++) {
-            reinterpret_cast<uint16_t *>(p)[2u * j] = (uint16_t)v[j];
-            reinterpret_cast<uint16_t *>(p)[2u * j + 1u] = (uint16_t)(v[j] >> 16);
-        }
-    }
-}
-// 16 bf16 values to out[at ...]
-K3_DEVINL void store_16_values(uint16_t *out, uint64_t at, const uint32_t (&v)[8]) {
-    store_32_bytes(out + at, v, (reinterpret_cast<uintptr_t>(out) & 31u) == 0);     // rows are multiples of 512 columns
-}
-
-// One result row's columns c .. c + 31 (tile 0, low halves of `pair`) and the same of tile 1
-// (high halves): activation, two-term split and stores, or plain stores.
-template <int kE>
-K3_DEVINL void store_row(const GmxArgs &a, uint64_t row, uint32_t c, uint32_t (&pair)[32]) {
-    uint32_t v[8];
-    if (kE == kEAct) {
-        uint32_t mx = 0u;
-#pragma unroll
-        for (uint32_t j = 0; j < 16u; j++) {              // two bf16 results in one register
-            const uint32_t p0 = pair[2u * j], p1 = pair[2u * j + 1u];
-            const uint32_t b0 =
-                float_to_bf16_bits(activation(bf16_lo(p0), bf16_hi(p0), a.activation, a.beta, a.linear_beta));
-            const uint32_t b1 =
-                float_to_bf16_bits(activation(bf16_lo(p1), bf16_hi(p1), a.activation, a.beta, a.linear_beta));
-            mx = max(mx, max(b0 & 0x7fffu, b1 & 0x7fffu));
-            pair[j] = b0 | (b1 << 16);
-        }
-        if (a.out != nullptr) {
-#pragma unroll
-            for (uint32_t h = 0; h < 2u; h++) {
-#pragma unroll
-                for (uint32_t j = 0; j < 8u; j++) v[j] = pair[8u * h + j];
-                store_16_values(a.out, row * a.out_width + c + 16u * h, v);
-            }
-        }
-        const uint32_t be = min(max(mx >> 7, 8u), 254u);  // as block_scale()
-        const float mult = __uint_as_float((261u - be) << 23);
-        uint32_t lo[8];
-#pragma unroll
-        for (uint32_t j = 0; j < 8u; j++) {
-            const uint32_t p0 = split_pair(bf16_lo(pair[2u * j]) * mult, bf16_hi(pair[2u * j]) * mult);
-            const uint32_t p1 = split_pair(bf16_lo(pair[2u * j + 1u]) * mult, bf16_hi(pair[2u * j + 1u]) * mult);
-            v[j] = (p0 & 0xffffu) | (p1 << 16);
-            lo[j] = (p0 >> 16) | (p1 & 0xffff0000u);
-        }
-        store_32_bytes(a.act_hi + row * a.w_rows + c, v, true);      // buffers of the workspace: aligned
-        store_32_bytes(a.act_lo + row * a.w_rows + c, lo, true);
-        a.act_sf[row * (a.w_rows / 32u) + c / 32u] = (uint8_t)block_scale_byte(mx >> 7);
-    } else {
-#pragma unroll
-        for (uint32_t h = 0; h < 4u; h++) {               // tile 0's columns, then tile 1's
-#pragma unroll
-            for (uint32_t j = 0; j < 8u; j++)
-                v[j] = __byte_perm(pair[16u * (h & 1u) + 2u * j], pair[16u * (h & 1u) + 2u * j + 1u],
-                                   h < 2u ? 0x5410 : 0x7632);
-            store_16_values(a.out, row * a.out_width + c + (h >> 1) * BM + 16u * (h & 1u), v);
-        }
-    }
-}
-
-// kStages stages in flight: four where every group has at most 64 rows (the weight stream bounds
-// those), else three.  Weights and terms of a stage share their barriers: an issuer's commits
-// cost about 0.1 us each, and with separate rings (two commits per stage) 128 rows per expert
-// took 2.07 ms instead of 1.89.
-template <int kE, uint32_t kStages>
+// Weights and terms of a stage share their barriers.
+template <int kE, bool kMany>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char *base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    constexpr uint32_t kStageBytes = kRingBytes / kStages;
-    unsigned char *sf_smem = base + kRingBytes;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sf_smem + kSfSlots * kSfSlotBytes);
+    using C = Cfg<kMany>;
+    constexpr uint32_t kStages = C::kStages, kStageBytes = C::kStageBytes, kSfSlots = C::kSfSlots;
+    constexpr uint32_t kSfBatches = C::kSfBatches, kSfStages = C::kSfStages;
+    extern __shared__ __align__(1024) unsigned char base[];      // the swizzled stages start on multiples of 1024
+    unsigned char *sf_smem = base + kStages * kStageBytes;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sf_smem + kSfSlots * C::kSfSlotBytes);
     uint64_t *full = bars, *empty = full + kStages;
     uint64_t *sf_full = empty + kStages, *sf_empty = sf_full + kSfBatches;
     uint64_t *sfs_full = sf_empty + kSfBatches, *sfs_empty = sfs_full + kSfSlots;
@@ -342,6 +276,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
     volatile uint32_t *abort_flag = tmem_slot + 1;
     uint32_t *total_items_s = tmem_slot + 2;
     volatile uint32_t *item_box = tmem_slot + 3;          // [kItemSlots]
+    uint32_t *warp_tot = tmem_slot + 3 + kItemSlots;      // [kThreads / kWarp]
     uint32_t *prefix = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(bars) + kBarBytes);
     const uint32_t warp = warp_index(), lane = threadIdx.x % kWarp;
     const uint32_t steps = a.k / KS;
@@ -379,16 +314,14 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
     // everything before it, and nothing it writes is read here, so this kernel's blocks start as its
     // blocks leave and wait for it only before they end (so that who waits for this one waits for both).
     pdl_trigger();
-    {   // exclusive prefix of ceil(rows_g / BN) over the groups (<= 1024)
-        __shared__ uint32_t warp_tot[kThreads / kWarp];
+    {   // exclusive prefix of the groups' row tiles (<= 1024 groups)
         uint32_t v[2], incl[2], run = 0;
 #pragma unroll
         for (int j = 0; j < 2; j++) {
             const uint32_t g = threadIdx.x * 2u + j;
             const uint32_t n = g < a.groups ? a.offsets[g + 1u] - a.offsets[g] : 0u;
-            const GroupShape shape = n != 0u ? group_shape(a.parts, g, n) : GroupShape{0u, 0u};
-            v[j] = shape.whole > a.row_floor && shape.whole <= a.row_ceil
-                       ? (n - shape.stacked + BN - 1u) / BN + (shape.stacked != 0u ? 1u : 0u) : 0u;
+            const uint32_t whole = n != 0u ? pass_rows(a.parts, g, n) : 0u;
+            v[j] = whole > a.row_floor && whole <= a.row_ceil ? (n + C::kTileRows - 1u) / C::kTileRows : 0u;
             run += v[j];
             incl[j] = run;
         }
@@ -462,7 +395,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             uint32_t w = atomicAdd(a.item_counter, 1u);
             bool ok = publish(w);
             while (ok && w < total_items) {
-                const Item it = decode_item(w, prefix, a);
+                const Item it = decode_item<kMany>(w, prefix, a);
                 const int32_t y0 = (int32_t)(it.group * a.w_rows + it.m_item * tile_rows);
                 const int32_t y1 = kE == kEAct ? y0 : y0 + (int32_t)BM;
                 for (uint32_t st = 0; st < steps; st++) {
@@ -486,9 +419,9 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             uint32_t s = 0, ph = 0;
             bool ok = true;
             for (uint32_t w = next_item(); ok && w != kNoItem; w = next_item()) {
-                const Item it = decode_item(w, prefix, a);
+                const Item it = decode_item<kMany>(w, prefix, a);
                 const uint32_t boxes = (it.rows_valid + kBBox - 1u) / kBBox;
-                const TermLayout t = term_layout<kStages>(it);
+                const TermLayout t = term_layout<kMany>(it);
                 for (uint32_t st = 0; st < steps; st++) {
                     if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag)) { ok = false; break; }
                     const int32_t x = (int32_t)(st * KS);
@@ -506,23 +439,16 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         }
     } else if (warp == 1 || warp == 3) {
         // ==================================================== MMA issuers
-        // One thread's issue loop cannot keep the tensor pipe fed with K = 32 MMAs of N <= 128,
-        // so warp 1 issues the MMAs of weight tile 0 and warp 3 those of tile 1.  Both
-        // commit to the same stage / scale / accumulator barriers (count 2).  The MMAs of a
-        // larger tile all add into one accumulator: warp 1 issues them, warp 3 only arrives.
+        // One per weight tile; both commit to the same stage / scale / accumulator barriers (count 2).
         if (elect_one()) {
             const uint32_t q = warp == 1 ? 0u : 1u;
             uint32_t s = 0, ph = 0, sb = 0, sph = 0;
-            AccBuffers acc;
-            auto release = [](uint64_t *bar, bool bystander) {
-                if (bystander) mbar_arrive(bar); else mma_commit(bar);
-            };
+            AccBuffers<kMany> acc;
             bool ok = true;
             for (uint32_t w = next_item(); ok && w != kNoItem; w = next_item()) {
-                const Item it = decode_item(w, prefix, a);
-                const TermLayout t = term_layout<kStages>(it);
-                const uint32_t idesc = make_idesc_mx(t.n, 0u, !t.stacked);
-                const bool bystander = !t.stacked && q == 1u;
+                const Item it = decode_item<kMany>(w, prefix, a);
+                const TermLayout t = term_layout<kMany>(it);
+                const uint32_t idesc = make_idesc_mx(t.n);
                 const bool small = acc.small(it);
                 const uint32_t b0 = acc.first(small);
                 if (!mbar_wait(&acc_empty[b0], (acc.uses(b0) & 1u) ^ 1u, abort_flag) ||
@@ -530,10 +456,11 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                     break;
                 }
                 tc_fence_after();
-                const uint32_t d = tmem + kAccCol + acc.column(small, b0, q);
+                const uint32_t d = tmem + acc.column(small, b0, q);
                 for (uint32_t st = 0; st < steps; st++) {
+                    const uint32_t in_batch = st % kSfStages;
                     if (!mbar_wait(&full[s], ph, abort_flag) ||
-                        ((st & 3u) == 0u && !mbar_wait(&sf_full[sb], sph, abort_flag))) {
+                        (in_batch == 0u && !mbar_wait(&sf_full[sb], sph, abort_flag))) {
                         ok = false;
                         break;
                     }
@@ -541,52 +468,50 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                     const unsigned char *src = base + s * kStageBytes;
                     const uint64_t dw = make_desc_sw128(smem_u32(src + q * kATile));
                     const uint64_t dhi = make_desc_sw128(smem_u32(src + 2u * kATile));
-                    const uint32_t sfw = tmem + kSfwCol + sb * 32u + (st & 3u) * 8u;
-                    const uint32_t sft = tmem + kSftCol + sb * 16u + (st & 3u) * 4u;
-                    if (t.stacked) {
+                    const uint32_t sfw = tmem + C::kSfwCol + (sb * kSfStages + in_batch) * 8u + 4u * q;
+                    const uint32_t sft = tmem + C::kSftCol + (sb * kSfStages + in_batch) * C::kSftStage;
+                    if (kMany) {
+                        const uint64_t dlo = make_desc_sw128(smem_u32(src + 2u * kATile + C::kTileRows * 128u));
 #pragma unroll
                         for (uint32_t j = 0; j < 4u; j++) {          // K blocks of 32 inside the stage
-                            mma_mx(d, dw + 2u * j, dhi + 2u * j, idesc + j * kNextScaleByte, sfw + 4u * q, sft,
+                            mma_mx(d, dw + 2u * j, dhi + 2u * j, idesc + j * kNextScaleByte, sfw, sft,
                                    (st | j) != 0u ? 1u : 0u);
+                            mma_mx(d, dw + 2u * j, dlo + 2u * j, idesc + j * kNextScaleByte, sfw, sft, 1u);
                         }
-                    } else if (!bystander) {
-                        // weight tiles 0 and 1 lie one behind the other: 256 rows of one operand
-                        const uint64_t dlo = make_desc_sw128(smem_u32(src + 2u * kATile + kBTile));
+                    } else {
 #pragma unroll
-                        for (uint32_t j = 0; j < 4u; j++) {
-                            mma_mx(d, dhi + 2u * j, dw + 2u * j, idesc + j * kNextScaleByte, sft, sfw,
+                        for (uint32_t j = 0; j < 4u; j++)
+                            mma_mx(d, dw + 2u * j, dhi + 2u * j, idesc + j * kNextScaleByte, sfw, sft,
                                    (st | j) != 0u ? 1u : 0u);
-                            mma_mx(d, dlo + 2u * j, dw + 2u * j, idesc + j * kNextScaleByte, sft, sfw, 1u);
-                        }
                     }
-                    release(&empty[s], bystander);
+                    mma_commit(&empty[s]);
                     if (++s == kStages) { s = 0; ph ^= 1u; }
-                    if ((st & 3u) == 3u) {
-                        release(&sf_empty[sb], bystander);
+                    if (in_batch == kSfStages - 1u) {
+                        mma_commit(&sf_empty[sb]);
                         if (++sb == kSfBatches) { sb = 0; sph ^= 1u; }
                     }
                 }
                 if (!ok) break;
-                release(&acc_full[b0], bystander);
-                if (!small) release(&acc_full[1], bystander);
+                mma_commit(&acc_full[b0]);
+                if (!small) mma_commit(&acc_full[1]);
                 acc.advance(small, b0);
             }
         }
     } else if (warp < 8) {
         // ================== scale writers: global -> shared -> tensor memory
         // A scale column holds rows 32c .. 32c+31 (lane = row % 32), the same in every
-        // lane quadrant; each warp fills its own quadrant.  One batch = 4 stages =
-        // 16 columns per table.  A thread fetches the 16 scale bytes of one row of each table, three
-        // batches before they are stored: by TMA boxes of 128 x 16 bytes, issued with the
+        // lane quadrant; each warp fills its own quadrant.  One batch = kSfStages stages.  A thread
+        // fetches the batch's scale bytes of one row of each table, kSfAhead batches
+        // before they are stored: as TMA boxes of 128 rows x 16 bytes, issued with the
         // weights of the batch's first stage, they came late (the batch has three stages to get here)
-        // and took a sixth of the copy unit's rows (256 rows per expert: gate/up and down 2.81 ms,
-        // 2.21 without any scales).
+        // and took a sixth of the rows that the copy unit moves (with the elected issue, both products
+        // of 192 experts, back to back: 128 rows 1935 -> 1717 us, 64 rows 1288 -> 1196).
         const uint32_t quad = warp & 3u;
         const uint32_t lane_base = (32u * quad) << 16;
         const uint32_t row = 32u * quad + lane, kb = a.k / 32u;
         uint32_t sb = 0, sph = 0, ss = 0, ssph = 0;
         uint32_t fs = 0, fph = 0, left = 0, pending = 0;       // fetching side: slot, batches left in its item
-        const uint8_t *p0 = nullptr, *p1 = nullptr, *pt = nullptr;
+        const uint8_t *p0 = nullptr, *p1 = nullptr, *pt = nullptr, *pu = nullptr;
         bool ok = true, more = true;
         // One batch's copies.  While batches are pending it does not wait for an item that is not
         // published yet: the items in front would then wait for scales that this warp holds back.
@@ -595,56 +520,83 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                 if (pending != 0u && !item_published()) return false;
                 const uint32_t w = next_item_warp();
                 if (w == kNoItem) { more = false; return false; }
-                const Item it = decode_item(w, prefix, a);
+                const Item it = decode_item<kMany>(w, prefix, a);
                 const uint64_t y0 = (uint64_t)it.group * a.w_rows + it.m_item * tile_rows + row;
                 p0 = a.sfa0 + y0 * kb;
                 p1 = a.sfa1 + (kE == kEAct ? y0 : y0 + BM) * kb;
                 // a stacked operand's lo rows have the scales of its hi rows; rows past the end repeat the last
-                const uint32_t r = min(row & (term_layout<kStages>(it).block - 1u), it.rows_valid - 1u);
+                const uint32_t r = min(kMany ? row : row & (term_layout<kMany>(it).block - 1u), it.rows_valid - 1u);
                 pt = a.sfb + (uint64_t)(it.row_start + r) * kb;
-                left = steps / 4u;
+                if (kMany) pu = a.sfb + (uint64_t)(it.row_start + min(BM + lane, it.rows_valid - 1u)) * kb;
+                left = steps / kSfStages;
             }
             if (!mbar_wait(&sfs_empty[fs], fph ^ 1u, abort_flag)) { ok = false; return false; }
-            unsigned char *dst = sf_smem + fs * kSfSlotBytes + row * 16u;
-            cp_async_16(dst, p0);
-            cp_async_16(dst + kSfKind, p1);
-            cp_async_16(dst + 2u * kSfKind, pt);
+            unsigned char *dst = sf_smem + fs * C::kSfSlotBytes + row * C::kSfRow;
+            cp_async<C::kSfRow>(dst, p0);
+            cp_async<C::kSfRow>(dst + BM * C::kSfRow, p1);
+            cp_async<C::kSfRow>(dst + 2u * BM * C::kSfRow, pt);
+            if (kMany && quad == 0u) {                       // token rows 128 .. 159
+                cp_async<C::kSfRow>(dst + 3u * BM * C::kSfRow, pu);
+                pu += C::kSfRow;
+            }
             cp_async_arrive(&sfs_full[fs]);
-            p0 += 16;
-            p1 += 16;
-            pt += 16;
+            p0 += C::kSfRow;
+            p1 += C::kSfRow;
+            pt += C::kSfRow;
             left--;
             pending++;
             if (++fs == kSfSlots) { fs = 0; fph ^= 1u; }
             return true;
         };
         while (true) {
-            while (ok && more && pending + 1u < kSfSlots && fetch()) {
+            while (ok && more && pending < C::kSfAhead && fetch()) {
             }
             if (!ok || pending == 0u) break;
             if (!mbar_wait(&sfs_full[ss], ssph, abort_flag)) break;
-            const unsigned char *src = sf_smem + ss * kSfSlotBytes;
-            auto rows_of = [&](uint32_t t, uint4 (&v)[4]) {
+            const unsigned char *src = sf_smem + ss * C::kSfSlotBytes;
+            const uint32_t wcol = tmem + lane_base + C::kSfwCol + sb * kSfStages * 8u;
+            const uint32_t tcol = tmem + lane_base + C::kSftCol + sb * kSfStages * C::kSftStage;
+            if constexpr (kMany) {
+                auto at = [&](uint32_t r) { return *reinterpret_cast<const uint2 *>(src + r * 8u); };
+                uint2 v0[4], v1[4];
 #pragma unroll
-                for (uint32_t c = 0; c < 4u; c++)
-                    v[c] = *reinterpret_cast<const uint4 *>(src + t * kSfKind + (32u * c + lane) * 16u);
-            };
-            uint4 v0[4], v1[4];
-            rows_of(0u, v0);
-            rows_of(1u, v1);
-            if (!mbar_wait(&sf_empty[sb], sph ^ 1u, abort_flag)) break;
-            tc_fence_after();
-            // a stage's columns: tile 0 | tile 1 side by side (rows 0..255 of one operand)
-            const uint32_t w01[16] = {v0[0].x, v0[1].x, v0[2].x, v0[3].x, v1[0].x, v1[1].x, v1[2].x, v1[3].x,
-                                      v0[0].y, v0[1].y, v0[2].y, v0[3].y, v1[0].y, v1[1].y, v1[2].y, v1[3].y};
-            tmem_st_32x16(tmem + lane_base + kSfwCol + sb * 32u, w01);
-            const uint32_t w23[16] = {v0[0].z, v0[1].z, v0[2].z, v0[3].z, v1[0].z, v1[1].z, v1[2].z, v1[3].z,
-                                      v0[0].w, v0[1].w, v0[2].w, v0[3].w, v1[0].w, v1[1].w, v1[2].w, v1[3].w};
-            tmem_st_32x16(tmem + lane_base + kSfwCol + sb * 32u + 16u, w23);
-            rows_of(2u, v0);
-            const uint32_t tok[16] = {v0[0].x, v0[1].x, v0[2].x, v0[3].x, v0[0].y, v0[1].y, v0[2].y, v0[3].y,
-                                      v0[0].z, v0[1].z, v0[2].z, v0[3].z, v0[0].w, v0[1].w, v0[2].w, v0[3].w};
-            tmem_st_32x16(tmem + lane_base + kSftCol + sb * 16u, tok);
+                for (uint32_t c = 0; c < 4u; c++) {
+                    v0[c] = at(32u * c + lane);
+                    v1[c] = at(BM + 32u * c + lane);
+                }
+                if (!mbar_wait(&sf_empty[sb], sph ^ 1u, abort_flag)) break;
+                tc_fence_after();
+                const uint32_t w01[16] = {v0[0].x, v0[1].x, v0[2].x, v0[3].x, v1[0].x, v1[1].x, v1[2].x, v1[3].x,
+                                          v0[0].y, v0[1].y, v0[2].y, v0[3].y, v1[0].y, v1[1].y, v1[2].y, v1[3].y};
+                tmem_st_32x16(wcol, w01);
+                uint2 v[5];
+#pragma unroll
+                for (uint32_t c = 0; c < 5u; c++) v[c] = at(2u * BM + 32u * c + lane);
+                const uint32_t tok[16] = {v[0].x, v[1].x, v[2].x, v[3].x, v[4].x, 0u, 0u, 0u,
+                                          v[0].y, v[1].y, v[2].y, v[3].y, v[4].y, 0u, 0u, 0u};
+                tmem_st_32x16(tcol, tok);
+            } else {
+                auto rows_of = [&](uint32_t t, uint4 (&v)[4]) {
+#pragma unroll
+                    for (uint32_t c = 0; c < 4u; c++)
+                        v[c] = *reinterpret_cast<const uint4 *>(src + (t * BM + 32u * c + lane) * 16u);
+                };
+                uint4 v0[4], v1[4];
+                rows_of(0u, v0);
+                rows_of(1u, v1);
+                if (!mbar_wait(&sf_empty[sb], sph ^ 1u, abort_flag)) break;
+                tc_fence_after();
+                const uint32_t w01[16] = {v0[0].x, v0[1].x, v0[2].x, v0[3].x, v1[0].x, v1[1].x, v1[2].x, v1[3].x,
+                                          v0[0].y, v0[1].y, v0[2].y, v0[3].y, v1[0].y, v1[1].y, v1[2].y, v1[3].y};
+                tmem_st_32x16(wcol, w01);
+                const uint32_t w23[16] = {v0[0].z, v0[1].z, v0[2].z, v0[3].z, v1[0].z, v1[1].z, v1[2].z, v1[3].z,
+                                          v0[0].w, v0[1].w, v0[2].w, v0[3].w, v1[0].w, v1[1].w, v1[2].w, v1[3].w};
+                tmem_st_32x16(wcol + 16u, w23);
+                rows_of(2u, v0);
+                const uint32_t tok[16] = {v0[0].x, v0[1].x, v0[2].x, v0[3].x, v0[0].y, v0[1].y, v0[2].y, v0[3].y,
+                                          v0[0].z, v0[1].z, v0[2].z, v0[3].z, v0[0].w, v0[1].w, v0[2].w, v0[3].w};
+                tmem_st_32x16(tcol, tok);
+            }
             // The shared-memory slot is given back only now: the stores above consumed every
             // loaded register, so the loads have completed (an arrive right after issuing
             // them would not wait for that).
@@ -661,20 +613,17 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         cp_async_wait_all();
     } else {
         // ======================================================== epilogue
-        // Sixteen warps: quadrant = warp % 4 (tensor-memory lanes), the accumulators' columns in
-        // four parts.  A warp takes its part of both accumulators out of tensor memory at once,
-        // rounded to bf16 (which both modes do anyway) and packed in pairs, and frees the
-        // accumulators before it computes anything: a tile of more than 32 rows has no second
-        // buffer, so the MMAs of the next item wait for exactly this.  Lanes are weight rows
-        // and columns token rows, or, in a tile of more than 64 rows, the other way round: a
-        // thread then holds 32 neighbouring columns of one result row (a whole scale block)
-        // and stores them in 32-byte pieces.
+        // Sixteen warps: quadrant = warp % 4 (tensor-memory lanes: weight rows), the accumulators'
+        // columns (token rows) in four parts.  A warp takes its part of both accumulators out of
+        // tensor memory at once, rounded to bf16 (which both modes do anyway) and packed in pairs, and
+        // frees the accumulators before it computes anything: a tile of more than 32 rows has no
+        // second buffer, so the MMAs of the next item wait for exactly this.
         const uint32_t quad = warp & 3u;
         const uint32_t part = (warp - 8u) >> 2;
-        const uint32_t m = 32u * quad + lane;            // tensor-memory lane: weight row, or token row
-        AccBuffers acc;
+        const uint32_t m = 32u * quad + lane;            // weight row inside the tile
+        AccBuffers<kMany> acc;
         for (uint32_t w = next_item_warp(); w != kNoItem; w = next_item_warp()) {
-            const Item it = decode_item(w, prefix, a);
+            const Item it = decode_item<kMany>(w, prefix, a);
             const bool small = acc.small(it);
             const uint32_t b0 = acc.first(small);
             if (!mbar_wait(&acc_full[b0], acc.uses(b0) & 1u, abort_flag) ||
@@ -683,21 +632,21 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
             }
             acc.advance(small, b0);
             tc_fence_after();
-            const uint32_t t0 = tmem + ((32u * quad) << 16) + kAccCol + acc.column(small, b0, 0u);
+            const uint32_t t0 = tmem + ((32u * quad) << 16) + acc.column(small, b0, 0u);
             const uint32_t tile1 = acc.column(small, b0, 1u) - acc.column(small, b0, 0u);
             const uint32_t col0 = it.m_item * tile_rows + m;
             const uint32_t col1 = kE == kEAct ? col0 : col0 + BM;
             const bool in0 = col0 < a.w_rows, in1 = col1 < a.w_rows;
-            const TermLayout t = term_layout<kStages>(it);
-            const uint32_t span = t.block / 4u, c = span * part;         // this warp's token rows
-            uint32_t pair[32];                                           // bf16 of tile 0 | tile 1 << 16
+            const TermLayout t = term_layout<kMany>(it);
+            const uint32_t span = kMany ? (it.rows_valid + 31u) / 32u * 8u : t.block / 4u, c = span * part;   // this warp's token rows
+            uint32_t pair[C::kSpan];                                     // bf16 of tile 0 | tile 1 << 16
 #pragma unroll
-            for (uint32_t i = 0; i < 32u; i += 8u) {
-                if (t.stacked && (i >= span || c + i >= it.rows_valid)) break;
+            for (uint32_t i = 0; i < C::kSpan; i += 8u) {
+                if (i >= span || c + i >= it.rows_valid) break;
                 uint32_t r0[8], r1[8];
                 tmem_ld_32x8(t0 + c + i, r0);
                 tmem_ld_32x8(t0 + tile1 + c + i, r1);
-                if (t.stacked) {
+                if (!kMany) {
                     uint32_t lo[8];
                     tmem_ld_32x8(t0 + t.block + c + i, lo);
                     tmem_ld_wait();
@@ -722,16 +671,11 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                 mbar_arrive(&acc_empty[b0]);
                 if (!small) mbar_arrive(&acc_empty[1]);
             }
-            if (!t.stacked) {
-                if (m < it.rows_valid) store_row<kE>(a, (uint64_t)(it.row_start + m), it.m_item * tile_rows + c, pair);
-                __syncwarp();
-                continue;
-            }
             if (c >= it.rows_valid) continue;
             const uint32_t n_here = min(span, it.rows_valid - c);
             if (kE == kEAct) {
 #pragma unroll
-                for (uint32_t j = 0; j < 32u; j += 2u) {
+                for (uint32_t j = 0; j < C::kSpan; j += 2u) {
                     if (j >= n_here) break;                              // uniform across the warp
                     const uint64_t row = (uint64_t)(it.row_start + c + j);
                     float av[2];
@@ -758,7 +702,7 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
                 }
             } else {
 #pragma unroll
-                for (uint32_t j = 0; j < 32u; j++) {
+                for (uint32_t j = 0; j < C::kSpan; j++) {
                     if (j >= n_here) break;
                     const uint64_t row = (uint64_t)(it.row_start + c + j);
                     if (in0) a.out[row * a.out_width + col0] = (uint16_t)pair[j];
@@ -820,7 +764,7 @@ split_rows_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t *_
             const uint32_t mid = (g + end) >> 1;
             if (offsets[mid] <= r) g = mid; else end = mid;
         }
-        if (group_shape(parts, g, offsets[g + 1u] - offsets[g]).whole <= k3_mx4_rows) continue;
+        if (pass_rows(parts, g, offsets[g + 1u] - offsets[g]) <= k3_mx4_rows) continue;
         const uint16_t *src = x + (uint64_t)(index ? index[r] : r) * k;
         for (uint32_t c = lane * 16u; c < k; c += 512u) {
             const SplitColumns t = split_columns(src + c);
@@ -860,25 +804,6 @@ split_tokens_kernel(uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, uint8_t 
         }
     }
     pdl_wait();
-}
-
-// One thread per group: the group's line of k3_group_parts.  The places of a group's rows ascend,
-// so its rows in the pass's stacked tile are its last ones.
-__global__ void __launch_bounds__(256)
-group_parts_kernel(uint32_t *table, const uint32_t *group_rows, const uint32_t *place, const uint32_t *offsets,
-                   uint32_t groups) {
-    pdl_wait();
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= groups) return;
-    const uint32_t begin = offsets[g], rows = offsets[g + 1u] - begin;
-    const uint32_t whole = max(group_rows[g], rows), large = whole - stacked_rows(whole);
-    uint32_t lo = 0u, hi = rows;                           // first row whose place is in the stacked tile
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (place[begin + mid] < large) lo = mid + 1u; else hi = mid;
-    }
-    table[2u * g] = whole;
-    table[2u * g + 1u] = min(rows - lo, kStackedRows);     // the limit holds for any places
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -932,7 +857,7 @@ struct MapKey {
 };
 
 template <int kE>
-bool launch(const Operands &op, GmxArgs args, bool few, cudaStream_t stream) {
+bool launch(const Operands &op, GmxArgs args, bool many, cudaStream_t stream) {
     constexpr size_t kCachedSets = 256;
     static std::mutex map_lock;
     static std::map<MapKey, GmxMaps> cached;
@@ -966,9 +891,10 @@ bool launch(const Operands &op, GmxArgs args, bool few, cudaStream_t stream) {
             maps = it->second;
         }
     }
-    auto kernel = few ? grouped_mx_kernel<kE, 4> : grouped_mx_kernel<kE, 3>;
-    if (!set_max_dynamic_smem((const void *)kernel, kSmemBytes)) return false;
-    return launch_chained(kernel, sm_count(), kThreads, kSmemBytes, stream, maps, args);
+    auto kernel = many ? grouped_mx_kernel<kE, true> : grouped_mx_kernel<kE, false>;
+    const uint32_t smem = many ? Cfg<true>::kSmemBytes : Cfg<false>::kSmemBytes;
+    if (!set_max_dynamic_smem((const void *)kernel, smem)) return false;
+    return launch_chained(kernel, sm_count(), kThreads, smem, stream, maps, args);
 }
 
 inline size_t up256(size_t v) { return (v + 255u) & ~(size_t)255u; }
@@ -977,7 +903,6 @@ struct Scratch {
     uint8_t *x_hi, *x_lo, *x_sf;       // per product row
     uint8_t *a_hi, *a_lo, *a_sf;       // activation, per product row
     uint32_t *counters;                // item counters of the six launches (zeroed per call)
-    uint32_t *parts;                   // k3_group_parts of a call that is a part of a pass
     void *few;                         // scratch of the kernel for few rows per group
     size_t total;
 };
@@ -999,7 +924,6 @@ Scratch carve_scratch(const k3_moe_layer_desc *d, uint32_t rows, uint32_t source
     s.a_lo = take(R * I);
     s.a_sf = take(R * (I / 32u));
     s.counters = (uint32_t *)take(256);
-    s.parts = (uint32_t *)take(2u * sizeof(uint32_t) * d->local_expert_count);
     s.few = take(k3_grouped_mx4_workspace_bytes(d, rows, source_rows ? source_rows : rows));
     s.total = off + 256u;
     return s;
@@ -1045,9 +969,8 @@ constexpr uint32_t kFewRows = k3_mx4_rows, kSomeRows = kStackedRows;
 // when index == nullptr, source_rows == 0).  `act` bf16 [rows, I] is written when
 // not null; rows_out bf16 [rows, H].
 //
-// A group's kernel and, above 64 rows, the tile a row lies in decide the order in which the row's
-// sums are added.  A caller that cuts a pass into parts and wants the pass's bits says with `pass`
-// what the groups are in the whole pass.
+// A group's kernel decides the order in which its rows' sums are added.  A caller that cuts a pass
+// into parts and wants the pass's bits says with `pass` how many rows the groups have in the whole pass.
 bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act, const void *rows_in,
                            const void *index, uint32_t source_rows, const void *offsets, uint32_t rows,
                            void *workspace, cudaStream_t stream, const k3_token_routes *routes,
@@ -1058,12 +981,7 @@ bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act
     const Scratch s = carve_scratch(d, rows, index ? source_rows : 0u, workspace);
     const uint32_t conv_rows = index ? source_rows : rows;
     const bool few = max_group_rows > kFewRows, many = max_group_rows > kSomeRows;   // launches beyond the packed one
-    const k3_group_parts parts{pass ? s.parts : nullptr};
-    if (pass && !launch_chained(group_parts_kernel, (d->local_expert_count + 255u) / 256u, 256, 0, stream, s.parts,
-                                (const uint32_t *)pass->group_rows, (const uint32_t *)pass->place,
-                                (const uint32_t *)offsets, d->local_expert_count)) {
-        return false;
-    }
+    const k3_group_parts parts{pass ? (const uint32_t *)pass->group_rows : nullptr};
     if (!k3_grouped_mx4_terms(d, rows_in, conv_rows, rows, routes ? routes->ids : nullptr, offsets, s.few, s.counters,
                               stream)) {
         return false;
@@ -1096,11 +1014,11 @@ bool k3_grouped_mx_experts(const k3_moe_layer_desc *d, void *rows_out, void *act
         b.row_floor = kFewRows;
         b.row_ceil = kSomeRows;
         b.item_counter = counters;
-        if (few && !launch<kE>(op, b, true, stream)) return false;
+        if (few && !launch<kE>(op, b, false, stream)) return false;
         b.row_floor = kSomeRows;
         b.row_ceil = 0xffffffffu;
         b.item_counter = counters + 8;
-        return !many || launch<kE>(op, b, false, stream);
+        return !many || launch<kE>(op, b, true, stream);
     };
     // gate/up + activation
     a.out = (uint16_t *)act;

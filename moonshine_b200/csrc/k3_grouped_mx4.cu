@@ -246,7 +246,7 @@ grouped_mx4_kernel(const __grid_constant__ Mx4Maps maps, Mx4Args a) {
         for (int j = 0; j < 2; j++) {
             const uint32_t g = threadIdx.x * 2u + j;
             const uint32_t n = g < a.groups ? a.offsets[g + 1u] - a.offsets[g] : 0u;
-            const uint32_t whole = a.parts.table != nullptr && g < a.groups ? a.parts.table[2u * g] : n;
+            const uint32_t whole = a.parts.table != nullptr && g < a.groups ? max(a.parts.table[g], n) : n;
             v[j] = n != 0u && whole <= kTileRows ? 1u : 0u;
             run += v[j];
             incl[j] = run;

@@ -394,7 +394,7 @@ extern "C" bool k3_moe_experts_grouped_part(const k3_moe_layer_desc *d, void *ro
     }
     const size_t need = k3_moe_experts_workspace_bytes(d, rows, index ? source_rows : 0u);
     if (need == 0 || workspace_bytes < need) return false;
-    const k3_part_of_pass pass{group_rows, place};
+    const k3_part_of_pass pass{group_rows};
     return k3_grouped_mx_experts(d, rows_out, act, rows_in, index, source_rows, offsets, rows, workspace,
                                  (cudaStream_t)stream, nullptr, &pass);
 }

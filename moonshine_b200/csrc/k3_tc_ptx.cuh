@@ -142,9 +142,15 @@ K3_DEVINL void tma_prefetch_2d(const void *map, int32_t x, int32_t y) {
 }
 
 // ------------------------------------------------------------- asynchronous copies
-// 16 bytes global -> shared memory of one thread (both 16-byte aligned)
-K3_DEVINL void cp_async_16(void *dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+// kBytes (8 or 16) global -> shared memory of one thread, both aligned to them
+template <uint32_t kBytes>
+K3_DEVINL void cp_async(void *dst, const void *src) {
+    if constexpr (kBytes == 16u) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    } else {
+        static_assert(kBytes == 8u, "8 or 16 bytes");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    }
 }
 // one arrival of this thread on `bar` (counted in its initial value) when its copies so far are done
 K3_DEVINL void cp_async_arrive(uint64_t *bar) {
