@@ -154,16 +154,20 @@ exact_q8_kernel(uint16_t *__restrict__ out, const int8_t *q, const void *scales,
 // A pair of warps covers the 256 lanes of a 256-column step, four columns per thread:
 // warp h of the pair holds lanes 128 h + 4 lane + i.  kSR x kSV pairs per block, each with
 // its own kR weight rows and kV input rows.
+template <int kR, int kV, int kSR, int kSV>
+constexpr uint32_t exact_bf16_smem_floats() { return kSR * kSV * (kR * kV < 8 ? kR * kV : 8) * 4 * 32; }
+
+// One block's work (64 * kSR * kSV threads): block_x along the weight rows, block_y along the input
+// rows; `smem` holds exact_bf16_smem_floats floats.
 template <typename Out, int kR, int kV, int kSR, int kSV>
-__global__ void __launch_bounds__(64 * kSR * kSV)
-exact_bf16_kernel(Out *__restrict__ out, const uint16_t *w, const uint16_t *x,
-                  uint32_t vectors, uint32_t rows, uint32_t columns) {
+K3_DEVINL void exact_bf16_block(Out *__restrict__ out, const uint16_t *w, const uint16_t *x, uint32_t vectors,
+                                uint32_t rows, uint32_t columns, uint32_t block_x, uint32_t block_y, float *smem) {
     constexpr int kPhase = kR * kV < 8 ? kR * kV : 8;      // outputs whose halves meet per pass over shared memory
-    __shared__ float half_sum[kSR * kSV][kPhase][4][32];
+    float(*half_sum)[kPhase][4][32] = reinterpret_cast<float(*)[kPhase][4][32]>(smem);
     const uint32_t lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
     const uint32_t h = warp & 1u, pair = warp >> 1;
-    const uint32_t row0 = (blockIdx.x * kSR + pair % kSR) * kR, v0 = (blockIdx.y * kSV + pair / kSR) * kV;
-    if (blockIdx.y == 0 && lane == 0 && h == 0 && row0 < rows)
+    const uint32_t row0 = (block_x * kSR + pair % kSR) * kR, v0 = (block_y * kSV + pair / kSR) * kV;
+    if (block_y == 0 && lane == 0 && h == 0 && row0 < rows)
         prefetch_l2(w + (uint64_t)row0 * columns, (uint64_t)min((uint32_t)kR, rows - row0) * columns * 2u);
     pdl_wait();
     const uint16_t *wr[kR];
@@ -238,6 +242,14 @@ exact_bf16_kernel(Out *__restrict__ out, const uint16_t *w, const uint16_t *x,
             }
         }
     }
+}
+
+template <typename Out, int kR, int kV, int kSR, int kSV>
+__global__ void __launch_bounds__(64 * kSR * kSV)
+exact_bf16_kernel(Out *__restrict__ out, const uint16_t *w, const uint16_t *x,
+                  uint32_t vectors, uint32_t rows, uint32_t columns) {
+    __shared__ float smem[exact_bf16_smem_floats<kR, kV, kSR, kSV>()];
+    exact_bf16_block<Out, kR, kV, kSR, kSV>(out, w, x, vectors, rows, columns, blockIdx.x, blockIdx.y, smem);
 }
 
 }  // namespace k3

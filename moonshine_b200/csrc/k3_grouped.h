@@ -26,6 +26,16 @@ bool k3_q8_few_product(void *out, const void *q, const void *scales, const void 
                        uint32_t columns, uint32_t block, int scale_type, cudaStream_t stream);
 bool k3_q8_few_gateup(const k3_moe_layer_desc *desc, void *act, void *gate, void *up, const void *x, uint32_t vectors,
                       cudaStream_t stream);
+// Router logits, gate/up with the activation and (latent not null) the latent projection bf16 [vectors,
+// latent_width] of 1 to 31 rows in one launch, each with the bits of its own kernel.  False, with
+// nothing launched, for shapes it does not take.
+bool k3_q8_few_front(const k3_moe_layer_desc *desc, void *logits, void *act, void *gate, void *up, const void *x,
+                     uint32_t vectors, void *latent, const void *down_q, const void *down_s, uint32_t latent_width,
+                     cudaStream_t stream);
+// out bf16 [vectors, rows] = bf16(x0 W0^T) + bf16(x1 W1^T), 1 to 31 rows; false as above.
+bool k3_q8_few_sum_of_two(void *out, const void *q0, const void *s0, const void *x0, uint32_t columns0, const void *q1,
+                          const void *s1, const void *x1, uint32_t columns1, uint32_t vectors, uint32_t rows,
+                          uint32_t block, int scale_type, cudaStream_t stream);
 
 // One Q8 projection as a plain bf16 tensor-core GEMM: the table is converted to bf16
 // once into weight_scratch (rows * cols * 2 bytes).  False when the shape or the

@@ -127,14 +127,24 @@ extern "C" bool k3_moe_latent_layer_forward(const k3_moe_latent_desc *d, void *o
     const uint32_t H = l.hidden, L = d->latent;
 
     // router on the full-width token, experts on the latent projection
-    if (!k3_moe_route(&l, w.ids, w.weights, w.logits, x, tokens, stream)) return false;
-    if (!(w.proj_w && k3_grouped_q8_dense_bf16(w.latent, d->down_q, d->down_s, x, tokens, L, H, l.q8_block,
+    // (a few tokens: with the shared expert's gate and up in one launch, its down projection with
+    // the routed one's at the end)
+    const bool front = tokens < 32u && w.sh_bytes == 0 && l.router_bias && l.shared_down_q && l.shared_down_s &&
+                       k3_q8_few_front(&l, w.logits, w.sh_act, w.sh_gate, w.sh_up, x, tokens, w.latent, d->down_q, d->down_s,
+                                       L, stream);
+    if (!(front ? k3_rocm_router_topk_f32_batch(w.ids, w.weights, w.logits, l.router_bias, tokens, l.expert_count, l.top_k,
+                                                l.route_scale, stream)
+                : k3_moe_route(&l, w.ids, w.weights, w.logits, x, tokens, stream))) {
+        return false;
+    }
+    if (!front &&
+        !(w.proj_w && k3_grouped_q8_dense_bf16(w.latent, d->down_q, d->down_s, x, tokens, L, H, l.q8_block,
                                                l.q8_scale_type, w.proj_w, stream)) &&
         !k3_grouped_q8_bf16(w.latent, d->down_q, d->down_s, x, tokens, L, H, l.q8_block, l.q8_scale_type,
                             stream)) {
         return false;
     }
-    if (l.shared_hidden) {
+    if (l.shared_hidden && !front) {
         const bool ok = w.sh_bytes != 0
                             ? k3_grouped_shared_expert(&l, w.sh_out, w.sh_act, x, tokens, w.sh_ws, stream)
                             : k3_moe_shared_expert(&l, w.sh_out, w.sh_gate, w.sh_up, w.sh_act, x, tokens, stream);
@@ -171,14 +181,22 @@ extern "C" bool k3_moe_latent_layer_forward(const k3_moe_latent_desc *d, void *o
         !k3_rocm_rms_norm_bf16(w.routed_norm, w.routed, d->norm_weight, tokens, L, d->norm_epsilon, stream)) {
         return false;
     }
+    const bool summed = front && k3_q8_few_sum_of_two(out, d->up_q, d->up_s, w.routed_norm, L, l.shared_down_q,
+                                                      l.shared_down_s, w.sh_act, l.shared_hidden, tokens, H, l.q8_block,
+                                                      l.q8_scale_type, stream);
+    if (front && !summed &&
+        !k3_grouped_q8_bf16(w.sh_out, l.shared_down_q, l.shared_down_s, w.sh_act, tokens, H, l.shared_hidden, l.q8_block,
+                            l.q8_scale_type, stream)) {
+        return false;
+    }
     void *full = l.shared_hidden ? (void *)w.routed_full : out;
-    if (!(w.proj_w && k3_grouped_q8_dense_bf16(full, d->up_q, d->up_s, w.routed_norm, tokens, H, L, l.q8_block,
+    if (!summed && !(w.proj_w && k3_grouped_q8_dense_bf16(full, d->up_q, d->up_s, w.routed_norm, tokens, H, L, l.q8_block,
                                                l.q8_scale_type, w.proj_w, stream)) &&
         !k3_grouped_q8_bf16(full, d->up_q, d->up_s, w.routed_norm, tokens, H, L, l.q8_block, l.q8_scale_type,
                             stream)) {
         return false;
     }
-    if (l.shared_hidden && !k3_rocm_add_bf16(out, w.routed_full, w.sh_out, (uint64_t)tokens * H, stream)) {
+    if (l.shared_hidden && !summed && !k3_rocm_add_bf16(out, w.routed_full, w.sh_out, (uint64_t)tokens * H, stream)) {
         return false;
     }
     if (ids_out && cudaMemcpyAsync(ids_out, w.ids, (size_t)routes * 4u, cudaMemcpyDefault, stream) != cudaSuccess) {

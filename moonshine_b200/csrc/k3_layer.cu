@@ -496,9 +496,24 @@ bool layer_forward_impl(const k3_moe_layer_desc *d, void *out, const void *x, ui
             return false;
         }
     } else {
-        if (!k3_moe_route(d, w.ids, w.weights, w.logits, x, tokens, stream)) return false;
+        // 9 to 31 tokens: what depends on them alone (router logits, the shared expert's gate and up)
+        // goes together, before the first event (24 tokens: 56 -> 40 us; with 5 tokens 22 -> 23, so
+        // up to 8 rows keep a launch each, gate and up with twice the warps)
+        const bool front = tokens > 8u && w.sh_bytes == 0 && d->router_bias && d->shared_down_q && d->shared_down_s &&
+                           k3_q8_few_front(d, w.logits, w.sh_act, w.sh_gate, w.sh_up, x, tokens, nullptr, nullptr, nullptr,
+                                           0u, stream);
+        if (!(front ? k3_rocm_router_topk_f32_batch(w.ids, w.weights, w.logits, d->router_bias, tokens, d->expert_count,
+                                                    d->top_k, d->route_scale, stream)
+                    : k3_moe_route(d, w.ids, w.weights, w.logits, x, tokens, stream))) {
+            return false;
+        }
         if (!mark(events, 1, stream)) return false;
-        if (d->shared_hidden &&
+        if (front) {
+            if (!k3_grouped_q8_bf16(w.sh_out, d->shared_down_q, d->shared_down_s, w.sh_act, tokens, d->hidden,
+                                    d->shared_hidden, d->q8_block, d->q8_scale_type, stream)) {
+                return false;
+            }
+        } else if (d->shared_hidden &&
             !(w.sh_bytes != 0
                   ? k3_grouped_shared_expert(d, w.sh_out, w.sh_act, x, tokens, w.sh_ws, stream)
                   : k3_moe_shared_expert(d, w.sh_out, w.sh_gate, w.sh_up, w.sh_act, x, tokens, stream))) {
