@@ -387,8 +387,7 @@ def kind_peaks(torch) -> dict:
         b.record()
         torch.cuda.synchronize()
         out[name] = {"burst_tflops": best, "sustained_tflops": launches * flop.value / (a.elapsed_time(b) * 1e-3) / 1e12}
-    # the same instruction at the N extents the prefill kernel issues (a row tile has at most 128
-    # rows): a chain of MMAs into one accumulator costs ~55 ns each for every N <= 128
+    # the same instruction at N extents of the prefill kernel's row tiles
     by_n = {}
     for n in (128, 64, 32):
         flop = C.c_double()

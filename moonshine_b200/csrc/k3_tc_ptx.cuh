@@ -13,12 +13,11 @@ K3_DEVINL uint32_t smem_u32(const void *p) {
 
 // ---------------------------------------------------------------- one thread of a warp
 // TMA, MMA and commit instructions take their operands from uniform registers.  A branch on
-// lane == 0 does not tell the compiler that one thread runs it, so every operand goes through a
-// loop over the values that the active lanes might hold; behind elect.sync, in a warp whose index
-// is the same in all lanes for the compiler too (warp_index), it moves them directly.  Measured,
-// one thread issuing back to back: a block-scaled MMA of N = 128 every 36 ns instead of 57 (its
-// operand fetch: N = 64 28 ns instead of 54), a bf16 MMA of N = 32 with A in tensor memory 11 instead
-// of 51, a TMA box every 14 instead of 32 to 60.
+// lane == 0 does not tell the compiler that one thread runs it; elect.sync does, in a warp whose
+// index is the same in all lanes for the compiler too (warp_index).  Measured, one thread issuing
+// back to back, lane == 0 / elected: block-scaled MMA of N = 16 31 / 23 ns, N = 64 33 / 28, N = 128 39 / 36;
+// TMA box of 64 x 32 bf16 32 to 62 / 19 to 43 (by boxes per stage), gather4 47 / 9.  Branches on run-time
+// values between the instructions cost as much again (N = 128 57 ns), so issue loops are straight-line.
 K3_DEVINL uint32_t warp_index() { return __shfl_sync(0xffffffffu, threadIdx.x / kWarp, 0); }
 
 // true in one lane of a converged warp, the same lane each time
