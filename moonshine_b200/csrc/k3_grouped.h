@@ -10,6 +10,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+// Sizes, activation and scale of a layer description, as every layer entry point wants them before
+// its first launch (pointers are checked where they are used).
+bool k3_layer_desc_ok(const k3_moe_layer_desc *desc);
+
 // logits f32 [tokens, rows] = x bf16 [tokens, cols] * W bf16 [rows, cols]^T
 bool k3_grouped_dense_bf16_f32(void *out, const void *weights, const void *x, uint32_t tokens,
                                uint32_t rows, uint32_t cols, void *stream);

@@ -114,7 +114,7 @@ extern "C" size_t k3_moe_latent_workspace_bytes(const k3_moe_latent_desc *d, uin
 extern "C" bool k3_moe_latent_layer_forward(const k3_moe_latent_desc *d, void *out, const void *x,
                                             uint32_t tokens, void *workspace, size_t workspace_bytes,
                                             void *ids_out, void *weights_out, void *stream_pointer) {
-    if (!latent_ok(d) || !out || !x || !workspace || tokens == 0 || tokens > 65535u ||
+    if (!latent_ok(d) || !k3_layer_desc_ok(&d->layer) || !out || !x || !workspace || tokens == 0 || tokens > 65535u ||
         d->layer.local_expert_first != 0 || d->layer.local_expert_count != d->layer.expert_count) {
         return false;
     }

@@ -275,6 +275,8 @@ bool slot_pointers_aligned(const k3_moe_layer_desc *d) {
 
 }  // namespace
 
+bool k3_layer_desc_ok(const k3_moe_layer_desc *d) { return desc_ok(d); }
+
 extern "C" const char *k3_moe_version(void) { return "k3moe-b200 0.1.0"; }
 
 extern "C" bool k3_moe_store_admit(const k3_moe_layer_desc *d, uint32_t slot, const void *span,

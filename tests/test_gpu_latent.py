@@ -101,3 +101,26 @@ def test_latent_layer_matches_oracle(oracle, tokens):
     # a null descriptor field is refused before any launch
     desc.norm_weight = None
     assert not ops.k3_moe_latent_layer_forward(desc, out, G.dev(x), tokens, ws, need, ids, wts)
+
+
+@pytest.mark.parametrize("tokens", [1, 5, 8, 9, 24, 31, 40])
+def test_bad_layer_descriptions_are_refused_before_any_launch(tokens):
+    """Few tokens take other launches than many; what is refused does not depend on that."""
+    x, ws = torch.zeros((tokens, H), dtype=torch.bfloat16, device="cuda"), torch.zeros(1 << 26, dtype=torch.uint8, device="cuda")
+    tables = torch.zeros(E * I * L, dtype=torch.uint8, device="cuda")
+    desc = _native.LatentDesc(latent=L, norm_epsilon=EPS,
+                              **{n: tables.data_ptr() for n in ("down_q", "down_s", "norm_weight", "up_q", "up_s")})
+    for n in ("router_weight", "router_bias", "w1_packed", "w1_scales", "w3_packed", "w3_scales", "w2_packed", "w2_scales",
+              "shared_gate_q", "shared_gate_s", "shared_up_q", "shared_up_s", "shared_down_q", "shared_down_s"):
+        setattr(desc.layer, n, tables.data_ptr())
+    good = dict(hidden=H, expert_hidden=I, expert_count=E, local_expert_count=E, top_k=K, shared_hidden=S, q8_block=BLOCK,
+                q8_scale_type=ST, activation=ops.ACT_SITU, beta=4.0, linear_beta=25.0, route_scale=1.0)
+    out = torch.full((tokens, H), 7.0, dtype=torch.bfloat16, device="cuda")
+    for bad in ({"activation": 7}, {"beta": 0.0}, {"linear_beta": float("nan")}, {"route_scale": 0.0},
+                {"route_scale": float("nan")}, {"top_k": 0}, {"top_k": E + 1}, {"expert_hidden": I + 1},
+                {"expert_count": 1025, "local_expert_count": 1025}):
+        for n, v in dict(good, **bad).items():
+            setattr(desc.layer, n, v)
+        ws.fill_(0x5A)
+        assert not ops.k3_moe_latent_layer_forward(desc, out, x, tokens, ws, ws.numel(), None, None), bad
+        assert (out == 7.0).all() and (ws == 0x5A).all(), bad
