@@ -218,7 +218,9 @@ bool k3_moe_layer_forward(const k3_moe_layer_desc *desc, void *out,
 /* Same as k3_moe_layer_forward, recording caller-created cudaEvent_t handles
  * (as void *, NULL entries skipped) on `stream` at the phase boundaries:
  * events[0] start, [1] router done, [2] shared expert done, [3] dispatch and
- * row gather done, [4] grouped expert products done, [5] combine done.  This is
+ * row gather done, [4] grouped expert products done, [5] combine done.  (9 to 31
+ * tokens: with events[1] given the router and the shared expert keep a launch
+ * each, where k3_moe_layer_forward joins them; the results are the same.)  This is
  * the device-timed form of the reference's host phase ledger
  * (router_seconds, routed_expert_pipeline_seconds, moe_tail_seconds of
  * k3_engine_prefill_stats, k3_engine.h:69-99). */

@@ -499,9 +499,10 @@ bool layer_forward_impl(const k3_moe_layer_desc *d, void *out, const void *x, ui
         }
     } else {
         // 9 to 31 tokens: what depends on them alone (router logits, the shared expert's gate and up)
-        // goes together, before the first event (24 tokens: 56 -> 40 us; with 5 tokens 22 -> 23, so
-        // up to 8 rows keep a launch each, gate and up with twice the warps)
-        const bool front = tokens > 8u && w.sh_bytes == 0 && d->router_bias && d->shared_down_q && d->shared_down_s &&
+        // goes together (24 tokens: 56 -> 40 us; with 5 tokens 22 -> 23, so up to 8 rows keep a launch
+        // each, gate and up with twice the warps).  A caller that asks when the router is done gets the
+        // separate launches, which compute the same bits.
+        const bool front = tokens > 8u && !(events && events[1]) && w.sh_bytes == 0 && d->router_bias && d->shared_down_q && d->shared_down_s &&
                            k3_q8_few_front(d, w.logits, w.sh_act, w.sh_gate, w.sh_up, x, tokens, nullptr, nullptr, nullptr,
                                            0u, stream);
         if (!(front ? k3_rocm_router_topk_f32_batch(w.ids, w.weights, w.logits, d->router_bias, tokens, d->expert_count,

@@ -124,6 +124,54 @@ def test_phase_ledger_accumulates_under_the_reference_names():
         ops.k3_moe_event_destroy(e)
 
 
+@pytest.mark.parametrize("tokens", [8, 9, 24, 31, 32])
+def test_the_shared_expert_is_not_booked_under_the_router(tokens):
+    """A shared expert of 32768 (three tables of 128 MiB, 20 us each or more) beside a router of 64 rows."""
+    h, s, e, i = 4096, 32768, 64, 512
+    t = {n: torch.zeros(c, dtype=torch.uint8, device=G.DEV) for n, c in (
+        ("router", e * h * 2), ("packed", e * i * h // 2), ("scales", e * i * h // 32), ("shared_q", s * h),
+        ("shared_s", s * h // 32 * 2))}
+    desc = _native.LayerDesc(hidden=h, expert_hidden=i, expert_count=e, top_k=2, shared_hidden=s, q8_block=32,
+                             q8_scale_type=ops.Q8_F16, activation=ops.ACT_SWIGLU, route_scale=1.0, local_expert_count=e,
+                             router_weight=t["router"].data_ptr(), router_bias=t["router"].data_ptr())
+    for n in ("w1", "w3", "w2"):
+        setattr(desc, n + "_packed", t["packed"].data_ptr())
+        setattr(desc, n + "_scales", t["scales"].data_ptr())
+    for n in ("gate", "up", "down"):
+        setattr(desc, f"shared_{n}_q", t["shared_q"].data_ptr())
+        setattr(desc, f"shared_{n}_s", t["shared_s"].data_ptr())
+    need = ops.k3_moe_layer_workspace_bytes(desc, tokens)
+    ws = torch.empty(need, dtype=torch.uint8, device=G.DEV)
+    x = torch.zeros((tokens, h), dtype=torch.bfloat16, device=G.DEV)
+    out = torch.empty_like(x)
+    events = [ops.k3_moe_event_create() for _ in range(6)]
+    arr = (C.c_void_p * 6)(*events)
+    for _ in range(3):
+        assert ops.k3_moe_layer_forward_events(desc, out, x, tokens, ws, need, arr)
+    stats = _native.PhaseStats()
+    for _ in range(5):
+        assert ops.k3_moe_layer_forward_events(desc, out, x, tokens, ws, need, arr)
+        assert ops.k3_moe_phase_stats_add(stats, arr)
+    for v in events:
+        ops.k3_moe_event_destroy(v)
+    assert stats.router_seconds < 0.5 * stats.shared_expert_seconds
+
+
+@pytest.mark.parametrize("tokens", [9, 24, 31])
+def test_events_do_not_change_the_results(tokens):
+    cfg = synth.baseline_config(hidden=4096, expert_hidden=512, experts=32, top_k=4, shared_hidden=512)
+    layer = MoELayer(cfg, synth.make_layer(cfg, 5), seed=5, device=G.DEV, max_tokens=tokens)
+    x = G.dev(synth.activations(5, tokens, 4096)).view(torch.bfloat16)
+    want, out = layer.forward(x), torch.empty_like(x)
+    events = [ops.k3_moe_event_create() for _ in range(6)]
+    for some in (events, [events[0]] + [None] * 4 + [events[5]]):
+        arr = (C.c_void_p * 6)(*some)
+        assert ops.k3_moe_layer_forward_events(layer.desc, out, x, tokens, layer.workspace, layer.workspace.numel(), arr)
+        assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+    for v in events:
+        ops.k3_moe_event_destroy(v)
+
+
 RING_SHAPE = dict(hidden=2048, expert_hidden=1024, experts=32, top_k=8, shared_hidden=1024)
 
 
