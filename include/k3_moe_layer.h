@@ -151,8 +151,8 @@ bool k3_moe_experts_grouped_ws(const k3_moe_layer_desc *desc, void *rows_out,
  * up to 64, more), so a part that is computed by itself differs from the whole
  * pass in the last bits.  group_rows: u32 [local_expert_count] on the device,
  * rows of each group in the whole pass; place: u32 [rows], place of each row in
- * its group there, ascending within a group (no longer read: all row tiles of a
- * group add a row's sums in one order).  Fails where
+ * its group there, ascending within a group (not read, since all row tiles of a
+ * group add a row's sums in one order, but NULL is refused).  Fails where
  * k3_moe_experts_workspace_bytes is 0 (fewer than 32 rows, or a shape that does
  * not suit the path) or the workspace is smaller. */
 bool k3_moe_experts_grouped_part(const k3_moe_layer_desc *desc, void *rows_out,

@@ -111,7 +111,7 @@ class NativeBackend:
     def experts(self, rows, offsets_local, index, whole=None):
         """Expert products of rows[index] (grouped by local expert as offsets_local says).
         ``whole`` = (group_rows, place) of ``k3_moe_experts_grouped_part`` when the rows are a
-        part of a pass."""
+        part of a pass; the places are not read, any table of the rows' length will do."""
         n, d, i = index.numel(), self.cfg["hidden"], self.cfg["expert_hidden"]
         out = self._buf("eo", (n, d), rows.dtype)
         act = self._buf("ea", (n, i), rows.dtype)
@@ -183,7 +183,8 @@ def part_of_pass(counts, piece: int, first: int, per: int):
     [world, E] matrix of rows each rank routes to each expert (host tensors).  The whole
     pass groups its rows by (expert asc, source asc, piece asc, route asc).  Returns the
     rows of each local expert in the whole pass [per] and, per (expert, source) block of
-    this piece, the place of its first row in the expert's group [per * world]."""
+    this piece, the place of its first row in the expert's group [per * world] (for a host that
+    fills the ``place`` argument of ``k3_moe_experts_grouped_part``; no kernel reads it)."""
     mine = torch.stack([c[:, first:first + per] for c in counts])    # [piece, source, local expert]
     blocks = mine.transpose(0, 1).reshape(-1, per)                   # (source asc, piece asc)
     before = torch.cumsum(blocks, 0) - blocks
@@ -280,7 +281,7 @@ def _ep_steps(backend, x, cfg: dict, group, once_per_destination=None, pieces=No
         for counted, _ in pieces:
             if counted is not None:
                 counted.synchronize()
-        group_rows, block_place = part_of_pass([c[:, :e] for _, c in pieces], piece, first, per)
+        whole, _ = part_of_pass([c[:, :e] for _, c in pieces], piece, first, per)
 
     rows_send = rows_send[:sum(send_unique)]
     rows_recv = torch.empty((n_unique, x.shape[1]), dtype=x.dtype, device=dev)
@@ -306,11 +307,8 @@ def _ep_steps(backend, x, cfg: dict, group, once_per_destination=None, pieces=No
                  + torch.arange(n_recv, device=dev)).to(torch.int32)
         inverse = torch.empty_like(order)
         inverse[order.long()] = torch.arange(n_recv, device=dev, dtype=torch.int32)
-        if pieces is not None and getattr(backend, "takes_parts", False):
-            passed = torch.cat([group_rows, block_place]).to(dev)
-            place = (torch.repeat_interleave(passed[per:] - dest_base, lengths_d, output_size=n_recv)
-                     + torch.arange(n_recv, device=dev)).to(torch.int32)
-            whole = (passed[:per].to(torch.int32), place)
+        if whole is not None:
+            whole = (whole.to(torch.int32).to(dev), order)
         # first received row of each source, repeated for each of its routes
         if dedup:
             base_of_route = torch.repeat_interleave(base_of_source, recv_d, output_size=n_recv)
