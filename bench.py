@@ -291,7 +291,8 @@ def launches_per_step(tokens: int, shared: bool) -> int:
     if tokens == 1:
         return 4                                   # shared-expert ring kernel, router rows, experts, tail
     route, combine = 2, 1
-    shared_k = 0 if not shared else 5 if tokens >= 32 else 2      # 3 conversions and 2 GEMMs; gate/up and down
+    # 3 conversions and 2 GEMMs; gate/up (9 to 31 tokens: in the router's launch) and down
+    shared_k = 0 if not shared else 5 if tokens >= 32 else 1 if tokens > 8 else 2
     dispatch = 1 if tokens * 16 <= 4096 else 3
     # row terms, gate/up and down of the packed kernel; two-term rows and the two-term kernel's
     # launches where an expert can have more than 16 rows; those for more than 64
