@@ -300,6 +300,12 @@ def launches_per_step(tokens: int, shared: bool) -> int:
     return route + shared_k + dispatch + experts + combine
 
 
+def latent_launches_per_step(tokens: int, shared: bool) -> int:
+    """The same for a latent-shape pass of 32 and more tokens: conversion and GEMM of either projection, the
+    norm and (with a shared expert) the add besides; the weighted sum takes the combine's place."""
+    return launches_per_step(tokens, shared) + 5 + (1 if shared else 0)
+
+
 def time_decode(call, cfg, device, torch, iters: int = 40):
     """One-token decode with a cold L2: distinct tokens round-robin and a buffer
     larger than L2 rewritten between iterations; each iteration timed by its own
@@ -486,7 +492,7 @@ def run_latent(args, cfg, tokens, device, peaks, torch):
         "config": {"workload": args.workload, "tokens": tokens, "experts": e, "top_k": k, "hidden": d,
                    "latent": latent, "expert_hidden": i, "shared_hidden": s, "router_bias": "zipf",
                    "l2": "inputs larger than L2"},
-        "gpu_launches": (launches_per_step(tokens, bool(s)) + 4) * args.steps, "clocks": clocks,
+        "gpu_launches": latent_launches_per_step(tokens, bool(s)) * args.steps, "clocks": clocks,
         "roofline": {"bound": "tensor", "kernel": "whole layer pass", "achieved": achieved,
                      "peak": peaks["bf16_tflops_sustained"], "unit": "TFLOP/s",
                      "frac": achieved / peaks["bf16_tflops_sustained"], "traffic": None,
