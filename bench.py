@@ -278,10 +278,10 @@ def run_config(args, cfg, tokens, world):
 
 
 # DRAM bytes per launch measured with ncu on these workloads (one-pass metrics,
-# summary kept under profiles/): prefill = the six grouped expert launches (gate/up 17.22 GB,
-# down 9.41 GB, the launches for groups that this load does not have nothing); decode = the
+# summary kept under profiles/): prefill = the six grouped expert launches (gate/up 16.64 GB,
+# down 9.39 GB, the launches for groups that this load does not have nothing); decode = the
 # four kernels of one token.
-PREFILL_TRAFFIC_BYTES = 26.63e9
+PREFILL_TRAFFIC_BYTES = 26.03e9
 DECODE_TRAFFIC_BYTES = 434.9e6
 
 

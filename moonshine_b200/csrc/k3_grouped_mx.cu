@@ -63,10 +63,19 @@ constexpr uint32_t kStackedRows = 64;
 // block of 32 is one MMA per weight tile and the 8-bit weight containers are read from shared
 // memory once.  Larger groups: row tiles of up to 160 rows, the hi and the lo MMA adding into the
 // same columns.  A tile of 160 rows takes the weights through the copy unit once where a tile
-// of 128 and a remainder took them twice: with 8192 tokens most experts have 129 to 160 rows, and
-// their remainders of a few rows were 29 % of the expert phase.  160 is what fits: three
+// of 128 and a remainder took them twice: with 8192 tokens and a Zipf router bias most experts (573
+// of 896) have 129 to 160 rows, and their remainders of a few rows were 29 % of the expert phase (with
+// a uniform bias or four hot experts few have).  160 is what fits: three
 // stages of 72 KB, two accumulators of 160 columns beside the scales (192 rows in two stages of
-// 80 KB ran at 1250 useful TFLOP/s, 160 in three at 1300; both operand orders alike).
+// 80 KB ran at 1250 useful TFLOP/s, 160 in three at 1300; both operand orders alike).  192 experts,
+// whole calls back to back, tiles of 128 and a remainder / these: 129 rows 3579 / 2863 us, 146 3746 / 3148,
+// 161 4014 / 3907, 176 4101 / 3995, 192 4250 / 4198, 193 4774 / 4367, 224 4928 / 4660, 256 5135 / 5099,
+// 320 6660 / 6139.
+// One accumulator for hi and lo has twice the additions of two, which a remainder of up to 64 rows had
+// in the kernel with tiles of 128.  Against 64 bits, remainder rows of 18 group sizes, two / one: bf16
+// activations on the wrong side of a rounding line 0.098 / 0.114 % at K = 7168 and 0.099 / 0.103 at 3584 (all
+// other rows of such groups, both kernels: 0.123, 0.103), down products 0.61 / 0.61; the layer of 8192
+// and 16384 tokens is as far from 64 bits as before (rel-L2 0.004098 both, six inputs: -5e-6 to +1e-5 of it).
 template <bool kMany>
 struct Cfg {
     static constexpr uint32_t kTileRows = kMany ? 160u : kStackedRows;
@@ -504,8 +513,12 @@ grouped_mx_kernel(const __grid_constant__ GmxMaps maps, GmxArgs a) {
         // fetches the batch's scale bytes of one row of each table, kSfAhead batches
         // before they are stored: as TMA boxes of 128 rows x 16 bytes, issued with the
         // weights of the batch's first stage, they came late (the batch has three stages to get here)
-        // and took a sixth of the rows that the copy unit moves (with the elected issue, both products
-        // of 192 experts, back to back: 128 rows 1935 -> 1717 us, 64 rows 1288 -> 1196).
+        // and took a sixth of the rows that the copy unit moves (with the elected issue and, above 64
+        // rows, still the terms as the A operand, both products of 192 experts, back to back: 128 rows
+        // 1935 -> 1717 us, 64 rows 1288 -> 1196).  This kernel has not waited when it reads the token
+        // scales, and the 8-byte copies go through L1 (they have no other form): both are safe because the
+        // scales were complete before this kernel was launched.  The packed kernel, which is first
+        // of a projection's launches, triggers only after its own wait for whoever wrote them.
         const uint32_t quad = warp & 3u;
         const uint32_t lane_base = (32u * quad) << 16;
         const uint32_t row = 32u * quad + lane, kb = a.k / 32u;
@@ -957,12 +970,14 @@ bool k3_grouped_mx_supported(const k3_moe_layer_desc *d, uint32_t rows) {
            ((((uintptr_t)d->w1_scales) | ((uintptr_t)d->w3_scales) | ((uintptr_t)d->w2_scales)) & 15u) == 0;
 }
 
-// Which kernel a group goes to, by its rows (device time of both projections of 192 experts at
-// 7168 x 2048; the weights alone are 0.69 ms of HBM time):
-//   rows                   1     8     16    24    32    48    64    96    128
-//   packed                 0.70  0.73  0.81  1.28  1.38  1.94
-//   two-term, four stages  0.97  0.99  1.00  1.01  1.03  1.21  1.28
-//   two-term, three        1.10        1.14  1.15  1.17  1.27  1.37  1.70  1.95
+// Which kernel a group goes to, by its rows (ms of a whole call with 192 experts at 7168 x 2048, back to
+// back; the weights alone are 0.69 ms of HBM time):
+//   rows                   1     8     16    17    24    32    48    64    65    96    128
+//   packed                 0.69  0.80  0.97
+//   two-term, 64 rows                        1.15  1.15  1.20  1.49  1.66
+//   two-term, 160 rows                       1.24  1.32  1.38  1.62  1.81  1.91  2.24  2.70
+// Both products alone, before the elected issue of TMA and MMA instructions: packed with 8 / 16 / 24 / 32
+// rows 0.73 / 0.81 / 1.28 / 1.38, two-term for up to 64 rows 0.99 / 1.00 / 1.01 / 1.03.
 constexpr uint32_t kFewRows = k3_mx4_rows, kSomeRows = kStackedRows;
 
 // rows_in bf16 [source_rows, H]; product row r reads rows_in[index[r]] (or row r

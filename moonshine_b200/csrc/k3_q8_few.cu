@@ -194,6 +194,8 @@ q8_few_kernel(Q8FewArgs a) {
 // warp at a fourth of the memory rate; together their blocks fill the chip once, two of 512 threads
 // per SM for up to 8 rows.  Latent shape, one token: 39 us in three launches, 25 here (three column steps
 // in flight spill: 27; one block per SM with four: 31); 24 tokens without the projection 56 -> 40.
+// Whole latent layer with a launch each / joined (its last two products too): 1 token 115 / 102 us, 2
+// 175 / 161, 5 282 / 273, 8 380 / 365, 9 420 / 411, 16 566 / 556, 24 697 / 684, 31 812 to 840 / 791 to 815.
 // Every product keeps the order of sums of its own kernel, so it has the same bits.
 struct FrontArgs {
     Q8FewArgs gateup, project;

@@ -16,7 +16,7 @@ K3_DEVINL uint32_t smem_u32(const void *p) {
 // lane == 0 does not tell the compiler that one thread runs it; elect.sync does, in a warp whose
 // index is the same in all lanes for the compiler too (warp_index).  Measured, one thread issuing
 // back to back, lane == 0 / elected: block-scaled MMA of N = 16 31 / 23 ns, N = 64 33 / 28, N = 128 39 / 36;
-// TMA box of 64 x 32 bf16 32 to 62 / 19 to 43 (by boxes per stage), gather4 47 / 9.  Branches on run-time
+// TMA box of 64 x 32 bf16 32 to 62 / 19 to 43 (by boxes per stage).  Branches on run-time
 // values between the instructions cost as much again (N = 128 57 ns), so issue loops are straight-line.
 K3_DEVINL uint32_t warp_index() { return __shfl_sync(0xffffffffu, threadIdx.x / kWarp, 0); }
 
